@@ -21,7 +21,7 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = ["engine.cu", "nofma.cu", "tables.cpp", "capi.cpp", "fortran_abi.cpp", "noalloc.cu"]
 # libgrpp is built without floating-point contraction; the angular sums round as its do
 EXTRA = {"nofma.cu": ["-fmad=false"]}
-HEADERS = ["grpp_common.cuh", "specfunc.cuh", "mmd.cuh", "radial.cuh", "angular.cuh", "level_model.cuh", "gradient.cuh", "tables.h",
+HEADERS = ["grpp_common.cuh", "specfunc.cuh", "mmd.cuh", "mmd_tables.h", "radial.cuh", "angular.cuh", "level_model.cuh", "gradient.cuh", "tables.h",
            "engine.h", "onee.cuh", "nucmodel.h", "nofma_launch.h", "exp_rn.h"]
 
 

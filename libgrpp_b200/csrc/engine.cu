@@ -30,6 +30,7 @@
 #define GRPP_NO_RADIAL_TABLE_KERNELS  // ftab_kernel, wu_table_kernel: compiled in nofma.cu
 #include "radial.cuh"
 #include "mmd.cuh"
+#include "mmd_tables.h"
 #define GRPP_NO_ANGULAR_KERNELS  // the angular kernels are compiled in nofma.cu (no contraction)
 #include "angular.cuh"
 #include "nofma_launch.h"
@@ -130,6 +131,8 @@ struct DeviceState {
     std::vector<int64_t> atab_off;
     bool atab_dirty = true;  // atab_off has entries the device copy lacks
     DevBuf atab_off_dev;
+    MmdArgs mmd{};                       // type 1 class tables (pointers only)
+    std::vector<MmdClass> mmd_cls;
     std::vector<cudaEvent_t> gev[2];     // per buffer set: boundaries of the assembly launches (autotuning)
     std::map<int, int> fin_tune;         // assembly class -> block size picked by the autotuner
     std::mutex mu;
@@ -187,10 +190,17 @@ int init_device_state(DeviceState &st, int device)
                                 cudaHostAllocDefault));
     }
     st.atab_off.assign((kMaxL + 2) * (kMaxL + 2), -1);
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmdSmem));
+    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmdSmem));
+    MmdTables mt;
+    mmd_build_classes(mt);
+    st.mmd_cls = mt.classes;
+    GRPP_CUDA(upload_vec(st, mt.classes, &st.mmd.classes));
+    GRPP_CUDA(upload_vec(st, mt.levels, &st.mmd.levels));
+    GRPP_CUDA(upload_vec(st, mt.etab, &st.mmd.etab));
+    GRPP_CUDA(upload_vec(st, mt.otab, &st.mmd.otab));
+    GRPP_CUDA(upload_vec(st, mt.rtab, &st.mmd.rtab));
+    GRPP_CUDA(upload_vec(st, mt.ztab, &st.mmd.ztab));
     GRPP_CUDA(cudaFuncSetAttribute(radial_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GRPP_CUDA(ang_set_final_max_smem((int)kFinSmemMax));
     GRPP_CUDA(cudaFuncSetAttribute(type1_num_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -238,97 +248,6 @@ struct Packer {
         return off;
     }
 };
-
-// Slot schedule of the Cartesian pairs of one (bra, ket) table class for mmd_kernel. Pairs
-// with equal (tx, uy, vz) = (ax+bx, ay+by, az+bz) have the same contraction loops: they are
-// coupled two by two into slots (2h, 2h+1) of one lane (an odd one out takes a slot couple
-// alone), and the couples fill the slot rows in (tx, uy, vz) order, so the 32 lanes of a row
-// run equal or nearly equal loops. Appends 32 x kpl slots to out; returns the rows in use.
-static int mmd_pair_schedule(const int8_t *ca, int nA, const int8_t *cb, int nB, int kpl, std::vector<uint16_t> &out)
-{
-    std::map<int, std::vector<int>> groups;  // key (tx * 32 + uy) * 32 + vz, ascending
-    for (int m = 0; m < nA; m++)
-        for (int n = 0; n < nB; n++) {
-            const int tx = ca[3 * m] + cb[3 * n], uy = ca[3 * m + 1] + cb[3 * n + 1], vz = ca[3 * m + 2] + cb[3 * n + 2];
-            groups[(tx * 32 + uy) * 32 + vz].push_back(m * nB + n);
-        }
-    std::vector<std::pair<int, int>> units;
-    for (auto &g : groups)
-        for (size_t i = 0; i < g.second.size(); i += 2)
-            units.push_back({g.second[i], i + 1 < g.second.size() ? g.second[i + 1] : -1});
-    const size_t base = out.size();
-    out.resize(base + 32 * (size_t)kpl, kMmdNoPair);
-    if ((int)units.size() > 16 * kpl) {  // more units than slot couples: plain order, unequal couples
-        for (int pr = 0; pr < nA * nB; pr++) out[base + pr] = (uint16_t)pr;
-        return (nA * nB + 63) / 64;
-    }
-    for (size_t r = 0; r < units.size(); r++) {
-        const int row = (int)(r / 32), lane = (int)(r % 32);
-        out[base + (2 * row) * 32 + lane] = (uint16_t)units[r].first;
-        if (units[r].second >= 0) out[base + (2 * row + 1) * 32 + lane] = (uint16_t)units[r].second;
-    }
-    return (int)(units.size() + 31) / 32;
-}
-
-// Update programs of mmd_kernel's Hermite coefficients for every (la, lb) with la, lb <= lmax,
-// and of its R^n_tuv tables for every S = 1..smax (mmd_e_code / MmdArgs::rtab).
-static void mmd_update_tables(int lmax, int smax, std::vector<int> &etab, std::vector<int> &etab_off,
-                              std::vector<int2> &rtab, std::vector<int> &rtab_off)
-{
-    etab_off.assign((kMaxL + 1) * (kMaxL + 1), 0);
-    for (int la = 0; la <= lmax; la++)
-        for (int lb = 0; lb <= lmax; lb++) {
-            etab_off[la * (kMaxL + 1) + lb] = (int)etab.size();
-            const int S = la + lb, la1 = la + 1, lb1 = lb + 1, S1 = S + 1;
-            for (int w = 0; w <= S; w++) {
-                const int ilo = std::max(0, w - lb), ihi = std::min(la, w), per_axis = (ihi - ilo + 1) * (w + 1);
-                for (int e = 0; e < 3 * per_axis; e++) {
-                    const int ax = e / per_axis, r = e % per_axis, i = ilo + r / (w + 1), t = r % (w + 1), j = w - i;
-                    etab.push_back(mmd_e_code(((ax * la1 + i) * lb1 + j) * S1 + t, ax, i, j, t));
-                }
-            }
-        }
-    rtab_off.assign(2 * kMaxL + 1, 0);
-    for (int S = 1; S <= smax; S++) {
-        rtab_off[S] = (int)rtab.size();
-        std::vector<int> lvl(S + 1);
-        for (int s = 0, o = 0; s <= S; s++) {
-            lvl[s] = o;
-            o += (s + 1) * (s + 2) / 2 * (S - s + 1);
-        }
-        rtab.resize(rtab.size() + mmd_r_size(S), int2{0, 0});
-        int2 *tab = rtab.data() + rtab_off[S];
-        for (int s = 1; s <= S; s++) {
-            const int ne = (s + 1) * (s + 2) / 2, nn = S - s + 1, ne1 = s * (s + 1) / 2, ne2 = (s - 1) * s / 2;
-            const int o1 = lvl[s - 1], o2 = s >= 2 ? lvl[s - 2] : 0;
-            for (int e = 0; e < ne * nn; e++) {
-                const int n = e / ne, idx = e % ne;
-                int kk = 0;
-                while ((kk + 1) * (kk + 2) / 2 <= idx) kk++;
-                const int v = idx - kk * (kk + 1) / 2, u = kk - v, t = s - kk;
-                // step down along z if t = u = 0, else along y if t = 0, else along x
-                int uu = u, vv = v, kq, ax;
-                if (t + u == 0) {
-                    vv = v - 1;
-                    kq = v;
-                    ax = 2;
-                } else if (t == 0) {
-                    uu = u - 1;
-                    kq = u;
-                    ax = 1;
-                } else {
-                    kq = t;
-                    ax = 0;
-                }
-                const int src1 = o1 + n * ne1 + r_in_level(uu, vv);
-                int src2 = 0;
-                if (kq > 1) src2 = o2 + n * ne2 + r_in_level(uu == u ? u : u - 2, vv == v ? v : v - 2);
-                const int r0d = n == 0 ? r0_row(S, t, u) + v : kMmdNoR0;
-                tab[lvl[s] + e] = int2{src1 | (src2 << 16), kq | (ax << 5) | (r0d << 7)};
-            }
-        }
-    }
-}
 
 // Positions of work items in decreasing order of estimated work (buckets of a quarter
 // octave; items of one bucket keep their order), for the kernels' dynamic queues.
@@ -549,7 +468,7 @@ struct Plan {
     int8_t *stop_level = nullptr, *pred_level = nullptr;  // per radial item
     int *order = nullptr, *lm_ctl = nullptr;               // learned mode: item order; n_order, queue, cursor[9]
     MmdArgs mmd;
-    int mmd_blocks = 0, mmd_threads = 128, mmd_kpl = 32;
+    int mmd_blocks = 0;
     size_t mmd_smem = 0;
     OcProjArgs ocp;
     int ocp_blocks = 0;
@@ -903,9 +822,11 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     proj_off[projs.size()] = sph_tot;
     const int64_t out_tot = out_off[nt];
 
-    // Cartesian pair schedules of the type 1 items, one per (bra, ket) table class
-    const int mmd_kpl = ncart(mmd_lmax) * ncart(mmd_lmax) <= 256 ? 8 : 32;
-    std::vector<uint16_t> mmd_sched;
+    // Cartesian pair tables of the type 1 items, one per (bra, ket) table class
+    std::vector<int4> mmd_pairs;
+    size_t mmd_smem = 0;
+    CHECK_INPUT(items.empty() || (mmd_lmax <= kMmdMaxL && mmd_accept_bytes(mmd_lmax, mmd_smax) <= 200 * 1024),
+                "type 1 workspace of this batch's angular momenta exceeds one block's shared memory");
     {
         std::map<std::vector<int8_t>, int> tab_id;  // a shell's Cartesian table -> class
         std::vector<int> sh_tab(ns);
@@ -915,20 +836,30 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             sh_tab[i] = ins.first->second;
         }
         const int ntab = (int)tab_id.size();
-        std::vector<std::pair<int, int>> sched_of((size_t)ntab * ntab, {-1, 0});  // (bra, ket) class -> (offset, rows)
+        std::vector<int> pairs_of((size_t)ntab * ntab, -1);
         for (auto &it : items) {
-            const int nA = ncart(sh_L[it.bra]), nB = ncart(sh_L[it.ket]);
-            CHECK_INPUT(nA * nB <= 32 * mmd_kpl, "type 1 block larger than one pass of the pair schedule");
-            std::pair<int, int> &f = sched_of[(size_t)sh_tab[it.bra] * ntab + sh_tab[it.ket]];
-            if (f.first < 0) {
-                const int off = (int)mmd_sched.size();
-                const int rows = mmd_pair_schedule(cart.data() + 3 * sh_co[it.bra], nA, cart.data() + 3 * sh_co[it.ket],
-                                                   nB, mmd_kpl, mmd_sched);
-                f = {off, rows};
+            const int la = sh_L[it.bra], lb = sh_L[it.ket];
+            CHECK_INPUT(ncart(la) * ncart(lb) <= kFinMaxPairs, "type 1 block larger than 1024 Cartesian pairs");
+            int &f = pairs_of[(size_t)sh_tab[it.bra] * ntab + sh_tab[it.ket]];
+            if (f < 0) {
+                f = (int)mmd_pairs.size();
+                mmd_pair_table(cart.data() + 3 * sh_co[it.bra], la, cart.data() + 3 * sh_co[it.ket], lb, mmd_pairs);
             }
-            it.sched = f.first;
-            it.sched_rows = f.second;
+            it.pairs = f;
+            it.cls = la * kMmdCls + lb;
+            mmd_smem = std::max(mmd_smem, (size_t)mmd_smem_doubles(st.mmd_cls[it.cls]) * sizeof(double));
         }
+    }
+    // per potential, the order of its terms that takes the n = 2 terms first
+    std::vector<int> p_perm(p_c.size()), p_n2(np, 0);
+    for (int p = 0; p < np; p++) {
+        int k = p_off[p];
+        for (int pass = 0; pass < 2; pass++)
+            for (int q = 0; q < p_n[p]; q++)
+                if ((p_pw[p_off[p] + q] == 2) == (pass == 0)) {
+                    p_perm[k++] = q;
+                    p_n2[p] += pass == 0;
+                }
     }
     // estimated work per type 1 item: primitive triples x (Hermite + R entries + contraction terms)
     std::vector<int> mmd_order;
@@ -1021,10 +952,6 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             fin_groups[gi].smem = fin_smem_bytes(fs);
         }
     }
-    std::vector<int> mmd_etab, mmd_etab_off, mmd_rtab_off;
-    std::vector<int2> mmd_rtab;
-    mmd_update_tables(mmd_lmax, mmd_smax, mmd_etab, mmd_etab_off, mmd_rtab, mmd_rtab_off);
-
     // F_l(r) tables per (shell, centre) pair: (lmax + 1) rows of grid points each, when they
     // stay below 8 GiB
     std::vector<int64_t> fp_off(fp_shell.size() + 1, 0);
@@ -1082,13 +1009,11 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                  o_ucls = pk.add(ucls), o_ulist = pk.add(ulist), o_sbig = pk.add(scr_big), o_ssmall = pk.add(scr_small),
                  o_suo = pk.add(su_off);
     const size_t o_bs = pk.add(blk_shell), o_bo = pk.add(blk_oc), o_bco = pk.add(blk_cart_off), o_bso = pk.add(blk_sph_off),
-                 o_poffp = pk.add(proj_off), o_msch = pk.add(mmd_sched);
+                 o_poffp = pk.add(proj_off), o_mpair = pk.add(mmd_pairs), o_pperm = pk.add(p_perm), o_pn2 = pk.add(p_n2);
     const size_t o_fps = pk.add(fp_shell), o_fpc = pk.add(fp_centre), o_fpl = pk.add(fp_lmax), o_fpo = pk.add(fp_off),
                  o_ifa = pk.add(item_fa), o_ifb = pk.add(item_fb), o_omo = pk.add(om_off), o_tfa = pk.add(task_fpa),
                  o_tfb = pk.add(task_fpb);
-    const size_t o_met = pk.add(mmd_etab), o_meto = pk.add(mmd_etab_off), o_mrt = pk.add(mmd_rtab),
-                 o_mrto = pk.add(mmd_rtab_off), o_mord = pk.add(mmd_order), o_ford = pk.add(fin_order);
-    std::vector<int8_t> stop_dummy;
+    const size_t o_mord = pk.add(mmd_order), o_ford = pk.add(fin_order);
     DevBuf *bin = own_buffers ? &P.in : &st.in[set], *bscr = own_buffers ? &P.scratch : &st.scratch[set],
            *bout = own_buffers ? &P.out : &st.out[set];
     GRPP_CUDA(bin->ensure(pk.buf.size()));
@@ -1155,52 +1080,36 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
 
     // ---------------------------------------------------------------- 2. MMD
     if (!items.empty()) {
-        MmdArgs m{};
+        MmdArgs m = st.mmd;
         m.items = at<MmdItem>(ib, o_items);
         m.n_items = (int)items.size();
         m.shell_L = at<int>(ib, o_shL);
         m.shell_nprim = at<int>(ib, o_shnp);
         m.shell_prim_off = at<int>(ib, o_shpo);
-        m.shell_cart_off = at<int>(ib, o_shco);
         m.prim_coef = at<double>(ib, o_pc);
         m.prim_alpha = at<double>(ib, o_pa);
         m.shell_origin = at<double>(ib, o_sor);
-        m.cart = at<int8_t>(ib, o_cart);
         m.pot_nprim = at<int>(ib, o_pn);
         m.pot_prim_off = at<int>(ib, o_poff);
         m.pot_powers = at<int>(ib, o_ppw);
         m.pot_coef = at<double>(ib, o_pcoef);
         m.pot_alpha = at<double>(ib, o_palpha);
+        m.pot_perm = at<int>(ib, o_pperm);
+        m.pot_n2 = at<int>(ib, o_pn2);
         m.centre_origin = at<double>(ib, o_cor);
         m.out[0] = o_arep;
         m.out[1] = Ucd;
         m.out[2] = Scd;
-        m.lmax = mmd_lmax;
-        m.smax = mmd_smax;
-        m.status = statusd;
         m.counters = (unsigned long long *)(statusd + 16);
-        m.sched = at<uint16_t>(ib, o_msch);
-        m.etab = at<int>(ib, o_met);
-        m.etab_off = at<int>(ib, o_meto);
-        m.rtab = at<int2>(ib, o_mrt);
-        m.rtab_off = at<int>(ib, o_mrto);
+        m.pairs = at<int4>(ib, o_mpair);
         m.order = at<int>(ib, o_mord);
         m.queue = statusd + 8;
-        const int wpb = 4;
-        P.mmd_kpl = mmd_kpl;
-        // per warp: the workspace, then 32 x KPL pair descriptors (8 bytes each)
-        const size_t smem = (size_t)wpb * (mmd_ws_size(mmd_lmax, mmd_smax) + 32 * P.mmd_kpl) * sizeof(double);
-        CHECK_INPUT(smem <= 200 * 1024, "type 1 workspace of this batch's angular momenta exceeds one block's shared memory");
         P.mmd = m;
         // persistent grid: the resident blocks pop items until the queue is empty
         int mmd_occ = 0;
-        if (mmd_kpl == 8)
-            GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<8, false>, 32 * wpb, smem));
-        else
-            GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<32, false>, 32 * wpb, smem));
-        P.mmd_blocks = (int)std::min<int64_t>(((int64_t)items.size() + wpb - 1) / wpb, (int64_t)nsm * std::max(mmd_occ, 1));
-        P.mmd_threads = 32 * wpb;
-        P.mmd_smem = smem;
+        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<false>, kMmdThreads, mmd_smem));
+        P.mmd_blocks = (int)std::min<int64_t>((int64_t)items.size(), (int64_t)nsm * std::max(mmd_occ, 1));
+        P.mmd_smem = mmd_smem;
     }
 
     // ---------------------------------------------------------------- 3. outercore projections
@@ -1410,13 +1319,8 @@ int plan_launch(Plan &P)
     GRPP_CUDA(cudaMemsetAsync(P.status, 0, 64 * sizeof(int), s));  // status, counters, assembly queues
     GRPP_CUDA(cudaEventRecord(ev[0], s));
     if (P.mmd_blocks > 0) {
-        if (P.count_ops) {
-            if (P.mmd_kpl == 8) mmd_kernel<8, true><<<P.mmd_blocks, P.mmd_threads, P.mmd_smem, s>>>(P.mmd);
-            else mmd_kernel<32, true><<<P.mmd_blocks, P.mmd_threads, P.mmd_smem, s>>>(P.mmd);
-        } else {
-            if (P.mmd_kpl == 8) mmd_kernel<8, false><<<P.mmd_blocks, P.mmd_threads, P.mmd_smem, s>>>(P.mmd);
-            else mmd_kernel<32, false><<<P.mmd_blocks, P.mmd_threads, P.mmd_smem, s>>>(P.mmd);
-        }
+        if (P.count_ops) mmd_kernel<true><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, s>>>(P.mmd);
+        else mmd_kernel<false><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, s>>>(P.mmd);
         GRPP_CUDA(cudaGetLastError());
     }
     GRPP_CUDA(cudaEventRecord(ev[1], s));

@@ -1,21 +1,41 @@
-// Type 1 (radially local) GRPP integrals by McMurchie-Davidson, and
-// two-centre overlaps by Obara-Saika, one warp per work item.
+// Type 1 (radially local) GRPP integrals by McMurchie-Davidson, and two-centre overlaps by
+// Obara-Saika, one thread block per work item.
 //
 // Reference algorithm: libgrpp/type1_mcmurchie_davidson.c:107-622 and
-// libgrpp/type1_integrals.c:43-78 (sum over potential terms k of c_k times
-// the primitive-pair contraction), libgrpp/overlap.c:39-139.
+// libgrpp/type1_integrals.c:43-78 (sum over potential terms k of c_k times the
+// primitive-pair contraction), libgrpp/overlap.c:39-139.
 //
-// A work item is <bra| c r^(n-2) exp(-zeta r^2) (centred at C) |ket> summed
-// over the terms of one potential, or the overlap <bra|ket>. Per primitive
-// pair and term the warp builds
-//   E[axis][i][j][t]  Hermite expansion coefficients, by wavefronts w = i+j
-//                     (each E^{ij} depends on E^{i-1,j} or E^{i,j-1} only),
-//   R^n_{tuv}         auxiliary integrals (Boys for n=1, G_n for n=0), by
-//                     levels s = t+u+v (each level depends on s-1, s-2 only),
-// in shared memory, then each lane accumulates its Cartesian pairs
-//   sum_{tuv} E^x_t E^y_u E^z_v R^0_{tuv}.
-// The contraction order (terms outer, primitive pairs inner, c_i c_j then
-// c_k applied as in the reference's daxpy calls) is kept.
+// A work item is <bra| c r^(n-2) exp(-zeta r^2) (centred at C) |ket> summed over the terms of
+// one potential, or the overlap <bra|ket>. For a primitive triple (i, j, k) with exponents
+// a, b, zeta, q = a + b + zeta, Q = (a A + b B + zeta C) / q and K_d the Gaussian product
+// factor of axis d:
+//   n = 2, and the overlap (zeta = 0):  (pi/q)^(3/2) prod_d S_d[i_d][j_d], Obara-Saika tables;
+//   n = 1, n = 0:                       sum_tuv E^x_t E^y_u E^z_v R^0_tuv,
+// E[axis][i][j][t] the Hermite expansion coefficients and R^n_tuv the auxiliary integrals, by
+// levels s = t + u + v (level s from s-1 and s-2) from (-2q)^n F_n (Boys) for n = 1 and from
+// (2q)^n G_n for n = 0. The n = 0 levels are differences R^(n+1) - 2q R^n that cancel for tight
+// exponents far from C; G_n, the powers of 2q and the levels therefore keep libgrpp's operations
+// one by one, so that the lost digits are the same ones.
+//
+// Mapping. A block takes the item's triples in groups of up to 64, for which it forms scalars
+// (a thread per triple and axis) and auxiliary values (four threads per triple), and these in
+// batches of T (a power of two per (la, lb) and kind, MmdClass). Every phase of a batch runs
+// over (entry, triple) pairs with the triple fastest: tables are laid out [entry][T], so the
+// lanes of a warp work on few different entries, addresses are consecutive and the update
+// programs (which entry comes from which) are read once per T triples. Per batch: step
+// s = 1..S does the E wavefront i + j = s and the R level s together (one barrier each), then
+// X[t,u][az,bz] = sum_v E^z_v R^0_tuv and, per Cartesian pair, sum_t E^x_t sum_u E^y_u X.
+// Splitting the contraction at z makes it about 4 operations per pair where the triple sum
+// needs 14 (g x g) to 60 (i x i).
+// Triples whose Gaussian product exponents sum to more than 800 are dropped: K_x K_y K_z < 1e-347
+// there, so their contributions underflow.
+//
+// What bounds it: shared-memory latency between the barriers of the S steps (FP64 is mostly
+// idle). Three blocks of 256 threads per SM with 70 kB each (T as large as fits) measured faster
+// than two with 104 kB (11.6 ms), four with 52 kB (10.3) or one with 204 kB (20.0) on the 65536
+// tasks of the s..g workload: 10.0 ms, against 40.7 ms for one warp per item walking its triples
+// one by one. The matrices of a 15-atom molecule with i shells, whose largest class set the registers
+// and shared memory of every item there: 51.9 -> 6.6 ms; a 200-task molecule: 2.0 -> 0.19 ms.
 #pragma once
 
 #include "grpp_common.cuh"
@@ -31,75 +51,134 @@ struct MmdItem {
     int pot;             // potential index, or -1 for an overlap
     int out_kind;        // 0: arep output, 1: outercore U scratch, 2: outercore S scratch
     int64_t out_off;     // offset of the nbra x nket row-major block
-    int sched;           // offset of the item's Cartesian pair schedule (MmdArgs::sched)
-    int sched_rows;      // slot couples (2h, 2h+1) of the schedule in use
+    int pairs;           // offset of the item's Cartesian pair table (MmdArgs::pairs)
+    int cls;             // class index la * kMmdCls + lb
+};
+
+constexpr int kMmdThreads = 256;
+constexpr int kMmdMaxL = 8;               // largest angular momentum whose tables are built
+constexpr int kMmdCls = kMmdMaxL + 1;
+constexpr int kMmdMaxPrims = 64;          // primitives per shell (the engine's limit)
+constexpr int kMmdMaxLgT = 6;
+constexpr int kMmdSmem = 70 * 1024;       // dynamic shared memory at most: three blocks per SM
+constexpr int kMmdGroup = 64;             // triples whose scalars and auxiliary values are formed together
+constexpr int kMmdRing = 512;             // live triples waiting: at most kMmdGroup - 1 + kMmdThreads
+constexpr double kMmdDropArg = 800.0;     // sum of the Gaussian product exponents that underflows
+constexpr double kPi15 = 5.568327996831708;  // pi^(3/2), correctly rounded
+static_assert(4 * kMmdGroup == kMmdThreads && (1 << kMmdMaxLgT) <= kMmdGroup, "four threads per triple of a group");
+
+// Tables of one (la, lb), built once per device (mmd_build_classes)
+struct MmdClass {
+    int la, lb, S;
+    int nE;              // Hermite coefficients of the three axes, [ax][(i, j)][t <= i + j]
+    int nR0;             // R^0_tuv, rows (t, u) of consecutive v
+    int nX;              // X[(az, bz)][t][u], t + u <= S - az - bz
+    int maxlev;          // largest level of R^n_tuv
+    int e_off, o_off, z_off, r_off;  // programs: E, Obara-Saika, X, R
+    int lv;              // level starts in MmdArgs::levels: S + 2 each of E, Obara-Saika, R
+    int lgT[2];          // log2 of the triples per batch: [0] n = 2 and overlap, [1] n = 0, 1
 };
 
 struct MmdArgs {
     const MmdItem *items;
     int n_items;
-    const int *shell_L, *shell_nprim, *shell_prim_off, *shell_cart_off;
+    const int *shell_nprim, *shell_prim_off, *shell_L;
     const double *prim_coef, *prim_alpha, *shell_origin;
-    const int8_t *cart;
     const int *pot_nprim, *pot_prim_off, *pot_powers;
     const double *pot_coef, *pot_alpha;
+    const int *pot_perm, *pot_n2;  // per potential: term order with the n = 2 terms first, their number
     const double *centre_origin;
     double *out[3];
-    int smax;            // max la+lb over the items (sizes the shared workspace)
-    int lmax;            // max l over the items
-    int *status;
     unsigned long long *counters;  // kRadCntMmdTriples / kRadCntMmdFlops slots (may be null)
-    // per class of (bra, ket) Cartesian tables, 32 x KPL slots: slot (q, lane) at q * 32 + lane
-    // holds the pair index m * nket + n the lane owns in its q-th register, or kMmdNoPair. Slots
-    // (2h, 2h+1) of a lane hold pairs with equal (ax+bx, ay+by, az+bz), or one pair and an empty
-    // slot; the 32 lanes of a slot row hold pairs of equal or adjacent (ax+bx, ay+by, az+bz)
-    const uint16_t *sched;
-    // update programs of the Hermite coefficients, per (la, lb) at etab_off[la * (kMaxL + 1) + lb]:
-    // one int per coefficient in wavefront order (see mmd_e_code); and of the R^n_tuv table, per
-    // S at rtab_off[S]: one int2 per entry of levels s >= 1, at the entry's own index (see mmd_r_code)
-    const int *etab, *etab_off;
-    const int2 *rtab;
-    const int *rtab_off;
-    // dynamic schedule: warps pop positions from *queue (zeroed before the launch) and take
+    const MmdClass *classes;
+    const int *levels;
+    // update programs, one int2 per entry (mmd_e_code, mmd_o_code, mmd_r_code, mmd_z_code)
+    const int2 *etab, *otab, *rtab, *ztab;
+    // per class of (bra, ket) Cartesian tables, one int4 per pair (mmd_pair)
+    const int4 *pairs;
+    // dynamic schedule: blocks pop positions from *queue (zeroed before the launch) and take
     // item order[position]; the host orders items by decreasing estimated work
     const int *order;
     int *queue;
 };
-constexpr uint16_t kMmdNoPair = 0xffff;
 
-// Hermite coefficient E[ax][i][j][t] (row-major over (ax, i, j, t), extents 3, la+1, lb+1, S+1):
-// bits 0-12 its index, 13-14 ax, 15-18 i, 19-22 j, 23-27 t, 28-30 the recurrence form
-// (type1_mcmurchie_davidson.c:569-622):
-//   0: K[ax] (i = j = 0)           1: (Q-A)[ax] E[ax][0][0][0] (i = 1, j = 0)
-//   2: (Q-B)[ax] E[ax][0][0][0] (i = 0, j = 1)
-//   3: (Q-B)[ax] E[ax][0][j-1][0] + E[ax][0][j-1][1] (i = 0, j >= 2)
-//   4: (Q-A)[ax] E[ax][i-1][j][0] + E[ax][i-1][j][1] (other t = 0)
-//   5: (i E[ax][i-1][j][t-1] + j E[ax][i][j-1][t-1]) / (2 q t) (t >= 1), each term as f i E
-__host__ __device__ inline int mmd_e_code(int dst, int ax, int i, int j, int t)
+__host__ __device__ inline int mmd_tet(int m) { return (m + 1) * (m + 2) * (m + 3) / 6; }
+// first t of E[ax][i][j] among the axis' coefficients
+__host__ __device__ inline int mmd_e_row(int lb, int i, int j)
 {
-    int ty;
-    if (t > 0) ty = 5;
-    else if (i == 0 && j == 0) ty = 0;
-    else if (i == 1 && j == 0) ty = 1;
-    else if (i == 0 && j == 1) ty = 2;
-    else if (i == 0) ty = 3;
-    else ty = 4;
-    return dst | (ax << 13) | (i << 15) | (j << 19) | (t << 23) | (ty << 28);
+    const int lb1 = lb + 1;
+    return lb1 * i * (i - 1) / 2 + i * (lb1 * (lb1 + 1) / 2) + j * i + j * (j + 1) / 2;
 }
-constexpr int kMmdNoR0 = 4095;  // R^n_tuv entry with n > 0: not an R^0 value
+__host__ __device__ inline int mmd_e_axis(int la, int lb) { return (la + 1) * (lb + 1) * (la + lb + 2) / 2; }
+// start of row (t, u) in the R^0 layout: rows ordered t-major, then u
+__host__ __device__ __forceinline__ int r0_row(int S, int t, int u)
+{
+    return mmd_tet(S) - mmd_tet(S - t) + u * (S - t + 1) - u * (u - 1) / 2;
+}
+// index of (u + v = k, v) within level s
+__host__ __device__ __forceinline__ int r_in_level(int u, int v) { return (u + v) * (u + v + 1) / 2 + v; }
 
+// doubles of shared memory: per triple of a group (scalars and R^n_000), and of a batch (tables)
+__host__ __device__ inline int mmd_group_doubles(const MmdClass &c) { return 15 + c.S + 1; }
+__host__ __device__ inline int mmd_batch_doubles(const MmdClass &c, int kind)
+{
+    if (kind == 0) return 3 * (c.la + 1) * (c.lb + 1);
+    const int u = c.nX > 3 * c.maxlev ? c.nX : 3 * c.maxlev;
+    return c.nE + c.nR0 + u;
+}
+// sums of the Cartesian pairs: one per 32 triples of a batch
+__host__ __device__ inline int mmd_sum_groups(const MmdClass &c)
+{
+    const int lg = c.lgT[0] > c.lgT[1] ? c.lgT[0] : c.lgT[1];
+    return lg > 5 ? 1 << (lg - 5) : 1;
+}
+__host__ __device__ inline int mmd_smem_doubles(const MmdClass &c)
+{
+    const int a = mmd_batch_doubles(c, 0) << c.lgT[0], b = mmd_batch_doubles(c, 1) << c.lgT[1];
+    return ncart(c.la) * ncart(c.lb) * mmd_sum_groups(c) + mmd_group_doubles(c) * kMmdGroup + (a > b ? a : b);
+}
 
-// FP64 operations of one primitive triple, by phase (FMA = 2, exp/div/sqrt/pow = 1):
-// setup (q, 3 mu, 3 Q, 9 exponentials, K) 40; a Hermite coefficient 5; an auxiliary
-// function value 16 (Boys, 6th-order Taylor) or 100 per G_n series; an R^n_tuv entry 5;
-// a term E_x E_y E_z R of the contraction 3, plus 3 per Cartesian pair.
+// ---- update programs (host-built)
+// Hermite coefficient (type1_mcmurchie_davidson.c:569-622), t = 0:
+//   P E[src] + (second ? E[src + 1] : 0), P = (Q-A)[ax] or (Q-B)[ax] (side 1)
+// t >= 1: (i E[src1] + j E[src2]) / (2 q t)
+inline int2 mmd_e_code0(int dst, int src, int ax, int side, bool second)
+{
+    return int2{dst | (src << 13) | (1 << 30), (ax << 13) | (side << 20) | ((second ? 1 : 0) << 24)};
+}
+inline int2 mmd_e_code(int dst, int src1, int src2, int ax, int i, int j, int t)
+{
+    return int2{dst | (src1 << 13), src2 | (ax << 13) | (t << 15) | (i << 20) | (j << 24)};
+}
+// Obara-Saika table (overlap.c:92-120): P S[s1] + (n2 S[s2] + n3 S[s3]) / (2q)
+inline int2 mmd_o_code(int dst, int s1, int s2, int s3, int n2, int n3, int ax, int side)
+{
+    return int2{dst | (s1 << 10) | (s2 << 20), s3 | (n2 << 10) | (n3 << 14) | (ax << 18) | (side << 20)};
+}
+// R^n_tuv at level s (type1_mcmurchie_davidson.c:457-564): (k - 1) D2 + (Q-C)[ax] D1 with
+// D1 = prev1[src1 + ne1] (- 2q prev1[src1] for the 1/r^2 terms), D2 likewise from prev2 (k > 1)
+inline int2 mmd_r_code(int src1, int src2, int dst_r0, int k, int ax)
+{
+    return int2{src1 | (src2 << 16), dst_r0 | (k << 14) | (ax << 19)};
+}
+constexpr int kMmdNoR0 = 8191;  // order n > 0: not an R^0 value
+// X entry: sum_{v <= vz} E[zrow + v] R0[row + v]
+inline int2 mmd_z_code(int row, int zrow, int vz) { return int2{row | (zrow << 16), vz}; }
+// Cartesian pair: E rows of axes x and y; start of its X rows, their count W + 1 and tx, uy; the
+// three Obara-Saika entries; index in the output block
+inline int4 mmd_pair(int ex, int ey, int xbase, int W, int tx, int uy, int o0, int o1, int o2, int out)
+{
+    return int4{ex | (ey << 16), xbase | (W << 16) | (tx << 21) | (uy << 26), o0 | (o1 << 10) | (o2 << 20), out};
+}
+
+// FP64 operations of one primitive triple of libgrpp's algorithm, by phase (FMA = 2, exp/div/sqrt/pow
+// = 1), for the counting build: setup 40; a Hermite coefficient 5; an auxiliary function value
+// 16 (Boys, 6th-order Taylor) or 100 per G_n series; an R^n_tuv entry 5; a term
+// E_x E_y E_z R of the contraction 3, plus 3 per Cartesian pair.
 __host__ __device__ inline unsigned long long mmd_e_count(int la, int lb)
 {
     return 3ull * ((la + 1) * (lb + 1) + (lb + 1) * la * (la + 1) / 2 + (la + 1) * lb * (lb + 1) / 2);
 }
-
-// shared workspace per warp, in doubles
-__host__ __device__ inline int mmd_e_size(int lmax) { return 3 * (lmax + 1) * (lmax + 1) * (2 * lmax + 1); }
 __host__ __device__ inline int mmd_r_size(int smax)
 {
     // sum over levels s of (s+1)(s+2)/2 entries x (smax-s+1) orders
@@ -107,397 +186,285 @@ __host__ __device__ inline int mmd_r_size(int smax)
     for (int s = 0; s <= smax; s++) tot += (s + 1) * (s + 2) / 2 * (smax - s + 1);
     return tot;
 }
-constexpr int kMmdMaxPrims = 64;     // primitives per shell (the engine's limit)
-constexpr double kPi15 = 5.568327996831708;  // pi^(3/2), correctly rounded
 
-// R^0_tuv (t+u+v <= S) in rows (t, u) of consecutive v: tet(S) = (S+1)(S+2)(S+3)/6 values
-__host__ __device__ inline int mmd_tet(int m) { return (m + 1) * (m + 2) * (m + 3) / 6; }
-__host__ __device__ inline int mmd_ws_size(int lmax, int smax)
-{
-    return mmd_e_size(lmax) + mmd_r_size(smax) + mmd_tet(smax) + 2 * (smax + 2) + 16 + 2 * kMmdMaxPrims + 12 +
-           (smax + 1) + 7 * 32;
-}
-
-// start of row (t, u) in the R^0 layout: rows ordered t-major, then u
-__host__ __device__ __forceinline__ int r0_row(int S, int t, int u)
-{
-    return mmd_tet(S) - mmd_tet(S - t) + u * (S - t + 1) - u * (u - 1) / 2;
-}
-
-// sum_{t<=tx, u<=uy, v<=vz} E^x_t E^y_u E^z_v R^0_tuv for two pairs with equal (tx, uy, vz),
-// side by side on shared R^0 loads; each sum in the reference's (t, u, v) order
-__device__ __forceinline__ void mmd_contract2(const double *E, const double *R0, int S, int2 d0, int2 d1, double &s0,
-                                              double &s1)
-{
-    const int tx = (d0.y >> 16) & 31, uy = (d0.y >> 21) & 31, vz = (d0.y >> 26) & 31;
-    const int ox0 = d0.x & 0xffff, oy0 = (int)((unsigned)d0.x >> 16);
-    const int ox1 = d1.x & 0xffff, oy1 = (int)((unsigned)d1.x >> 16);
-    const double *ez0 = E + (d0.y & 0xffff), *ez1 = E + (d1.y & 0xffff);
-    s0 = 0.0;
-    s1 = 0.0;
-    for (int t = 0; t <= tx; t++) {
-        const double ex0 = E[ox0 + t], ex1 = E[ox1 + t];
-        for (int u = 0; u <= uy; u++) {
-            const double exy0 = ex0 * E[oy0 + u], exy1 = ex1 * E[oy1 + u];
-            const double *r0 = R0 + r0_row(S, t, u);
-#pragma unroll 4
-            for (int v = 0; v <= vz; v++) {
-                const double rv = r0[v];
-                s0 += exy0 * ez0[v] * rv;
-                s1 += exy1 * ez1[v] * rv;
-            }
-        }
-    }
-}
-
-constexpr int kMmdMaxPairsPerLane = 32;  // up to 1024 Cartesian pairs per pass (KPL = 32 variant)
-
-__device__ __forceinline__ int eidx(int lb1, int S1, int ax, int i, int j, int t, int la1)
-{
-    return ((ax * la1 + i) * lb1 + j) * S1 + t;
-}
-
-// level offsets of the R table: lvl_off[s] = sum_{s'<s} ne(s') (S-s'+1)
-__device__ __forceinline__ int r_level_off(int S, int s)
-{
-    int o = 0;
-    for (int q = 0; q < s; q++) o += (q + 1) * (q + 2) / 2 * (S - q + 1);
-    return o;
-}
-
-// index of (u+v = k, v) within level s: tri(k) + v
-__host__ __device__ __forceinline__ int r_in_level(int u, int v) { return (u + v) * (u + v + 1) / 2 + v; }
-
-// KPL: Cartesian pairs held per lane per pass (8: up to 256 pairs, 32: up to 1024)
 // COUNT: keep the operation counters (a separate instantiation, so the timed kernel carries none)
-template <int KPL, bool COUNT>
-__global__ void __launch_bounds__(128) mmd_kernel(MmdArgs a)
+template <bool COUNT>
+__global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
 {
     extern __shared__ double smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wpb = blockDim.x >> 5;
-    const int ws = mmd_ws_size(a.lmax, a.smax);
-    double *E = smem + warp * ws;
-    double *R = E + mmd_e_size(a.lmax);
-    double *R0 = R + mmd_r_size(a.smax);
-    double *aux = R0 + mmd_tet(a.smax);
-    int *lvl = (int *)(aux + (a.smax + 2));
-    double *normA = aux + 2 * (a.smax + 2) + 16, *normB = normA + kMmdMaxPrims;  // per item
-    // per primitive triple: (Q-A)[3], (Q-B)[3], K[3], (Q-C)[3], then 1/(2 q t) for t = 1..S
-    double *sQA = normB + kMmdMaxPrims, *sQB = sQA + 3, *sK = sQB + 3, *sQC = sK + 3, *finv = sQC + 3;
-    // per chunk of 32 primitive pairs, lane l's pair: q, Q[3], K[3] at spre[v * 32 + l]
-    double *spre = finv + (a.smax + 1);
-    // lane-private descriptors of the Cartesian pairs of the current pass (after all warps'
-    // workspaces): x = E row of axis x | E row of axis y << 16, y = E row of axis z |
-    // (ax+bx) << 16 | (ay+by) << 21 | (az+bz) << 26 — each pair is decoded once per pass,
-    // not once per primitive triple
-    int2 *pdesc = reinterpret_cast<int2 *>(smem + wpb * ws) + warp * 32 * KPL;
-
-    unsigned long long c_trip = 0, c_fl = 0;  // operation counters of this lane
+    __shared__ int ring[kMmdRing];
+    __shared__ int s_cnt[kMmdThreads / 32];
+    __shared__ int s_item;
+    __shared__ double normA[kMmdMaxPrims], normB[kMmdMaxPrims];
+    __shared__ double rcp[2 * kMmdMaxL + 1];  // 1/t
+    __shared__ unsigned long long s_fl;
+    constexpr int NT = kMmdThreads, NW = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long c_trip = 0, c_fl = 0;  // operation counters of this thread
+    if (tid <= 2 * kMmdMaxL) rcp[tid] = 1.0 / max(tid, 1);
     for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(a.queue, 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= a.n_items) break;
-        const MmdItem item = a.items[a.order[k]];
-        const int la = a.shell_L[item.bra], lb = a.shell_L[item.ket];
-        const int nA = ncart(la), nB = ncart(lb), S = la + lb;
-        const int la1 = la + 1, lb1 = lb + 1, S1 = S + 1;
+        if (tid == 0) {
+            const int k = atomicAdd(a.queue, 1);
+            s_item = k < a.n_items ? a.order[k] : -1;
+        }
+        __syncthreads();
+        const int it = s_item;
+        if (it < 0) break;
+        const MmdItem item = a.items[it];
+        const MmdClass &cl = a.classes[item.cls];
+        const int la = cl.la, lb = cl.lb, S = cl.S, npairs = ncart(la) * ncart(lb);
+        const int G = mmd_sum_groups(cl);
+        const int *lv = a.levels + cl.lv;
         const double *Ao = a.shell_origin + 3 * item.bra;
         const double *Bo = item.ket_at_centre ? a.centre_origin + 3 * item.centre : a.shell_origin + 3 * item.ket;
         const double *Co = a.centre_origin + 3 * item.centre;
-        const double A[3] = {Ao[0], Ao[1], Ao[2]}, B[3] = {Bo[0], Bo[1], Bo[2]}, C[3] = {Co[0], Co[1], Co[2]};
-        const int8_t *ca = a.cart + 3 * a.shell_cart_off[item.bra];
-        const int8_t *cb = a.cart + 3 * a.shell_cart_off[item.ket];
-        const int npA = a.shell_nprim[item.bra], npB = a.shell_nprim[item.ket];
+        const int npA = a.shell_nprim[item.bra], npB = a.shell_nprim[item.ket], np2 = npA * npB;
         const double *cA = a.prim_coef + a.shell_prim_off[item.bra], *xA = a.prim_alpha + a.shell_prim_off[item.bra];
         const double *cB = a.prim_coef + a.shell_prim_off[item.ket], *xB = a.prim_alpha + a.shell_prim_off[item.ket];
         const bool overlap = item.pot < 0;
-        const int nterms = overlap ? 1 : a.pot_nprim[item.pot];
-        double *out = a.out[item.out_kind] + item.out_off;
-
-        __syncwarp();  // the previous item's readers of lvl and the norms are done
-        if (lane == 0) {
-            int o = 0;
-            for (int s = 0; s <= S; s++) {
-                lvl[s] = o;
-                o += (s + 1) * (s + 2) / 2 * (S - s + 1);
+        const int poff = overlap ? 0 : a.pot_prim_off[item.pot];
+        const int nterms = overlap ? 1 : a.pot_nprim[item.pot], n2 = overlap ? 1 : a.pot_n2[item.pot];
+        const int4 *pt = a.pairs + item.pairs;
+        double *acc = smem, *ws = smem + npairs * G;
+        for (int p = tid; p < npairs * G; p += NT) acc[p] = 0.0;
+        if (tid < npA) normA[tid] = gaussian_norm(la, xA[tid]);
+        else if (tid >= kMmdMaxPrims && tid < kMmdMaxPrims + npB) normB[tid - kMmdMaxPrims] = gaussian_norm(lb, xB[tid - kMmdMaxPrims]);
+        if (COUNT && tid == 0) s_fl = 0;
+        __syncthreads();
+        if (COUNT) {  // operations of one triple's contraction over the item's Cartesian pairs
+            unsigned long long f = 0;
+            for (int p = tid; p < npairs; p += NT) {
+                const int y = pt[p].y, W = (y >> 16) & 31, tx = (y >> 21) & 31, uy = (int)((unsigned)y >> 26);
+                f += 3ull * (tx + 1) * (uy + 1) * (S - W + 1) + 3ull;
             }
+            atomicAdd(&s_fl, f);
+            __syncthreads();
         }
-        // primitive norms depend on (shell, primitive) only: once per item, one per lane
-        for (int q = lane; q < npA; q += 32) normA[q] = gaussian_norm(la, xA[q]);
-        for (int q = lane; q < npB; q += 32) normB[q] = gaussian_norm(lb, xB[q]);
-        __syncwarp();
-
-        const int npairs = nA * nB;
-        {  // one pass over all pairs: npairs <= 32 x KPL (the host checks it)
-            const int pass = 0;
-            // operations of one primitive triple's contraction over this pass's Cartesian pairs (counters)
-            const int pend = min(npairs, pass + 32 * KPL);
-            unsigned long long contract_fl = 0;
-            if (COUNT) {
-                for (int pr = pass + lane; pr < pend; pr += 32) {
-                    const int m = pr / nB, n = pr % nB;
-                    contract_fl += 3ull * (ca[3 * m] + cb[3 * n] + 1) * (ca[3 * m + 1] + cb[3 * n + 1] + 1) *
-                                       (ca[3 * m + 2] + cb[3 * n + 2] + 1) + 3ull;
-                }
-                for (int o = 16; o > 0; o >>= 1) contract_fl += __shfl_xor_sync(0xffffffffu, contract_fl, o);
-            }
-            const uint16_t *sch = a.sched + item.sched;
-            const int nslots = 2 * item.sched_rows;
+        // group arrays, [..][kMmdGroup]: Q-A, Q-B, Q-C, K per axis, w = c_k c_i c_j N_i N_j x
+        // prefactor, 1/(2q), 2q of the 1/r^2 terms (else 0), R^n_000
+        constexpr int GS = kMmdGroup;
+        double *sQA = ws, *sQB = sQA + 3 * GS, *sQC = sQB + 3 * GS, *sK = sQC + 3 * GS, *sW = sK + 3 * GS, *sI = sW + GS,
+               *sC = sI + GS, *sR = sC + GS, *E = sR + (S + 1) * GS;
+        for (int kind = 0; kind < 2; kind++) {
+            const int k0 = kind == 0 ? 0 : n2, ncand = (kind == 0 ? n2 : nterms - n2) * np2;
+            const int lg = cl.lgT[kind], T = 1 << lg, tr = tid & (T - 1), e0 = tid >> lg, est = NT >> lg;
+            const int nax = kind == 0 ? (la + 1) * (lb + 1) : mmd_e_axis(la, lb);
+            double *R0 = E + cl.nE * T, *X = R0 + cl.nR0 * T, *Rb = X;  // kind 1; X shares the R levels' space
+            int head = 0, tail = 0, base = 0;
+            for (;;) {
+                if (tail - head < GS && base < ncand) {
+                    // the next NT triples (term outer, primitive pair inner): keep the live ones, in order
+                    const int c = base + tid;
+                    bool live = false;
+                    if (c < ncand) {
+                        const int k = c / np2, r = c - k * np2, i = r / npB, j = r - i * npB;
+                        if (overlap || (!(fabs(cA[i]) < kZeroThresh) && !(fabs(cB[j]) < kZeroThresh))) {
+                            const double al = xA[i], be = xB[j];
+                            const double z = overlap ? 0.0 : a.pot_alpha[poff + a.pot_perm[poff + k0 + k]];
+                            double ab = 0.0, ac = 0.0, bc = 0.0;
 #pragma unroll
-            for (int qq = 0; qq < KPL; qq++) {
-                if (qq >= nslots) break;
-                const int pr = sch[qq * 32 + lane];
-                if (pr == kMmdNoPair) {
-                    pdesc[qq * 32 + lane] = make_int2(0, -1);  // empty slot
+                            for (int d = 0; d < 3; d++) {
+                                const double u = Ao[d] - Bo[d], v = Ao[d] - Co[d], w = Bo[d] - Co[d];
+                                ab += u * u;
+                                ac += v * v;
+                                bc += w * w;
+                            }
+                            live = !(al * be * ab + al * z * ac + be * z * bc > kMmdDropArg * (al + be + z));
+                        }
+                    }
+                    const unsigned m = __ballot_sync(0xffffffffu, live);
+                    if (lane == 0) s_cnt[warp] = __popc(m);
+                    __syncthreads();
+                    int pre = 0, tot = 0;
+#pragma unroll
+                    for (int w = 0; w < NW; w++) {
+                        const int v = s_cnt[w];
+                        pre += w < warp ? v : 0;
+                        tot += v;
+                    }
+                    if (live) ring[(tail + pre + __popc(m & ((1u << lane) - 1))) & (kMmdRing - 1)] = c;
+                    tail += tot;
+                    base += NT;
+                    __syncthreads();
                     continue;
                 }
-                const int m = pr / nB, n = pr % nB;
-                const int ax = ca[3 * m], ay = ca[3 * m + 1], az = ca[3 * m + 2];
-                const int bx = cb[3 * n], by = cb[3 * n + 1], bz = cb[3 * n + 2];
-                pdesc[qq * 32 + lane] =
-                    make_int2(eidx(lb1, S1, 0, ax, bx, 0, la1) | (eidx(lb1, S1, 1, ay, by, 0, la1) << 16),
-                              eidx(lb1, S1, 2, az, bz, 0, la1) | ((ax + bx) << 16) | ((ay + by) << 21) | ((az + bz) << 26));
-            }
-            double res[KPL];
-#pragma unroll
-            for (int q = 0; q < KPL; q++) res[q] = 0.0;
-
-            for (int k = 0; k < nterms; k++) {
-                const double zeta = overlap ? 0.0 : a.pot_alpha[a.pot_prim_off[item.pot] + k];
-                const int npow = overlap ? 3 : a.pot_powers[a.pot_prim_off[item.pot] + k];
-                double accp[KPL];
-#pragma unroll
-                for (int q = 0; q < KPL; q++) accp[q] = 0.0;
-
-                // primitive pairs (i, j) in the reference's order, 32 at a time: first each lane
-                // evaluates the scalars of one pair (q, Q, the Gaussian factors K per axis,
-                // K[d] = e(d,ab) e(d,ac) e(d,bc)); pairs with a zero coefficient (|c| < 1e-14)
-                // or a K[d] that underflowed to exactly 0 add exact zeros and are dropped
-                const int np2 = npA * npB;
-                for (int base = 0; base < np2; base += 32) {
-                    const int rr = base + lane;
-                    bool live = false;
-                    __syncwarp();  // the previous chunk's readers of spre are done
-                    if (rr < np2) {
-                        const int i = rr / npB, j = rr - i * npB;
-                        if (overlap) {
-                            live = true;
-                        } else if (!(fabs(cA[i]) < kZeroThresh) && !(fabs(cB[j]) < kZeroThresh)) {
-                            const double al = xA[i], be = xB[j];
-                            const double q = al + be + zeta;
-                            const double muab = (al * be) / q, muac = (al * zeta) / q, mubc = (be * zeta) / q;
-                            spre[lane] = q;
-#pragma unroll
-                            for (int d = 0; d < 3; d++) {
-                                // each product rounded, as the reference's (a A + b B + c C) / q
-                                // (type1_mcmurchie_davidson.c:198); no contraction into an FMA
-                                spre[(1 + d) * 32 + lane] =
-                                    __dadd_rn(__dadd_rn(__dmul_rn(al, A[d]), __dmul_rn(be, B[d])), __dmul_rn(zeta, C[d])) / q;
-                                const double dab = A[d] - B[d], dac = A[d] - C[d], dbc = B[d] - C[d];
-                                const double Kd = exp(-muab * dab * dab) * exp(-muac * dac * dac) * exp(-mubc * dbc * dbc);
-                                spre[(4 + d) * 32 + lane] = Kd;
-                                live = d == 0 ? Kd != 0.0 : (live && Kd != 0.0);
-                            }
-                        }
-                    }
-                    unsigned live_mask = __ballot_sync(0xffffffffu, live);
-                    __syncwarp();
-                    while (live_mask) {
-                        const int bl = __ffs(live_mask) - 1;
-                        live_mask &= live_mask - 1;
-                        const int i = (base + bl) / npB, j = (base + bl) - i * npB;
-                        const double ci = cA[i], cj = cB[j];
-                        const double al = xA[i], be = xB[j];
-                        const double NA = normA[i], NB = normB[j];
-                        double pref;
-                        if (!overlap) {
-                            // ---- Hermite E by wavefronts (type1_mcmurchie_davidson.c:569-622)
-                            const double q = spre[bl];
-                            double Q[3], K[3];
-#pragma unroll
-                            for (int d = 0; d < 3; d++) {
-                                Q[d] = spre[(1 + d) * 32 + bl];
-                                K[d] = spre[(4 + d) * 32 + bl];
-                            }
-                            if (COUNT && lane == 0) {
-                                c_trip++;
-                                c_fl += 40 + 5 * mmd_e_count(la, lb);
-                                if (npow != 2)
-                                    c_fl += (npow == 1 ? 16ull * (S + 1) : 100ull) + 2ull * (S + 1) +
-                                            5ull * (mmd_r_size(S) - (S + 1)) + contract_fl;
-                                else
-                                    c_fl += 4ull * (pend - pass);
-                            }
-                            // per-triple scalars shared by the coefficient updates (the same
-                            // expressions the updates would evaluate)
-                            if (lane < 3) {
-                                const double Qd = lane == 0 ? Q[0] : (lane == 1 ? Q[1] : Q[2]);
-                                const double Ad = lane == 0 ? A[0] : (lane == 1 ? A[1] : A[2]);
-                                const double Bd = lane == 0 ? B[0] : (lane == 1 ? B[1] : B[2]);
-                                const double Cd = lane == 0 ? C[0] : (lane == 1 ? C[1] : C[2]);
-                                sQA[lane] = Qd - Ad;
-                                sQB[lane] = Qd - Bd;
-                                sQC[lane] = Qd - Cd;
-                                sK[lane] = lane == 0 ? K[0] : (lane == 1 ? K[1] : K[2]);
-                            }
-                            if (lane >= 1 && lane <= S) finv[lane] = 1.0 / (2.0 * q * lane);
-                            __syncwarp();
-                            const int *ecode = a.etab + __ldg(a.etab_off + la * (kMaxL + 1) + lb);
-                            const int sj = S1, si = lb1 * S1;  // index steps of j and i
-                            for (int w = 0, wo = 0; w <= S; w++) {
-                                // entries (axis, i, j=w-i, t<=w)
-                                const int ilo = max(0, w - lb), ihi = min(la, w);
-                                const int tot = 3 * (ihi - ilo + 1) * (w + 1);
-                                for (int e = lane; e < tot; e += 32) {
-                                    const int c = __ldg(ecode + wo + e);
-                                    const int dst = c & 8191, ax = (c >> 13) & 3, ty = c >> 28;
-                                    const int e000 = ax * la1 * lb1 * S1;
-                                    double v;
-                                    if (ty == 0) v = sK[ax];
-                                    else if (ty == 1) v = sQA[ax] * E[e000];
-                                    else if (ty == 2) v = sQB[ax] * E[e000];
-                                    else if (ty == 3) v = sQB[ax] * E[dst - sj] + E[dst - sj + 1];
-                                    else if (ty == 4) v = sQA[ax] * E[dst - si] + E[dst - si + 1];
-                                    else {
-                                        const int ii = (c >> 15) & 15, jj = (c >> 19) & 15, t = (c >> 23) & 31;
-                                        const double f = finv[t];
-                                        v = 0.0;
-                                        if (ii > 0) v += f * ii * E[dst - si - 1];
-                                        if (jj > 0) v += f * jj * E[dst - sj - 1];
-                                    }
-                                    E[dst] = v;
-                                }
-                                wo += tot;
-                                __syncwarp();
-                            }
-                            const double p15 = npow == 2 ? pow(kPi / q, 1.5) : 0.0;  // once per primitive triple
-                            if (npow == 2) {
-                                pref = 0.0;
-                            } else {
-                                // ---- auxiliary functions and R by levels (type1_mcmurchie_davidson.c:457-564)
-                                const double dx = Q[0] - C[0], dy = Q[1] - C[1], dz = Q[2] - C[2];
-                                const double x = q * (dx * dx + dy * dy + dz * dz);
-                                if (npow == 1) {
-                                    if (lane <= S) aux[lane] = boys(lane, x);
-                                } else {
-                                    gfun_values_warp(x, S, aux, lane);
-                                }
-                                __syncwarp();
-                                const bool isg = npow == 0;
-                                const double q2 = isg ? 2.0 * q : -2.0 * q;
-                                if (lane <= S) R[lane] = pow(q2, lane) * aux[lane];  // level 0: n = 0..S
-                                if (lane == 0) R0[0] = R[0];
-                                __syncwarp();
-                                const int2 *rcode = a.rtab + __ldg(a.rtab_off + S);
-                                for (int s = 1; s <= S; s++) {
-                                    const int ne = (s + 1) * (s + 2) / 2, nn = S - s + 1, tot = ne * nn;
-                                    const int o = lvl[s], ne1 = s * (s + 1) / 2, ne2 = (s - 1) * s / 2;
-                                    for (int e = lane; e < tot; e += 32) {
-                                        // entry (t, u, v) of order n from its step down along one axis
-                                        // (the first of z, y, x with t+u, t, ... as in the reference)
-                                        const int2 c = __ldg(rcode + o + e);
-                                        const int src1 = c.x & 0xffff, src2 = (int)((unsigned)c.x >> 16);
-                                        const int kq = c.y & 31, ax = (c.y >> 5) & 3, r0d = (c.y >> 7) & 4095;
-                                        const double X = sQC[ax];
-                                        const double r1n1 = R[src1 + ne1], r1n = R[src1];
-                                        double val = 0.0;
-                                        if (kq > 1) {
-                                            const double r2n1 = R[src2 + ne2], r2n = R[src2];
-                                            if (isg) val += (kq - 1) * (r2n1 - 2.0 * q * r2n);
-                                            else val += (kq - 1) * r2n1;
-                                        }
-                                        if (isg) val += X * (r1n1 - 2.0 * q * r1n);
-                                        else val += X * r1n1;
-                                        R[o + e] = val;
-                                        if (r0d != kMmdNoR0) R0[r0d] = val;
-                                    }
-                                    __syncwarp();
-                                }
-                                pref = npow == 1 ? NA * NB * 2.0 * kPi / q : NA * NB * 2.0 * kPi15 / sqrt(q);
-                            }
-                            // ---- Cartesian pairs of this lane, by slot couples (2h, 2h+1) of equal
-                            // (tx, uy, vz); a lone pair runs with itself as partner, so every lane of a
-                            // row takes the same path
-#pragma unroll
-                            for (int h = 0; h < KPL; h += 2) {
-                                if (h >= nslots) break;
-                                const int2 d0 = pdesc[h * 32 + lane], d1 = pdesc[(h + 1) * 32 + lane];
-                                if (d0.y < 0) continue;
-                                if (npow == 2) {
-                                    accp[h] += (ci * cj) * (NA * NB * E[d0.x & 0xffff] * E[(int)((unsigned)d0.x >> 16)] *
-                                                            E[d0.y & 0xffff] * p15);
-                                    if (d1.y >= 0)
-                                        accp[h + 1] += (ci * cj) * (NA * NB * E[d1.x & 0xffff] *
-                                                                    E[(int)((unsigned)d1.x >> 16)] * E[d1.y & 0xffff] * p15);
-                                    continue;
-                                }
-                                const bool same = (d1.y >> 16) == (d0.y >> 16);  // false for an empty d1
-                                double s0, s1;
-                                mmd_contract2(E, R0, S, d0, same ? d1 : d0, s0, s1);
-                                accp[h] += (ci * cj) * (s0 * pref);
-                                if (same) accp[h + 1] += (ci * cj) * (s1 * pref);
-                                else if (d1.y >= 0) {  // unequal couple (not produced by the schedule builder)
-                                    mmd_contract2(E, R0, S, d1, d1, s0, s1);
-                                    accp[h + 1] += (ci * cj) * (s0 * pref);
-                                }
-                            }
-                        } else {
-                            // ---- overlap: 1D Obara-Saika tables per axis (overlap.c:92-120)
-                            const double p = al + be, mu = al * be / p, pf = 1.0 / (2.0 * p);
-                            if (lane < 3) {
-                                const int ax = lane;
-                                const double P = (al * A[ax] + be * B[ax]) / p, xab = A[ax] - B[ax];
-                                const double xpa = P - A[ax], xpb = P - B[ax];
-                                for (int ii = 0; ii <= la; ii++)
-                                    for (int jj = 0; jj <= lb; jj++) {
-                                        double s = 0.0;
-                                        if (ii + jj == 0) {
-                                            E[eidx(lb1, S1, ax, 0, 0, 0, la1)] = sqrt(kPi / p) * exp(-mu * xab * xab);
-                                            continue;
-                                        }
-                                        if (ii == 0) {
-                                            s += xpb * E[eidx(lb1, S1, ax, ii, jj - 1, 0, la1)];
-                                            if (jj - 1 > 0) s += (jj - 1) * pf * E[eidx(lb1, S1, ax, ii, jj - 2, 0, la1)];
-                                        } else {
-                                            s += xpa * E[eidx(lb1, S1, ax, ii - 1, jj, 0, la1)];
-                                            if (ii - 1 > 0) s += (ii - 1) * pf * E[eidx(lb1, S1, ax, ii - 2, jj, 0, la1)];
-                                            if (jj > 0) s += jj * pf * E[eidx(lb1, S1, ax, ii - 1, jj - 1, 0, la1)];
-                                        }
-                                        E[eidx(lb1, S1, ax, ii, jj, 0, la1)] = s;
-                                    }
-                            }
-                            __syncwarp();
-                            if (COUNT && lane == 0) {
-                                c_trip++;
-                                c_fl += 12ull * (la + 1) * (lb + 1) + 10 + 4ull * (pend - pass);  // Obara-Saika + pairs
-                            }
-#pragma unroll
-                            for (int qq = 0; qq < KPL; qq++) {
-                                if (qq >= nslots) break;
-                                const int2 dsc = pdesc[qq * 32 + lane];
-                                if (dsc.y < 0) continue;
-                                const double buf = NA * NB * E[dsc.x & 0xffff] * E[(int)((unsigned)dsc.x >> 16)] *
-                                                   E[dsc.y & 0xffff];
-                                accp[qq] += (ci * cj) * buf;
-                            }
-                        }
-                        __syncwarp();
+                if (tail == head) break;
+                const int ng = min(GS, tail - head);
+                {  // ---- scalars of the group: one thread per (triple, axis), a fourth one for the weight
+                    const int t = tid & (GS - 1), d = tid / GS;
+                    const bool have = t < ng;
+                    const int c = ring[(head + (have ? t : 0)) & (kMmdRing - 1)];
+                    const int k = c / np2, r = c - k * np2, i = r / npB, j = r - i * npB;
+                    const double al = xA[i], be = xB[j];
+                    const int ko = overlap ? 0 : poff + a.pot_perm[poff + k0 + k];
+                    const double z = overlap ? 0.0 : a.pot_alpha[ko], q = al + be + z;
+                    if (d < 3) {
+                        const double A = Ao[d], B = Bo[d], C = Co[d];
+                        // each product rounded, as the reference's (a A + b B + c C) / q
+                        // (type1_mcmurchie_davidson.c:198); no contraction into an FMA
+                        const double Q = __dadd_rn(__dadd_rn(__dmul_rn(al, A), __dmul_rn(be, B)), __dmul_rn(z, C)) / q;
+                        const double ab = A - B, ac = A - C, bc = B - C;
+                        const double K = exp(-((al * be) / q * ab * ab + (al * z) / q * ac * ac + (be * z) / q * bc * bc));
+                        sQA[d * GS + t] = Q - A;
+                        sQB[d * GS + t] = Q - B;
+                        sQC[d * GS + t] = Q - C;
+                        sK[d * GS + t] = K;
+                    } else {
+                        const double ck = overlap ? 1.0 : a.pot_coef[ko];
+                        const int n = overlap ? 2 : a.pot_powers[ko];
+                        const double pq = kPi / q;
+                        const double pref = n == 2 ? pq * sqrt(pq) : (n == 1 ? 2.0 * pq : 2.0 * kPi15 / sqrt(q));
+                        sW[t] = have ? ck * (cA[i] * cB[j]) * (normA[i] * normB[j] * pref) : 0.0;
+                        sI[t] = 1.0 / (2.0 * q);
+                        sC[t] = n == 0 ? 2.0 * q : 0.0;
+                        sR[t] = q;
                     }
                 }
-                const double ck = overlap ? 1.0 : a.pot_coef[a.pot_prim_off[item.pot] + k];
-#pragma unroll
-                for (int qq = 0; qq < KPL; qq++) res[qq] += ck * accp[qq];
-            }
-#pragma unroll
-            for (int qq = 0; qq < KPL; qq++) {
-                if (qq >= nslots) break;
-                const int pr = sch[qq * 32 + lane];
-                if (pr != kMmdNoPair) out[pr] = res[qq];
+                __syncthreads();
+                if (COUNT && tid < ng) {
+                    const int c = ring[(head + tid) & (kMmdRing - 1)], k = c / np2;
+                    if (sK[tid] != 0.0 && sK[GS + tid] != 0.0 && sK[2 * GS + tid] != 0.0) {
+                        const int n = overlap ? 2 : a.pot_powers[poff + a.pot_perm[poff + k0 + k]];
+                        c_trip++;
+                        if (overlap) c_fl += 12ull * (la + 1) * (lb + 1) + 10 + 4ull * npairs;
+                        else {
+                            c_fl += 40 + 5 * mmd_e_count(la, lb);
+                            if (n != 2)
+                                c_fl += (n == 1 ? 16ull * (S + 1) : 100ull) + 2ull * (S + 1) + 5ull * (mmd_r_size(S) - (S + 1)) + s_fl;
+                            else
+                                c_fl += 4ull * npairs;
+                        }
+                    }
+                }
+                if (kind == 1) {  // ---- R^n_000, n = 0..S: four threads per triple
+                    const int t = tid >> 2, sub = tid & 3;
+                    const double q = sR[t], dx = sQC[t], dy = sQC[GS + t], dz = sQC[2 * GS + t];
+                    const bool isg = sC[t] != 0.0;
+                    const double x = q * (dx * dx + dy * dy + dz * dz), q2 = isg ? 2.0 * q : -2.0 * q;
+                    __syncwarp();  // q is read before sR takes the values
+                    if (t < ng) {
+                        if (isg) gfun_values4(x, S, sR + t, GS, sub);
+                        __syncwarp(0xfu << (tid & 28));
+                        for (int n = sub; n <= S; n += 4) sR[n * GS + t] = pow(q2, n) * (isg ? sR[n * GS + t] : boys(n, x));
+                    }
+                    __syncthreads();
+                }
+                for (int b0 = 0; b0 < ng; b0 += T) {
+                    const int g = b0 + tr;  // this thread's triple in the group arrays
+                    const bool have = g < ng;
+                    for (int e = e0; e < 3; e += est) E[e * nax * T + tr] = have ? sK[e * GS + g] : 0.0;
+                    if (kind == 1)
+                        for (int n = e0; n <= S; n += est) {
+                            const double v = have ? sR[n * GS + g] : 0.0;
+                            Rb[n * T + tr] = v;
+                            if (n == 0) R0[tr] = v;
+                        }
+                    __syncthreads();
+                    const double f = sI[g];
+                    if (kind == 0) {
+                        const int *ol = lv + (S + 2);
+                        for (int s = 1; s <= S; s++) {
+                            const int n1 = ol[s + 1];
+                            for (int e = ol[s] + e0; e < n1; e += est) {
+                                const int2 c = __ldg(a.otab + cl.o_off + e);
+                                const int ax = (c.y >> 18) & 3;
+                                const double P = ((c.y >> 20) & 1 ? sQB : sQA)[ax * GS + g];
+                                const double n2f = (c.y >> 10) & 15, n3f = (c.y >> 14) & 15;
+                                double v = P * E[((c.x >> 10) & 1023) * T + tr];
+                                v += f * (n2f * E[((c.x >> 20) & 1023) * T + tr] + n3f * E[(c.y & 1023) * T + tr]);
+                                E[(c.x & 1023) * T + tr] = v;
+                            }
+                            __syncthreads();
+                        }
+                    } else {
+                        // ---- step s: E wavefront i + j = s and R level s
+                        const int *rl = lv + 2 * (S + 2);
+                        const double c2q = sC[g];
+                        const bool isg = c2q != 0.0;
+                        for (int s = 1; s <= S; s++) {
+                            const int n1 = lv[s + 1];
+                            for (int e = lv[s] + e0; e < n1; e += est) {
+                                const int2 c = __ldg(a.etab + cl.e_off + e);
+                                const int ax = (c.y >> 13) & 3, src = (c.x >> 13) & 8191;
+                                double v;
+                                if (c.x & (1 << 30)) {
+                                    v = ((c.y >> 20) & 1 ? sQB : sQA)[ax * GS + g] * E[src * T + tr];
+                                    if ((c.y >> 24) & 1) v += E[(src + 1) * T + tr];
+                                } else {
+                                    const double ii = (c.y >> 20) & 15, jj = (c.y >> 24) & 15;
+                                    v = f * rcp[(c.y >> 15) & 31] * (ii * E[src * T + tr] + jj * E[(c.y & 8191) * T + tr]);
+                                }
+                                E[(c.x & 8191) * T + tr] = v;
+                            }
+                            double *dst = Rb + (s % 3) * cl.maxlev * T;
+                            const double *p1 = Rb + ((s + 2) % 3) * cl.maxlev * T, *p2 = Rb + ((s + 1) % 3) * cl.maxlev * T;
+                            const int m0 = rl[s], m1 = rl[s + 1], ne1 = s * (s + 1) / 2, ne2 = (s - 1) * s / 2;
+                            for (int e = m0 + e0; e < m1; e += est) {
+                                const int2 c = __ldg(a.rtab + cl.r_off + e);
+                                const int k = (c.y >> 14) & 31, r0d = c.y & 8191, s1 = c.x & 0xffff, s2 = (int)((unsigned)c.x >> 16);
+                                double v = 0.0;
+                                if (k > 1) {
+                                    double d2 = p2[(s2 + ne2) * T + tr];
+                                    if (isg) d2 = __fma_rn(-c2q, p2[s2 * T + tr], d2);
+                                    v = (k - 1) * d2;
+                                }
+                                double d1 = p1[(s1 + ne1) * T + tr];
+                                if (isg) d1 = __fma_rn(-c2q, p1[s1 * T + tr], d1);
+                                v = __fma_rn(sQC[((c.y >> 19) & 3) * GS + g], d1, v);
+                                dst[(e - m0) * T + tr] = v;
+                                if (r0d != kMmdNoR0) R0[r0d * T + tr] = v;
+                            }
+                            __syncthreads();
+                        }
+                        // ---- X[(az, bz)][t][u] = sum_v E^z_v R^0_tuv (the R levels are consumed)
+                        for (int e = e0; e < cl.nX; e += est) {
+                            const int2 c = __ldg(a.ztab + cl.z_off + e);
+                            const double *r = R0 + (c.x & 0xffff) * T + tr, *z = E + ((unsigned)c.x >> 16) * T + tr;
+                            double v = z[0] * r[0];
+                            for (int u = 1; u <= c.y; u++) v += z[u * T] * r[u * T];
+                            X[e * T + tr] = v;
+                        }
+                        __syncthreads();
+                    }
+                    // ---- Cartesian pairs: one thread per (pair, triple); the batch's triples are added by a
+                    // shuffle tree, then to the pair's running sum
+                    const double w = sW[g];
+                    const int rounds = (npairs * T + NT - 1) / NT;
+                    for (int rd = 0, p = e0; rd < rounds; rd++, p += est) {
+                        double s = 0.0;
+                        if (p < npairs) {
+                            const int4 d = __ldg(pt + p);
+                            if (kind == 0) {
+                                s = E[(d.z & 1023) * T + tr] * E[((d.z >> 10) & 1023) * T + tr] * E[((d.z >> 20) & 1023) * T + tr];
+                            } else {
+                                const double *ex = E + (d.x & 0xffff) * T + tr, *ey = E + ((unsigned)d.x >> 16) * T + tr;
+                                const double *x = X + (d.y & 0xffff) * T + tr;
+                                const int W = (d.y >> 16) & 31, tx = (d.y >> 21) & 31, uy = (int)((unsigned)d.y >> 26);
+                                for (int t = 0; t <= tx; t++) {
+                                    double sy = ey[0] * x[0];
+                                    for (int u = 1; u <= uy; u++) sy += ey[u * T] * x[u * T];
+                                    s += ex[t * T] * sy;
+                                    x += (W + 1 - t) * T;
+                                }
+                            }
+                            s *= w;
+                        }
+                        for (int o = min(T, 32) >> 1; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+                        if (p < npairs && (tr & 31) == 0) acc[p * G + (tr >> 5)] += s;
+                    }
+                    __syncthreads();  // the batch's tables are consumed
+                }
+                head += ng;
             }
         }
-        __syncwarp();
+        __syncthreads();
+        double *out = a.out[item.out_kind] + item.out_off;
+        for (int p = tid; p < npairs; p += NT) {
+            double s = acc[p * G];
+            for (int g = 1; g < G; g++) s += acc[p * G + g];
+            out[__ldg(pt + p).w] = s;
+        }
+        __syncthreads();  // acc and s_item are consumed
     }
     if (COUNT && a.counters) {
         for (int o = 16; o > 0; o >>= 1) {

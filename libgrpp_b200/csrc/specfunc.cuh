@@ -6,7 +6,7 @@
 //   bessel_scaled_row  the same for all orders 0..lmax at one x (one table row)
 //   boys               F_n(x), 6th-order Taylor on a 0.1 grid below 30, asymptotic above
 //                      (libgrpp/specfunc_boys.c:21-47)
-//   gfun_values        G_n(x) = int_0^1 t^(2n) exp(-x(1-t^2)) dt: series + downward
+//   gfun_values4       G_n(x) = int_0^1 t^(2n) exp(-x(1-t^2)) dt: series + downward
 //                      recursion for x <= 12, Dawson + upward recursion above
 //                      (libgrpp/specfunc_gfun.c:40-93)
 //   dawson             Daw(y) for y >= 3: Taylor about a 1/32 grid with derivatives from
@@ -145,60 +145,47 @@ __device__ inline double dawson(double y)
     return s / (2.0 * y);
 }
 
-// g[0..nmax]
-__device__ inline void gfun_values(double x, int nmax, double *g)
+// G_n(x), n = 0..nmax, into g[n * stride], by four consecutive lanes of a warp (sub = 0..3; all
+// four call it with the same arguments and converge after it). For x <= 12 the series of the top
+// order: lane sub forms the terms k = sub, sub + 4, .. with the product chains of the serial loop
+// (x^k and k! by repeated multiplication from 1), and the terms are added in order up to the
+// first one below 1e-15, as the serial loop does; the recursions are lane 0's.
+__device__ inline void gfun_values4(double x, int nmax, double *g, int stride, int sub)
 {
-    if (x <= 12.0) {
-        double ex = exp(-x), sum = 0.0, xk = 1.0, fk = 1.0;
-        for (int k = 0; k < 100; k++) {
-            if (k > 0) {
-                xk *= x;
-                fk *= k;
-            }
-            double c = ex * xk / fk / (2.0 * nmax + 2.0 * k + 1.0);
-            sum += c;
-            if (fabs(c) < 1e-15) break;
-        }
-        g[nmax] = sum;
-        for (int n = nmax; n > 0; n--) g[n - 1] = (1.0 - 2.0 * x * g[n]) / (2.0 * n - 1.0);
-    } else {
-        double sx = sqrt(x);
-        g[0] = dawson(sx) / sx;
-        for (int n = 0; n < nmax; n++) g[n + 1] = (1.0 - (2 * n + 1) * g[n]) / (2.0 * x);
-    }
-}
-
-// gfun_values by one warp (all 32 lanes call it; g[] is written by lane 0). For x <= 12
-// lane k forms the series term k with the same product chains as the serial loop
-// (x^k and k! by repeated multiplication from 1), and lane 0 adds the terms in order up
-// to the first one below 1e-15, as the serial loop does; the recursions stay on lane 0.
-__device__ inline void gfun_values_warp(double x, int nmax, double *g, int lane)
-{
+    const unsigned quad = 0xfu << (threadIdx.x & 28);
     if (x <= 12.0) {
         const double ex = exp(-x);
-        double sum = 0.0;
-        for (int k0 = 0; k0 < 100; k0 += 32) {
-            const int k = k0 + lane;
-            double xk = 1.0, fk = 1.0;
-            for (int i = 1; i <= k; i++) {
-                xk *= x;
-                fk *= i;
-            }
+        double sum = 0.0, xk = 1.0, fk = 1.0;
+        for (int i = 1; i <= sub; i++) {
+            xk *= x;
+            fk *= i;
+        }
+        for (int k0 = 0; k0 < 100; k0 += 4) {
+            const int k = k0 + sub;
             const double c = ex * xk / fk / (2.0 * nmax + 2.0 * k + 1.0);
-            const unsigned stop = __ballot_sync(0xffffffffu, k >= 99 || fabs(c) < 1e-15);
-            const int last = stop ? __ffs(stop) - 1 : 31;  // last term added in this block
-            for (int j = 0; j <= last; j++) {
-                const double cj = __shfl_sync(0xffffffffu, c, j);
-                if (lane == 0) sum += cj;
+            bool stop = false;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const double cj = __shfl_sync(quad, c, j, 4);
+                if (!stop) sum += cj;
+                stop = stop || fabs(cj) < 1e-15;
             }
             if (stop) break;
+#pragma unroll
+            for (int i = 1; i <= 4; i++) {
+                xk *= x;
+                fk *= k + i;
+            }
         }
-        if (lane == 0) {
-            g[nmax] = sum;
-            for (int n = nmax; n > 0; n--) g[n - 1] = (1.0 - 2.0 * x * g[n]) / (2.0 * n - 1.0);
+        if (sub == 0) {
+            g[nmax * stride] = sum;
+            for (int n = nmax; n > 0; n--) g[(n - 1) * stride] = sum = (1.0 - 2.0 * x * sum) / (2.0 * n - 1.0);
         }
-    } else if (lane == 0) {
-        gfun_values(x, nmax, g);
+    } else if (sub == 0) {
+        const double sx = sqrt(x);
+        double v = dawson(sx) / sx;
+        g[0] = v;
+        for (int n = 0; n < nmax; n++) g[(n + 1) * stride] = v = (1.0 - (2 * n + 1) * v) / (2.0 * x);
     }
 }
 
