@@ -166,6 +166,10 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(upload_vec(st, h.bessel, &d.bessel));
     GRPP_CUDA(upload_vec(st, h.bessel_p, &d.bessel_p));
     GRPP_CUDA(upload_vec(st, h.rfun, &d.rfun));
+    GRPP_CUDA(upload_vec(st, h.ratio, &d.ratio));
+    GRPP_CUDA(upload_vec(st, h.ratio_y, &d.ratio_y));
+    GRPP_CUDA(upload_vec(st, h.bes_t, &d.bes_t));
+    GRPP_CUDA(upload_vec(st, h.bes_y, &d.bes_y));
     GRPP_CUDA(upload_vec(st, h.boys, &d.boys));
     GRPP_CUDA(upload_vec(st, h.dawson, &d.dawson));
     GRPP_CUDA(upload_vec(st, h.rsh_coef, &d.rsh_coef));
@@ -201,6 +205,8 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(upload_vec(st, mt.otab, &st.mmd.otab));
     GRPP_CUDA(upload_vec(st, mt.rtab, &st.mmd.rtab));
     GRPP_CUDA(upload_vec(st, mt.ztab, &st.mmd.ztab));
+    GRPP_CUDA(cudaFuncSetAttribute(radial_screen_unit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(kScrWarps * scr_warp_doubles(kRadMaxLam + 1) * sizeof(double))));
     GRPP_CUDA(cudaFuncSetAttribute(radial_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GRPP_CUDA(ang_set_final_max_smem((int)kFinSmemMax));
     GRPP_CUDA(cudaFuncSetAttribute(type1_num_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -652,7 +658,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     std::vector<int> proj_a(nt, -1), proj_b(nt, -1);
     std::vector<MmdItem> items;
     std::vector<int> rad_task;
-    std::vector<int64_t> rad_qoff, rad_uoff;
+    std::vector<int64_t> rad_qoff;
     // (shell, centre) pairs of the radial items, for the F_l(r) tables (ftab_kernel)
     // pair index per (shell, centre): a flat array when it is small next to the chunk (filling
     // it costs n_shells x n_centres per chunk), else a hash map
@@ -682,12 +688,12 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         }
         return idx;
     };
-    int64_t qtot = 0, utot = 0, rad_list_max = 0;
-    // screening runs: long runs of one (task, potential) to the unit kernel, short ones (and
-    // one-centre tasks) to the flat kernel
+    int64_t qtot = 0, rad_list_max = 0;
+    // screening runs of one (task, potential): one-centre tasks apart
     std::vector<ScrUnit> scr_big, scr_small;
     std::vector<int64_t> su_off(1, 0);
     int scr_lw = 2;
+    int64_t scr_entries = 0;
     std::vector<int2> ucls((kMaxL + 1) * (kMaxL + 1) * (kMaxL + 1), int2{0, 0});
     std::vector<uint8_t> ucls_set(ucls.size(), 0);
     std::vector<uint16_t> ulist;
@@ -716,7 +722,6 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             q_off[t] = qtot;
             rad_task.push_back((int)t);
             rad_qoff.push_back(qtot);
-            rad_uoff.push_back(utot);
             int e = 0, Lmx = 0;
             int64_t item_used = 0;
             double CA2 = 0.0, CB2 = 0.0;
@@ -742,17 +747,16 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                     ucls_set[key] = 1;
                 }
                 const int ne = ucls[key].y;
-                if (one_centre || ne < kScrUnitMin) {
+                if (one_centre) {
                     if (ne > 0) {
                         scr_small.push_back(ScrUnit{item, pot, pe, ucls[key].x, ne});
                         su_off.push_back(su_off.back() + ne);
                     }
-                } else {
-                    for (int o = 0; o < ne; o += kScrUnitThreads)
-                        scr_big.push_back(ScrUnit{item, pot, pe, ucls[key].x + o, std::min(kScrUnitThreads, ne - o)});
+                } else if (ne > 0) {
+                    scr_big.push_back(ScrUnit{item, pot, pe, ucls[key].x, ne});
+                    scr_entries += ne;
                     scr_lw = std::max(scr_lw, L + std::max(la, lb) + 1);
                 }
-                utot += ucls[key].y;
                 item_used += ucls[key].y;
                 rad_l1 = std::max(rad_l1, L + la);
                 rad_l2 = std::max(rad_l2, L + lb);
@@ -789,14 +793,27 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             }
         }
     }
-    // long screening runs, costliest first (entries x primitive triples), so the static
-    // round-robin over blocks ends evenly
+    // Screening runs: whole (task, potential) lists up to kScrRunMax entries share their staged
+    // triples; a batch with too few entries to give every warp of the chip (about 16 per
+    // SM) four runs is cut finer, down to 4 entries. Costliest first (entries x primitive triples).
     {
-        auto cost = [&](const ScrUnit &u) {
+        int run = kScrRunMax;
+        while (run > 4 && scr_entries < (int64_t)run * st.nsm * 64) run /= 2;
+        std::vector<ScrUnit> cut;
+        for (const ScrUnit &u : scr_big)
+            for (int o = 0; o < u.ne; o += run)
+                cut.push_back(ScrUnit{u.item, u.pot, u.pe, u.uo + o, std::min(run, u.ne - o)});
+        scr_big.swap(cut);
+        std::vector<double> cost(scr_big.size());
+        for (size_t i = 0; i < scr_big.size(); i++) {
+            const ScrUnit &u = scr_big[i];
             const int t = rad_task[u.item];
-            return (int64_t)u.ne * rp_n[ta[t]] * rp_n[tb[t]] * p_n[u.pot];
-        };
-        std::stable_sort(scr_big.begin(), scr_big.end(), [&](const ScrUnit &x, const ScrUnit &y) { return cost(x) > cost(y); });
+            cost[i] = (u.ne + 2.0) * rp_n[ta[t]] * rp_n[tb[t]] * p_n[u.pot];
+        }
+        cut.resize(scr_big.size());
+        const std::vector<int> ord = order_by_cost(cost);
+        for (size_t i = 0; i < ord.size(); i++) cut[i] = scr_big[ord[i]];
+        scr_big.swap(cut);
     }
     // outercore projection blocks
     std::vector<int> blk_shell, blk_oc;
@@ -1005,8 +1022,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     const size_t o_cor = pk.add(c_or), o_cg = pk.add(c_g);
     const size_t o_ta = pk.add(ta), o_tb = pk.add(tb), o_tc = pk.add(tc), o_too = pk.add(out_off), o_thul = pk.add(has_ul),
                  o_tqo = pk.add(q_off), o_tpa = pk.add(proj_a), o_tpb = pk.add(proj_b);
-    const size_t o_items = pk.add(items), o_rt = pk.add(rad_task), o_rq = pk.add(rad_qoff), o_ru = pk.add(rad_uoff),
-                 o_ucls = pk.add(ucls), o_ulist = pk.add(ulist), o_sbig = pk.add(scr_big), o_ssmall = pk.add(scr_small),
+    const size_t o_items = pk.add(items), o_rt = pk.add(rad_task), o_rq = pk.add(rad_qoff),
+                 o_ulist = pk.add(ulist), o_sbig = pk.add(scr_big), o_ssmall = pk.add(scr_small),
                  o_suo = pk.add(su_off);
     const size_t o_bs = pk.add(blk_shell), o_bo = pk.add(blk_oc), o_bco = pk.add(blk_cart_off), o_bso = pk.add(blk_sph_off),
                  o_poffp = pk.add(proj_off), o_mpair = pk.add(mmd_pairs), o_pperm = pk.add(p_perm), o_pn2 = pk.add(p_n2);
@@ -1162,13 +1179,11 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         r.pot_alpha = at<double>(ib, o_palpha);
         r.q_off = at<int64_t>(ib, o_rq);
         r.n_entries = qtot;
-        r.u_off = at<int64_t>(ib, o_ru);
-        r.n_used = utot;
-        r.ucls = at<int2>(ib, o_ucls);
         r.ulist = at<uint16_t>(ib, o_ulist);
         r.scr_units = at<ScrUnit>(ib, o_sbig);
         r.n_scr_units = (int)scr_big.size();
         r.scr_lw = scr_lw;
+        r.scr_queue = statusd + 10;
         r.su = at<ScrUnit>(ib, o_ssmall);
         r.su_off = at<int64_t>(ib, o_suo);
         r.n_su = (int)scr_small.size();
@@ -1215,13 +1230,11 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         P.wu_blocks = (int)std::min<int64_t>((wu_words + 255) / 256, (int64_t)nsm * 16);
         P.rad = r;
         P.rad_blocks = (int)std::min<int64_t>((int64_t)rad_task.size(), (int64_t)nsm * 16);
-        int scr_occ = 0;
-        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scr_occ, radial_screen_flat_kernel, kRadThreads, 0));
-        P.scr_blocks = (int)std::min<int64_t>((su_off.back() + kRadThreads - 1) / kRadThreads, (int64_t)nsm * std::max(scr_occ, 1));
-        P.scru_smem = (size_t)2 * kScrChunk * scr_lw * sizeof(double);
+        P.scr_blocks = (int)std::min<int64_t>((su_off.back() + kRadThreads - 1) / kRadThreads, (int64_t)nsm * 16);
+        P.scru_smem = (size_t)kScrWarps * scr_warp_doubles(scr_lw) * sizeof(double);
         int scru_occ = 0;
-        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scru_occ, radial_screen_unit_kernel, kScrUnitThreads, P.scru_smem));
-        P.scru_blocks = (int)std::min<int64_t>((int64_t)scr_big.size(), (int64_t)nsm * std::max(scru_occ, 1));
+        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scru_occ, radial_screen_unit_kernel, 32 * kScrWarps, P.scru_smem));
+        P.scru_blocks = (int)std::min<int64_t>(((int64_t)scr_big.size() + kScrWarps - 1) / kScrWarps, (int64_t)nsm * std::max(scru_occ, 1));
         P.rad_smem = smem;
     }
 
@@ -1331,11 +1344,11 @@ int plan_launch(Plan &P)
         GRPP_CUDA(cudaMemsetAsync(P.rad.walk, 0, (size_t)P.n_radial, s));
         GRPP_CUDA(cudaMemsetAsync(P.rad.eflag, 0, (size_t)P.n_entries, s));  // unread entries stay inactive
         if (P.scru_blocks > 0) {
-            radial_screen_unit_kernel<<<P.scru_blocks, kScrUnitThreads, P.scru_smem, s>>>(P.rad);
+            radial_screen_unit_kernel<<<P.scru_blocks, 32 * kScrWarps, P.scru_smem, s>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
         }
         if (P.scr_blocks > 0) {
-            radial_screen_flat_kernel<<<P.scr_blocks, kRadThreads, 0, s>>>(P.rad);
+            radial_one_centre_kernel<<<P.scr_blocks, kRadThreads, 0, s>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
         }
         GRPP_CUDA(cudaEventRecord(ev[4], s));

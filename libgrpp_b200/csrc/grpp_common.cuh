@@ -15,6 +15,12 @@ constexpr int kMaxL = 10;          // basis and projector angular momentum (libg
 constexpr int kBesL = 40;          // Bessel table orders 0..kBesL-1 (even: the pair layout)
 constexpr int kBesNX = 1601;       // x = 0.00 .. 16.00 step 0.01 (specfunc_bessel_table.c:14-17)
 constexpr int kRfunL = 40;         // asymptotic R_l coefficients (specfunc_scaled_mod_sph_bessel.c:163-190)
+constexpr int kRatL = 26;          // screening ratio tables: orders 0..kRatL-1
+constexpr int kRatYN = 66;         // y = 1/x = 0 .. 65/1024 (x > 16)
+constexpr double kRatYInv = 1024.0;
+constexpr int kBesYN = 258;         // y = 0 .. 257/4096
+constexpr double kBesYInv = 4096.0;
+constexpr double kRatXmin = 1.25;  // the tables are read from here on
 constexpr int kBoysNX = 301;       // x = 0.0 .. 30.0 step 0.1 (specfunc_boys.c:24)
 constexpr int kBoysNN = 40;
 constexpr int kRshL = 32;          // real spherical harmonic tables l = 0..kRshL
@@ -40,6 +46,10 @@ struct DeviceTables {
     const double *bessel;     // [kBesNX][kBesL][5]: value + 4 derivatives
     const double *bessel_p;   // the same values as [kBesNX][kBesL/2][5][2]: orders 2p, 2p+1 side by side
     const double *rfun;       // [kRfunL][kRfunL]
+    const double *ratio;      // [kBesNX][kRatL][5]: Taylor coefficients of T_l(x) about x = 0.01 i
+    const double *ratio_y;    // [kRatYN][kRatL][5]: of T_l(1/y) - 1/y about y = i / 1024
+    const double *bes_t;      // [kBesNX][kRatL][5]: Taylor coefficients of M_l(x) about x = 0.01 i
+    const double *bes_y;      // [kBesYN][kRatL][5]: of 2x M_l(x) in y = 1/x about y = i / 4096
     const double *boys;       // [kBoysNX][kBoysNN]
     const double *dawson;     // [kDawNY]
     const double *rsh_coef;   // concatenated per l: [(2l+1)][ncomb(l)]

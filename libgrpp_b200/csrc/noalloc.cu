@@ -131,6 +131,7 @@ int setup(int dev)
     if ((rc = copy_table(g_bessel, h.bessel, kNaBessel, &d.bessel))) return rc;
     if ((rc = copy_table(g_bessel_p, h.bessel_p, kNaBessel, &d.bessel_p))) return rc;
     if ((rc = copy_table(g_rfun, h.rfun, (size_t)kRfunL * kRfunL, &d.rfun))) return rc;
+    d.ratio = d.ratio_y = d.bes_t = d.bes_y = nullptr;  // not read by this path's screening kernel
     if ((rc = copy_table(g_boys, h.boys, (size_t)kBoysNX * kBoysNN, &d.boys))) return rc;
     if ((rc = copy_table(g_dawson, h.dawson, (size_t)kDawNY, &d.dawson))) return rc;
     if ((rc = copy_table(g_rsh_coef, h.rsh_coef, kNaRsh, &d.rsh_coef))) return rc;

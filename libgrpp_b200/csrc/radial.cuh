@@ -13,12 +13,9 @@
 //     |S_L - S_{L-1}| <= 1e-16 unless |S|/|estimate| < 1e-3, capped at 8191 points.
 //
 // GPU mapping, two kernels:
-//  * radial_screen_flat_kernel: one thread per (task, entry) over the entries of the
-//    whole batch. A thread walks the primitive triples (i, j, k) of its entry in
-//    libgrpp's order and stops at the first failing one, exactly as libgrpp does,
-//    so the estimate and the gate decision are those of the reference, and no
-//    work is spent on triples libgrpp never evaluates. One-centre tasks get their
-//    analytic table here and need no grid walk.
+//  * radial_screen_unit_kernel: one warp per run of entries of one (task, potential), lanes over
+//    primitive triples, triples that cannot matter dropped first; the gate decisions are
+//    libgrpp's. One-centre tasks get their analytic table (radial_one_centre_kernel).
 //  * radial_walk_kernel: one CTA per task that has entries left. The grid is
 //    walked level by level in chunks of one point per thread; a point's
 //    integrand values
@@ -35,9 +32,6 @@
 namespace grpp {
 
 constexpr int kRadThreads = 128;
-#ifndef GRPP_SCR_MINB
-#define GRPP_SCR_MINB 5  // resident 128-thread blocks per SM asked of the flat screening kernel
-#endif
 constexpr int kRadMaxPrims = 64;     // primitives per shell on the radial path
 constexpr int kRadMaxPots = 24;      // semilocal potentials per centre
 constexpr int kRadMaxTerms = 256;    // potential terms per centre (all semilocal potentials)
@@ -49,9 +43,9 @@ constexpr int kRadMaxEntries = 16384;
 // entry flag bits
 constexpr uint8_t kEntActive = 1, kEntScrOk = 2;
 
-// A run of used entries of one semilocal potential of one task, screened by one block of
-// radial_screen_unit_kernel (or, for short runs, by the flat kernel): item, potential index,
-// offset of the potential's (l1, l2, N) box within the item's table, offset of the run in ulist,
+// A run of used entries of one semilocal potential of one task, screened by one warp of
+// radial_screen_unit_kernel (or, for a one-centre task, evaluated by radial_one_centre_kernel):
+// item, potential index, offset of the potential's (l1, l2, N) box within the item's table, offset of the run in ulist,
 // number of entries.
 struct ScrUnit {
     int item, pot, pe, uo, ne;
@@ -92,18 +86,15 @@ struct RadialArgs {
     const int64_t *fp_off;
     const int *fp_shell, *fp_centre, *fp_lmax, *item_fa, *item_fb;
     int n_fpairs;
-    // entries the angular sums read, per item: u_off[item] = first used index; per class
-    // (L, la, lb) ucls = {offset into ulist, count}; ulist = entry offsets within a potential's block
-    const int64_t *u_off;
-    int64_t n_used;
-    const int2 *ucls;
+    // entries the angular sums read: offsets within a potential's (l1, l2, N) block, per class
+    // (L, la, lb) one list
     const uint16_t *ulist;
-    // screening split: runs of at least kScrUnitMin entries go to radial_screen_unit_kernel
-    // (scr_units), the others to the flat kernel through su, with prefix entry offsets su_off
-    // (su_off null: the flat kernel covers every used entry of every item through u_off);
-    // scr_lw: orders 0..scr_lw-1 of the unit kernel's Bessel tables
+    // screening: runs of entries of one (task, potential) for radial_screen_unit_kernel, popped
+    // from *scr_queue (zeroed before the launch); scr_lw: orders 0..scr_lw-1 of its Bessel tables
     const ScrUnit *scr_units;
     int n_scr_units, scr_lw;
+    int *scr_queue;
+    // runs of one-centre tasks, with prefix entry offsets su_off (radial_one_centre_kernel)
     const ScrUnit *su;
     const int64_t *su_off;
     int n_su;
@@ -268,20 +259,6 @@ __device__ __forceinline__ void scr_ratio_parts(int l, double x, double &num, do
     }
 }
 
-// M_l(x) with one reciprocal of x in the asymptotic range (bessel_scaled divides twice there)
-__device__ __forceinline__ double bessel_scaled_1r(int n, double x)
-{
-    if (x <= 16.0) return bessel_scaled(n, x);
-    const double inv = 1.0 / x, ninv = -inv;
-    const double *c = c_tab.rfun + n * kRfunL;
-    double pw = 1.0, sum = 0.0;
-    for (int k = 0; k <= n; k++) {
-        sum += __ldg(c + k) * pw;
-        pw *= ninv;
-    }
-    return sum * (0.5 * inv);
-}
-
 // Gaussian integral int_0^inf r^n exp(-p r^2) dr (screening.c:255-265): the
 // screening estimate of two s functions on the centre and the one-centre analytic table
 __device__ __forceinline__ double scr_gaussian_integral(int n, double p)
@@ -296,79 +273,60 @@ __device__ __forceinline__ double scr_gaussian_integral(int n, double p)
     return f / (2.0 * pow(p, k + 1));
 }
 
+// T_l(x) = x M_(l-1)(x) / M_l(x), T_0(x) = x M_1(x) / M_0(x): what the fixed-point step of
+// screening.c:329-362 takes of each side. Tabulated (tables.cpp) as Taylor coefficients in x up to
+// x = 16 and of T_l - x in y = 1/x above, so a step costs one short polynomial per side and no
+// division (two Taylor sums or asymptotic series per side and a division before); relative error
+// below 3e-12 at every order. Below x = 1.25 libgrpp's own 4th-order
+// Taylor sums of M_l lose digits (down to 0/0 for high l near 0, an undefined estimate): there
+// its quotient is formed as libgrpp does. inv_x: 1/x, read for x > 16 only.
+__device__ __forceinline__ double scr_poly(const double *c, double h)
+{
+    return __ldg(c) + h * (__ldg(c + 1) + h * (__ldg(c + 2) + h * (__ldg(c + 3) + h * __ldg(c + 4))));
+}
+__device__ __forceinline__ double scr_t(int l, double x, double inv_x)
+{
+    if (x < kRatXmin) {
+        double num, den;
+        scr_ratio_parts(l, x, num, den);
+        return num * x / den;
+    }
+    // one polynomial for both ranges, so that lanes on either side of 16 stay together
+    const bool lo = x <= 16.0;
+    const int i = lo ? (int)(x * 100.0 + 0.5) : (int)(inv_x * kRatYInv + 0.5);
+    const double h = lo ? x - i * 0.01 : inv_x - i * (1.0 / kRatYInv);
+    return (lo ? 0.0 : x) + scr_poly((lo ? c_tab.ratio : c_tab.ratio_y) + (i * kRatL + l) * 5, h);
+}
+// M_l(x) of the envelope: Taylor in x up to 16, above of 2x M_l (a polynomial of degree l in 1/x) in y = 1/x
+__device__ __forceinline__ double scr_m(int l, double x, double inv_x)
+{
+    const bool lo = x <= 16.0;
+    const int i = lo ? (int)(x * 100.0 + 0.5) : (int)(inv_x * kBesYInv + 0.5);
+    const double h = lo ? x - i * 0.01 : inv_x - i * (1.0 / kBesYInv);
+    return scr_poly((lo ? c_tab.bes_t : c_tab.bes_y) + (i * kRatL + l) * 5, h) * (lo ? 1.0 : 0.5 * inv_x);
+}
+
 // The envelope of screening.c:308-318 at the fixed point r0, with sqpi = sqrt(pi / p) and
 // sqp = sqrt(p). Every factor is finite and non-negative: a Gaussian factor that underflowed to
 // exactly 0 makes the product exactly 0, so the other factors are not needed; and 1 + erf(z) is
-// exactly 2 once erfc(z) < 2^-54 (z > 5.9), taken here as p r0^2 > 49 (z > 7). The product keeps
+// exactly 2 once erfc(z) < 2^-54 (z > 5.9), taken here as p r0^2 > 36 (z > 6). The product keeps
 // libgrpp's order (screening.c:333-338).
 __device__ __forceinline__ double scr_envelope(int l1, int l2, int n, double CA, double CB, double aA, double aB,
-                                               double eta, double p, double k1, double k2, double r0, double sqpi,
-                                               double sqp)
+                                               double eta, double p, double k1, double k2, double ik1, double ik2,
+                                               double r0, double sqpi, double sqp)
 {
     const double e1 = r0 - CA, e2 = r0 - CB;
     const double ex = exp(-eta * r0 * r0 - aA * e1 * e1 - aB * e2 * e2);
     if (ex == 0.0) return 0.0;
     const double z2 = p * r0 * r0;
-    const double erf_part = z2 > 49.0 ? 2.0 : 1 + erf(sqp * r0);
-    return sqpi * ipow(r0, n) * bessel_scaled_1r(l1, k1 * r0) * bessel_scaled_1r(l2, k2 * r0) * ex * 0.5 * erf_part;
+    const double erf_part = z2 > 36.0 ? 2.0 : 1 + erf(sqp * r0);
+    const double ir = 1.0 / r0;
+    return sqpi * ipow(r0, n) * scr_m(l1, k1 * r0, ik1 * ir) * scr_m(l2, k2 * r0, ik2 * ir) * ex * 0.5 * erf_part;
 }
 
-// The fixed-point update of screening.c:329-362 from the Bessel ratio parts (n1/d1 = M_a/M_b of
-// side A at x1, n2/d2 of side B at x2): r0' = sqrt(s / (2p)),
-// s = M_a1/M_b1 x1 + M_a2/M_b2 x2 + n - (l1 + 1 if l1 > 0) - (l2 + 1 if l2 > 0),
-// the two ratios over one common denominator
-__device__ __forceinline__ double scr_update(int l1, int l2, int n, double n1, double d1, double n2, double d2,
-                                             double x1, double x2, double inv2p)
-{
-    double s = (n1 * x1 * d2 + n2 * x2 * d1) / (d1 * d2) + n;
-    if (l1 > 0) s = s - l1 - 1;
-    if (l2 > 0) s = s - l2 - 1;
-    return sqrt(s * inv2p);
-}
-
-// One fixed-point step from r0
-__device__ __forceinline__ double scr_step(int l1, int l2, int n, double k1, double k2, double inv2p, double r0)
-{
-    const double x1 = k1 * r0, x2 = k2 * r0;
-    double n1, d1, n2, d2;
-    scr_ratio_parts(l1, x1, n1, d1);
-    scr_ratio_parts(l2, x2, n2, d2);
-    return scr_update(l1, l2, n, n1, d1, n2, d2, x1, x2, inv2p);
-}
-
-// Primitive screening estimate (screening.c:243-318) with CA, CB as distances.
-// Returns true on failure (no fixed point in 4 steps). *iters: steps taken, negative
-// (-(steps)-1) when the envelope was evaluated.
-__device__ __forceinline__ bool scr_prim_flat(int l1, int l2, int n, double CA, double CB, double aA, double aB,
-                                              double k1, double k2, double eta, double *val, int *iters)
-{
-    *val = 0.0;
-    *iters = 0;
-    if (l1 >= 1 && fabs(k1) <= kZeroThresh) return false;
-    if (l2 >= 1 && fabs(k2) <= kZeroThresh) return false;
-    const double p = aA + aB + eta;
-    if (l1 == 0 && l2 == 0 && fabs(k1) <= kZeroThresh && fabs(k2) <= kZeroThresh) {
-        *val = exp(-aA * CA * CA - aB * CB * CB) * scr_gaussian_integral(n, p);
-        return false;
-    }
-    // one reciprocal of p serves the start point, the fixed-point step and the envelope
-    // (libgrpp divides by p three times; the estimate only feeds threshold tests)
-    const double inv_p = 1.0 / p, inv2p = 0.5 * inv_p;
-    double r0 = (aA * CA + aB * CB) * inv_p, r0p;
-    int steps = 0;
-    do {
-        steps++;
-        if (steps == 5) {
-            *iters = steps - 1;
-            return true;
-        }
-        r0p = r0;
-        r0 = scr_step(l1, l2, n, k1, k2, inv2p, r0);
-    } while (fabs(r0 - r0p) > 1e-2);
-    *iters = -steps - 1;
-    *val = scr_envelope(l1, l2, n, CA, CB, aA, aB, eta, p, k1, k2, r0, sqrt(kPi * inv_p), sqrt(p));
-    return false;
-}
+// The fixed-point update of screening.c:329-362: r0'^2 = s / (2p),
+// s = T_l1(x1) + T_l2(x2) + n - (l1 + 1 if l1 > 0) - (l2 + 1 if l2 > 0); cn = n - (..) - (..)
+__device__ __forceinline__ double scr_next(double t1, double t2, int cn, double inv2p) { return (t1 + t2 + cn) * inv2p; }
 
 // One-centre entry (CA = CB = 0): libgrpp's analytic table (radial_type2_integral.c:126-155),
 // only l1 = l2 = 0 non-zero
@@ -411,188 +369,104 @@ __device__ __forceinline__ void scr_store(const RadialArgs &a, int item, int64_t
 }
 
 #ifndef GRPP_RADIAL_TABLES_ONLY
-// Screening of (task, entry) pairs, one thread per entry over a flattened entry space (entries
-// of one task are consecutive, tasks in item order): no per-task barrier and no ragged last
-// round. With a.su_off the space is the short runs of a.su (the long ones go to
-// radial_screen_unit_kernel); without it, every used entry of every item. A thread follows
-// screening.c:193-220 for its entry: primitive triples (i, j, k) in libgrpp's order, stopping at
-// the first failure. The outcome per entry is written to Q (value if screened out), scr
-// (estimate) and eflag; walk[item] is set to 1 when any entry of the item needs the grid (walk[]
-// is zeroed by the host before the launch). One-centre tasks get their analytic table.
-__global__ void __launch_bounds__(kRadThreads, GRPP_SCR_MINB) radial_screen_flat_kernel(RadialArgs a)
+// Entries of one-centre tasks (CA = CB = 0): libgrpp's analytic table, one thread per entry over
+// the flattened runs of a.su.
+__global__ void __launch_bounds__(kRadThreads) radial_one_centre_kernel(RadialArgs a)
 {
-    const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const long long t0 = clock64();
-    unsigned long long c_combo = 0, c_iter = 0, c_final = 0;
-    const int64_t n_flat = a.su_off ? a.n_su_entries : a.n_used;
-    for (int64_t gu = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gu < n_flat; gu += stride) {
-        int item, pot, e;
-        int64_t pe = 0;
-        if (a.su_off) {
-            int lo = 0, hi = a.n_su - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(a.su_off + mid) <= gu) lo = mid;
-                else hi = mid - 1;
-            }
-            const ScrUnit &U = a.su[lo];
-            item = U.item;
-            pot = U.pot;
-            pe = U.pe;
-            e = a.ulist[U.uo + (int)(gu - __ldg(a.su_off + lo))];
-        } else {
-            int lo = 0, hi = a.n_items - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(a.u_off + mid) <= gu) lo = mid;
-                else hi = mid - 1;
-            }
-            item = lo;
-            int ku = (int)(gu - __ldg(a.u_off + item));
-            const int t = __ldg(a.item_task + item);
-            const int sa = __ldg(a.task_a + t), sb = __ldg(a.task_b + t), c = __ldg(a.task_c + t);
-            const int la = __ldg(a.shell_L + sa), lb = __ldg(a.shell_L + sb), dn = la + lb + 1;
-            const int gr = __ldg(a.centre_grpp + c), npot = __ldg(a.grpp_sl_n + gr), slo = __ldg(a.grpp_sl_off + gr);
-            // libgrpp tabulates the whole (l1, l2, N) box of every potential, but its angular sums
-            // read only the entries with N = n1 + n2 (n1 <= la, n2 <= lb), l1 in [max(L-n1,0), L+n1]
-            // of the parity of L+n1, l2 likewise (type2_integrals.c:169-184,
-            // spin_orbit_integrals.c:189-204). Only those are screened and walked: the others cannot
-            // change an output, and every entry's walk and stop level are its own
-            // (radial_type2_integral.c:242-318). The host lists them per class (L, la, lb).
-            pot = -1;
-            e = 0;
-            for (int p = 0; p < npot; p++) {
-                pot = __ldg(a.sl_pot + slo + p);
-                const int Lp = __ldg(a.pot_L + pot);
-                const int2 cls = a.ucls[(Lp * (kMaxL + 1) + la) * (kMaxL + 1) + lb];
-                if (ku < cls.y) {
-                    e = a.ulist[cls.x + ku];
-                    break;
-                }
-                ku -= cls.y;
-                pe += (Lp + la + 1) * (Lp + lb + 1) * dn;
-            }
+    for (int64_t gu = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; gu < a.n_su_entries; gu += stride) {
+        int lo = 0, hi = a.n_su - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(a.su_off + mid) <= gu) lo = mid;
+            else hi = mid - 1;
         }
-        const int t = __ldg(a.item_task + item);
-        const int sa = __ldg(a.task_a + t), sb = __ldg(a.task_b + t), c = __ldg(a.task_c + t);
-        const double *Ao = a.shell_origin + 3 * sa, *Bo = a.shell_origin + 3 * sb, *Co = a.centre_origin + 3 * c;
-        double CA2 = 0.0, CB2 = 0.0;
-        for (int d = 0; d < 3; d++) {
-            const double u = __ldg(Co + d) - __ldg(Ao + d), v = __ldg(Co + d) - __ldg(Bo + d);
-            CA2 += u * u;
-            CB2 += v * v;
-        }
+        const ScrUnit &U = a.su[lo];
+        const int e = a.ulist[U.uo + (int)(gu - __ldg(a.su_off + lo))];
+        const int t = __ldg(a.item_task + U.item), sa = __ldg(a.task_a + t), sb = __ldg(a.task_b + t);
         const int la = __ldg(a.shell_L + sa), lb = __ldg(a.shell_L + sb), dn = la + lb + 1;
-        const int Lp = __ldg(a.pot_L + pot);
-        const int64_t g = __ldg(a.q_off + item) + pe + e;
-        const int d2 = Lp + lb + 1;
-        const int l1 = e / (d2 * dn), rem = e - l1 * d2 * dn, l2 = rem / dn, N = rem - l2 * dn;
-        const int nk = __ldg(a.pot_nprim + pot), po = __ldg(a.pot_prim_off + pot);
-        if (CA2 < 1e-14 && CB2 < 1e-14) {
-            a.Q[g] = scr_one_centre_entry(a, sa, sb, la, lb, l1, l2, N, nk, po);
-            a.eflag[g] = 0;
-            continue;
-        }
-        const double CA = sqrt(CA2), CB = sqrt(CB2);
-        const int na = __ldg(a.rp_n + sa), nb = __ldg(a.rp_n + sb);
-        const double *ca = a.rp_coef + __ldg(a.rp_off + sa), *xa = a.rp_alpha + __ldg(a.rp_off + sa);
-        const double *cb = a.rp_coef + __ldg(a.rp_off + sb), *xb = a.rp_alpha + __ldg(a.rp_off + sb);
-        // screening.c:193-220: triples in (bra, ket, potential term) order, stop at the first failure
-        double sum = 0.0;
-        bool fail = false;
-        for (int i = 0; i < na && !fail; i++) {
-            const double aA = __ldg(xa + i), ci = __ldg(ca + i), k1 = 2 * aA * CA;
-            for (int j = 0; j < nb && !fail; j++) {
-                const double aB = __ldg(xb + j), cij = ci * __ldg(cb + j), k2 = 2 * aB * CB;
-                for (int k = 0; k < nk; k++) {
-                    double v;
-                    int it;
-                    const bool f = scr_prim_flat(l1, l2, N + __ldg(a.pot_powers + po + k), CA, CB, aA, aB, k1, k2,
-                                                 __ldg(a.pot_alpha + po + k), &v, &it);
-                    c_combo++;
-                    if (it < 0) {
-                        c_final++;
-                        it = -it - 1;
-                    }
-                    c_iter += it;
-                    if (f) {
-                        fail = true;
-                        break;
-                    }
-                    sum += cij * __ldg(a.pot_coef + po + k) * v;
-                }
-            }
-        }
-        scr_store(a, item, g, sum, fail);
-    }
-    if (a.counters) {
-        unsigned long long v[3] = {c_combo, c_iter, c_final};
-        for (int k = 0; k < 3; k++)
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        if (lane == 0) {
-            atomicAdd(a.counters + kRadCntScrCombos, v[0]);
-            atomicAdd(a.counters + kRadCntScrIters, v[1]);
-            atomicAdd(a.counters + kRadCntScrFinal, v[2]);
-            atomicAdd(a.counters + kRadCntScreenCycles, (unsigned long long)(clock64() - t0));
-        }
+        const int d2 = __ldg(a.pot_L + U.pot) + lb + 1, l1 = e / (d2 * dn), rem = e - l1 * d2 * dn, l2 = rem / dn;
+        const int64_t g = __ldg(a.q_off + U.item) + U.pe + e;
+        a.Q[g] = scr_one_centre_entry(a, sa, sb, la, lb, l1, l2, rem - l2 * dn, __ldg(a.pot_nprim + U.pot),
+                                      __ldg(a.pot_prim_off + U.pot));
+        a.eflag[g] = 0;
     }
 }
 
-// ---- screening of long runs: radial_screen_unit_kernel ----------------------------------------
+// ---- screening: radial_screen_unit_kernel ------------------------------------------------------
 //
-// A block screens one run of entries of one (task, semilocal potential) (ScrUnit), a thread per
-// entry. Everything of a primitive triple (i, j, k) that does not depend on the entry
-// (l1, l2, N) is formed once per block, a triple per thread, kScrChunk triples at a time, into
-// shared memory: p = a_A + a_B + eta, 1/p, sqrt(pi/p), sqrt(p), k = 2 a C, the fixed point's start
-// r0 = (a_A CA + a_B CB)/p and its arguments x = k r0, and the Bessel parts of the first step for
-// every order 0..lw-1 of both sides (the first step's arguments do not depend on the entry).
-// Every entry then runs libgrpp's per-triple estimate (screening.c:193-220, 243-362) over the
-// staged triples in libgrpp's order, reading its first step from the tables: the same
-// expressions, operands and order as the flat kernel, so the estimates and gate decisions are
-// the same.
-constexpr int kScrUnitThreads = 64;  // threads per block = entries per run at most
-constexpr int kScrUnitMin = 32;      // runs with fewer entries stay in the flat kernel
-constexpr int kScrChunk = 64;        // primitive triples staged per round (one per thread)
-static_assert(kScrChunk == kScrUnitThreads, "one staged triple per thread");
+// A warp screens one run of entries (l1, l2, N) of one (task, semilocal potential): for each entry
+// libgrpp's estimate, the sum over primitive triples (i, j, k) of c times a primitive estimate
+// (screening.c:193-220, 243-362), which decides whether the entry is walked.
+//
+//  * Triples that cannot matter are dropped first, for the whole run. The primitive estimate is
+//    an envelope at the fixed point r' of r'^2 = r^2 + c / (2p), started at r = (a_A CA + a_B CB)/p;
+//    the Bessel ratios obey x - 1 <= x M_(l-1)/M_l - l - 1 <= x + l, so n - 2 <= c <= n + l1 + l2.
+//    When both ends keep |r' - r| below 1e-2, libgrpp's iteration stops after one step and cannot
+//    fail; and the envelope is at most sqrt(pi/p) max(1, r + 0.01)^n times the Gaussian factor at
+//    r, its largest value. Where that bound times |c| is below e^-92 = 1e-40 the triple cannot
+//    change a sum that is compared with 1e-16 (scr_dead). This removes two thirds of the triples
+//    of the 64-atom s..g workload and half of those of a 15-atom molecule.
+//  * The remaining triples are staged in shared memory, 32 at a time: everything that does not
+//    depend on the entry, including the first step's T_l of every order (its arguments k r do
+//    not depend on the entry).
+//  * Lanes take entries, each walking the staged triples in order; where the run's entries leave
+//    lanes idle each entry gets a group of G = 2, 4 or 8 lanes that share its triples (values added by a
+//    shuffle tree; the sum's order then differs from libgrpp's in the last bits, which matter
+//    only to an estimate within them of a threshold). More lanes per entry would spread the
+//    Bessel table reads over as many rows. A triple that fails ends the entry (it is then walked).
+// What bounds it: FP64 latency with about half of the lanes active (entries need different
+// numbers of steps). Five blocks per SM (96 registers) against four and six: 17.4, 18.3, 16.9 ms
+// on the 65536 tasks of the s..g workload, where the previous pair of kernels (a thread per entry,
+// every triple, two Bessel sums per side and a division per step) took 49.5 ms; the matrices
+// of a 15-atom molecule 24.7 -> 12.8 ms, of three atoms 1.24 -> 0.44 ms. Lanes over triples
+// throughout (32 per entry) measured 53.7 ms on the first: the table rows of 32 different
+// arguments do not stay in L1.
+constexpr int kScrWarps = 4;    // warps per block, each on its own run
+constexpr int kScrRunMax = 64;  // entries per run
+constexpr int kScrArr = 13;     // staged scalars per triple
+// shared memory of a warp, in doubles: T_l [side][order][32], scalars, sums, then ints
+// (r power, waiting triples, failed entries)
+__host__ __device__ inline int scr_warp_doubles(int lw) { return 2 * lw * 32 + kScrArr * 32 + kScrRunMax + (32 + 64 + kScrRunMax) / 2; }
 
-// Bessel parts of orders 0..n-1 at x, as scr_ratio_parts forms them: the value (x <= 16) or, above
-// x = 16, the asymptotic sum without its 1/(2x) factor (it cancels in the ratio of two orders)
-__device__ __forceinline__ void scr_parts_row(int n, double x, double *out)
+// Whether a triple's estimate is below 1e-40 and its iteration ends at the first step, for every
+// entry with l1 <= l1m, l2 <= l2m and N between nlo and nhi (pw: the term's power; c: the triple's
+// coefficient). The bounds on the Bessel ratios hold for the tabulated values too when their
+// arguments are at least 0.5 (or the side's distance is 0, where entries with l > 0 are 0) and
+// the orders at most 16: their relative error is then below 1e-6, against a margin of 0.5%.
+__device__ __forceinline__ bool scr_dead(double CA, double CB, double aA, double aB, double eta, double c, int pw, int l1m,
+                                         int l2m, int nlo, int nhi)
 {
-    if (x <= 1e-7) {
-        for (int l = 0; l < n; l++) out[l] = bessel_small(l, x);
-    } else if (x <= 16.0) {
-        const int i0 = (int)(round(x * 100) + 1e-5);
-        const double dx = x - i0 * 0.01;
-        const double *row = c_tab.bessel + (size_t)i0 * kBesL * 5;
-        for (int l = 0; l < n; l++) out[l] = taylor4(row + 5 * l, dx);
-    } else {
-        const double ninv = -1.0 / x;
-        for (int l = 0; l < n; l++) {
-            const double *cl = c_tab.rfun + l * kRfunL;
-            double pw = 1.0, sum = 0.0;
-            for (int k = 0; k <= l; k++) {
-                sum += __ldg(cl + k) * pw;
-                pw *= ninv;
-            }
-            out[l] = sum;
-        }
-    }
+    const double p = aA + aB + eta, inv_p = 1.0 / p, inv2p = 0.5 * inv_p;
+    const double r = (aA * CA + aB * CB) * inv_p, k1 = 2 * aA * CA, k2 = 2 * aB * CB;
+    const bool in1 = k1 * r >= 0.5, in2 = k2 * r >= 0.5;
+    if (!(in1 || k1 <= kZeroThresh) || !(in2 || k2 <= kZeroThresh) || !(in1 || in2) || l1m > 16 || l2m > 16) return false;
+    if (!((nhi + pw + l1m + l2m) * inv2p <= 0.0199 * r + 0.99e-4) || !((2 - nlo - pw) * inv2p <= 0.0199 * r - 1e-4)) return false;
+    const double eA = r - CA, eB = r - CB;
+    const float g = (float)(-eta * r * r - aA * eA * eA - aB * eB * eB);
+    const float b = 0.5f * __logf(3.1416f * (float)inv_p) + (nhi + pw) * __logf(fmaxf(1.f, (float)r + 0.01f)) +
+                    __logf(fmaxf((float)fabs(c), 1e-37f));
+    return g + b < -92.f;
 }
 
-__global__ void __launch_bounds__(kScrUnitThreads, 10) radial_screen_unit_kernel(RadialArgs a)
+__global__ void __launch_bounds__(32 * kScrWarps, 5) radial_screen_unit_kernel(RadialArgs a)
 {
-    extern __shared__ double ptab[];  // [kScrChunk][2][scr_lw]: Bessel parts, sides A and B
-    __shared__ double t_aA[kScrChunk], t_aB[kScrChunk], t_eta[kScrChunk], t_p[kScrChunk], t_ip[kScrChunk],
-        t_sqpi[kScrChunk], t_sqp[kScrChunk], t_k1[kScrChunk], t_k2[kScrChunk], t_r0[kScrChunk], t_x1[kScrChunk],
-        t_x2[kScrChunk], t_c[kScrChunk];
-    __shared__ int t_pw[kScrChunk];
-    const int tid = threadIdx.x, lane = tid & 31, lw = a.scr_lw;
+    extern __shared__ double scr_sm[];
+    const int lane = threadIdx.x & 31, lw = a.scr_lw;
+    double *PA = scr_sm + (threadIdx.x >> 5) * scr_warp_doubles(lw), *PB = PA + lw * 32;
+    double *t_aA = PB + lw * 32, *t_aB = t_aA + 32, *t_eta = t_aB + 32, *t_p = t_eta + 32, *t_i2p = t_p + 32, *t_sqpi = t_i2p + 32,
+           *t_sqp = t_sqpi + 32, *t_k1 = t_sqp + 32, *t_k2 = t_k1 + 32, *t_r0 = t_k2 + 32, *t_ik1 = t_r0 + 32, *t_ik2 = t_ik1 + 32,
+           *t_c = t_ik2 + 32, *s_sum = t_c + 32;
+    int *t_pw = (int *)(s_sum + kScrRunMax), *list = t_pw + 32, *s_bad = list + 64;
     const long long t0 = clock64();
     unsigned long long c_combo = 0, c_iter = 0, c_final = 0;
-    for (int u = blockIdx.x; u < a.n_scr_units; u += gridDim.x) {
-        const int item = a.scr_units[u].item, pot = a.scr_units[u].pot, ne = a.scr_units[u].ne;
+    for (;;) {
+        int u = 0;
+        if (lane == 0) u = atomicAdd(a.scr_queue, 1);
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= a.n_scr_units) break;
+        const ScrUnit U = a.scr_units[u];
+        const int item = U.item, pot = U.pot, ne = U.ne;
         const int t = __ldg(a.item_task + item);
         const int sa = __ldg(a.task_a + t), sb = __ldg(a.task_b + t), c = __ldg(a.task_c + t);
         const double *Ao = a.shell_origin + 3 * sa, *Bo = a.shell_origin + 3 * sb, *Co = a.centre_origin + 3 * c;
@@ -602,111 +476,146 @@ __global__ void __launch_bounds__(kScrUnitThreads, 10) radial_screen_unit_kernel
             CA2 += uu * uu;
             CB2 += vv * vv;
         }
+        const double CA = sqrt(CA2), CB = sqrt(CB2);
         const int la = __ldg(a.shell_L + sa), lb = __ldg(a.shell_L + sb), dn = la + lb + 1;
         const int Lp = __ldg(a.pot_L + pot), d2 = Lp + lb + 1;
         const int nk = __ldg(a.pot_nprim + pot), po = __ldg(a.pot_prim_off + pot);
-        const bool have = tid < ne;
-        int l1 = 0, l2 = 0, N = 0;
-        int64_t g = 0;
-        if (have) {
-            const int e = a.ulist[a.scr_units[u].uo + tid];
-            g = __ldg(a.q_off + item) + a.scr_units[u].pe + e;
-            l1 = e / (d2 * dn);
-            const int rem = e - l1 * d2 * dn;
-            l2 = rem / dn;
-            N = rem - l2 * dn;
-        }
-        if (CA2 < 1e-14 && CB2 < 1e-14) {  // one-centre tasks are the flat kernel's; kept for safety
-            if (have) {
-                a.Q[g] = scr_one_centre_entry(a, sa, sb, la, lb, l1, l2, N, nk, po);
-                a.eflag[g] = 0;
-            }
-            continue;
-        }
-        const double CA = sqrt(CA2), CB = sqrt(CB2);
-        const int na = __ldg(a.rp_n + sa), nb = __ldg(a.rp_n + sb);
+        const int na = __ldg(a.rp_n + sa), nb = __ldg(a.rp_n + sb), T = na * nb * nk;
         const double *ca = a.rp_coef + __ldg(a.rp_off + sa), *xa = a.rp_alpha + __ldg(a.rp_off + sa);
         const double *cb = a.rp_coef + __ldg(a.rp_off + sb), *xb = a.rp_alpha + __ldg(a.rp_off + sb);
-        // orders of the first step's ratios (screening.c:329-346): (1, 0) for l = 0, else (l-1, l)
-        const int oa1 = l1 == 0 ? 1 : l1 - 1, ob1 = l1 == 0 ? 0 : l1, oa2 = l2 == 0 ? 1 : l2 - 1, ob2 = l2 == 0 ? 0 : l2;
-        const int nA = max(2, Lp + la + 1), nB = max(2, Lp + lb + 1);  // orders the run's entries can use
-        double sum = 0.0;
-        bool fail = !have;
-        const int T = na * nb * nk;
-        for (int c0 = 0; c0 < T; c0 += kScrChunk) {
-            const int nc = min(kScrChunk, T - c0);
-            __syncthreads();  // the previous round's tables are consumed
-            if (tid < nc) {
-                const int q = c0 + tid, i = q / (nb * nk), j = (q / nk) % nb, k = q % nk;
+        const int64_t g0 = __ldg(a.q_off + item) + U.pe;
+        __syncwarp();  // the previous run's shared arrays are consumed
+        int l1m = 0, l2m = 0, nlo = dn, nhi = 0;
+        for (int q = lane; q < ne; q += 32) {
+            const int e = a.ulist[U.uo + q], l1 = e / (d2 * dn), rem = e - l1 * d2 * dn, l2 = rem / dn, N = rem - l2 * dn;
+            l1m = max(l1m, l1);
+            l2m = max(l2m, l2);
+            nlo = min(nlo, N);
+            nhi = max(nhi, N);
+            s_sum[q] = 0.0;
+            s_bad[q] = 0;
+        }
+        l1m = __reduce_max_sync(0xffffffffu, l1m);
+        l2m = __reduce_max_sync(0xffffffffu, l2m);
+        nlo = __reduce_min_sync(0xffffffffu, nlo);
+        nhi = __reduce_max_sync(0xffffffffu, nhi);
+        // lanes per entry: the fewest that leave at most an eighth of the lanes without an entry
+        int lg = 0;
+        while (lg < 3 && ((ne + (32 >> lg) - 1) & ~((32 >> lg) - 1)) * 7 > 8 * ne) lg++;
+        const int G = 1 << lg;
+        int pos = 0, nl = 0;
+        unsigned n_dead = 0;
+        for (;;) {
+            // the next triples in libgrpp's (i, j, k) order that are not dropped
+            while (nl < 32 && pos < T) {
+                const int q = pos + lane;
+                bool live = false;
+                if (q < T) {
+                    const int i = q / (nb * nk), r = q - i * nb * nk, j = r / nk, k = r - j * nk;
+                    live = !scr_dead(CA, CB, __ldg(xa + i), __ldg(xb + j), __ldg(a.pot_alpha + po + k),
+                                     __ldg(ca + i) * __ldg(cb + j) * __ldg(a.pot_coef + po + k), __ldg(a.pot_powers + po + k), l1m,
+                                     l2m, nlo, nhi);
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, live);
+                if (live) list[nl + __popc(m & ((1u << lane) - 1))] = q;
+                n_dead += min(32, T - pos) - __popc(m);
+                nl += __popc(m);
+                pos += 32;
+            }
+            if (nl == 0) break;
+            const int nc = min(32, nl);
+            __syncwarp();
+            if (lane < nc) {
+                const int q = list[lane], i = q / (nb * nk), r = q - i * nb * nk, j = r / nk, k = r - j * nk;
                 const double aA = __ldg(xa + i), aB = __ldg(xb + j), eta = __ldg(a.pot_alpha + po + k);
                 const double k1 = 2 * aA * CA, k2 = 2 * aB * CB;
                 const double p = aA + aB + eta, inv_p = 1.0 / p;
                 const double r0 = (aA * CA + aB * CB) * inv_p;
-                const double cij = __ldg(ca + i) * __ldg(cb + j);
-                t_aA[tid] = aA;
-                t_aB[tid] = aB;
-                t_eta[tid] = eta;
-                t_p[tid] = p;
-                t_ip[tid] = inv_p;
-                t_sqpi[tid] = sqrt(kPi * inv_p);
-                t_sqp[tid] = sqrt(p);
-                t_k1[tid] = k1;
-                t_k2[tid] = k2;
-                t_r0[tid] = r0;
-                t_x1[tid] = k1 * r0;
-                t_x2[tid] = k2 * r0;
-                t_c[tid] = cij * __ldg(a.pot_coef + po + k);
-                t_pw[tid] = __ldg(a.pot_powers + po + k);
-                scr_parts_row(nA, k1 * r0, ptab + (size_t)(2 * tid) * lw);
-                scr_parts_row(nB, k2 * r0, ptab + (size_t)(2 * tid + 1) * lw);
+                t_aA[lane] = aA;
+                t_aB[lane] = aB;
+                t_eta[lane] = eta;
+                t_p[lane] = p;
+                t_i2p[lane] = 0.5 * inv_p;
+                t_sqpi[lane] = sqrt(kPi * inv_p);
+                t_sqp[lane] = sqrt(p);
+                t_k1[lane] = k1;
+                t_k2[lane] = k2;
+                t_r0[lane] = r0;
+                t_ik1[lane] = 1.0 / k1;
+                t_ik2[lane] = 1.0 / k2;
+                t_c[lane] = __ldg(ca + i) * __ldg(cb + j) * __ldg(a.pot_coef + po + k);
+                t_pw[lane] = __ldg(a.pot_powers + po + k);
+                const double i1 = 1.0 / (k1 * r0), i2 = 1.0 / (k2 * r0);
+                for (int l = 0; l <= l1m; l++) PA[l * 32 + lane] = scr_t(l, k1 * r0, i1);
+                for (int l = 0; l <= l2m; l++) PB[l * 32 + lane] = scr_t(l, k2 * r0, i2);
             }
-            __syncthreads();
-            if (fail) continue;
-            for (int q = 0; q < nc; q++) {
-                const double k1 = t_k1[q], k2 = t_k2[q];
-                double v = 0.0;
-                int it = 0;
-                bool f = false;
-                if (!(l1 >= 1 && fabs(k1) <= kZeroThresh) && !(l2 >= 1 && fabs(k2) <= kZeroThresh)) {
-                    const int n = N + t_pw[q];
-                    const double p = t_p[q];
-                    if (l1 == 0 && l2 == 0 && fabs(k1) <= kZeroThresh && fabs(k2) <= kZeroThresh) {
-                        v = exp(-t_aA[q] * CA * CA - t_aB[q] * CB * CB) * scr_gaussian_integral(n, p);
-                    } else {
-                        const double inv2p = 0.5 * t_ip[q];
-                        const double *PA = ptab + (size_t)(2 * q) * lw, *PB = PA + lw;
+            __syncwarp();
+            for (int e0 = 0; e0 < ne; e0 += 32 >> lg) {
+                const int ei = e0 + (lane >> lg);
+                const bool on = ei < ne && !s_bad[ei < ne ? ei : 0];
+                const int e = a.ulist[U.uo + (ei < ne ? ei : 0)];
+                const int l1 = e / (d2 * dn), rem = e - l1 * d2 * dn, l2 = rem / dn, N = rem - l2 * dn;
+                const int cl = N - (l1 > 0 ? l1 + 1 : 0) - (l2 > 0 ? l2 + 1 : 0);
+                double sum = 0.0;
+                bool fail = false;
+                for (int q0 = 0; q0 < nc; q0 += G) {
+                    const int q = q0 + (lane & (G - 1));
+                    const bool go = on && !fail && q < nc;
+                    const double k1 = t_k1[q & 31], k2 = t_k2[q & 31], p = t_p[q & 31];
+                    const bool z1 = fabs(k1) <= kZeroThresh, z2 = fabs(k2) <= kZeroThresh, ss = l1 == 0 && l2 == 0 && z1 && z2;
+                    bool step = go && !(l1 >= 1 && z1) && !(l2 >= 1 && z2) && !ss, conv = false;
+                    const int pw = t_pw[q & 31], n = N + pw;
+                    c_combo += go;
+                    double r0 = 0.0;
+                    if (step) {
+                        const double inv2p = t_i2p[q], ik1 = t_ik1[q], ik2 = t_ik2[q];
                         double r0p = t_r0[q];
-                        double r0 = scr_update(l1, l2, n, PA[oa1], PA[ob1], PB[oa2], PB[ob2], t_x1[q], t_x2[q], inv2p);
+                        r0 = sqrt(scr_next(PA[l1 * 32 + q], PB[l2 * 32 + q], cl + pw, inv2p));
                         int steps = 1;
-                        while (fabs(r0 - r0p) > 1e-2) {
+                        while (fabs(r0 - r0p) > 1e-2 && steps < 4) {
                             steps++;
-                            if (steps == 5) {
-                                f = true;
-                                break;
-                            }
                             r0p = r0;
-                            r0 = scr_step(l1, l2, n, k1, k2, inv2p, r0);
+                            const double ir = 1.0 / r0;  // a factor of both sides' 1/x
+                            r0 = sqrt(scr_next(scr_t(l1, k1 * r0, ik1 * ir), scr_t(l2, k2 * r0, ik2 * ir), cl + pw, inv2p));
                         }
-                        if (f) {
-                            it = steps - 1;
-                        } else {
-                            it = steps;
-                            c_final++;
-                            v = scr_envelope(l1, l2, n, CA, CB, t_aA[q], t_aB[q], t_eta[q], p, k1, k2, r0, t_sqpi[q],
-                                             t_sqp[q]);
-                        }
+                        c_iter += steps;
+                        fail = fabs(r0 - r0p) > 1e-2;  // no fixed point in four steps
+                        conv = !fail;
                     }
+                    __syncwarp();
+                    if (conv) {
+                        c_final++;
+                        sum += t_c[q] * scr_envelope(l1, l2, n, CA, CB, t_aA[q], t_aB[q], t_eta[q], p, k1, k2, t_ik1[q], t_ik2[q], r0,
+                                                     t_sqpi[q], t_sqp[q]);
+                    } else if (go && ss) {
+                        sum += t_c[q] * exp(-t_aA[q] * CA * CA - t_aB[q] * CB * CB) * scr_gaussian_integral(n, p);
+                    }
+                    __syncwarp();
                 }
-                c_combo++;
-                c_iter += it;
-                if (f) {
-                    fail = true;
-                    break;
+                const unsigned bad = __ballot_sync(0xffffffffu, fail) >> (lane & ~(G - 1)) & ((1u << G) - 1);
+                for (int o = G >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (on && (lane & (G - 1)) == 0) {
+                    s_sum[ei] += sum;
+                    if (bad) s_bad[ei] = 1;
                 }
-                sum += t_c[q] * v;
+                __syncwarp();
+            }
+            // the triples that still wait move to the front
+            const int rest = nl - nc;
+            const int keep = lane < rest ? list[nc + lane] : 0;
+            __syncwarp();
+            if (lane < rest) list[lane] = keep;
+            nl = rest;
+            __syncwarp();
+        }
+        for (int q = lane; q < ne; q += 32) {
+            scr_store(a, item, g0 + a.ulist[U.uo + q], s_sum[q], s_bad[q] != 0);
+            if (!s_bad[q]) {  // a dropped triple is one step and one envelope of libgrpp's
+                c_combo += n_dead;
+                c_iter += n_dead;
+                c_final += n_dead;
             }
         }
-        if (have) scr_store(a, item, g, sum, fail);
     }
     if (a.counters) {
         unsigned long long v[3] = {c_combo, c_iter, c_final};

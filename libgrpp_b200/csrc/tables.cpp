@@ -6,6 +6,8 @@
 //   exp(-x) i_l(x) = exp(-x) x^l/(2l+1)!! sum_k (x^2/2)^k / (k! prod_{j<=k} (2l+2j+1))
 //   F_n(x)         = exp(-x) sum_k (2x)^k / prod_{j<=k} (2n+2j+1)
 //   Daw(y)         = exp(-y^2) sum_k y^(2k+1) / (k! (2k+1))
+// The screening's ratios T_l(x) = x M_(l-1)/M_l are tabulated with the Taylor coefficients that
+// their Riccati equation gives.
 // Derivatives of M_l follow the exact recurrence
 //   M_l' = l/(2l+1) M_{l-1} + (l+1)/(2l+1) M_{l+1} - M_l
 // (libgrpp/specfunc_scaled_mod_sph_bessel.c:135-156).
@@ -53,6 +55,53 @@ long double boys_series(int n, long double x)
         if (term < 1e-24L * sum) break;
     }
     return expl(-x) * sum;
+}
+
+// Taylor coefficients of T(x) = x i_(l-1)/i_l (l = 0: x i_1/i_0) about x0 > 0 from T(x0), by
+// x T' = x^2 + beta T - T^2, beta = 2l + 1 (l = 0: -1)
+void ratio_taylor_x(long double beta, long double x0, long double t0, double *c)
+{
+    long double t[6] = {t0};
+    for (int k = 0; k < 4; k++) {
+        long double r = beta * t[k] - k * t[k];
+        if (k == 0) r += x0 * x0;
+        if (k == 1) r += 2 * x0;
+        if (k == 2) r += 1;
+        for (int i = 0; i <= k; i++) r -= t[i] * t[k - i];
+        t[k + 1] = r / (x0 * (k + 1));
+    }
+    for (int k = 0; k < 5; k++) c[k] = (double)t[k];
+}
+
+// the same of a(y) = T(1/y) - 1/y about y0 from a(y0): y^2 a' = 1 - beta + 2a + y (a^2 - beta a);
+// at y0 = 0 the equation gives every coefficient, a(0) = (beta - 1) / 2
+void ratio_taylor_y(long double beta, long double y0, long double a0, double *c)
+{
+    long double a[6] = {y0 > 0 ? a0 : (beta - 1) / 2}, b[6];  // b = a^2 - beta a
+    for (int k = 0; k < 5; k++) {
+        if (y0 == 0 && k > 0) a[k] = ((k - 1) * a[k - 1] - b[k - 1]) / 2;
+        b[k] = -beta * a[k];
+        for (int i = 0; i <= k; i++) b[k] += a[i] * a[k - i];
+        if (y0 > 0) {
+            long double r = 2 * a[k] + y0 * b[k] - 2 * y0 * k * a[k];
+            if (k == 0) r += 1 - beta;
+            if (k > 0) r += b[k - 1] - (k - 1) * a[k - 1];
+            a[k + 1] = r / (y0 * y0 * (k + 1));
+        }
+    }
+    for (int k = 0; k < 5; k++) c[k] = (double)a[k];
+}
+
+// T_l(x), l = 0..n-1: downward T_l = 2l + 1 + x^2 / T_(l+1) from an order where T ~ 2l + 1 + x^2/..
+void ratio_values(int n, long double x, long double *t)
+{
+    long double v = 0;
+    const int top = n + 60 + (int)x;
+    for (int l = top; l >= 1; l--) {
+        v = 2.0L * l + 1.0L + (l == top ? 0.0L : x * x / v);
+        if (l < n) t[l] = v;
+    }
+    t[0] = x * x / v;
 }
 
 long double dawson_series(long double y)
@@ -243,6 +292,39 @@ void build_host_tables(HostTables &t)
     t.boys.assign(kBoysNX * kBoysNN, 0.0);
     for (int i = 0; i < kBoysNX; i++)
         for (int n = 0; n < kBoysNN; n++) t.boys[i * kBoysNN + n] = (double)boys_series(n, 0.1L * i);
+
+    t.ratio.assign((size_t)kBesNX * kRatL * 5, 0.0);
+    t.ratio_y.assign((size_t)kRatYN * kRatL * 5, 0.0);
+    std::vector<long double> tl(kRatL);
+    for (int i = 1; i < kBesNX; i++) {
+        ratio_values(kRatL, 0.01L * i, tl.data());
+        for (int l = 0; l < kRatL; l++)
+            ratio_taylor_x(l ? 2.0L * l + 1.0L : -1.0L, 0.01L * i, tl[l], &t.ratio[((size_t)i * kRatL + l) * 5]);
+    }
+    for (int i = 0; i < kRatYN; i++) {
+        const long double y = i / (long double)kRatYInv, x = i ? 1.0L / y : 0.0L;
+        if (i) ratio_values(kRatL, x, tl.data());
+        for (int l = 0; l < kRatL; l++)
+            ratio_taylor_y(l ? 2.0L * l + 1.0L : -1.0L, y, i ? tl[l] - x : 0.0L, &t.ratio_y[((size_t)i * kRatL + l) * 5]);
+    }
+
+    t.bes_t.assign((size_t)kBesNX * kRatL * 5, 0.0);
+    t.bes_y.assign((size_t)kBesYN * kRatL * 5, 0.0);
+    const double inv_fact[5] = {1.0, 1.0, 0.5, 1.0 / 6.0, 1.0 / 24.0};
+    for (int i = 0; i < kBesNX; i++)
+        for (int l = 0; l < kRatL; l++)
+            for (int k = 0; k < 5; k++)
+                t.bes_t[((size_t)i * kRatL + l) * 5 + k] = t.bessel[((size_t)i * kBesL + l) * 5 + k] * inv_fact[k];
+    for (int i = 0; i < kBesYN; i++)
+        for (int l = 0; l < kRatL; l++) {
+            const long double y = i / (long double)kBesYInv;
+            for (int m = 0; m < 5 && m <= l; m++) {  // Taylor shift of sum_k c_k (-y)^k
+                long double v = 0, pw = 1;
+                for (int k = m; k <= l; k++, pw *= y)
+                    v += (k & 1 ? -1 : 1) * (long double)t.rfun[l * kRfunL + k] * (long double)binom_d(k, m) * pw;
+                t.bes_y[((size_t)i * kRatL + l) * 5 + m] = (double)v;
+            }
+        }
 
     t.dawson.assign(kDawNY, 0.0);
     for (int j = 0; j < kDawNY; j++) t.dawson[j] = (double)dawson_series((long double)kDawY0 + (long double)j / 32.0L);
