@@ -46,6 +46,17 @@ __host__ __device__ inline int lam_slots(int L, int l)
     return m;
 }
 
+// Omega tables: omega[abc][slot][m], rows of om_row(L) values (2L + 1 and a zero: 16-byte rows), with
+// om_stride(L, l) values per abc, an odd number of 16-byte units, so that the lanes of a warp reading
+// different abc meet different shared-memory banks
+__host__ __device__ inline int om_row(int L) { return 2 * L + 2; }
+__host__ __device__ inline int om_stride(int L, int l)
+{
+    const int s = lam_slots(L, l) * om_row(L);
+    return (s / 2) & 1 ? s : s + 2;
+}
+__host__ __device__ inline int om_size(int L, int l) { return n_abc(l) * om_stride(L, l); }
+
 // Atab layout per (L, l): [abc][slot][mu (0..2*lmax_lam)][m (0..2L)], lmax_lam = L + l
 __host__ __device__ inline int64_t atab_size(int L, int l)
 {
@@ -128,6 +139,8 @@ struct OcProjArgs {
     const int8_t *cart;
     const double *S_cart, *U_cart;
     double *S_sph, *U_sph;
+    double *LS, *SL;             // [3][sph_tot]: sum_m2 L(m1, m2) S(m2) and sum_m1 S(m1) L(m1, m2)
+    int64_t sph_tot;
 };
 
 __device__ inline double sph_coef_oc(int L, int m, int r, int s, int t)
@@ -143,13 +156,22 @@ __device__ inline double sph_coef_oc(int L, int m, int r, int s, int t)
     return y / an;
 }
 
+__device__ __forceinline__ double lmat_val(int L, int comp, int m1, int m2)
+{
+    const int d = 2 * L + 1;
+    return c_tab.lmat[c_tab.lmat_off[L] + comp * d * d + (m1 + L) * d + (m2 + L)];
+}
+
 #ifndef GRPP_NO_ANGULAR_KERNELS
+// The products of an outercore block with the L matrices depend on one shell only: formed here
+// once per (shell, centre), not per task and element of the assembly.
 __global__ void oc_proj_kernel(OcProjArgs a)
 {
     for (int blk = blockIdx.x; blk < a.n; blk += gridDim.x) {
         const int s = a.blk_shell[blk], o = a.blk_ocshell[blk];
         const int ns = ncart(a.shell_L[s]), L = a.shell_L[o], no = ncart(L), d = 2 * L + 1;
         const int8_t *co = a.cart + 3 * a.shell_cart_off[o];
+        const int64_t off = a.blk_sph_off[blk];
         for (int e = threadIdx.x; e < ns * d; e += blockDim.x) {
             const int i = e / d, m = e % d - L;
             double ss = 0.0, su = 0.0;
@@ -158,9 +180,20 @@ __global__ void oc_proj_kernel(OcProjArgs a)
                 ss += u * a.S_cart[a.blk_cart_off[blk] + i * no + ic];
                 su += u * a.U_cart[a.blk_cart_off[blk] + i * no + ic];
             }
-            a.S_sph[a.blk_sph_off[blk] + i * d + m + L] = ss;
-            a.U_sph[a.blk_sph_off[blk] + i * d + m + L] = su;
+            a.S_sph[off + i * d + m + L] = ss;
+            a.U_sph[off + i * d + m + L] = su;
         }
+        __syncthreads();
+        for (int e = threadIdx.x; e < 3 * ns * d; e += blockDim.x) {
+            const int comp = e / (ns * d), r = e - comp * ns * d, i = r / d, m = r - i * d;
+            const double *S = a.S_sph + off + i * d;
+            double ls = 0.0, sl = 0.0;
+            for (int q = 0; q < d; q++) ls += lmat_val(L, comp, m - L, q - L) * S[q];
+            for (int q = 0; q < d; q++) sl += S[q] * lmat_val(L, comp, q - L, m - L);
+            a.LS[comp * a.sph_tot + off + r] = ls;
+            a.SL[comp * a.sph_tot + off + r] = sl;
+        }
+        __syncthreads();
     }
 }
 #endif  // GRPP_NO_ANGULAR_KERNELS
@@ -169,9 +202,9 @@ __global__ void oc_proj_kernel(OcProjArgs a)
 
 constexpr int kFinThreads = 128;       // omega tables; the assembly kernel is instantiated for 128, 256, 512
 constexpr int kFinMaxPairs = 1024;     // Cartesian pairs of one task block (i x i = 784)
-constexpr int kFinElemPerThread = kFinMaxPairs / kFinThreads;
 constexpr int kFinMaxLam = 24;
-constexpr int kLmatPairs = 100;  // (m1, m2) pairs of the L matrices with a non-zero component: 10L - 4 <= 96 for L <= 10
+constexpr int kFinMaxCart = 66;         // components of L = 10
+constexpr int kFinTile = 4;            // rows of V per thread of the V table
 constexpr int kFinMaxSl = 24;         // semilocal potentials per centre
 constexpr int kFinMaxOc = 32;         // outercore shells per centre
 
@@ -197,6 +230,8 @@ struct FinalArgs {
     const double *atab;
     const int64_t *proj_off;          // per projection: offset of its first oc block in S_sph / U_sph
     const double *S_sph, *U_sph;
+    const double *LS, *SL;            // [3][sph_tot] (oc_proj_kernel)
+    int64_t sph_tot;
     int raw_so;                       // 1: spin-orbit output without the 2/(2L+1) factor
     double *arep, *so_x, *so_y, *so_z;
     int *status;
@@ -205,81 +240,106 @@ struct FinalArgs {
     const int *order;
     int *queue;
     // omega tables per (shell, centre) pair (omega_tab_kernel): for each semilocal potential
-    // of the centre's GRPP in order, omega[abc][slot][m] of that side, from om_off[pair];
+    // of the centre's GRPP in order, om_size values of that side, from om_off[pair];
     // task_fpa / task_fpb: the pairs (A, C) and (B, C) of a task. omtab null: computed here
     const double *omtab;
     const int64_t *om_off;
     const int *task_fpa, *task_fpb;
 };
 
-// RSH values S_{l mu}(k/|k|) for l = 0..lmax (spherical_harmonics.c:227-280); out[l*(2*kFinMaxLam+1) + mu + l]
-__device__ void rsh_values(int lmax, const double *k, double *out, int tid, int nthr)
-{
-    const double len = sqrt(k[0] * k[0] + k[1] * k[1] + k[2] * k[2]);
-    double ux = 0.0, uy = 0.0, uz = 0.0;
-    if (len > kZeroThresh) {
-        const double inv = 1.0 / len;
-        ux = k[0] * inv;
-        uy = k[1] * inv;
-        uz = k[2] * inv;
-    }
-    for (int e = tid; e < (lmax + 1) * (2 * kFinMaxLam + 1); e += nthr) {
-        const int l = e / (2 * kFinMaxLam + 1), mu = e % (2 * kFinMaxLam + 1) - l;
-        if (mu > l) continue;
-        const int nc = ncart(l);
-        const int8_t *cc = c_tab.rsh_comb + 3 * c_tab.rsh_comb_off[l];
-        const double *y = c_tab.rsh_coef + c_tab.rsh_off[l] + (mu + l) * nc;
-        double v = 0.0;
-        for (int q = 0; q < nc; q++) {
-            double px = 1.0, py = 1.0, pz = 1.0;
-            for (int i = 0; i < cc[3 * q]; i++) px *= ux;
-            for (int i = 0; i < cc[3 * q + 1]; i++) py *= uy;
-            for (int i = 0; i < cc[3 * q + 2]; i++) pz *= uz;
-            v += y[q] * (px * py * pz);
-        }
-        out[e] = v;
-    }
-}
-
-}  // namespace grpp
-
-namespace grpp {
-
 struct FinalSmem {
-    // offsets (in doubles) of the dynamic shared regions, computed on the host
+    // sizes (in doubles) of the dynamic shared regions, computed on the host
     int rsh_stride;  // 2*lam_max+1
-    int n_rsh;       // (lam_max+1) * rsh_stride
-    int n_omega;     // per side
-    int n_q;
-    int n_v;
-    int n_w;         // W[j][abc][comp] of the factored re-centring sum (0: not used)
+    int n_rsh;       // (lam_max+1) * rsh_stride per side (0: omega tables come from global memory)
+    int n_task;      // a task's own tables (fin_task_doubles), the largest of the launch
+    int n_v;         // rows of V
+    int n_w;         // W of the factored re-centring sum (0: not used)
 };
 
-__device__ __forceinline__ double lmat_val(int L, int comp, int m1, int m2)
+// Binomial terms of the Cartesian components of one shell: sum over its components of
+// (x+1)(y+1)(z+1) entries
+__host__ __device__ inline int fin_terms(const int8_t *cart, int n)
 {
-    const int d = 2 * L + 1;
-    return c_tab.lmat[c_tab.lmat_off[L] + comp * d * d + (m1 + L) * d + (m2 + L)];
+    int t = 0;
+    for (int i = 0; i < n; i++) t += (cart[3 * i] + 1) * (cart[3 * i + 1] + 1) * (cart[3 * i + 2] + 1);
+    return t;
+}
+// doubles of a task's own tables: both sides' omega of the largest potential, its radial table,
+// and the binomial terms (a factor and a packed index each)
+__host__ __device__ inline int fin_task_doubles(int n_omega, int n_q, int n_terms) { return n_omega + ((n_q + 1) & ~1) + n_terms + (n_terms + 1) / 2; }
+// row length of V (odd: lanes over rows meet different banks)
+__host__ __device__ inline int fin_v_row(int nabB, int ncomp) { return (nabB * ncomp) | 1; }
+__host__ __device__ inline int fin_v_rows(int n_v, int nabA, int nabB, int ncomp)
+{
+    const int r = n_v / fin_v_row(nabB, ncomp);
+    return r < 1 ? 1 : (r < nabA ? r : nabA);
+}
+__host__ __device__ inline int fin_w_size(int nB, int rows, int ncomp) { return nB * (((rows * ncomp) | 1) + (rows | 1)); }
+
+// A binomial term (abc) of a component (x, y, z): index of abc, product of the three binomials
+// (at most 252 for l <= 10, exact), powers x - a, y - b, z - c
+__device__ __forceinline__ unsigned fin_term(int abc, int c, int ex, int ey, int ez)
+{
+    return abc | (c << 9) | (ex << 17) | (ey << 21) | (ez << 25);
+}
+
+// |abc| of an abc index
+__device__ inline int abc_degree(int l, int idx)
+{
+    int aa, bb;
+    for (aa = 0; aa <= l; aa++) {
+        const int cnt = (l - aa + 1) * (l - aa + 2) / 2;
+        if (idx < cnt) break;
+        idx -= cnt;
+    }
+    for (bb = 0; bb <= l - aa; bb++) {
+        const int cnt = l - aa - bb + 1;
+        if (idx < cnt) break;
+        idx -= cnt;
+    }
+    return aa + bb + idx;
+}
+
+// omega[abc][slot][m] = sum_mu S_{lam mu} Atab (angular_integrals.c:78-108), |abc| = n
+__device__ __forceinline__ double omega_value(int L, int n, int slot, int m, int sl, int nmu, int nm, int abc, const double *At,
+                                              const double *rsh, int rs)
+{
+    double w = 0.0;
+    if (slot < lam_count(L, n)) {
+        const int lam = lam_lo(L, n) + 2 * slot;
+        const double *S = rsh + lam * rs;
+        const double *Ap = At + ((int64_t)(abc * sl + slot) * nmu) * nm + m;
+        for (int mu = -lam; mu <= lam; mu++) {
+            const double rv = S[mu + lam];
+            if (fabs(rv) < kZeroThresh) continue;
+            w += Ap[(int64_t)(mu + lam) * nm] * rv;
+        }
+    }
+    return w;
 }
 
 #ifndef GRPP_NO_ANGULAR_KERNELS
-// Omega tables of one side for every (shell, centre) pair: a CTA per pair computes the
-// real spherical harmonics of the unit vector along k = -2 a (C - S) (a the shell's first
-// exponent) and, for each semilocal potential of the centre's GRPP in order,
-// omega[abc][slot][m] = sum_mu S_{lam mu} Atab[abc][slot][mu][m] with the skips of
-// angular_integrals.c:78-108 — the same expressions as final_kernel's own evaluation.
-// Dynamic shared memory: (lam_max + 1) x sm.rsh_stride doubles.
+// Omega tables of one side for every (shell, centre) pair and semilocal potential of the centre's
+// GRPP, a CTA each: the real spherical harmonics of the unit vector along k = -2 a (C - S) (a the
+// shell's first exponent), then omega[abc][slot][m] = sum_mu S_{lam mu} Atab[abc][slot][mu][m] with
+// the skips of angular_integrals.c:78-108 — the same expressions as final_kernel's own
+// evaluation. (A CTA per pair, all potentials one after another, left small calls waiting for one
+// CTA.) Dynamic shared memory: (lam_max + 1) x sm.rsh_stride doubles.
 __global__ void __launch_bounds__(kFinThreads) omega_tab_kernel(FinalArgs a, FinalSmem sm, const int *op_shell,
-                                                                const int *op_centre, int n_pairs, double *omtab)
+                                                                const int *op_centre, int n_pairs, int max_sl, double *omtab)
 {
     extern __shared__ double rsh[];
     __shared__ double upow[3][kFinMaxLam + 1];
     __shared__ int8_t nabc[n_abc(kMaxL)];
     const int tid = threadIdx.x, rs = sm.rsh_stride;
-    for (int pr = blockIdx.x; pr < n_pairs; pr += gridDim.x) {
+    for (int64_t blk = blockIdx.x; blk < (int64_t)n_pairs * max_sl; blk += gridDim.x) {
+        const int pr = (int)(blk / max_sl), p = (int)(blk % max_sl);
         const int sx = op_shell[pr], c = op_centre[pr], l = a.shell_L[sx], g = a.centre_grpp[c];
-        const int nsl = a.grpp_sl_n[g];
-        int lam_max = 0;
-        for (int p = 0; p < nsl; p++) lam_max = max(lam_max, a.pot_L[a.sl_pot[a.grpp_sl_off[g] + p]] + l);
+        if (p >= a.grpp_sl_n[g]) continue;
+        const int *pots = a.sl_pot + a.grpp_sl_off[g];
+        const int L = a.pot_L[pots[p]], lam_max = L + l;
+        int64_t off = a.om_off[pr];
+        for (int q = 0; q < p; q++) off += om_size(a.pot_L[pots[q]], l);
         double k[3];
         const double al = a.prim_alpha[a.shell_prim_off[sx]];
         for (int d = 0; d < 3; d++) k[d] = -2.0 * (al * (a.centre_origin[3 * c + d] - a.shell_origin[3 * sx + d]));
@@ -289,7 +349,7 @@ __global__ void __launch_bounds__(kFinThreads) omega_tab_kernel(FinalArgs a, Fin
             const double inv = 1.0 / len;
             for (int d = 0; d < 3; d++) u[d] = k[d] * inv;
         }
-        __syncthreads();  // the previous pair's readers of upow, nabc and rsh are done
+        __syncthreads();  // the previous table's readers of upow, nabc and rsh are done
         if (tid < 3) {
             const double ud = tid == 0 ? u[0] : (tid == 1 ? u[1] : u[2]);
             double pw = 1.0;
@@ -299,20 +359,7 @@ __global__ void __launch_bounds__(kFinThreads) omega_tab_kernel(FinalArgs a, Fin
                 upow[tid][i] = pw;
             }
         }
-        for (int e = tid; e < n_abc(l); e += kFinThreads) {
-            int idx = e, aa, bb;
-            for (aa = 0; aa <= l; aa++) {
-                const int cnt = (l - aa + 1) * (l - aa + 2) / 2;
-                if (idx < cnt) break;
-                idx -= cnt;
-            }
-            for (bb = 0; bb <= l - aa; bb++) {
-                const int cnt = l - aa - bb + 1;
-                if (idx < cnt) break;
-                idx -= cnt;
-            }
-            nabc[e] = (int8_t)(aa + bb + idx);
-        }
+        for (int e = tid; e < n_abc(l); e += kFinThreads) nabc[e] = (int8_t)abc_degree(l, e);
         __syncthreads();
         const int nlm = (lam_max + 1) * (lam_max + 1);
         for (int e = tid; e < nlm; e += kFinThreads) {
@@ -328,51 +375,51 @@ __global__ void __launch_bounds__(kFinThreads) omega_tab_kernel(FinalArgs a, Fin
             rsh[ll * rs + mu + ll] = v;
         }
         __syncthreads();
-        int64_t off = a.om_off[pr];
-        for (int p = 0; p < nsl; p++) {
-            const int L = a.pot_L[a.sl_pot[a.grpp_sl_off[g] + p]];
-            const int sl = lam_slots(L, l), nab = n_abc(l), nm = 2 * L + 1, nmu = 2 * (L + l) + 1;
-            const double *At = a.atab + a.atab_off[L * (kMaxL + 2) + l];
-            for (int e = tid; e < nab * sl * nm; e += kFinThreads) {
-                const int m = e % nm, slot = (e / nm) % sl, abc = e / (nm * sl);
-                const int n = nabc[abc];
-                double w = 0.0;
-                if (slot < lam_count(L, n)) {
-                    const int lam = lam_lo(L, n) + 2 * slot;
-                    const double *S = rsh + lam * rs;
-                    const double *Ap = At + ((int64_t)(abc * sl + slot) * nmu) * nm + m;
-                    for (int mu = -lam; mu <= lam; mu++) {
-                        const double rv = S[mu + lam];
-                        if (fabs(rv) < kZeroThresh) continue;
-                        w += Ap[(int64_t)(mu + lam) * nm] * rv;
-                    }
-                }
-                omtab[off + e] = w;
-            }
-            off += (int64_t)nab * sl * nm;
+        const int sl = lam_slots(L, l), nab = n_abc(l), nm = 2 * L + 1, nmu = 2 * (L + l) + 1, row = om_row(L), st = om_stride(L, l);
+        const double *At = a.atab + a.atab_off[L * (kMaxL + 2) + l];
+        for (int e = tid; e < nab * sl * row; e += kFinThreads) {
+            const int m = e % row, slot = (e / row) % sl, abc = e / (row * sl);
+            omtab[off + abc * st + slot * row + m] = m < nm ? omega_value(L, nabc[abc], slot, m, sl, nmu, nm, abc, At, rsh, rs) : 0.0;
         }
     }
 }
 
+// The assembly of one task per block: T1 + sum type 2 + sum 2/(2L+1) SO + outercore.
+//
+// The sums that cancel (V and the term-by-term re-centring) keep libgrpp's operands and order; how
+// they are shared out does not matter to them:
+//  * V: a thread forms kFinTile rows abc of one |abc| at one def, lanes over def sorted by |def|,
+//    so that the loops over (l1, l2) are those of the whole warp, the radial value is read once
+//    per kFinTile entries and omega_A is a broadcast; omega rows are padded to 16-byte units with
+//    an odd stride (om_stride): no bank conflicts. Values of omega_A below libgrpp's skip threshold
+//    are zeroed when they are loaded, which adds exact zeros in place of the skip.
+//  * spin-orbit: each (m1, m2) pair has one non-zero L matrix component; the pairs come from a host
+//    table per component, in libgrpp's order.
+//  * re-centring: the binomial terms of every component of both shells are listed once per task
+//    (a factor and packed exponents), not per potential, row and element.
+//  * outercore: products with the L matrices come from oc_proj_kernel.
+// Bound by FP64 and shared-memory loads of V on high l, by the latency of a task's phases on low l.
+// The matrices of a 15-atom molecule (l <= 6, projectors l <= 5, spin-orbit): 49.1 -> 14.8 ms; the
+// derivative blocks of a 6-atom gradient 23.8 -> 4.7; 65536 s..g tasks 13.9 -> 7.3; a 200-task
+// molecule 1.00 -> 0.27.
 template <int NT>
-__global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
+__global__ void __launch_bounds__(NT, NT == 128 ? 5 : (NT == 256 ? 3 : 1)) final_kernel(FinalArgs a, FinalSmem sm)
 {
     constexpr int EPT = kFinMaxPairs / NT;  // Cartesian pairs per thread
-    extern __shared__ double dsm[];
+    extern __shared__ __align__(16) double dsm[];
     __shared__ double powA[3][kMaxL + 2], powB[3][kMaxL + 2];
     __shared__ double sCA[3], sCB[3];
     // powers u^0..u^lam of the unit vectors along kA, kB: [side][axis][power], each the same
     // chain of products 1 * u * u ... as the reference's per-term loops
     __shared__ double upow[2][3][kFinMaxLam + 1];
     __shared__ int8_t nabcA[n_abc(kMaxL)], nabcB[n_abc(kMaxL)];  // |abc| of each abc index
-    // spin-orbit: the (m1, m2) pairs, in m1-major order, at which some L matrix component is
-    // non-zero (spin_orbit_integrals.c:206-222 skips the others), with the three values
-    __shared__ int8_t lpm1[kLmatPairs], lpm2[kLmatPairs];
-    __shared__ double lpv[3][kLmatPairs];
-    __shared__ int s_npair;
+    __shared__ int16_t ordA[n_abc(kMaxL)], ordB[n_abc(kMaxL)];   // abc indices by |abc|, ascending within one
+    __shared__ int begA[kMaxL + 2];                              // first of each |abc| in ordA
+    __shared__ int tile_lo[kMaxL + 1], tile_n[kMaxL + 1], tile_first[kMaxL + 2];  // of a chunk of V's rows
+    __shared__ int offLA[kFinMaxCart + 1], offLB[kFinMaxCart + 1];  // binomial terms of each component
+    __shared__ int ocL[kFinMaxOc], ocJ[kFinMaxOc];
     const int tid = threadIdx.x;
-    double *rshA = dsm, *rshB = rshA + sm.n_rsh, *omA = rshB + sm.n_rsh, *omB = omA + sm.n_omega, *Qs = omB + sm.n_omega,
-           *V = Qs + sm.n_q;
+    double *rshA = dsm, *rshB = rshA + sm.n_rsh, *V = rshB + sm.n_rsh, *W = V + sm.n_v, *tab = W + ((sm.n_w + 1) & ~1);
     const int rs = sm.rsh_stride;
 
     __shared__ int s_next;
@@ -395,6 +442,7 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
         }
         const int sa = a.task_a[t], sb = a.task_b[t], c = a.task_c[t];
         const int la = a.shell_L[sa], lb = a.shell_L[sb], nA = ncart(la), nB = ncart(lb), nel = nA * nB;
+        const int nabA = n_abc(la), nabB = n_abc(lb);
         const int8_t *cA = a.cart + 3 * a.shell_cart_off[sa], *cB = a.cart + 3 * a.shell_cart_off[sb];
         const int g = a.centre_grpp[c];
         const int64_t oo = a.task_out_off[t];
@@ -404,12 +452,15 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
             sCB[tid] = a.centre_origin[3 * c + tid] - a.shell_origin[3 * sb + tid];
         }
         __syncthreads();
-        if (tid < 3) {
-            for (int k = 0; k <= la; k++) powA[tid][k] = pow(sCA[tid], k);
-            for (int k = 0; k <= lb; k++) powB[tid][k] = pow(sCB[tid], k);
+        if (tid < 3 * (kMaxL + 1)) {
+            const int d = tid % 3, k = tid / 3;
+            if (k <= la) powA[d][k] = pow(sCA[d], k);
+            if (k <= lb) powB[d][k] = pow(sCB[d], k);
         }
         double acc[4][EPT];
-#pragma unroll
+        // indexed in loops that are not unrolled (local memory): a copy of the loop bodies per element
+        // took 250 registers and one block per SM
+#pragma unroll 1
         for (int q = 0; q < EPT; q++) {
             const int e = tid + q * NT;
             acc[0][q] = (e < nel && a.task_has_ul[t]) ? a.arep[oo + e] : 0.0;
@@ -418,38 +469,61 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
 
         const int nsl = a.grpp_sl_n[g];
         if (nsl > 0 && a.task_q_off[t] >= 0) {
-            int lam_max = 0;
+            const int *pots = a.sl_pot + a.grpp_sl_off[g];
+            const bool omt = a.omtab != nullptr;
+            int lam_max = 0, n_om = 0, n_q = 0;
             for (int p = 0; p < nsl; p++) {
-                const int Lp = a.pot_L[a.sl_pot[a.grpp_sl_off[g] + p]];
+                const int Lp = a.pot_L[pots[p]];
                 lam_max = max(lam_max, Lp + max(la, lb));
+                n_om = max(n_om, om_size(Lp, la) + om_size(Lp, lb));
+                n_q = max(n_q, (Lp + la + 1) * (Lp + lb + 1) * (la + lb + 1));
             }
-            double kA[3], kB[3];
-            const double alA = a.prim_alpha[a.shell_prim_off[sa]], alB = a.prim_alpha[a.shell_prim_off[sb]];
-            for (int d = 0; d < 3; d++) {
-                kA[d] = -2.0 * (alA * (a.centre_origin[3 * c + d] - a.shell_origin[3 * sa + d]));
-                kB[d] = -2.0 * (alB * (a.centre_origin[3 * c + d] - a.shell_origin[3 * sb + d]));
+            double *Qs = tab + n_om, *FA = Qs + ((n_q + 1) & ~1);
+            for (int e = tid; e < nabA + nabB; e += NT) {
+                if (e < nabA) nabcA[e] = (int8_t)abc_degree(la, e);
+                else nabcB[e - nabA] = (int8_t)abc_degree(lb, e - nabA);
+            }
+            // first binomial term of each component
+            for (int e = tid; e < nA + nB + 2; e += NT) {
+                if (e <= nA) offLA[e] = fin_terms(cA, e);
+                else offLB[e - nA - 1] = fin_terms(cB, e - nA - 1);
             }
             __syncthreads();
-            // RSH values with stride rs (rsh_values uses 2*kFinMaxLam+1; use a local variant)
-            const bool omt = a.omtab != nullptr;
-            if (omt) {  // only the |abc| tables are needed: omega comes from the pair tables
-                for (int e = tid; e < n_abc(la) + n_abc(lb); e += NT) {
-                    const bool sideB = e >= n_abc(la);
-                    const int l = sideB ? lb : la;
-                    int idx = sideB ? e - n_abc(la) : e, aa, bb;
-                    for (aa = 0; aa <= l; aa++) {
-                        const int cnt = (l - aa + 1) * (l - aa + 2) / 2;
-                        if (idx < cnt) break;
-                        idx -= cnt;
-                    }
-                    for (bb = 0; bb <= l - aa; bb++) {
-                        const int cnt = l - aa - bb + 1;
-                        if (idx < cnt) break;
-                        idx -= cnt;
-                    }
-                    (sideB ? nabcB : nabcA)[sideB ? e - n_abc(la) : e] = (int8_t)(aa + bb + idx);
+            const int nLA = offLA[nA], nLB = offLB[nB];
+            double *FB = FA + nLA;
+            unsigned *IA = (unsigned *)(FB + nLB), *IB = IA + nLA;
+            // binomial terms, in libgrpp's loop order (a, b, c): four threads per component
+            for (int e = tid; e < 4 * (nA + nB); e += NT) {
+                const bool sideB = (e >> 2) >= nA;
+                const int i = sideB ? (e >> 2) - nA : e >> 2, l = sideB ? lb : la;
+                const int8_t *cc = (sideB ? cB : cA) + 3 * i;
+                const int x = cc[0], y = cc[1], z = cc[2], n = (x + 1) * (y + 1) * (z + 1), o = sideB ? offLB[i] : offLA[i];
+                const double(*pw)[kMaxL + 2] = sideB ? powB : powA;
+                for (int q = e & 3; q < n; q += 4) {
+                    const int aa = q / ((y + 1) * (z + 1)), r = q - aa * (y + 1) * (z + 1), bb = r / (z + 1), c3 = r - bb * (z + 1);
+                    const double bin = c_tab.binom[x * kBinN + aa] * c_tab.binom[y * kBinN + bb] * c_tab.binom[z * kBinN + c3];
+                    (sideB ? FB : FA)[o + q] = bin * pw[0][x - aa] * pw[1][y - bb] * pw[2][z - c3];
+                    (sideB ? IB : IA)[o + q] = fin_term(min(abc_index(l, aa, bb, c3), n_abc(l) - 1), (int)bin, x - aa, y - bb, z - c3);
                 }
-            } else {
+            }
+            // abc indices by degree: position = smaller degrees, then equal ones of smaller index
+            for (int e = tid; e < nabA + nabB; e += NT) {
+                const bool sideB = e >= nabA;
+                const int i = sideB ? e - nabA : e;
+                const int8_t *nn = sideB ? nabcB : nabcA;
+                const int n = nn[i];
+                int pos = n > 0 ? n_abc(n - 1) : 0;  // abc of degree < n: as many as n_abc(n - 1)
+                for (int q = 0; q < i; q++) pos += nn[q] == n;
+                (sideB ? ordB : ordA)[pos] = (int16_t)i;
+            }
+            if (tid <= la + 1) begA[tid] = tid > 0 ? n_abc(tid - 1) : 0;
+            if (!omt) {
+                double kA[3], kB[3];
+                const double alA = a.prim_alpha[a.shell_prim_off[sa]], alB = a.prim_alpha[a.shell_prim_off[sb]];
+                for (int d = 0; d < 3; d++) {
+                    kA[d] = -2.0 * (alA * (a.centre_origin[3 * c + d] - a.shell_origin[3 * sa + d]));
+                    kB[d] = -2.0 * (alB * (a.centre_origin[3 * c + d] - a.shell_origin[3 * sb + d]));
+                }
                 const double lenA = sqrt(kA[0] * kA[0] + kA[1] * kA[1] + kA[2] * kA[2]);
                 const double lenB = sqrt(kB[0] * kB[0] + kB[1] * kB[1] + kB[2] * kB[2]);
                 double uA[3] = {0, 0, 0}, uB[3] = {0, 0, 0};
@@ -471,22 +545,6 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                         pw *= ud;
                         upow[side][d][i] = pw;
                     }
-                }
-                for (int e = tid; e < n_abc(la) + n_abc(lb); e += NT) {
-                    const bool sideB = e >= n_abc(la);
-                    const int l = sideB ? lb : la;
-                    int idx = sideB ? e - n_abc(la) : e, aa, bb;
-                    for (aa = 0; aa <= l; aa++) {
-                        const int cnt = (l - aa + 1) * (l - aa + 2) / 2;
-                        if (idx < cnt) break;
-                        idx -= cnt;
-                    }
-                    for (bb = 0; bb <= l - aa; bb++) {
-                        const int cnt = l - aa - bb + 1;
-                        if (idx < cnt) break;
-                        idx -= cnt;
-                    }
-                    (sideB ? nabcB : nabcA)[sideB ? e - n_abc(la) : e] = (int8_t)(aa + bb + idx);
                 }
                 __syncthreads();
                 // (l, mu) pairs e = l^2 + l + mu of both sides
@@ -527,118 +585,140 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
             int64_t omoA = omt ? a.om_off[a.task_fpa[t]] : 0, omoB = omt ? a.om_off[a.task_fpb[t]] : 0;
             const int n_arep = a.grpp_n_arep[g];
             for (int p = 0; p < nsl; p++) {
-                const int L = a.pot_L[a.sl_pot[a.grpp_sl_off[g] + p]];
+                const int L = a.pot_L[pots[p]];
                 const bool so = p >= n_arep;
-                const int d1 = L + la + 1, d2 = L + lb + 1, dn = la + lb + 1, nm = 2 * L + 1;
+                const int d1 = L + la + 1, d2 = L + lb + 1, dn = la + lb + 1, nm = 2 * L + 1, row = om_row(L);
                 const int slA = lam_slots(L, la), slB = lam_slots(L, lb);
-                const int nabA = n_abc(la), nabB = n_abc(lb);
-                const int nmuA = 2 * (L + la) + 1, nmuB = 2 * (L + lb) + 1;
-                const double *AtA = a.atab + a.atab_off[L * (kMaxL + 2) + la];
-                const double *AtB = a.atab + a.atab_off[L * (kMaxL + 2) + lb];
+                const int stA = om_stride(L, la), stB = om_stride(L, lb);
+                const double thrF = so ? kZeroThresh : 1e-13, thrQ = so ? kZeroThresh : 1e-16, thrW = so ? kZeroThresh : 1e-16;
+                double *omA = tab, *omB = omA + nabA * stA;
                 __syncthreads();
-                // omega tables: omega[abc][slot][m] = sum_mu S_{lam mu} Atab (angular_integrals.c:78-108)
                 if (omt) {
-                    for (int e = tid; e < nabA * slA * nm; e += NT) omA[e] = a.omtab[omoA + e];
-                    for (int e = tid; e < nabB * slB * nm; e += NT) omB[e] = a.omtab[omoB + e];
-                    omoA += nabA * slA * nm;
-                    omoB += nabB * slB * nm;
-                }
-                for (int e = tid; !omt && e < nabA * slA * nm + nabB * slB * nm; e += NT) {
-                    const bool sideB = e >= nabA * slA * nm;
-                    const int r = sideB ? e - nabA * slA * nm : e;
-                    const int sl = sideB ? slB : slA, nab = sideB ? nabB : nabA, l = sideB ? lb : la;
-                    const int m = r % nm, slot = (r / nm) % sl, abc = r / (nm * sl);
-                    (void)nab;
-                    (void)l;
-                    const int n = sideB ? nabcB[abc] : nabcA[abc];
-                    double w = 0.0;
-                    if (slot < lam_count(L, n)) {
-                        const int lam = lam_lo(L, n) + 2 * slot;
-                        const double *S = (sideB ? rshB : rshA) + lam * rs;
-                        const double *At = (sideB ? AtB : AtA) + ((int64_t)(abc * sl + slot) * (sideB ? nmuB : nmuA)) * nm + m;
-                        for (int mu = -lam; mu <= lam; mu++) {
-                            const double rv = S[mu + lam];
-                            if (fabs(rv) < kZeroThresh) continue;
-                            w += At[(int64_t)(mu + lam) * nm] * rv;
-                        }
+                    const double2 *gA = (const double2 *)(a.omtab + omoA), *gB = (const double2 *)(a.omtab + omoB);
+                    for (int e = tid; e < nabA * stA / 2; e += NT) {
+                        double2 v = __ldg(gA + e);
+                        if (fabs(v.x) < thrW) v.x = 0.0;
+                        if (fabs(v.y) < thrW) v.y = 0.0;
+                        ((double2 *)omA)[e] = v;
                     }
-                    (sideB ? omB : omA)[r] = w;
+                    for (int e = tid; e < nabB * stB / 2; e += NT) ((double2 *)omB)[e] = __ldg(gB + e);
+                    omoA += nabA * stA;
+                    omoB += nabB * stB;
+                } else {
+                    const double *AtA = a.atab + a.atab_off[L * (kMaxL + 2) + la];
+                    const double *AtB = a.atab + a.atab_off[L * (kMaxL + 2) + lb];
+                    for (int e = tid; e < (nabA * slA + nabB * slB) * row; e += NT) {
+                        const bool sideB = e >= nabA * slA * row;
+                        const int r = sideB ? e - nabA * slA * row : e, sl = sideB ? slB : slA;
+                        const int m = r % row, slot = (r / row) % sl, abc = r / (row * sl);
+                        double w = 0.0;
+                        if (m < nm)
+                            w = omega_value(L, sideB ? nabcB[abc] : nabcA[abc], slot, m, sl, 2 * (L + (sideB ? lb : la)) + 1, nm, abc,
+                                            sideB ? AtB : AtA, sideB ? rshB : rshA, rs);
+                        if (!sideB && fabs(w) < thrW) w = 0.0;
+                        (sideB ? omB + abc * stB : omA + abc * stA)[slot * row + m] = w;
+                    }
                 }
                 for (int e = tid; e < d1 * d2 * dn; e += NT) Qs[e] = a.Q[qbase + qoff + e];
                 qoff += (int64_t)d1 * d2 * dn;
-                if (so && tid == 0) {
-                    int np = 0;
-                    for (int m1 = -L; m1 <= L; m1++)
-                        for (int m2 = -L; m2 <= L; m2++) {
-                            const double lx = lmat_val(L, 0, m1, m2), ly = lmat_val(L, 1, m1, m2), lz = lmat_val(L, 2, m1, m2);
-                            if (fabs(lx) < kZeroThresh && fabs(ly) < kZeroThresh && fabs(lz) < kZeroThresh) continue;
-                            if (np < kLmatPairs) {
-                                lpm1[np] = (int8_t)(m1 + L);
-                                lpm2[np] = (int8_t)(m2 + L);
-                                lpv[0][np] = lx;
-                                lpv[1][np] = ly;
-                                lpv[2][np] = lz;
-                            }
-                            np++;
-                        }
-                    s_npair = np;  // never above kLmatPairs for L <= 10 (10L - 4 pairs)
-                }
-                __syncthreads();
 
-                const int ncomp = so ? 3 : 1;
-                const double thrF = so ? kZeroThresh : 1e-13, thrQ = so ? kZeroThresh : 1e-16, thrW = so ? kZeroThresh : 1e-16;
-                const int rows = max(1, min(nabA, sm.n_v / (nabB * ncomp)));
+                const int ncomp = so ? 3 : 1, vrow = fin_v_row(nabB, ncomp);
+                const int rows = fin_v_rows(sm.n_v, nabA, nabB, ncomp);
                 double gam[3][EPT];
-#pragma unroll
+#pragma unroll 1
                 for (int q = 0; q < EPT; q++) gam[0][q] = gam[1][q] = gam[2][q] = 0.0;
 
                 for (int r0 = 0; r0 < nabA; r0 += rows) {
-                    const int r1 = min(nabA, r0 + rows);
+                    const int r1 = min(nabA, r0 + rows), nrow = r1 - r0;
+                    __syncthreads();  // the tables are loaded; the previous chunk's V and W are consumed
+                    // tiles of kFinTile rows of equal |abc| within the chunk
+                    if (tid <= la) {
+                        int lo = begA[tid], hi = begA[tid + 1];
+                        while (lo < hi && ordA[lo] < r0) lo++;
+                        while (hi > lo && ordA[hi - 1] >= r1) hi--;
+                        tile_lo[tid] = lo;
+                        tile_n[tid] = hi - lo;
+                    }
+                    __syncthreads();
+                    if (tid == 0) {
+                        int f = 0;
+                        for (int n = 0; n <= la; n++) {
+                            tile_first[n] = f;
+                            f += (tile_n[n] + kFinTile - 1) / kFinTile;
+                        }
+                        tile_first[la + 1] = f;
+                    }
                     __syncthreads();
                     // V[abc][def] (type2_integrals.c:174-196, spin_orbit_integrals.c:197-224)
-                    for (int e = tid; e < (r1 - r0) * nabB; e += NT) {
-                        const int abc = r0 + e / nabB, def = e % nabB;
-                        const int n1 = nabcA[abc], n2 = nabcB[def], N = n1 + n2;
-                        double v0 = 0.0, v1 = 0.0, v2 = 0.0;
-                        const int c1 = lam_count(L, n1), c2 = lam_count(L, n2);
-                        for (int s1 = 0; s1 < c1; s1++) {
-                            const int l1 = lam_lo(L, n1) + 2 * s1;
-                            const double *w1 = omA + (abc * slA + s1) * nm;
-                            for (int s2 = 0; s2 < c2; s2++) {
-                                const int l2 = lam_lo(L, n2) + 2 * s2;
-                                const double QN = Qs[(l1 * d2 + l2) * dn + N];
-                                if (fabs(QN) < thrQ) continue;
-                                const double *w2 = omB + (def * slB + s2) * nm;
-                                if (!so) {
-                                    double sa2 = 0.0;
-                                    for (int m = 0; m < nm; m++) {
-                                        if (fabs(w1[m]) < thrW) continue;
-                                        sa2 += w1[m] * w2[m];
+                    for (int e = tid; e < tile_first[la + 1] * nabB; e += NT) {
+                        const int tile = e / nabB, def = ordB[e - tile * nabB];
+                        int n1 = 0;
+                        while (tile_first[n1 + 1] <= tile) n1++;
+                        const int first = (tile - tile_first[n1]) * kFinTile, cnt = min(kFinTile, tile_n[n1] - first);
+                        const int n2 = nabcB[def], N = n1 + n2, c1 = lam_count(L, n1), c2 = lam_count(L, n2);
+                        int ab[kFinTile];
+#pragma unroll
+                        for (int q = 0; q < kFinTile; q++) ab[q] = ordA[tile_lo[n1] + first + min(q, cnt - 1)];
+                        const double *w2b = omB + def * stB;
+                        const double *Qp = Qs + (lam_lo(L, n1) * d2 + lam_lo(L, n2)) * dn + N;
+                        if (!so) {
+                            double v[kFinTile];
+#pragma unroll
+                            for (int q = 0; q < kFinTile; q++) v[q] = 0.0;
+                            for (int s1 = 0; s1 < c1; s1++)
+                                for (int s2 = 0; s2 < c2; s2++) {
+                                    const double QN = Qp[(2 * s1 * d2 + 2 * s2) * dn];
+                                    if (fabs(QN) < thrQ) continue;
+                                    const double2 *w2 = (const double2 *)(w2b + s2 * row);
+                                    double sa2[kFinTile];
+#pragma unroll
+                                    for (int q = 0; q < kFinTile; q++) sa2[q] = 0.0;
+                                    for (int m = 0; m <= L; m++) {
+                                        const double2 y = w2[m];
+#pragma unroll
+                                        for (int q = 0; q < kFinTile; q++) {
+                                            const double2 x = ((const double2 *)(omA + ab[q] * stA + s1 * row))[m];
+                                            sa2[q] += x.x * y.x;
+                                            sa2[q] += x.y * y.y;
+                                        }
                                     }
-                                    v0 += QN * sa2;
-                                } else {
-                                    // the non-zero (m1, m2) pairs in the reference's loop order: the same terms,
-                                    // added in the same order, as the dense double loop with its skip
-                                    double sx = 0.0, sy = 0.0, sz = 0.0;
-                                    const int npair = min(s_npair, kLmatPairs);
-                                    for (int q = 0; q < npair; q++) {
-                                        const double o1 = w1[lpm1[q]];
-                                        if (fabs(o1) < kZeroThresh) continue;
-                                        const double o2 = w2[lpm2[q]];
-                                        sx += o1 * o2 * lpv[0][q];
-                                        sy += o1 * o2 * lpv[1][q];
-                                        sz += o1 * o2 * lpv[2][q];
-                                    }
-                                    v0 += QN * sx;
-                                    v1 += QN * sy;
-                                    v2 += QN * sz;
+#pragma unroll
+                                    for (int q = 0; q < kFinTile; q++) v[q] += QN * sa2[q];
                                 }
+#pragma unroll
+                            for (int q = 0; q < kFinTile; q++)
+                                if (q < cnt) V[(ab[q] - r0) * vrow + def] = v[q];
+                        } else {
+                            // per component the non-zero (m1, m2) pairs in the reference's loop order: the same
+                            // terms, added in the same order, as the dense double loop with its skip
+                            const int *lp = c_tab.lpair_off + 4 * L;
+                            for (int comp = 0; comp < 3; comp++) {
+                                const int p0 = __ldg(lp + comp), p1 = __ldg(lp + comp + 1);
+                                double v[kFinTile];
+#pragma unroll
+                                for (int q = 0; q < kFinTile; q++) v[q] = 0.0;
+                                for (int s1 = 0; s1 < c1; s1++)
+                                    for (int s2 = 0; s2 < c2; s2++) {
+                                        const double QN = Qp[(2 * s1 * d2 + 2 * s2) * dn];
+                                        if (fabs(QN) < thrQ) continue;
+                                        const double *w2 = w2b + s2 * row;
+                                        double sx[kFinTile];
+#pragma unroll
+                                        for (int q = 0; q < kFinTile; q++) sx[q] = 0.0;
+                                        for (int k = p0; k < p1; k++) {
+                                            const int mm = __ldg(c_tab.lpair_m + k);
+                                            const double lv = __ldg(c_tab.lpair_v + k), o2 = w2[mm >> 8];
+                                            const int o1 = s1 * row + (mm & 255);
+#pragma unroll
+                                            for (int q = 0; q < kFinTile; q++) sx[q] += omA[ab[q] * stA + o1] * o2 * lv;
+                                        }
+#pragma unroll
+                                        for (int q = 0; q < kFinTile; q++) v[q] += QN * sx[q];
+                                    }
+#pragma unroll
+                                for (int q = 0; q < kFinTile; q++)
+                                    if (q < cnt) V[(ab[q] - r0) * vrow + def * 3 + comp] = v[q];
                             }
-                        }
-                        V[e * ncomp] = v0;
-                        if (so) {
-                            V[e * ncomp + 1] = v1;
-                            V[e * ncomp + 2] = v2;
                         }
                     }
                     __syncthreads();
@@ -646,66 +726,57 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                     unsigned tbt = fact ? 0u : ~0u;
                     if (fact) {
                         // W[j][abc] = sum_def F_B V[abc][def] and Wa[j][abc] = sum_def |F_B| max_c |V[abc][def]|
-                        double *W = V + sm.n_v;
-                        const int nrow = r1 - r0;
-                        double *Wa = W + nB * nrow * ncomp;
+                        const int wrow = (nrow * ncomp) | 1, arow = nrow | 1;
+                        double *Wa = W + nB * wrow;
                         for (int e = tid; e < nB * nrow; e += NT) {
-                            const int j = e / nrow, ar = e % nrow;
-                            const int bx = cB[3 * j], by = cB[3 * j + 1], bz = cB[3 * j + 2];
+                            const int j = e / nrow, ar = e - j * nrow;
+                            const double *vr = V + ar * vrow;
                             double w0 = 0.0, w1 = 0.0, w2 = 0.0, wa = 0.0;
-                            for (int dd = 0; dd <= bx; dd++)
-                                for (int ee = 0; ee <= by; ee++)
-                                    for (int ff = 0; ff <= bz; ff++) {
-                                        const double fb = c_tab.binom[bx * kBinN + dd] * c_tab.binom[by * kBinN + ee] *
-                                                          c_tab.binom[bz * kBinN + ff] * powB[0][bx - dd] * powB[1][by - ee] *
-                                                          powB[2][bz - ff];
-                                        if (fb == 0.0) continue;
-                                        const double *vv = V + (ar * nabB + abc_index(lb, dd, ee, ff)) * ncomp;
-                                        w0 += fb * vv[0];
-                                        double vm = fabs(vv[0]);
-                                        if (so) {
-                                            w1 += fb * vv[1];
-                                            w2 += fb * vv[2];
-                                            vm = fmax(vm, fmax(fabs(vv[1]), fabs(vv[2])));
-                                        }
-                                        wa += fabs(fb) * vm;
-                                    }
-                            double *ww = W + (j * nrow + ar) * ncomp;
+                            const int k1 = offLB[j + 1];
+                            for (int k = offLB[j]; k < k1; k++) {
+                                const double fb = FB[k];
+                                const double *vv = vr + (IB[k] & 511) * ncomp;
+                                const double x = vv[0];
+                                w0 += fb * x;
+                                double vm = fabs(x);
+                                if (so) {
+                                    const double y = vv[1], z = vv[2];
+                                    w1 += fb * y;
+                                    w2 += fb * z;
+                                    vm = fmax(vm, fmax(fabs(y), fabs(z)));
+                                }
+                                wa += fabs(fb) * vm;
+                            }
+                            double *ww = W + j * wrow + ar * ncomp;
                             ww[0] = w0;
                             if (so) {
                                 ww[1] = w1;
                                 ww[2] = w2;
                             }
-                            Wa[j * nrow + ar] = wa;
+                            Wa[j * arow + ar] = wa;
                         }
                         __syncthreads();
-#pragma unroll
+#pragma unroll 1
                         for (int q = 0; q < EPT; q++) {
                             const int el = tid + q * NT;
                             if (el >= nel) continue;
-                            const int i = el / nB, j = el % nB;
-                            const int ax = cA[3 * i], ay = cA[3 * i + 1], az = cA[3 * i + 2];
-                            const int bx = cB[3 * j], by = cB[3 * j + 1], bz = cB[3 * j + 2];
+                            const int i = el / nB, j = el - i * nB;
                             double g0 = 0.0, g1 = 0.0, g2 = 0.0, ga = 0.0;
                             int nta = 0;
-                            for (int aa = 0; aa <= ax; aa++)
-                                for (int bb = 0; bb <= ay; bb++)
-                                    for (int cc = 0; cc <= az; cc++) {
-                                        const int abc = abc_index(la, aa, bb, cc);
-                                        if (abc < r0 || abc >= r1) continue;
-                                        const double fa = c_tab.binom[ax * kBinN + aa] * c_tab.binom[ay * kBinN + bb] *
-                                                          c_tab.binom[az * kBinN + cc] * powA[0][ax - aa] * powA[1][ay - bb] *
-                                                          powA[2][az - cc];
-                                        if (fa == 0.0) continue;
-                                        nta++;
-                                        const double *ww = W + (j * nrow + abc - r0) * ncomp;
-                                        g0 += fa * ww[0];
-                                        if (so) {
-                                            g1 += fa * ww[1];
-                                            g2 += fa * ww[2];
-                                        }
-                                        ga += fabs(fa) * Wa[j * nrow + abc - r0];
-                                    }
+                            const int k1 = offLA[i + 1];
+                            for (int k = offLA[i]; k < k1; k++) {
+                                const int ar = (int)(IA[k] & 511) - r0;
+                                const double fa = FA[k];
+                                if (ar < 0 || ar >= nrow || fa == 0.0) continue;
+                                nta++;
+                                const double *ww = W + j * wrow + ar * ncomp;
+                                g0 += fa * ww[0];
+                                if (so) {
+                                    g1 += fa * ww[1];
+                                    g2 += fa * ww[2];
+                                }
+                                ga += fabs(fa) * Wa[j * arow + ar];
+                            }
                             // Both this sum and libgrpp's term-by-term sum of the same terms are within
                             // (n + 12) u sum|terms| of the exact value, n = the number of terms and 12 u the
                             // rounding of a term's factors; the two differ by at most twice that. The
@@ -713,7 +784,7 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                             // 1e-11 absolute or 1e-10 of the partial sum itself (a tenth of the 1e-10 / 1e-9
                             // comparator); otherwise, where the re-centring sum cancels, the element is summed
                             // term by term in libgrpp's order.
-                            const double nterm = (double)nta * (double)((bx + 1) * (by + 1) * (bz + 1));
+                            const double nterm = (double)nta * (double)(offLB[j + 1] - offLB[j]);
                             const double bound = 2.0 * (nterm + 12.0) * 1.1102230246251565e-16 * ga * (16 * kPi * kPi);
                             const double gmax = fmax(fabs(g0), fmax(fabs(g1), fabs(g2)));
                             if (bound <= fmax(1e-11, 1e-10 * gmax * (16 * kPi * kPi))) {
@@ -726,38 +797,33 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                         }
                     }
                     // Cartesian pairs: binomial re-centring sums over (a..f) in the reference's loop order
-#pragma unroll
+                    // (a factor is the exact product of six binomials times six powers, left to right)
+#pragma unroll 1
                     for (int q = 0; q < EPT; q++) {
                         const int el = tid + q * NT;
                         if (el >= nel || !((tbt >> q) & 1u)) continue;
-                        const int i = el / nB, j = el % nB;
-                        const int ax = cA[3 * i], ay = cA[3 * i + 1], az = cA[3 * i + 2];
-                        const int bx = cB[3 * j], by = cB[3 * j + 1], bz = cB[3 * j + 2];
+                        const int i = el / nB, j = el - i * nB;
                         double g0 = gam[0][q], g1 = gam[1][q], g2 = gam[2][q];
-                        for (int aa = 0; aa <= ax; aa++)
-                            for (int bb = 0; bb <= ay; bb++)
-                                for (int cc = 0; cc <= az; cc++) {
-                                    const int abc = abc_index(la, aa, bb, cc);
-                                    if (abc < r0 || abc >= r1) continue;
-                                    const double cabc = c_tab.binom[ax * kBinN + aa] * c_tab.binom[ay * kBinN + bb] *
-                                                        c_tab.binom[az * kBinN + cc];
-                                    for (int dd = 0; dd <= bx; dd++)
-                                        for (int ee = 0; ee <= by; ee++)
-                                            for (int ff = 0; ff <= bz; ff++) {
-                                                const double f = cabc * c_tab.binom[bx * kBinN + dd] * c_tab.binom[by * kBinN + ee] *
-                                                                 c_tab.binom[bz * kBinN + ff] * powA[0][ax - aa] * powA[1][ay - bb] *
-                                                                 powA[2][az - cc] * powB[0][bx - dd] * powB[1][by - ee] *
-                                                                 powB[2][bz - ff];
-                                                if (fabs(f) < thrF) continue;
-                                                const int def = abc_index(lb, dd, ee, ff);
-                                                const double *vv = V + ((abc - r0) * nabB + def) * ncomp;
-                                                g0 += f * vv[0];
-                                                if (so) {
-                                                    g1 += f * vv[1];
-                                                    g2 += f * vv[2];
-                                                }
-                                            }
+                        const int k1 = offLA[i + 1], b0 = offLB[j], b1 = offLB[j + 1];
+                        for (int k = offLA[i]; k < k1; k++) {
+                            const unsigned ta = IA[k];
+                            const int ar = (int)(ta & 511) - r0, ca = (ta >> 9) & 255;
+                            if (ar < 0 || ar >= nrow) continue;
+                            const double a0 = powA[0][(ta >> 17) & 15], a1 = powA[1][(ta >> 21) & 15], a2 = powA[2][ta >> 25];
+                            const double *vr = V + ar * vrow;
+                            for (int kb = b0; kb < b1; kb++) {
+                                const unsigned tb = IB[kb];
+                                const double f = (double)(ca * (int)((tb >> 9) & 255)) * a0 * a1 * a2 * powB[0][(tb >> 17) & 15] *
+                                                 powB[1][(tb >> 21) & 15] * powB[2][tb >> 25];
+                                if (fabs(f) < thrF) continue;
+                                const double *vv = vr + (tb & 511) * ncomp;
+                                g0 += f * vv[0];
+                                if (so) {
+                                    g1 += f * vv[1];
+                                    g2 += f * vv[2];
                                 }
+                            }
+                        }
                         gam[0][q] = g0;
                         gam[1][q] = g1;
                         gam[2][q] = g2;
@@ -765,7 +831,7 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                 }
                 const double pi16 = 16 * kPi * kPi;
                 const double fso = a.raw_so ? 1.0 : 2.0 / (2 * L + 1);
-#pragma unroll
+#pragma unroll 1
                 for (int q = 0; q < EPT; q++) {
                     if (!so) {
                         acc[0][q] += 1.0 * (gam[0][q] * pi16);
@@ -784,19 +850,25 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
             const int64_t pa = a.proj_off[a.task_proj_a[t]], pb = a.proj_off[a.task_proj_b[t]];
             const int ocoff = a.grpp_oc_off[g];
             const double *dl = a.oc_delta + a.grpp_delta_off[g];
-#pragma unroll
+            __syncthreads();
+            if (tid < noc) {
+                ocL[tid] = a.oc_L[ocoff + tid];
+                ocJ[tid] = a.oc_J[ocoff + tid];
+            }
+            __syncthreads();
+#pragma unroll 1
             for (int q = 0; q < EPT; q++) {
                 const int el = tid + q * NT;
                 if (el >= nel) continue;
                 const int i = el / nB, j = el % nB;
-                double oa = 0.0, ox = 0.0, oy = 0.0, oz = 0.0;
+                double oa = 0.0, oso[3] = {0.0, 0.0, 0.0};
                 // part 1
                 int64_t offA = pa, offB = pb;
                 for (int k = 0; k < noc; k++) {
-                    const int L = a.oc_L[ocoff + k], d = 2 * L + 1;
-                    const double J = a.oc_J[ocoff + k] / 2.0;
-                    const double *SA = a.S_sph + offA + i * d, *UA = a.U_sph + offA + i * d;
-                    const double *SB = a.S_sph + offB + j * d, *UB = a.U_sph + offB + j * d;
+                    const int L = ocL[k], d = 2 * L + 1;
+                    const double J = ocJ[k] / 2.0;
+                    const int64_t rA = offA + i * d, rB = offB + j * d;
+                    const double *SA = a.S_sph + rA, *UA = a.U_sph + rA, *SB = a.S_sph + rB, *UB = a.U_sph + rB;
                     const double farep = (J < L) ? (L / (2.0 * L + 1)) : ((L + 1) / (2.0 * L + 1));
                     const double fso = (J < L) ? (-2.0 / (2 * L + 1)) : (+2.0 / (2 * L + 1));
                     double s1 = 0.0, s2 = 0.0;
@@ -806,29 +878,17 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                     buf += s1;
                     buf += s2;
                     oa += farep * buf;
-                    double *oso[3] = {&ox, &oy, &oz};
+#pragma unroll
                     for (int comp = 0; comp < 3; comp++) {
                         // so_buf = U_a (L S_b) + (S_a L) U_b
-                        double t1 = 0.0;
-                        for (int m1 = 0; m1 < d; m1++) {
-                            double tm = 0.0;
-                            for (int m2 = 0; m2 < d; m2++) tm += lmat_val(L, comp, m1 - L, m2 - L) * SB[m2];
-                            double tmp = 0.0;
-                            tmp += tm;
-                            t1 += UA[m1] * tmp;
-                        }
+                        const double *LSB = a.LS + comp * a.sph_tot + rB, *SLA = a.SL + comp * a.sph_tot + rA;
+                        double t1 = 0.0, t2 = 0.0;
+                        for (int m = 0; m < d; m++) t1 += UA[m] * LSB[m];
+                        for (int m = 0; m < d; m++) t2 += SLA[m] * UB[m];
                         double sob = 0.0;
                         sob += t1;
-                        double t2 = 0.0;
-                        for (int m = 0; m < d; m++) {
-                            double tm = 0.0;
-                            for (int k2 = 0; k2 < d; k2++) tm += SA[k2] * lmat_val(L, comp, k2 - L, m - L);
-                            double tmp = 0.0;
-                            tmp += tm;
-                            t2 += tmp * UB[m];
-                        }
                         sob += t2;
-                        *oso[comp] += fso * sob;
+                        oso[comp] += fso * sob;
                     }
                     offA += (int64_t)nA * d;
                     offB += (int64_t)nB * d;
@@ -836,36 +896,30 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                 // part 2
                 int64_t offA1 = pa;
                 for (int k1 = 0; k1 < noc; k1++) {
-                    const int L1 = a.oc_L[ocoff + k1], d = 2 * L1 + 1;
+                    const int L = ocL[k1], d = 2 * L + 1;
                     int64_t offB2 = pb;
                     for (int k2 = 0; k2 < noc; k2++) {
-                        const int L2 = a.oc_L[ocoff + k2];
-                        const int d2 = 2 * L2 + 1;
-                        if (L1 == L2 && a.oc_J[ocoff + k1] == a.oc_J[ocoff + k2]) {
+                        const int d2 = 2 * ocL[k2] + 1;
+                        if (L == ocL[k2] && ocJ[k1] == ocJ[k2]) {
                             const double delta = dl[k1 * noc + k2];
-                            const double J = a.oc_J[ocoff + k1] / 2.0;
-                            const int L = L1;
+                            const double J = ocJ[k1] / 2.0;
                             const double farep = (J < L) ? (L / (2.0 * L + 1)) : ((L + 1) / (2.0 * L + 1));
                             const double fso = (J < L) ? (-2.0 / (2 * L + 1)) : (+2.0 / (2 * L + 1));
-                            const double *SA = a.S_sph + offA1 + i * d, *SB = a.S_sph + offB2 + j * d;
+                            const int64_t rB = offB2 + j * d;
+                            const double *SA = a.S_sph + offA1 + i * d, *SB = a.S_sph + rB;
                             double s = 0.0;
                             for (int m = 0; m < d; m++) s += SA[m] * SB[m];
                             double buf = 0.0;
                             buf += s;
                             oa += (-1.0) * delta * farep * buf;
-                            double *oso[3] = {&ox, &oy, &oz};
+#pragma unroll
                             for (int comp = 0; comp < 3; comp++) {
+                                const double *LSB = a.LS + comp * a.sph_tot + rB;
                                 double t1 = 0.0;
-                                for (int m1 = 0; m1 < d; m1++) {
-                                    double tm = 0.0;
-                                    for (int m2 = 0; m2 < d; m2++) tm += lmat_val(L, comp, m1 - L, m2 - L) * SB[m2];
-                                    double tmp = 0.0;
-                                    tmp += tm;
-                                    t1 += SA[m1] * tmp;
-                                }
+                                for (int m = 0; m < d; m++) t1 += SA[m] * LSB[m];
                                 double sob = 0.0;
                                 sob += t1;
-                                *oso[comp] += (-1.0) * delta * fso * sob;
+                                oso[comp] += (-1.0) * delta * fso * sob;
                             }
                         }
                         offB2 += (int64_t)nB * d2;
@@ -873,12 +927,12 @@ __global__ void __launch_bounds__(NT) final_kernel(FinalArgs a, FinalSmem sm)
                     offA1 += (int64_t)nA * d;
                 }
                 acc[0][q] += 1.0 * oa;
-                acc[1][q] += 1.0 * ox;
-                acc[2][q] += 1.0 * oy;
-                acc[3][q] += 1.0 * oz;
+                acc[1][q] += 1.0 * oso[0];
+                acc[2][q] += 1.0 * oso[1];
+                acc[3][q] += 1.0 * oso[2];
             }
         }
-#pragma unroll
+#pragma unroll 1
         for (int q = 0; q < EPT; q++) {
             const int e = tid + q * NT;
             if (e < nel) {

@@ -21,6 +21,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <set>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -178,6 +179,9 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(upload_vec(st, h.rsh_comb_off, &d.rsh_comb_off));
     GRPP_CUDA(upload_vec(st, h.lmat, &d.lmat));
     GRPP_CUDA(upload_vec(st, h.lmat_off, &d.lmat_off));
+    GRPP_CUDA(upload_vec(st, h.lpair_off, &d.lpair_off));
+    GRPP_CUDA(upload_vec(st, h.lpair_m, &d.lpair_m));
+    GRPP_CUDA(upload_vec(st, h.lpair_v, &d.lpair_v));
     GRPP_CUDA(upload_vec(st, h.dfact, &d.dfact));
     GRPP_CUDA(upload_vec(st, h.binom, &d.binom));
     GRPP_CUDA(upload_vec(st, h.grid, &d.grid));
@@ -273,47 +277,51 @@ static std::vector<int> order_by_cost(const std::vector<double> &cost)
 }
 
 // Assembly classes and shared-memory layouts. A class is (la, lb, largest semilocal L, spin-orbit
-// terms or not); the layout holds the task's RSH rows, both sides' omega tables, its radial
-// table, the V rows of one potential (all rows when they fit in 6144 values) and W of the
-// factored re-centring sum. W holds ncart(lb) x rows x (components + 1) values (the sums and the
-// sums of absolute terms), rows chosen by the kernel so that nabB x rows x components fits in V;
-// its size is set per launch group from the group's tasks.
+// terms or not); the layout holds the task's own tables (both sides' omega tables and the radial
+// table of one potential, the binomial terms), the V rows of one potential (all rows when they
+// fit in 6144 values) and W of the factored re-centring sum (fin_w_size, for the rows that the
+// kernel takes from V's size); both are set per launch group.
 static int fin_class_key(int la, int lb, int Lmax, bool so) { return ((la * 16 + lb) * 16 + Lmax) * 2 + (so ? 1 : 0); }
 
-static int fin_default_nt(int la, int lb)
+// Block size of a class without an entry in the autotuner's table. 512 threads pay from about 1000 V
+// entries on (g x g: 0.31 ms against 0.40 with 128 threads for 576 tasks; g x f with 700: 0.23 against
+// 0.19; i x i 3.4 against 8.4 for 125), and for every class when the whole batch has at most two
+// tasks per SM, where a task's own latency is what is waited for (200 tasks: 0.27 against 0.40 ms).
+static int fin_default_nt(int la, int lb, int64_t n_tasks, int nsm)
 {
-    const int w = n_abc(la) * n_abc(lb);
-    return w < 1000 ? 128 : (w < 3000 ? 256 : 512);
+    return n_abc(la) * n_abc(lb) >= 1000 || n_tasks <= 2 * nsm ? 512 : 128;
 }
 
-static FinalSmem fin_layout(int lam, int n_omega, int n_q, int nabA, int nabB, int ncomp)
+// Limit of the supported classes: what a launch may need with dense omega rows on both sides, the
+// harmonics, the radial table and 6144 values of V
+struct FinNeed {
+    int n_rsh = 0, n_omega = 0, n_q = 0, n_v = 0;
+    size_t bytes() const { return (size_t)(2 * n_rsh + 2 * n_omega + n_q + n_v) * sizeof(double); }
+};
+
+static FinNeed fin_need(int lam, int n_omega, int n_q, int nabA, int nabB, int ncomp)
 {
-    FinalSmem fs{};
-    fs.rsh_stride = 2 * lam + 1;
-    fs.n_rsh = (lam + 1) * fs.rsh_stride;
-    fs.n_omega = n_omega;
-    fs.n_q = n_q;
-    fs.n_v = std::min(6144, std::max(nabA * nabB * ncomp, 3 * std::max(nabA, nabB)));
-    fs.n_v = std::max(fs.n_v, 3 * std::max(nabA, nabB));
-    fs.n_w = 0;  // set per launch group
-    return fs;
+    FinNeed f;
+    f.n_rsh = (lam + 1) * (2 * lam + 1);
+    f.n_omega = n_omega;
+    f.n_q = n_q;
+    f.n_v = std::max(std::min(6144, nabA * nabB * ncomp), 3 * std::max(nabA, nabB));
+    return f;
 }
 
-static FinalSmem fin_merge(const FinalSmem &x, const FinalSmem &y)
+static FinNeed fin_merge(const FinNeed &x, const FinNeed &y)
 {
-    FinalSmem m{};
-    m.rsh_stride = std::max(x.rsh_stride, y.rsh_stride);
+    FinNeed m;
     m.n_rsh = std::max(x.n_rsh, y.n_rsh);
     m.n_omega = std::max(x.n_omega, y.n_omega);
     m.n_q = std::max(x.n_q, y.n_q);
     m.n_v = std::max(x.n_v, y.n_v);
-    m.n_w = std::max(x.n_w, y.n_w);
     return m;
 }
 
 static size_t fin_smem_bytes(const FinalSmem &fs)
 {
-    return (size_t)(2 * fs.n_rsh + 2 * fs.n_omega + fs.n_q + fs.n_v + fs.n_w) * sizeof(double);
+    return (size_t)(2 * fs.n_rsh + fs.n_task + fs.n_v + ((fs.n_w + 1) & ~1)) * sizeof(double);
 }
 
 template <typename T>
@@ -488,7 +496,7 @@ struct Plan {
     size_t ft_smem = 0;
     double *omtab = nullptr;  // omega tables per (shell, centre) pair (scratch), omega_tab_kernel
     const int *om_shell = nullptr, *om_centre = nullptr;
-    int om_pairs = 0, om_blocks = 0;
+    int om_pairs = 0, om_blocks = 0, om_sl = 0;
     size_t om_smem = 0;
     size_t rad_smem = 0;
     FinalArgs fin;
@@ -894,6 +902,21 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         mmd_order = order_by_cost(cost);
     }
 
+    // omega tables per (shell, centre) pair (omega_tab_kernel): per semilocal potential of the
+    // centre's GRPP, om_size values; below 2 GiB
+    std::vector<int64_t> om_off(fp_shell.size() + 1, 0);
+    for (size_t k = 0; k < fp_shell.size(); k++) {
+        const int l = sh_L[fp_shell[k]], g = b->centre_grpp[fp_centre[k]];
+        int64_t w = 0;
+        for (int i = 0; i < g_sl_n[g]; i++) {
+            const int L = p_L[sl_pot[g_sl_off[g] + i]];
+            w += om_size(L, l);
+        }
+        om_off[k + 1] = om_off[k] + w;
+    }
+    int64_t om_words = rad_task.empty() ? 0 : om_off.back();
+    if (om_words * (int64_t)sizeof(double) > (int64_t(2) << 30)) om_words = 0;
+
     // Assembly launch groups. Per task: its class, the block size for the class (the caller's,
     // the autotuner's table, or the default rule) and the shared memory its tables need. Tasks of
     // one block size and one shared-memory tier form a group (one group per class when
@@ -905,13 +928,17 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         std::vector<double> cost(nt);
         std::map<int, int> gidx;
         std::vector<std::vector<int>> members;
+        std::vector<FinNeed> needs;
+        std::vector<int> v_min, sh_terms(ns);
+        for (int i = 0; i < ns; i++) sh_terms[i] = fin_terms(cart.data() + 3 * sh_co[i], ncart(sh_L[i]));
         for (int64_t t = 0; t < nt; t++) {
             const int la = sh_L[ta[t]], lb = sh_L[tb[t]], g = b->centre_grpp[tc[t]];
             cost[t] = 1.0 + (double)g_sl_n[g] * ((double)n_abc(la) * n_abc(lb) + 4.0 * ncart(la) * ncart(lb));
-            int lam = 0, nom = 1, nq = 1, Lmx = 0;
+            int lam = 0, nom = 1, nq = 1, Lmx = 0, om2 = 0;
             for (int i = 0; i < g_sl_n[g]; i++) {
                 const int L = p_L[sl_pot[g_sl_off[g] + i]];
                 Lmx = std::max(Lmx, L);
+                om2 = std::max(om2, om_size(L, la) + om_size(L, lb));
                 lam = std::max(lam, L + std::max(la, lb));
                 nom = std::max(nom, std::max(n_abc(la) * lam_slots(L, la), n_abc(lb) * lam_slots(L, lb)) * (2 * L + 1));
                 nq = std::max(nq, (L + la + 1) * (L + lb + 1) * (la + lb + 1));
@@ -921,11 +948,12 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             int ntb = opt.fin_nt;
             if (ntb == 0) {
                 auto it = st.fin_tune.find(cls);
-                ntb = it != st.fin_tune.end() ? it->second : fin_default_nt(la, lb);
+                ntb = it != st.fin_tune.end() ? it->second : fin_default_nt(la, lb, nt, st.nsm);
             }
             CHECK_INPUT(ntb == 128 || ntb == 256 || ntb == 512, "assembly block size must be 128, 256 or 512");
-            const FinalSmem fs = fin_layout(lam, nom, nq, n_abc(la), n_abc(lb), so ? 3 : 1);
-            const size_t bytes = fin_smem_bytes(fs);
+            const FinNeed fn = fin_need(lam, nom, nq, n_abc(la), n_abc(lb), so ? 3 : 1);
+            const int task_dbl = fin_task_doubles(om2, nq, sh_terms[ta[t]] + sh_terms[tb[t]]);
+            const size_t bytes = fn.bytes();
             const int tier = bytes <= 32 * 1024 ? 0 : (bytes <= 96 * 1024 ? 1 : 2);
             const int key = opt.fin_by_class ? cls * 8 + ntb / 128 : ntb * 4 + tier;
             auto it = gidx.find(key);
@@ -936,13 +964,18 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 FinGroup G;
                 G.nt = ntb;
                 G.key = opt.fin_by_class ? cls : -1;
-                G.fs = fs;
                 fin_groups.push_back(G);
                 members.emplace_back();
+                v_min.push_back(0);
+                needs.push_back(fn);
             } else {
                 gi = it->second;
-                fin_groups[gi].fs = fin_merge(fin_groups[gi].fs, fs);
+                needs[gi] = fin_merge(needs[gi], fn);
             }
+            FinalSmem &fs = fin_groups[gi].fs;
+            fs.n_task = std::max(fs.n_task, (task_dbl + 1) & ~1);
+            fs.n_v = std::max(fs.n_v, std::min(6144, n_abc(la) * fin_v_row(n_abc(lb), so ? 3 : 1)));
+            v_min[gi] = std::max(v_min[gi], fin_v_row(n_abc(lb), so ? 3 : 1));
             members[gi].push_back((int)t);
         }
         for (size_t gi = 0; gi < fin_groups.size(); gi++) {
@@ -952,19 +985,31 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             fin_groups[gi].count = (int)m.size();
             fin_order.insert(fin_order.end(), m.begin(), m.end());
             FinalSmem &fs = fin_groups[gi].fs;
-            // W of the factored re-centring sum: ncart(lb) x rows x (components + 1) values per
-            // potential, rows as the kernel takes them from the group's V size
-            int need = 0;
-            for (int t : m) {
-                const int la = sh_L[ta[t]], lb = sh_L[tb[t]];
-                const bool so = b->grpp_n_so[b->centre_grpp[tc[t]]] > 0;
-                for (int ncomp = 1; ncomp <= (so ? 3 : 1); ncomp += 2) {
-                    const int rows = std::max(1, std::min(n_abc(la), fs.n_v / (n_abc(lb) * ncomp)));
-                    need = std::max(need, ncart(lb) * rows * (ncomp + 1));
-                }
+            CHECK_INPUT(needs[gi].bytes() <= kFinSmemMax, "assembly tables of this batch exceed the shared memory of one block");
+            if (om_words == 0) {
+                fs.rsh_stride = 2 * fin_lam + 1;
+                fs.n_rsh = (fin_lam + 1) * fs.rsh_stride;
             }
-            fs.n_w = need;
-            if (fin_smem_bytes(fs) > kFinSmemMax) fs.n_w = 0;  // term-by-term re-centring only
+            std::set<std::array<int, 3>> shapes;  // (la, lb, components) of the group's tasks
+            for (int t : m) {
+                shapes.insert({sh_L[ta[t]], sh_L[tb[t]], 1});
+                if (b->grpp_n_so[b->centre_grpp[tc[t]]] > 0) shapes.insert({sh_L[ta[t]], sh_L[tb[t]], 3});
+            }
+            auto w_size = [&](int n_v) {
+                int need = 0;
+                for (const auto &q : shapes)
+                    need = std::max(need, fin_w_size(ncart(q[1]), fin_v_rows(n_v, n_abc(q[0]), n_abc(q[1]), q[2]), q[2]));
+                return need;
+            };
+            // V as large as leaves room for W, at least one row; term-by-term re-centring only if none does
+            const int vm = (v_min[gi] + 1) & ~1;
+            fs.n_v = std::max((fs.n_v + 1) & ~1, vm);
+            fs.n_w = w_size(fs.n_v);
+            while (fin_smem_bytes(fs) > kFinSmemMax && fs.n_v > vm) {
+                fs.n_v = std::max(vm, fs.n_v - 256);
+                fs.n_w = w_size(fs.n_v);
+            }
+            if (fin_smem_bytes(fs) > kFinSmemMax) fs.n_w = 0;
             CHECK_INPUT(fin_smem_bytes(fs) <= kFinSmemMax, "assembly tables of this batch exceed the shared memory of one block");
             fin_groups[gi].smem = fin_smem_bytes(fs);
         }
@@ -975,21 +1020,6 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     for (size_t k = 0; k < fp_shell.size(); k++) fp_off[k + 1] = fp_off[k] + (int64_t)(fp_lmax[k] + 1) * kRadGridPts;
     int64_t f_words = rad_task.empty() ? 0 : fp_off.back();
     if (f_words * (int64_t)sizeof(double) > (int64_t(8) << 30)) f_words = 0;
-    // omega tables per (shell, centre) pair (omega_tab_kernel): per semilocal potential of the
-    // centre's GRPP, n_abc(l) x slots x (2L+1) values; below 2 GiB
-    std::vector<int64_t> om_off(fp_shell.size() + 1, 0);
-    for (size_t k = 0; k < fp_shell.size(); k++) {
-        const int l = sh_L[fp_shell[k]], g = b->centre_grpp[fp_centre[k]];
-        int64_t w = 0;
-        for (int i = 0; i < g_sl_n[g]; i++) {
-            const int L = p_L[sl_pot[g_sl_off[g] + i]];
-            w += (int64_t)n_abc(l) * lam_slots(L, l) * (2 * L + 1);
-        }
-        om_off[k + 1] = om_off[k] + w;
-    }
-    int64_t om_words = rad_task.empty() ? 0 : om_off.back();
-    if (om_words * (int64_t)sizeof(double) > (int64_t(2) << 30)) om_words = 0;
-
     // angular tensors
     for (int L = 0; L <= kMaxL; L++)
         for (int l = 0; l <= kMaxL; l++)
@@ -1055,9 +1085,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     for (int g = 0; g < ng; g++) wu_npot = std::max(wu_npot, g_sl_n[g]);
     int64_t wu_words = rad_task.empty() ? 0 : (int64_t)ng * wu_npot * kRadGridPts;
     if (wu_words * (int64_t)sizeof(double) > (int64_t(256) << 20)) wu_words = 0;
-    const size_t scratch_bytes =
-        (size_t)(3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words + wu_words + f_words + om_words) *
-        sizeof(double);
+    const int64_t om_at = (3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words + wu_words + f_words + 1) & ~int64_t(1);
+    const int64_t ls_at = om_at + om_words;  // 16-byte aligned omega tables, then the L matrix products
+    const size_t scratch_bytes = (size_t)(ls_at + 6 * sn) * sizeof(double);
     GRPP_CUDA(bscr->ensure(scratch_bytes));
     GRPP_CUDA(bout->ensure((size_t)4 * std::max<int64_t>(out_tot, 1) * sizeof(double)));
     P.scratch_bytes = (int64_t)scratch_bytes;
@@ -1073,9 +1103,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     double *wud = wu_words > 0 ? (double *)bscr->p + (3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words) : nullptr;
     double *ftd = f_words > 0 ? (double *)bscr->p + (3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words + wu_words)
                               : nullptr;
-    double *omd = om_words > 0 ? (double *)bscr->p + (3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words + wu_words +
-                                                      f_words)
-                               : nullptr;
+    double *omd = om_words > 0 ? (double *)bscr->p + om_at : nullptr;
+    double *lsd = (double *)bscr->p + ls_at, *sld = lsd + 3 * sn;
     P.stop_level = stopd;
     P.pred_level = predd;
     P.order = orderd;
@@ -1144,6 +1173,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         o.U_cart = Ucd;
         o.S_sph = Ssd;
         o.U_sph = Usd;
+        o.LS = lsd;
+        o.SL = sld;
+        o.sph_tot = sn;
         P.ocp = o;
         P.ocp_blocks = (int)std::min<size_t>(blk_shell.size(), (size_t)nsm * 32);
     }
@@ -1275,6 +1307,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         f.proj_off = at<int64_t>(ib, o_poffp);
         f.S_sph = Ssd;
         f.U_sph = Usd;
+        f.LS = lsd;
+        f.SL = sld;
+        f.sph_tot = sn;
         f.raw_so = opt.raw_so;
         f.arep = o_arep;
         f.so_x = o_sx;
@@ -1297,7 +1332,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         P.om_shell = at<int>(ib, o_fps);
         P.om_centre = at<int>(ib, o_fpc);
         P.om_smem = (size_t)fs.n_rsh * sizeof(double);
-        P.om_blocks = (int)std::min<int64_t>((int64_t)fp_shell.size(), (int64_t)nsm * 8);
+        P.om_sl = wu_npot;
+        P.om_blocks = (int)std::min<int64_t>((int64_t)fp_shell.size() * wu_npot, (int64_t)nsm * 16);
         // persistent grid per assembly group over its part of the task queue
         for (auto &G : fin_groups) {
             int occ = 0;
@@ -1382,7 +1418,7 @@ int plan_launch(Plan &P)
     GRPP_CUDA(cudaEventRecord(ev[2], s));
     if (P.omtab) {
         GRPP_CUDA(ang_launch_omega_tab(P.om_blocks, kFinThreads, P.om_smem, s, &P.fin, sizeof(P.fin), &P.fin_smem_layout,
-                                       sizeof(P.fin_smem_layout), P.om_shell, P.om_centre, P.om_pairs, P.omtab));
+                                       sizeof(P.fin_smem_layout), P.om_shell, P.om_centre, P.om_pairs, P.om_sl, P.omtab));
     }
     for (size_t gi = 0; gi < P.fin_groups.size(); gi++) {
         const FinGroup &G = P.fin_groups[gi];

@@ -58,6 +58,9 @@ struct DeviceTables {
     const int *rsh_comb_off;  // [kRshL+1] offsets (in combos)
     const double *lmat;       // concatenated per L: 3 x (2L+1)^2 (x, y, z)
     const int *lmat_off;      // [kMaxL+2]
+    const int *lpair_off;     // [kMaxL+2][4]: first (m1, m2) pair of components x, y, z of L, and their end
+    const int *lpair_m;       // m1 + L | (m2 + L) << 8 of the pairs with a non-zero value, m1-major
+    const double *lpair_v;    // their values
     const double *dfact;      // dfact[n+1] = n!!, n = -1..kDfMax
     const double *binom;      // [kBinN][kBinN]
     const double *grid;       // [kGridRows][kGridPts] (null: the kernels compute r and w themselves)

@@ -61,6 +61,7 @@ namespace {
 using namespace grpp_noalloc::grpp;
 
 constexpr size_t kNoAllocScratchBytes = 32u << 20;  // 32 MiB
+constexpr size_t kNaFinSmem = 200 * 1024;  // dynamic shared memory of the assembly kernel
 constexpr int kMaxDevices = 64;
 
 // static constant tables (sizes of tables.cpp's layout for kRshL = 32, kMaxL = 10)
@@ -138,6 +139,8 @@ int setup(int dev)
     if ((rc = copy_table(g_rsh_off, h.rsh_off, (size_t)kRshL + 2, &d.rsh_off))) return rc;
     if ((rc = copy_table(g_rsh_comb, h.rsh_comb, kNaComb, &d.rsh_comb))) return rc;
     if ((rc = copy_table(g_rsh_comb_off, h.rsh_comb_off, (size_t)kRshL + 2, &d.rsh_comb_off))) return rc;
+    d.lpair_off = d.lpair_m = nullptr;  // no spin-orbit terms here
+    d.lpair_v = nullptr;
     if ((rc = copy_table(g_lmat, h.lmat, kNaLmat, &d.lmat))) return rc;
     if ((rc = copy_table(g_lmat_off, h.lmat_off, (size_t)kMaxL + 3, &d.lmat_off))) return rc;
     if ((rc = copy_table(g_dfact, h.dfact, (size_t)kDfMax + 2, &d.dfact))) return rc;
@@ -147,7 +150,7 @@ int setup(int dev)
     NA_CUDA(cudaGetSymbolAddress(&p, g_scratch));
     g_scratch_ptr[dev] = (unsigned char *)p;
     NA_CUDA(cudaFuncSetAttribute(radial_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-    NA_CUDA(cudaFuncSetAttribute(final_kernel<kFinThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    NA_CUDA(cudaFuncSetAttribute(final_kernel<kFinThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNaFinSmem));
     g_ready[dev] = true;
     return 0;
 }
@@ -286,7 +289,7 @@ int run(const libgrpp_b200_batch_t *b, double *h_arep)
     for (int64_t t = 0; t < nt; t++) {
         NA_CHECK(ta[t] >= 0 && ta[t] < ns && tb[t] >= 0 && tb[t] < ns && tc[t] >= 0 && tc[t] < b->n_centres, "task index out of range");
         const int la = sh_L[ta[t]], lb = sh_L[tb[t]], g = b->centre_grpp[tc[t]];
-        NA_CHECK(ncart(la) * ncart(lb) <= kFinThreads * kFinElemPerThread, "shell pair block larger than 1024 Cartesian pairs");
+        NA_CHECK(ncart(la) * ncart(lb) <= kFinMaxPairs, "shell pair block larger than 1024 Cartesian pairs");
         out_off[t + 1] = out_off[t] + (int64_t)ncart(la) * ncart(lb);
         if (g_sl_n[g] == 0) continue;
         int64_t e = 0;
@@ -440,15 +443,22 @@ int run(const libgrpp_b200_batch_t *b, double *h_arep)
     FinalSmem fs{};
     fs.rsh_stride = 2 * fin_lam + 1;
     fs.n_rsh = (fin_lam + 1) * fs.rsh_stride;
-    int n_om = 1, nabmax = 1;
+    int n_om = 1, n_om2 = 1, nabmax = 1, terms = 1;
     for (auto &lp : atab_need) {
         n_om = std::max(n_om, n_abc(lp.second) * lam_slots(lp.first, lp.second) * (2 * lp.first + 1));
+        n_om2 = std::max(n_om2, om_size(lp.first, lp.second));
         nabmax = std::max(nabmax, n_abc(lp.second));
     }
-    fs.n_omega = n_om;
-    fs.n_q = fin_nq;
-    fs.n_v = std::max(6144, 3 * nabmax);
-    const size_t smem = (size_t)(2 * fs.n_rsh + 2 * fs.n_omega + fs.n_q + fs.n_v) * sizeof(double);
+    for (int i = 0; i < b->n_shells; i++)
+        terms = std::max(terms, fin_terms(cart.data() + 3 * sh_co[i], ncart(sh_L[i])));
+    // the classes that fit: dense omega rows, the harmonics, the radial table and V
+    const size_t need = (size_t)(2 * fs.n_rsh + 2 * n_om + fin_nq + std::max(6144, 3 * nabmax)) * sizeof(double);
+    const int vmin = (fin_v_row(nabmax, 1) + 1) & ~1;
+    fs.n_task = (fin_task_doubles(2 * n_om2, fin_nq, 2 * terms) + 1) & ~1;
+    fs.n_v = std::max(6144, vmin);
+    auto bytes = [&]() { return (size_t)(2 * fs.n_rsh + fs.n_task + fs.n_v) * sizeof(double); };
+    while (bytes() > kNaFinSmem && fs.n_v > vmin) fs.n_v = std::max(vmin, fs.n_v - 256);
+    const size_t smem = std::max(bytes(), need > kNaFinSmem ? need : 0);  // refused by the launch when over the limit
     final_kernel<kFinThreads><<<(int)std::min<int64_t>(nt, (int64_t)nsm * 8), kFinThreads, smem>>>(f, fs);
     NA_CUDA(cudaGetLastError());
     NA_CUDA(cudaMemcpy(h_arep, P(o_arep), out_tot * sizeof(double), cudaMemcpyDeviceToHost));

@@ -78,13 +78,13 @@ cudaError_t ang_launch_oc_proj(int blocks, int threads, cudaStream_t s, const vo
 
 cudaError_t ang_launch_omega_tab(int blocks, int threads, size_t smem, cudaStream_t s, const void *fin, size_t fin_size,
                                  const void *layout, size_t layout_size, const int *op_shell, const int *op_centre,
-                                 int n_pairs, double *omtab)
+                                 int n_pairs, int max_sl, double *omtab)
 {
     AFin f;
     ASmem m;
     if (!unpack(f, fin, fin_size) || !unpack(m, layout, layout_size) || threads != grpp_ang::grpp::kFinThreads)
         return cudaErrorInvalidValue;
-    grpp_ang::grpp::omega_tab_kernel<<<blocks, threads, smem, s>>>(f, m, op_shell, op_centre, n_pairs, omtab);
+    grpp_ang::grpp::omega_tab_kernel<<<blocks, threads, smem, s>>>(f, m, op_shell, op_centre, n_pairs, max_sl, omtab);
     return cudaGetLastError();
 }
 

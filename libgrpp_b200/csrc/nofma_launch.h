@@ -33,7 +33,7 @@ cudaError_t ang_launch_atab(int blocks, int threads, cudaStream_t s, int L, int 
 cudaError_t ang_launch_oc_proj(int blocks, int threads, cudaStream_t s, const void *args, size_t size);
 cudaError_t ang_launch_omega_tab(int blocks, int threads, size_t smem, cudaStream_t s, const void *fin, size_t fin_size,
                                  const void *layout, size_t layout_size, const int *op_shell, const int *op_centre,
-                                 int n_pairs, double *omtab);
+                                 int n_pairs, int max_sl, double *omtab);
 // RadialArgs (radial.cuh) by address and size
 cudaError_t nofma_launch_ftab(int blocks, int threads, size_t smem, cudaStream_t s, const void *rad, size_t rad_size,
                               double *ftab);

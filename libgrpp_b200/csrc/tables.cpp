@@ -393,6 +393,20 @@ void build_host_tables(HostTables &t)
     }
     t.lmat_off[kMaxL + 2] = (int)t.lmat.size();
 
+    // per L and component (x, y, z) the (m1, m2) pairs with a non-zero value, m1 outer
+    t.lpair_off.assign(4 * (kMaxL + 2), 0);
+    for (int L = 0; L <= kMaxL + 1; L++)
+        for (int comp = 0; comp < 4; comp++) {
+            t.lpair_off[4 * L + comp] = (int)t.lpair_m.size();
+            const int d = 2 * L + 1;
+            for (int q = 0; q < d * d && comp < 3; q++) {
+                const double v = t.lmat[t.lmat_off[L] + comp * d * d + q];
+                if (std::fabs(v) < kZeroThresh) continue;
+                t.lpair_m.push_back(q / d | (q % d) << 8);
+                t.lpair_v.push_back(v);
+            }
+        }
+
     t.dfact.assign(kDfMax + 2, 1.0);
     for (int n = 1; n <= kDfMax; n++) t.dfact[n + 1] = n * (n >= 2 ? t.dfact[n - 1] : 1.0);
 
