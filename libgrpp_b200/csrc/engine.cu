@@ -212,6 +212,7 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(cudaFuncSetAttribute(radial_screen_unit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(kScrWarps * scr_warp_doubles(kRadMaxLam + 1) * sizeof(double))));
     GRPP_CUDA(cudaFuncSetAttribute(radial_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    GRPP_CUDA(cudaFuncSetAttribute(radial_walk_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GRPP_CUDA(ang_set_final_max_smem((int)kFinSmemMax));
     GRPP_CUDA(cudaFuncSetAttribute(type1_num_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)(t1_smem_doubles(kT1MaxLam) * sizeof(double))));
@@ -395,6 +396,27 @@ std::vector<uint16_t> used_entries(int L, int la, int lb)
     return out;
 }
 
+// The same entries as groups of the walk: up to kWalkN values of N of one (l1, l2); for given orders N
+// runs in steps of 2 from |l1 - L| + |l2 - L|.
+void walk_groups(int L, int la, int lb, std::vector<WalkGroup> &out)
+{
+    std::vector<WalkGroup> g;
+    for (int l1 = std::max(L - la, 0); l1 <= L + la; l1++)
+        for (int l2 = std::max(L - lb, 0); l2 <= L + lb; l2++) {
+            const int k1 = std::abs(l1 - L), k2 = std::abs(l2 - L);
+            // equal shares of the N values: 5 as 3 + 2
+            const int n = (la - k1) / 2 + (lb - k2) / 2 + 1, parts = (n + kWalkN - 1) / kWalkN;
+            for (int q = 0, k = 0; q < parts; q++) {
+                const int cnt = n / parts + (q < n % parts);
+                g.push_back(WalkGroup{(uint8_t)l1, (uint8_t)l2, (uint8_t)(k1 + k2 + 2 * k), (uint8_t)cnt});
+                k += cnt;
+            }
+        }
+    // groups of equal size side by side: the lanes of a warp advance as many entries as the largest
+    std::stable_sort(g.begin(), g.end(), [](const WalkGroup &x, const WalkGroup &y) { return x.cnt > y.cnt; });
+    out.insert(out.end(), g.begin(), g.end());
+}
+
 struct PotView {
     int L, J;
     std::vector<int> pw;
@@ -499,6 +521,9 @@ struct Plan {
     int om_pairs = 0, om_blocks = 0, om_sl = 0;
     size_t om_smem = 0;
     size_t rad_smem = 0;
+    bool walk_groups = false;  // radial_walk_group_kernel, else the walk that evaluates the integrands itself
+    WalkArgs wlk{};
+    size_t walk_smem = 0;
     FinalArgs fin;
     FinalSmem fin_smem_layout;  // batch-wide layout (omega tables)
     std::vector<FinGroup> fin_groups;
@@ -705,6 +730,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     std::vector<int2> ucls((kMaxL + 1) * (kMaxL + 1) * (kMaxL + 1), int2{0, 0});
     std::vector<uint8_t> ucls_set(ucls.size(), 0);
     std::vector<uint16_t> ulist;
+    std::vector<WalkGroup> wgroups;  // the same lists as groups of the walk
+    std::vector<int2> wcls(ucls.size(), int2{0, 0});
+    int64_t walk_list_max = 1;
     out_off[0] = 0;
     int mmd_lmax = 0, mmd_smax = 0;
     int rad_l1 = 0, rad_l2 = 0, rad_dn = 1, rad_npot = 0;
@@ -731,7 +759,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             rad_task.push_back((int)t);
             rad_qoff.push_back(qtot);
             int e = 0, Lmx = 0;
-            int64_t item_used = 0;
+            int64_t item_used = 0, item_groups = 0;
             double CA2 = 0.0, CB2 = 0.0;
             for (int d = 0; d < 3; d++) {
                 const double u = b->centre_origin[3 * C + d] - b->shell_origin[3 * A + d];
@@ -753,6 +781,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                     ucls[key] = int2{(int)ulist.size(), (int)u.size()};
                     ulist.insert(ulist.end(), u.begin(), u.end());
                     ucls_set[key] = 1;
+                    wcls[key].x = (int)wgroups.size();
+                    walk_groups(L, la, lb, wgroups);
+                    wcls[key].y = (int)wgroups.size() - wcls[key].x;
                 }
                 const int ne = ucls[key].y;
                 if (one_centre) {
@@ -766,6 +797,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                     scr_lw = std::max(scr_lw, L + std::max(la, lb) + 1);
                 }
                 item_used += ucls[key].y;
+                item_groups += wcls[key].y;
                 rad_l1 = std::max(rad_l1, L + la);
                 rad_l2 = std::max(rad_l2, L + lb);
                 fin_lam = std::max(fin_lam, L + std::max(la, lb));
@@ -781,6 +813,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             CHECK_INPUT(std::max(rad_l1, rad_l2) <= kRadMaxLam && la + lb + 1 <= kRadMaxN, "angular momentum too high for the radial path");
             qtot += e;
             rad_list_max = std::max(rad_list_max, item_used);
+            walk_list_max = std::max(walk_list_max, item_groups);
             rad_dn = std::max(rad_dn, la + lb + 1);
             rad_npot = std::max(rad_npot, g_sl_n[g]);
         }
@@ -822,6 +855,14 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         const std::vector<int> ord = order_by_cost(cost);
         for (size_t i = 0; i < ord.size(); i++) cut[i] = scr_big[ord[i]];
         scr_big.swap(cut);
+    }
+    // items by centre, for the walk
+    std::vector<int> walk_perm(rad_task.size());
+    {
+        std::vector<int> start(b->n_centres + 1, 0);
+        for (int t : rad_task) start[tc[t] + 1]++;
+        for (int c = 0; c < b->n_centres; c++) start[c + 1] += start[c];
+        for (size_t i = 0; i < rad_task.size(); i++) walk_perm[start[tc[rad_task[i]]]++] = (int)i;
     }
     // outercore projection blocks
     std::vector<int> blk_shell, blk_oc;
@@ -1053,7 +1094,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     const size_t o_ta = pk.add(ta), o_tb = pk.add(tb), o_tc = pk.add(tc), o_too = pk.add(out_off), o_thul = pk.add(has_ul),
                  o_tqo = pk.add(q_off), o_tpa = pk.add(proj_a), o_tpb = pk.add(proj_b);
     const size_t o_items = pk.add(items), o_rt = pk.add(rad_task), o_rq = pk.add(rad_qoff),
-                 o_ulist = pk.add(ulist), o_sbig = pk.add(scr_big), o_ssmall = pk.add(scr_small),
+                 o_ulist = pk.add(ulist), o_wgrp = pk.add(wgroups), o_wcls = pk.add(wcls), o_wperm = pk.add(walk_perm), o_sbig = pk.add(scr_big), o_ssmall = pk.add(scr_small),
                  o_suo = pk.add(su_off);
     const size_t o_bs = pk.add(blk_shell), o_bo = pk.add(blk_oc), o_bco = pk.add(blk_cart_off), o_bso = pk.add(blk_sph_off),
                  o_poffp = pk.add(proj_off), o_mpair = pk.add(mmd_pairs), o_pperm = pk.add(p_perm), o_pn2 = pk.add(p_n2);
@@ -1077,8 +1118,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     const int64_t qn = std::max<int64_t>(qtot, 1), cn = std::max<int64_t>(cart_tot, 1), sn = std::max<int64_t>(sph_tot, 1);
     const int64_t nrad = std::max<int64_t>((int64_t)rad_task.size(), 1);
     const int64_t flag_words = (qn + nrad + 2 * 8) / 8 + 1;  // entry flags + per-task walk flags, in doubles
-    // per radial item: stop level, predicted level (int8), order (int); learned-mode control words
-    const int64_t lm_words = (2 * nrad + 4 * nrad + 16 * 4) / 8 + 4;
+    // per radial item: stop level, predicted level (int8), order, deepest level (int); walk control words
+    const int64_t lm_words = (2 * nrad + 8 * nrad + 16 * 4) / 8 + 4;
     // table of w U_p(r) per GRPP, semilocal potential slot and grid point (wu_table_kernel),
     // when the batch walks a grid and the table stays below 256 MiB
     int wu_npot = 0;
@@ -1268,6 +1309,26 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&scru_occ, radial_screen_unit_kernel, 32 * kScrWarps, P.scru_smem));
         P.scru_blocks = (int)std::min<int64_t>(((int64_t)scr_big.size() + kScrWarps - 1) / kScrWarps, (int64_t)nsm * std::max(scru_occ, 1));
         P.rad_smem = smem;
+        // the walk over groups needs the tables; a batch of few items shares an item between up to
+        // 16 blocks, so that there are two blocks for every resident one, with 32 groups each
+        const int wrows = rad_npot + rad_l1 + 1 + rad_l2 + 1 + rad_dn;
+        const size_t gsmem = (size_t)wrows * kWalkRow * sizeof(double) + 8 * walk_list_max;
+        P.walk_groups = wud && ftd && gsmem <= 160 * 1024;
+        P.wlk.groups = at<WalkGroup>(ib, o_wgrp);
+        P.wlk.cls = at<int2>(ib, o_wcls);
+        P.wlk.perm = at<int>(ib, o_wperm);
+        P.wlk.nparts = opt.walk_parts > 0 ? opt.walk_parts
+                                          : (int)std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(16, walk_list_max / 32),
+                                                                                        (int64_t)10 * nsm / (int64_t)rad_task.size()));
+        P.wlk.list_max = (int)walk_list_max;
+        P.wlk.chunk_doubles = wrows * kWalkRow;
+        P.wlk.item_level = opt.radial_mode == LIBGRPP_B200_RADIAL_LEARNED && P.wlk.nparts > 1 ? lmctld + 16 : nullptr;
+        P.walk_smem = gsmem;
+        if (P.walk_groups) {
+            int occ = 0;
+            GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, radial_walk_group_kernel, kWalkThreads, gsmem));
+            P.rad_blocks = (int)std::min<int64_t>((int64_t)rad_task.size() * P.wlk.nparts, (int64_t)nsm * std::max(occ, 1));
+        }
     }
 
     // ---------------------------------------------------------------- 5. final assembly
@@ -1378,6 +1439,7 @@ int plan_launch(Plan &P)
     }
     if (P.rad_blocks > 0) {
         GRPP_CUDA(cudaMemsetAsync(P.rad.walk, 0, (size_t)P.n_radial, s));
+        GRPP_CUDA(cudaMemsetAsync(P.lm_ctl, 0, (16 + (P.wlk.item_level ? (size_t)P.n_radial : 0)) * sizeof(int), s));
         GRPP_CUDA(cudaMemsetAsync(P.rad.eflag, 0, (size_t)P.n_entries, s));  // unread entries stay inactive
         if (P.scru_blocks > 0) {
             radial_screen_unit_kernel<<<P.scru_blocks, 32 * kScrWarps, P.scru_smem, s>>>(P.rad);
@@ -1395,12 +1457,11 @@ int plan_launch(Plan &P)
                 return LIBGRPP_B200_ERR_INVALID;
             }
             // predict every walked task's level, order deepest first, walk from the queue
-            GRPP_CUDA(cudaMemsetAsync(P.lm_ctl, 0, 16 * sizeof(int), s));
             LevelModelDev lm{st.lm_norm, st.lm_w};
             const int pblocks = (int)std::min<int64_t>((P.n_radial + 3) / 4, (int64_t)st.nsm * 16);
             level_predict_kernel<<<pblocks, 128, 0, s>>>(P.rad, lm, P.pred_level);
             GRPP_CUDA(cudaGetLastError());
-            level_order_kernel<<<1, 256, 0, s>>>((int)P.n_radial, P.pred_level, P.order, P.lm_ctl, P.lm_ctl + 2);
+            level_order_kernel<<<1, 1024, 0, s>>>((int)P.n_radial, P.wlk.perm, P.pred_level, P.order, P.lm_ctl, P.lm_ctl + 2);
             GRPP_CUDA(cudaGetLastError());
             ra.order = P.order;
             ra.pred_level = P.pred_level;
@@ -1412,7 +1473,8 @@ int plan_launch(Plan &P)
         if (P.ftab) {
             GRPP_CUDA(nofma_launch_ftab(P.ft_blocks, kRadThreads, P.ft_smem, s, &P.rad, sizeof(P.rad), P.ftab));
         }
-        radial_walk_kernel<<<P.rad_blocks, kRadThreads, P.rad_smem, s>>>(ra);
+        if (P.walk_groups) radial_walk_group_kernel<<<P.rad_blocks, kWalkThreads, P.walk_smem, s>>>(ra, P.wlk);
+        else radial_walk_kernel<<<P.rad_blocks, kRadThreads, P.rad_smem, s>>>(ra);
         GRPP_CUDA(cudaGetLastError());
     }
     GRPP_CUDA(cudaEventRecord(ev[2], s));
@@ -1713,6 +1775,7 @@ int level_samples(const libgrpp_b200_batch_t *b, float *features, int8_t *levels
     if (!stp) return rc;
     std::lock_guard<std::mutex> lk(stp->mu);
     RunOptions opt;
+    opt.walk_parts = 1;  // a block per item writes its stop level
     Plan P;
     rc = plan_build(*stp, b, opt, false, P);
     if (rc) return rc;

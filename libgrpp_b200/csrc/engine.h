@@ -14,6 +14,7 @@ struct RunOptions {
     int radial_mode = LIBGRPP_B200_RADIAL_PLAIN;
     int raw_so = 0;          // spin-orbit output without the 2/(2L+1) factor (libgrpp_spin_orbit_integrals)
     int fin_nt = 0;          // assembly block size for every task (128, 256, 512); 0: tuning table, else default rule
+    int walk_parts = 0;      // blocks that share a task's grid walk; 0: by the batch's size
     int fin_by_class = 0;    // one assembly launch per class, each timed (autotuning)
 };
 

@@ -181,9 +181,9 @@ __global__ void __launch_bounds__(128) level_predict_kernel(RadialArgs a, LevelM
     }
 }
 
-// Deepest-predicted-first order of the walked items: counting sort over levels 8..0.
-// cursor[0..9] must be zero on entry; one CTA of 256 threads.
-__global__ void level_order_kernel(int n_items, const int8_t *pred, int *order, int *n_order, int *cursor)
+// Deepest-predicted-first order of the walked items, within a level in the order of perm (items by
+// centre): counting sort over levels 8..0. cursor[0..9] must be zero on entry; one CTA of 256 threads.
+__global__ void level_order_kernel(int n_items, const int *perm, const int8_t *pred, int *order, int *n_order, int *cursor)
 {
     __shared__ int hist[kLmOut], start[kLmOut];
     if (threadIdx.x < kLmOut) hist[threadIdx.x] = 0;
@@ -200,11 +200,13 @@ __global__ void level_order_kernel(int n_items, const int8_t *pred, int *order, 
         *n_order = s;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n_items; i += blockDim.x)
+    for (int k = threadIdx.x; k < n_items; k += blockDim.x) {
+        const int i = perm[k];
         if (pred[i] >= 0) {
             const int l = min((int)pred[i], kLmOut - 1);
             order[start[l] + atomicAdd(&cursor[l], 1)] = i;
         }
+    }
 }
 
 // ---- training -----------------------------------------------------------------------------

@@ -1217,6 +1217,329 @@ __global__ void __launch_bounds__(kRadThreads, 5) radial_walk_kernel(RadialArgs 
         }
     }
 }
+
+// ---- the walk over tabulated integrands: radial_walk_group_kernel ------------------------------
+//
+// The same walk (points, per-level rules, sums: radial_walk_kernel above) when w U_p, F_l and r^N
+// come from tables. What it does differently:
+//  * A thread advances a group of up to kWalkN entries of one (p, l1, l2) whose N differ by 2:
+//    ((w U) F1) F2 is formed once per point for the group, and the entries' sums are independent
+//    chains: 3 + k shared loads, 2 + k products and k additions for k entries, where each entry took 4
+//    loads, 3 products and a dependent addition.
+//  * Most points belong to the deep levels of a few entries (63 active entries per point on the s..g
+//    workload), so what counts there is the latency of a chunk: the rows that are still needed are
+//    packed, and a chunk takes as many points as the block's shared memory holds of them (128 to
+//    1024, within one level), copied asynchronously, every row in flight at once.
+//  * Chunks start one before libgrpp's first point (a point of weight 0), so that levels 0 to 2 are the
+//    first 128 points and every later level starts and ends with a chunk; rows of an odd number of
+//    16-byte units, read two points at a time without bank conflicts.
+//  * Items are taken by centre, so that the F_l tables of one centre's shells stay in L2; a batch of
+//    few items shares the groups of an item between nparts CTAs.
+//  * The lists of active groups carry their entries' active bits; flags, previous sums and estimates
+//    are read at the ends of levels only.
+// Bound by shared-memory loads (75% of the cycles). Walk with its tables and ordering, four blocks
+// per SM against five: 26.6 and 26.5 ms on 65536 s..g tasks, 21.3 and 22.5 on a 15-atom molecule,
+// where the walk by single entries took 30.0 and 31.8; a 200-task molecule 1.21 -> 0.42 ms.
+// Groups of the four order pairs L -+ k1, L -+ k2 (a third of the loads) leave too few threads
+// busy: 35.7 ms on the first.
+constexpr int kWalkN = 4;
+constexpr int kWalkPts = 128;            // points of the smallest chunk
+constexpr int kWalkMaxPts = 1024;
+constexpr int kWalkRow = kWalkPts + 2;
+constexpr int kWalkThreads = 128;
+struct WalkGroup {
+    uint8_t l1, l2, n0, cnt;  // orders; N = n0, n0 + 2, .., cnt of them
+};
+
+struct WalkArgs {
+    const WalkGroup *groups;
+    const int2 *cls;     // per class (L, la, lb): offset into groups, count
+    const int *perm;     // items by potential centre
+    int nparts;          // CTAs per item
+    int list_max;        // capacity of the active-group lists (groups of one item at most)
+    int chunk_doubles;   // doubles of point rows before the lists
+    int *item_level;     // learned mode and nparts > 1: deepest level + 1 of an item so far (else null)
+};
+
+// 8 bytes from global to shared memory, asynchronously (zero: writes 0)
+__device__ __forceinline__ void copy8_async(double *dst, const double *src, bool zero)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(zero ? 0 : 8)
+                 : "memory");
+}
+
+// The sums of K entries over the point pairs x0..x1-1, each in point order: s += (((w U) F1) F2) r^N
+template <int K>
+__device__ __forceinline__ void walk_advance(int x0, int x1, const double2 *pw, const double2 *p1, const double2 *p2,
+                                             const double2 *const *pn, double *s)
+{
+#pragma unroll(K > 2 ? 2 : 4)
+    for (int x = x0; x < x1; x++) {
+        const double2 vw = pw[x], v1 = p1[x], v2 = p2[x];
+        const double tx = __dmul_rn(__dmul_rn(vw.x, v1.x), v2.x), ty = __dmul_rn(__dmul_rn(vw.y, v1.y), v2.y);
+#pragma unroll
+        for (int q = 0; q < K; q++) {
+            const double2 vn = pn[q][x];
+            s[q] = __dadd_rn(s[q], __dmul_rn(tx, vn.x));
+            s[q] = __dadd_rn(s[q], __dmul_rn(ty, vn.y));
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kWalkThreads, 4) radial_walk_group_kernel(RadialArgs a, WalkArgs w)
+{
+    extern __shared__ __align__(16) double wsm[];
+    __shared__ int pL[kRadMaxPots], pent[kRadMaxPots], pgrp[kRadMaxPots], gpre[kRadMaxPots + 1];
+    __shared__ int s_need[2][4];  // per buffer: max l1, max l2, max N of active entries, potential mask
+    __shared__ int s_cnt[2], s_lvl, s_item, s_part;
+    const int tid = threadIdx.x, lane = tid & 31, NT = blockDim.x;
+    // active groups: potential << 27 | index within the potential's groups << 4 | active entries
+    unsigned *lists[2] = {(unsigned *)(wsm + w.chunk_doubles), (unsigned *)(wsm + w.chunk_doubles) + w.list_max};
+    const int n_units = (a.order ? *a.n_order : a.n_items) * w.nparts;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) {
+            int item = -1, part = 0;
+            for (;;) {
+                const int u = atomicAdd(a.queue, 1);
+                if (u >= n_units) break;
+                const int k = u / w.nparts;
+                const int it = a.order ? a.order[k] : w.perm[k];
+                if (!a.order && !a.walk[it]) continue;
+                item = it;
+                part = u - k * w.nparts;
+                break;
+            }
+            s_item = item;
+            s_part = part;
+            s_lvl = 0;
+            s_cnt[0] = 0;
+        }
+        if (tid < 8) s_need[tid >> 2][tid & 3] = (tid & 3) == 3 ? 0 : -1;
+        __syncthreads();
+        const int item = s_item, part = s_part;
+        if (item < 0) break;
+        const int t = a.item_task[item], c = a.task_c[t], gr = a.centre_grpp[c];
+        const int la = a.shell_L[a.task_a[t]], lb = a.shell_L[a.task_b[t]], dn = la + lb + 1, npot = a.grpp_sl_n[gr];
+        if (tid < 32) {
+            int sz = 0, ng = 0;
+            if (tid < npot) {
+                const int L = a.pot_L[a.sl_pot[a.grpp_sl_off[gr] + tid]];
+                const int2 cl = w.cls[(L * (kMaxL + 1) + la) * (kMaxL + 1) + lb];
+                pL[tid] = L;
+                pgrp[tid] = cl.x;
+                sz = (L + la + 1) * (L + lb + 1) * dn;
+                ng = cl.y;
+            }
+            int es = sz, gs = ng;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int e = __shfl_up_sync(0xffffffffu, es, o), g = __shfl_up_sync(0xffffffffu, gs, o);
+                if (lane >= o) {
+                    es += e;
+                    gs += g;
+                }
+            }
+            if (tid < npot) {
+                pent[tid] = es - sz;
+                gpre[tid + 1] = gs;
+            }
+            if (tid == 0) gpre[0] = 0;
+        }
+        __syncthreads();
+        const int64_t qo = a.q_off[item];
+        double *Q = a.Q + qo, *Sp = a.S_prev + qo;
+        const double *SC = a.scr + qo;
+        uint8_t *EF = a.eflag + qo;
+        int l1m = 0, l2m = 0;
+        for (int p = 0; p < npot; p++) {
+            l1m = max(l1m, pL[p] + la);
+            l2m = max(l2m, pL[p] + lb);
+        }
+        const long long t0 = clock64();
+        unsigned long long c_acc = 0;
+        const int G = gpre[npot], glo = (int)((int64_t)G * part / w.nparts), ghi = (int)((int64_t)G * (part + 1) / w.nparts);
+        {  // groups with an entry left by the screening, and what they need of each point
+            int n1 = -1, n2 = -1, nN = -1, mask = 0;
+            for (int gb = glo + (tid & ~31); gb < ghi; gb += NT) {
+                const int g = gb + lane;
+                int p = 0, loc = 0;
+                unsigned on = 0;
+                WalkGroup W{};
+                if (g < ghi) {
+                    while (gpre[p + 1] <= g) p++;
+                    loc = g - gpre[p];
+                    W = w.groups[pgrp[p] + loc];
+                    const uint8_t *E = EF + pent[p] + (W.l1 * (pL[p] + lb + 1) + W.l2) * dn + W.n0;
+                    for (int q = 0; q < W.cnt; q++)
+                        if (E[2 * q] & kEntActive) on |= 1u << q;
+                }
+                const unsigned keep = __ballot_sync(0xffffffffu, on != 0);
+                int at = 0;
+                if (lane == 0 && keep) at = atomicAdd(&s_cnt[0], __popc(keep));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (!on) continue;
+                lists[0][at + __popc(keep & ((1u << lane) - 1))] = (unsigned)p << 27 | (unsigned)loc << 4 | on;
+                n1 = max(n1, (int)W.l1);
+                n2 = max(n2, (int)W.l2);
+                nN = max(nN, W.n0 + 2 * (W.cnt - 1));
+                mask |= 1 << p;
+            }
+            if (mask) {
+                atomicMax(&s_need[1][0], n1);
+                atomicMax(&s_need[1][1], n2);
+                atomicMax(&s_need[1][2], nN);
+                atomicOr(&s_need[1][3], mask);
+            }
+        }
+        __syncthreads();
+        const double *FA = a.ftab + a.fp_off[a.item_fa[item]], *FB = a.ftab + a.fp_off[a.item_fb[item]];
+        const double *wug = a.wu + (int64_t)gr * a.wu_npot * kRadGridPts;
+        const double *rng = c_tab.grid + (size_t)kGridRowPow0 * kGridPts;
+        int any = 0;
+        for (int q0 = 0, npts = 0, cur = 0; q0 <= kRadGridPts; q0 += npts, cur ^= 1) {
+            const int nb = cur ^ 1, ncur = s_cnt[cur];
+            any = ncur > 0;
+            if (!any) break;
+            const int u1 = s_need[nb][0], u2 = s_need[nb][1], uN = s_need[nb][2], umask = s_need[nb][3];
+            // what this chunk refills: nobody reads it before the next barrier
+            if (tid < 4) s_need[cur][tid] = tid == 3 ? 0 : -1;
+            if (tid == 0) s_cnt[nb] = 0;
+            // ---- the chunk: points q0 .. q0 + npts - 1 of one level (levels 0..2 for q0 = 0), column x
+            // being walk-order point q0 + x - 1
+            const int nw = __popc(umask), rows = nw + u1 + u2 + uN + 3;
+            npts = kWalkPts;
+            if (q0 > 0) {
+                const int left = (2 << (31 - __clz(q0))) - q0;  // points to the end of the level
+                while (2 * npts <= min(left, kWalkMaxPts) && rows * (2 * npts + 2) <= w.chunk_doubles) npts *= 2;
+            }
+            const int rst = npts + 2;
+            double *cf1 = wsm + nw * rst, *cf2 = cf1 + (u1 + 1) * rst, *crn = cf2 + (u2 + 1) * rst;
+            for (int x = tid; x < npts; x += NT) {
+                const int f = max(q0 + x - 1, 0);
+                const bool dummy = q0 + x == 0;
+                double *d = wsm + x;
+                for (int m = umask; m; m &= m - 1, d += rst)
+                    copy8_async(d, wug + (int64_t)(__ffs(m) - 1) * kRadGridPts + f, dummy);
+                for (int l = 0; l <= u1; l++, d += rst) copy8_async(d, FA + (int64_t)l * kRadGridPts + f, false);
+                for (int l = 0; l <= u2; l++, d += rst) copy8_async(d, FB + (int64_t)l * kRadGridPts + f, false);
+                for (int n = 0; n <= uN; n++, d += rst) copy8_async(d, rng + (size_t)n * kGridPts + f, false);
+            }
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            // level that ends with this chunk (q0 = 0: levels 0..2): -1 if none
+            const int qe = q0 + npts, lend = (qe & (qe - 1)) == 0 ? 31 - __clz(qe) - 5 : -1;
+            int n1 = -1, n2 = -1, nN = -1, mask = 0, my_lvl = 0;
+            for (int k0 = tid & ~31; k0 < ncur; k0 += NT) {
+                // a warp's lanes run together: the list keeps groups of equal size side by side
+                const bool have = k0 + lane < ncur;
+                const unsigned id = lists[cur][have ? k0 + lane : k0];
+                const int p = id >> 27;
+                const WalkGroup W = w.groups[pgrp[p] + ((id >> 4) & 0x7fffff)];
+                unsigned act = have ? id & 15u : 0u;
+                const int e0 = pent[p] + (W.l1 * (pL[p] + lb + 1) + W.l2) * dn + W.n0;
+                double sm[kWalkN];
+                const double2 *pw = (const double2 *)(wsm + __popc(umask & ((1 << p) - 1)) * rst),
+                              *p1 = (const double2 *)(cf1 + W.l1 * rst), *p2 = (const double2 *)(cf2 + W.l2 * rst), *pn[kWalkN];
+#pragma unroll
+                for (int q = 0; q < kWalkN; q++) {
+                    const bool on = (act >> q) & 1u;
+                    sm[q] = on ? Q[e0 + 2 * q] : 0.0;
+                    // an entry that is not active takes a row that is there; its sum is not stored
+                    pn[q] = (const double2 *)(crn + (on ? W.n0 + 2 * q : 0) * rst);
+                }
+                int x = 0;
+                for (int seg = 0; seg < 3; seg++) {
+                    // q0 = 0: levels 0, 1, 2 end after 32, 64, 128 points; else the whole chunk
+                    const int xe = q0 == 0 ? 16 << seg : npts / 2;
+                    c_acc += (unsigned)(2 * (xe - x) - (q0 + x == 0)) * __popc(act);
+                    const int K = __reduce_max_sync(0xffffffffu, 32 - __clz(act));  // of the warp's largest group
+                    if (K == 4) walk_advance<4>(x, xe, pw, p1, p2, pn, sm);
+                    else if (K == 3) walk_advance<3>(x, xe, pw, p1, p2, pn, sm);
+                    else if (K == 2) walk_advance<2>(x, xe, pw, p1, p2, pn, sm);
+                    else if (K == 1) walk_advance<1>(x, xe, pw, p1, p2, pn, sm);
+                    x = xe;
+                    const int L = q0 == 0 ? seg : lend;
+                    if (L >= 0) {
+                        // end of level L (radial_type2_integral.c:285-315); an entry that has converged
+                        // keeps its sum
+#pragma unroll
+                        for (int q = 0; q < kWalkN; q++)
+                            if ((act >> q) & 1u) {
+                                const int en = e0 + 2 * q;
+                                bool conv = false;
+                                if (L > 0) {
+                                    const bool forced = (EF[en] & kEntScrOk) && (fabs(sm[q]) / fabs(SC[en]) < 0.001);
+                                    conv = !forced && fabs(sm[q] - Sp[en]) <= 1e-16;
+                                }
+                                if (conv) {
+                                    act &= ~(1u << q);
+                                    Q[en] = sm[q];
+                                    EF[en] &= (uint8_t)~kEntActive;
+                                    my_lvl = max(my_lvl, L);
+                                } else if (L < kRadMaxLevel) {
+                                    Sp[en] = sm[q];
+                                    sm[q] = 0.5 * sm[q];
+                                }
+                            }
+                    }
+                    if (q0 > 0) break;
+                }
+#pragma unroll
+                for (int q = 0; q < kWalkN; q++)
+                    if ((act >> q) & 1u) Q[e0 + 2 * q] = sm[q];
+                const unsigned keep = __ballot_sync(0xffffffffu, act != 0);
+                int at = 0;
+                if (lane == 0 && keep) at = atomicAdd(&s_cnt[nb], __popc(keep));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (act) {
+                    lists[nb][at + __popc(keep & ((1u << lane) - 1))] = (id & ~15u) | act;
+                    n1 = max(n1, (int)W.l1);
+                    n2 = max(n2, (int)W.l2);
+                    nN = max(nN, W.n0 + 2 * (31 - __clz(act)));
+                    mask |= 1 << p;
+                }
+            }
+            if (mask) {
+                atomicMax(&s_need[cur][0], n1);
+                atomicMax(&s_need[cur][1], n2);
+                atomicMax(&s_need[cur][2], nN);
+                atomicOr(&s_need[cur][3], mask);
+            }
+            if (my_lvl) atomicMax(&s_lvl, my_lvl);
+            __syncthreads();  // the next list and needs are complete; the rows are consumed
+        }
+        // deepest level walked: the cap if the last chunk was walked, else the last convergence
+        const int level_reached = any ? kRadMaxLevel : s_lvl;
+        if (tid == 0) {
+            if (w.nparts == 1 && a.stop_level) a.stop_level[item] = (int8_t)level_reached;
+            if (a.pred_level && level_reached > a.pred_level[item] + 1 &&
+                (!w.item_level || atomicMax(w.item_level + item, level_reached + 1) <= a.pred_level[item] + 2))
+                atomicAdd(a.fallback_count, 1);
+        }
+        if (a.counters) {
+            unsigned long long v = c_acc;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) atomicAdd(a.counters + kRadCntAccum, v);
+            if (tid == 0) atomicAdd(a.counters + kRadCntQuadCycles, (unsigned long long)(clock64() - t0));
+            if (tid == 0 && part == 0) {
+                // algorithmic work of the shared grid up to the stop level (every point once,
+                // every order and potential term at every point)
+                const unsigned long long pts = (unsigned long long)((1 << (level_reached + 5)) - 1);
+                const int np_a = a.rp_n[a.task_a[t]], np_b = a.rp_n[a.task_b[t]];
+                int terms = 0;
+                for (int p = 0; p < npot; p++) terms += a.pot_nprim[a.sl_pot[a.grpp_sl_off[gr] + p]];
+                atomicAdd(a.counters + kRadCntPoints, pts);
+                atomicAdd(a.counters + kRadCntBessel, pts * (unsigned long long)(np_a * (l1m + 1) + np_b * (l2m + 1)));
+                atomicAdd(a.counters + kRadCntPrimPts, pts * (unsigned long long)(np_a + np_b));
+                atomicAdd(a.counters + kRadCntTermPts, pts * (unsigned long long)terms);
+                atomicAdd(a.counters + kRadCntPowPts, pts * (unsigned long long)dn);
+                atomicAdd(a.counters + kRadCntItems, 1ull);
+                atomicAdd(a.counters + kRadCntLevels, (unsigned long long)(level_reached + 1));
+            }
+        }
+    }
+}
 #endif  // GRPP_RADIAL_TABLES_ONLY
 
 }  // namespace grpp
