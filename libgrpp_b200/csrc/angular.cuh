@@ -232,6 +232,7 @@ struct FinalArgs {
     const double *S_sph, *U_sph;
     const double *LS, *SL;            // [3][sph_tot] (oc_proj_kernel)
     int64_t sph_tot;
+    int arep_only;                    // 1: no outercore spin-orbit parts
     int raw_so;                       // 1: spin-orbit output without the 2/(2L+1) factor
     double *arep, *so_x, *so_y, *so_z;
     int *status;
@@ -880,6 +881,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 5 : (NT == 256 ? 3 : 1)) final
                     oa += farep * buf;
 #pragma unroll
                     for (int comp = 0; comp < 3; comp++) {
+                        if (a.arep_only) break;
                         // so_buf = U_a (L S_b) + (S_a L) U_b
                         const double *LSB = a.LS + comp * a.sph_tot + rB, *SLA = a.SL + comp * a.sph_tot + rA;
                         double t1 = 0.0, t2 = 0.0;
@@ -914,6 +916,7 @@ __global__ void __launch_bounds__(NT, NT == 128 ? 5 : (NT == 256 ? 3 : 1)) final
                             oa += (-1.0) * delta * farep * buf;
 #pragma unroll
                             for (int comp = 0; comp < 3; comp++) {
+                                if (a.arep_only) break;
                                 const double *LSB = a.LS + comp * a.sph_tot + rB;
                                 double t1 = 0.0;
                                 for (int m = 0; m < d; m++) t1 += SA[m] * LSB[m];

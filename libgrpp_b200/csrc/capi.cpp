@@ -15,7 +15,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <tuple>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/libgrpp.h"
@@ -801,20 +801,21 @@ int libgrpp_b200_grpp_gradient_contract_symmetric(const libgrpp_b200_batch_t *b,
             if (std::fabs(D[(int64_t)i * n_bf + j] - D[(int64_t)j * n_bf + i]) > 1e-14 * dmax)
                 return invalid("gradient contraction: the density matrix is not symmetric");
     // fold (a, b, c) and (b, a, c) onto a <= b
-    std::map<std::tuple<int, int, int>, int> seen;
+    std::unordered_map<int64_t, int> seen;
+    seen.reserve((size_t)b->n_tasks);
     std::vector<int> fa, fb, fc;
     std::vector<double> w;
     for (int64_t t = 0; t < b->n_tasks; t++) {
         const int a = std::min(b->task_a[t], b->task_b[t]), bb = std::max(b->task_a[t], b->task_b[t]), c = b->task_c[t];
-        auto it = seen.find({a, bb, c});
-        if (it == seen.end()) {
-            seen[{a, bb, c}] = (int)fa.size();
+        if (a < 0 || bb >= b->n_shells || c < 0 || c >= b->n_centres) return invalid("task index out of range");
+        const auto ins = seen.insert({((int64_t)a * b->n_shells + bb) * b->n_centres + c, (int)fa.size()});
+        if (ins.second) {
             fa.push_back(a);
             fb.push_back(bb);
             fc.push_back(c);
             w.push_back(1.0);
         } else {
-            w[it->second] += 1.0;
+            w[ins.first->second] += 1.0;
         }
     }
     libgrpp_b200_batch_t v = *b;
@@ -931,48 +932,49 @@ static int grad_contract_impl(const libgrpp_b200_batch_t *b, int radial_mode, co
     sub.cart_list = cart.data();
     grpp::RunOptions opt;
     opt.radial_mode = radial_mode;
-    const int64_t chunk = 16384;
+    opt.arep_only = arep_only;
+    // chunks of tasks: the host describes one while the GPU works on the one before
+    const int64_t chunk = 4096, n_chunks = (b->n_tasks + chunk - 1) / chunk;
     std::vector<int> ta, tb, tc;
-    std::vector<grpp::GradTaskHost> gt;
-    std::vector<double> out24;
-    for (int64_t t0 = 0; t0 < b->n_tasks; t0 += chunk) {
-        const int64_t t1 = std::min<int64_t>(b->n_tasks, t0 + chunk);
+    auto fill = [&](int64_t c, grpp::GradChunk &ch) {
+        const int64_t t0 = c * chunk, t1 = std::min<int64_t>(b->n_tasks, t0 + chunk);
         ta.clear();
         tb.clear();
         tc.clear();
-        gt.clear();
-        auto add = [&](int x, int y, int c) {
+        ch.tasks.clear();
+        auto add = [&](int x, int y, int cc) {
             ta.push_back(x);
             tb.push_back(y);
-            tc.push_back(c);
+            tc.push_back(cc);
             return (int)ta.size() - 1;
         };
         for (int64_t t = t0; t < t1; t++) {
-            const int a = b->task_a[t], bb = b->task_b[t], c = b->task_c[t];
+            const int a = b->task_a[t], bb = b->task_b[t], cc = b->task_c[t];
             grpp::GradTaskHost h;
-            h.t_ad = dn[a] >= 0 ? add(dn[a], bb, c) : -1;
-            h.t_au = add(up[a], bb, c);
-            h.t_bd = dn[bb] >= 0 ? add(a, dn[bb], c) : -1;
-            h.t_bu = add(a, up[bb], c);
+            h.t_ad = dn[a] >= 0 ? add(dn[a], bb, cc) : -1;
+            h.t_au = add(up[a], bb, cc);
+            h.t_bd = dn[bb] >= 0 ? add(a, dn[bb], cc) : -1;
+            h.t_bu = add(a, up[bb], cc);
             h.la = sL[a];
             h.lb = sL[bb];
             h.d_row = bf_off[a];
             h.d_col = bf_off[bb];
-            gt.push_back(h);
+            ch.tasks.push_back(h);
         }
-        sub.n_tasks = (int64_t)ta.size();
-        sub.task_a = ta.data();
-        sub.task_b = tb.data();
-        sub.task_c = tc.data();
-        out24.assign((size_t)(t1 - t0) * 24, 0.0);
-        const int rc = grpp::run_grad_contract(&sub, opt, gt.data(), t1 - t0, tab.data(), D, n_bf, out24.data());
-        if (rc) return rc;
-        // which atoms receive which side, with which sign (grpp_integrals_gradient.c:280-393)
+        ch.batch = sub;
+        ch.batch.n_tasks = (int64_t)ta.size();
+        ch.batch.task_a = ta.data();
+        ch.batch.task_b = tb.data();
+        ch.batch.task_c = tc.data();
+    };
+    // which atoms receive which side, with which sign (grpp_integrals_gradient.c:280-393)
+    auto consume = [&](int64_t c, const double *out24) {
+        const int64_t t0 = c * chunk, t1 = std::min<int64_t>(b->n_tasks, t0 + chunk);
         for (int64_t t = t0; t < t1; t++) {
-            const int a = b->task_a[t], bb = b->task_b[t], c = b->task_c[t];
-            const double *A = b->shell_origin + 3 * a, *B = b->shell_origin + 3 * bb, *C = b->centre_origin + 3 * c;
-            const int atoms[3] = {shell_atom[a], shell_atom[bb], centre_atom[c]};
-            const double *o = out24.data() + (t - t0) * 24;
+            const int a = b->task_a[t], bb = b->task_b[t], cc = b->task_c[t];
+            const double *A = b->shell_origin + 3 * a, *B = b->shell_origin + 3 * bb, *C = b->centre_origin + 3 * cc;
+            const int atoms[3] = {shell_atom[a], shell_atom[bb], centre_atom[cc]};
+            const double *o = out24 + (t - t0) * 24;
             const double wt = task_weight ? task_weight[t] : 1.0;
             const int nm = arep_only ? 1 : 4;
             for (int q = 0; q < 3; q++) {
@@ -986,8 +988,9 @@ static int grad_contract_impl(const libgrpp_b200_batch_t *b, int radial_mode, co
                 }
             }
         }
-    }
-    return 0;
+    };
+    return grpp::run_grad_contract(n_chunks, std::min<int64_t>(chunk, std::max<int64_t>(b->n_tasks, 1)), fill, consume, opt, tab.data(),
+                                   D, n_bf);
 }
 
 int libgrpp_b200_plan_learned_stats(const libgrpp_b200_plan_t *plan, double *ms_predict, int64_t *fallbacks)

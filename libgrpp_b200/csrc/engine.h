@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <array>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -13,6 +14,7 @@ namespace grpp {
 struct RunOptions {
     int radial_mode = LIBGRPP_B200_RADIAL_PLAIN;
     int raw_so = 0;          // spin-orbit output without the 2/(2L+1) factor (libgrpp_spin_orbit_integrals)
+    int arep_only = 0;       // outercore terms: the arep part only (spin-orbit outputs hold no outercore part)
     int fin_nt = 0;          // assembly block size for every task (128, 256, 512); 0: tuning table, else default rule
     int walk_parts = 0;      // blocks that share a task's grid walk; 0: by the batch's size
     int fin_by_class = 0;    // one assembly launch per class, each timed (autotuning)
@@ -62,8 +64,15 @@ struct GradTaskHost {
 };
 constexpr int kGradMaxL = 10;      // component table rows L = 0..10 (the engine's kMaxL)
 constexpr int kGradTabCart = 66;   // components of L = 10
-int run_grad_contract(const libgrpp_b200_batch_t *sub, const RunOptions &opt, const GradTaskHost *tasks,
-                      int64_t n_tasks, const int *cart_tab, const double *D, int64_t n_bf, double *out24);
+// one chunk of the task list: its sub-task batch (arrays owned by the caller until the next fill) and tasks
+struct GradChunk {
+    libgrpp_b200_batch_t batch;
+    std::vector<GradTaskHost> tasks;
+};
+using GradFill = std::function<void(int64_t, GradChunk &)>;
+using GradConsume = std::function<void(int64_t, const double *)>;
+int run_grad_contract(int64_t n_chunks, int64_t max_tasks, const GradFill &fill, const GradConsume &consume, const RunOptions &opt,
+                      const int *cart_tab, const double *D, int64_t n_bf);
 
 // one-electron integrals (onee.cuh): kind 0 overlap, 1 kinetic (out0), 2 momentum (out0..2)
 int run_onee_batch(const libgrpp_b200_batch_t *b, int kind, double *out0, double *out1, double *out2);

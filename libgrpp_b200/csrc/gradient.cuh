@@ -35,6 +35,7 @@ struct GradArgs {
     const double *out[4];        // sub-task blocks of the four matrices
     const double *D;             // n_bf x n_bf, row-major
     int64_t n_bf;
+    int nm;                      // matrices contracted: 4, or 1 (arep; the other sums are zero)
     double *g;                   // [n_tasks][2][3][4]
 };
 
@@ -43,7 +44,8 @@ __device__ __forceinline__ const int *cart_entry(const int *tab, int L, int i, i
     return tab + ((L * kGradMaxCart + i) * 3 + k) * 3;
 }
 
-// one warp per task; lanes over the Cartesian pairs (i, j)
+// one warp per task; lanes over the Cartesian pairs (i, j); NM of the four matrices
+template <int NM>
 __global__ void __launch_bounds__(128) grad_contract_kernel(GradArgs a)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -51,9 +53,9 @@ __global__ void __launch_bounds__(128) grad_contract_kernel(GradArgs a)
         const GradTask T = a.tasks[t];
         const int nA = ncart(T.la), nB = ncart(T.lb);
         const int nBu = ncart(T.lb + 1), nBd = T.lb > 0 ? ncart(T.lb - 1) : 0;
-        double acc[24];
+        double acc[6 * NM];  // [side][k][m]
 #pragma unroll
-        for (int q = 0; q < 24; q++) acc[q] = 0.0;
+        for (int q = 0; q < 6 * NM; q++) acc[q] = 0.0;
         for (int pr = lane; pr < nA * nB; pr += 32) {
             const int i = pr / nB, j = pr % nB;
             const double d = a.D[(T.d_row + i) * a.n_bf + T.d_col + j];
@@ -63,21 +65,21 @@ __global__ void __launch_bounds__(128) grad_contract_kernel(GradArgs a)
                 const int *eb = cart_entry(a.cart_tab, T.la, i, k);
                 const int *ek = cart_entry(a.cart_tab, T.lb, j, k);
 #pragma unroll
-                for (int m = 0; m < 4; m++) {
+                for (int m = 0; m < NM; m++) {
                     double vb = a.out[m][a.sub_off[T.t_au] + (int64_t)eb[1] * nB + j];
                     if (eb[0] > 0 && T.t_ad >= 0) vb -= eb[0] * a.out[m][a.sub_off[T.t_ad] + (int64_t)eb[2] * nB + j];
                     double vk = a.out[m][a.sub_off[T.t_bu] + (int64_t)i * nBu + ek[1]];
                     if (ek[0] > 0 && T.t_bd >= 0) vk -= ek[0] * a.out[m][a.sub_off[T.t_bd] + (int64_t)i * nBd + ek[2]];
-                    acc[k * 4 + m] += d * vb;
-                    acc[12 + k * 4 + m] += d * vk;
+                    acc[k * NM + m] += d * vb;
+                    acc[3 * NM + k * NM + m] += d * vk;
                 }
             }
         }
 #pragma unroll
-        for (int q = 0; q < 24; q++) {
+        for (int q = 0; q < 6 * NM; q++) {
             double v = acc[q];
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) a.g[(int64_t)t * 24 + q] = v;
+            if (lane == 0) a.g[(int64_t)t * 24 + q / NM * 4 + q % NM] = v;
         }
     }
 }

@@ -27,3 +27,42 @@ def test_task_alone_equals_batch(gpu_lib, system, pairs, mode):
         for m in range(4):
             want = ref[m][off[t]:off[t + 1]]
             assert np.max(np.abs(one[m] - want)) <= 1e-13 * max(np.max(np.abs(want)), 1e-300), (a, b, c, m)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_tasks", [4095, 4096, 4097, 9000])
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_gradient_of_a_long_list(gpu_lib, n_tasks, symmetric):
+    """The gradient runs its list in chunks, the host one chunk ahead: a list that repeats a few
+    tasks gives their weighted sum. n equal addends in any order: n eps of the addends' sum."""
+    S = synthetic.config2(9, n_heavy=1, n_h=2, lmax=2, box=7.0, l_proj=2)
+    a, b, c = S.all_tasks()
+    n = S.n_basis()
+    D = np.random.default_rng(4).uniform(-1, 1, (n, n))
+    D = 0.5 * (D + D.T)
+    pick = np.arange(min(7, len(a)))
+    idx = pick[np.arange(n_tasks) % len(pick)]
+    got = gpu_lib.grad_contract(S, S.batch(a[idx], b[idx], c[idx]), D, symmetric=symmetric)
+    want, size = np.zeros_like(got), np.zeros_like(got)
+    for k, cnt in zip(pick, np.bincount(idx, minlength=len(pick))):
+        one = gpu_lib.grad_contract(S, S.batch(a[k:k + 1], b[k:k + 1], c[k:k + 1]), D, symmetric=symmetric)
+        want += cnt * one
+        size += cnt * np.abs(one)
+    assert np.all(np.abs(got - want) <= n_tasks * 2.3e-16 * size + 1e-13 * size.max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("copies", [1, 227, 228, 400])
+def test_outputs_with_the_status_or_after_it(gpu_lib, copies):
+    """Up to 8192 numbers per array return with the status words, more are copied on their own
+    (a block of two d shells: 36 numbers, the line at 227 copies)."""
+    S = synthetic.config2(9, n_heavy=1, n_h=2, lmax=2, box=7.0, l_proj=2)
+    a, b, c = S.all_tasks()
+    ncart = np.array([(s.L + 1) * (s.L + 2) // 2 for s in S.shells])
+    k = int(np.argmax(ncart[a] * ncart[b]))
+    one = gpu_lib.full_grpp_batch(S.batch(a[k:k + 1], b[k:k + 1], c[k:k + 1]))
+    assert len(one[0]) == 36
+    many = gpu_lib.full_grpp_batch(S.batch(*[np.repeat(x[k:k + 1], copies) for x in (a, b, c)]))
+    for x, y in zip(one, many):
+        y = y.reshape(copies, 36)
+        assert np.max(np.abs(y - x)) <= 1e-13 * max(np.max(np.abs(x)), 1e-300)
