@@ -227,8 +227,8 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(cudaFuncSetAttribute(radial_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GRPP_CUDA(cudaFuncSetAttribute(radial_walk_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
     GRPP_CUDA(ang_set_final_max_smem((int)kFinSmemMax));
-    GRPP_CUDA(cudaFuncSetAttribute(type1_num_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(t1_smem_doubles(kT1MaxLam) * sizeof(double))));
+    GRPP_CUDA(cudaFuncSetAttribute(t1_assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(t1_assemble_smem(kT1MaxLam) * sizeof(double))));
     GRPP_CUDA(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mlp_train_smem_bytes()));
     GRPP_CUDA(cudaDeviceGetAttribute(&st.nsm, cudaDevAttrMultiProcessorCount, device));
     st.device = device;
@@ -2317,14 +2317,51 @@ int run_type1_numeric_batch(const libgrpp_b200_batch_t *b, int model, const doub
     cudaStream_t s = stp->stream;
     const int64_t nt = b->n_tasks, nout = k.off[nt];
     const int Lt = k.lmax_pair;
+    // chunks of consecutive tasks: up to kT1Scratch doubles of per-pair scratch and kT1Slots centres
+    struct T1Chunk {
+        int64_t t0, t1, s0, s1;
+    };
+    constexpr int64_t kT1Scratch = int64_t(1) << 25;
+    constexpr int kT1Slots = 1024;
+    std::vector<int64_t> unit_off(nt + 1, 0), group_off(nt + 1, 0), scr_off(nt);
+    std::vector<int> slot(nt), slot_centre, slot_of(nc, -1);
+    std::vector<T1Chunk> chunks{T1Chunk{0, 0, 0, 0}};
+    int64_t scr = 0, scr_max = 1, slots_max = 1;
+    for (int64_t t = 0; t < nt; t++) {
+        const int la = k.sL[k.ta[t]], lb = k.sL[k.tb[t]], c = k.tc[t];
+        const int64_t nu = (int64_t)k.snp[k.ta[t]] * k.snp[k.tb[t]], need = nu * (t1_nq(la + lb) + ncart(la) * ncart(lb));
+        const bool full = slot_of[c] < 0 && (int64_t)slot_centre.size() - chunks.back().s0 >= kT1Slots;
+        if (t > chunks.back().t0 && (full || scr + need > kT1Scratch)) {
+            for (int64_t q = chunks.back().s0; q < (int64_t)slot_centre.size(); q++) slot_of[slot_centre[q]] = -1;
+            chunks.push_back(T1Chunk{t, t, (int64_t)slot_centre.size(), 0});
+            scr = 0;
+        }
+        T1Chunk &ck = chunks.back();
+        if (slot_of[c] < 0) {
+            slot_of[c] = (int)((int64_t)slot_centre.size() - ck.s0);
+            slot_centre.push_back(c);
+        }
+        slot[t] = slot_of[c];
+        scr_off[t] = scr;
+        scr += need;
+        unit_off[t + 1] = unit_off[t] + nu;
+        group_off[t + 1] = group_off[t] + (nu + kT1Group - 1) / kT1Group;
+        ck.t1 = t + 1;
+        ck.s1 = (int64_t)slot_centre.size();
+        scr_max = std::max(scr_max, scr);
+        slots_max = std::max(slots_max, ck.s1 - ck.s0);
+    }
     const int64_t n_ang = (int64_t)(Lt + 1) * (2 * Lt + 1) * n_abc(Lt);
     OneeUpload u;
     const size_t oL = u.add(k.sL), onp = u.add(k.snp), opo = u.add(k.spo), oco = u.add(k.sco), opc = u.add(k.pc),
                  opa = u.add(k.pa), oso = u.add(k.so), ocart = u.add(k.cart), ota = u.add(k.ta), otb = u.add(k.tb),
                  otc = u.add(k.tc), ooff = u.add(k.off), ocor = u.add(cor), ocpar = u.add(cpar), ocpo = u.add(cpo),
-                 ocpn = u.add(cpn), oppw = u.add(ppw), opco = u.add(pco), opal = u.add(pal);
+                 ocpn = u.add(cpn), oppw = u.add(ppw), opco = u.add(pco), opal = u.add(pal), ouo = u.add(unit_off),
+                 ogo = u.add(group_off), oso2 = u.add(scr_off), oslot = u.add(slot), osc = u.add(slot_centre);
     const size_t in_bytes = u.used;
-    const size_t oang = u.reserve(n_ang * sizeof(double)), oout = u.reserve(nout * sizeof(double));
+    const size_t oang = u.reserve(n_ang * sizeof(double)), oout = u.reserve(nout * sizeof(double)),
+                 opts = u.reserve((size_t)(Lt + 2) * kT1Pts * sizeof(double)), owp = u.reserve(slots_max * kT1Pts * sizeof(double)),
+                 oscr = u.reserve(scr_max * sizeof(double));
     GRPP_CUDA(stp->onee.ensure(u.used));
     u.dev = (char *)stp->onee.p;
     GRPP_CUDA(cudaMemcpyAsync(u.dev, u.host.data(), in_bytes, cudaMemcpyHostToDevice, s));
@@ -2357,9 +2394,38 @@ int run_type1_numeric_batch(const libgrpp_b200_batch_t *b, int model, const doub
     a.tol = tol;
     a.pair_skip = pair_skip;
     a.out = u.at<double>(oout);
-    const size_t smem = (size_t)t1_smem_doubles(Lt) * sizeof(double);
-    type1_num_kernel<<<(int)std::min<int64_t>(nt, (int64_t)stp->nsm * 8), kT1Threads, smem, s>>>(a);
+    a.points = u.at<double>(opts);
+    a.wpot = u.at<double>(owp);
+    a.scratch = u.at<double>(oscr);
+    t1_points_kernel<<<kT1Pts / 128, 128, 0, s>>>(a);
     cudaError_t e = cudaGetLastError();
+    for (const T1Chunk &ck : chunks) {
+        Type1NumArgs c = a;
+        c.n_tasks = (int)(ck.t1 - ck.t0);
+        c.task_a += ck.t0;
+        c.task_b += ck.t0;
+        c.task_c += ck.t0;
+        c.out_off += ck.t0;
+        c.unit_off = u.at<int64_t>(ouo) + ck.t0;
+        c.group_off = u.at<int64_t>(ogo) + ck.t0;
+        c.scr_off = u.at<int64_t>(oso2) + ck.t0;
+        c.slot = u.at<int>(oslot) + ck.t0;
+        c.slot_centre = u.at<int>(osc) + ck.s0;
+        c.n_slots = (int)(ck.s1 - ck.s0);
+        const int64_t units = unit_off[ck.t1] - unit_off[ck.t0], groups = group_off[ck.t1] - group_off[ck.t0];
+        if (units > 0) {
+            t1_wpot_kernel<<<dim3(kT1Pts / 128, std::min(c.n_slots, 64)), 128, 0, s>>>(c);
+            const unsigned blocks = (unsigned)((units + kT1Warps - 1) / kT1Warps);
+            const size_t smem = (size_t)t1_radial_smem(Lt) * sizeof(double);
+            if (t1_nq(Lt) > 64) t1_radial_kernel<3><<<blocks, 32 * kT1Warps, smem, s>>>(c, units);
+            else if (t1_nq(Lt) > 32) t1_radial_kernel<2><<<blocks, 32 * kT1Warps, smem, s>>>(c, units);
+            else t1_radial_kernel<1><<<blocks, 32 * kT1Warps, smem, s>>>(c, units);
+            t1_assemble_kernel<<<(unsigned)std::min<int64_t>(groups, (int64_t)1 << 30), kT1AsmThreads,
+                                 (size_t)t1_assemble_smem(Lt) * sizeof(double), s>>>(c, groups);
+        }
+        t1_sum_kernel<<<(int)std::min<int64_t>(c.n_tasks, (int64_t)stp->nsm * 64), 128, 0, s>>>(c);
+        if (e == cudaSuccess) e = cudaGetLastError();
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, a.out, nout * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {

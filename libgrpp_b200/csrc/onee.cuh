@@ -10,19 +10,19 @@
 //   type1_ang_kernel   k-independent angular factors of the numeric type 1 integral,
 //                      A1[lambda][mu][IJK] = sum_rst y_{lambda mu, rst} I(I+r, J+s, K+t)
 //                      (libgrpp/angular_integrals.c:35-56), once per batch.
-//   type1_num_kernel   numeric type 1 integrals <A| V(|r - C|) |B> of a radially local
-//                      potential: a GRPP's U_L, or the electrostatic potential of a point,
-//                      charged-ball, Gaussian, Fermi or Fermi-bubble nucleus
-//                      (libgrpp/nuclear_models.c). libgrpp's per-primitive-pair scheme
-//                      (type1_integrals.c:144-270, radial_type1_integral.c:73-325): the
-//                      radial integrals Q(lambda, N) of the pair on the nested Log3 grid
-//                      (2047 -> 4095 -> 8191 points, stop at |S_L - S_{L-1}| <= tol), then the
-//                      binomial re-centring of both shells on C with the angular factors of
-//                      k = -2 (a CA + b CB). One CTA per shell pair, primitive pairs in order:
-//                      threads evaluate the integrand at 128 grid points per chunk, then one
-//                      thread per (lambda, N) entry adds the chunk's terms in point order, so
-//                      each sum is formed in libgrpp's order; threads own Cartesian pairs for
-//                      the angular assembly.
+//   numeric type 1 integrals <A| V(|r - C|) |B> of a radially local potential: a GRPP's U_L, or
+//                      the electrostatic potential of a point, charged-ball, Gaussian, Fermi or
+//                      Fermi-bubble nucleus (libgrpp/nuclear_models.c), by libgrpp's
+//                      per-primitive-pair scheme (type1_integrals.c:144-270,
+//                      radial_type1_integral.c:73-325): radial integrals Q(lambda, N) of the
+//                      pair on the nested Log3 grid (2047 -> 4095 -> 8191 points, stop at
+//                      |S_L - S_{L-1}| <= tol), then the binomial re-centring of both shells on
+//                      C with the angular factors of k = -2 (a CA + b CB). Five kernels:
+//   t1_points_kernel   r and r^N of the 8191 grid points, once per call
+//   t1_wpot_kernel     weight x potential at every point, once per centre
+//   t1_radial_kernel   Q(lambda, N): one warp per primitive pair, every sum in point order
+//   t1_assemble_kernel re-centring: one block per four primitive pairs of a task
+//   t1_sum_kernel      the pairs' contributions added in libgrpp's order
 #pragma once
 
 #include "angular.cuh"
@@ -145,8 +145,11 @@ __global__ void __launch_bounds__(32 * kOneeWarps) onee_os_kernel(OneeArgs a)
 }
 
 // ------------------------------------------------------------------ numeric type 1
-constexpr int kT1Threads = 128;
 constexpr int kT1MaxLam = 12;       // L_A + L_B <= 12
+constexpr int kT1Pts = 8192;        // row length of the point tables (8191 points in order of evaluation)
+constexpr int kT1Warps = 4;         // warps of a radial block
+constexpr int kT1Group = 4;         // primitive pairs of an assembly block
+constexpr int kT1AsmThreads = 128;
 
 struct Type1NumArgs {
     int n_tasks, model;
@@ -165,8 +168,34 @@ struct Type1NumArgs {
     int lmax_tab;
     double tol;                        // radial stop tolerance (libgrpp_params.radial_tolerance)
     double pair_skip;                  // primitive pairs with |c_i c_j| below it are skipped
+    // one chunk of tasks (the task arrays above and these start at it)
+    const int64_t *unit_off, *group_off;  // [n_tasks + 1] first primitive pair / assembly block of a task
+    const int64_t *scr_off;               // per task: doubles into scratch, [pair][nq + block size]
+    const int *slot;                      // per task: row of wpot
+    const int *slot_centre;
+    int n_slots;
+    double *points;                       // r, then r^0 .. r^lmax_tab: rows of kT1Pts
+    double *wpot;                         // [n_slots][kT1Pts]
+    double *scratch;
     double *out;
 };
+
+// Q(lambda, N) entries that the angular factors read: lambda of N's parity (for the others every
+// integral over the sphere has an odd power and vanishes)
+__host__ __device__ inline int t1_row(int lmax) { return lmax / 2 + 1; }
+__host__ __device__ inline int t1_nq(int lmax) { return (lmax + 1) * t1_row(lmax); }
+
+// the task of item u, off[t] <= u < off[t + 1] counted from off[0]
+__device__ __forceinline__ int t1_find(const int64_t *off, int n, int64_t u)
+{
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int m = (lo + hi) / 2;
+        if (off[m] - off[0] <= u) lo = m;
+        else hi = m;
+    }
+    return lo;
+}
 
 // A1 layout for lmax_tab = Lt: [lambda (0..Lt)][mu (0..2 Lt)][IJK index among I+J+K <= Lt]
 __host__ __device__ inline int64_t ang1_index(int Lt, int lam, int mu_off, int ijk)
@@ -203,201 +232,331 @@ __global__ void type1_ang_kernel(int Lt, double *A1)
     }
 }
 
-// dynamic shared memory of type1_num_kernel (doubles)
-__host__ __device__ inline int t1_smem_doubles(int lmax)
+// grid points of the three levels in order of evaluation: 2047, then 2048 and 4096 new ones
+__device__ __forceinline__ void t1_point(int q, double &r, double &w)
 {
-    const int ne = (lmax + 1) * (lmax + 1);
-    return kT1Threads * (1 + 2 * (lmax + 1))   // wpg, M_lambda, r^N per chunk point
-           + 3 * ne                             // running sums, previous level sums, active flags
-           + (lmax + 1) * (2 * lmax + 1)        // S_lambda,mu(k)
-           + (lmax + 1) * n_abc(lmax);          // omega[lambda][IJK]
+    const int nr = q < 2047 ? 2047 : (q < 4095 ? 4095 : 8191);
+    const int ip = q < 2047 ? q + 1 : (q < 4095 ? 2 * (q - 2047) + 1 : 2 * (q - 4095) + 1);
+    const double xi = ip / (nr + 1.0), xi3 = xi * xi * xi, ln = log(1 - xi3);
+    const double R = 5.0, R3 = R * R * R;
+    w = 3 * R3 * xi * xi * ln * ln / ((1 - xi3) * (nr + 1.0));
+    r = -R * ln;
 }
 
-__global__ void __launch_bounds__(kT1Threads) type1_num_kernel(Type1NumArgs a)
+__global__ void t1_points_kernel(Type1NumArgs a)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= kT1Pts - 1) return;
+    double r, w;
+    t1_point(q, r, w);
+    a.points[q] = r;
+    for (int n = 0; n <= a.lmax_tab; n++) a.points[(int64_t)(1 + n) * kT1Pts + q] = pow(r, (double)n);
+}
+
+__global__ void t1_wpot_kernel(Type1NumArgs a)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= kT1Pts - 1) return;
+    double r, w;
+    t1_point(q, r, w);
+    for (int s = blockIdx.y; s < a.n_slots; s += gridDim.y) {
+        const int C = a.slot_centre[s];
+        double pot;
+        if (a.model == kPotGrpp) {
+            pot = 0.0;
+            const int o = a.centre_pot_off[C];
+            const double r2 = r * r;
+            for (int u = 0; u < a.centre_pot_n[C]; u++)
+                pot = rn_add(pot, rn_mul(rn_mul(a.pot_coef[o + u], pow(r, (double)(a.pot_pow[o + u] - 2))),
+                                         exp(-a.pot_alpha[o + u] * r2)));
+        } else {
+            pot = nuclear_potential(a.model, a.centre_param + 4 * C, r, a.fermi);
+        }
+        a.wpot[(int64_t)s * kT1Pts + q] = w * pot;
+    }
+}
+
+// geometry of one primitive pair, as every kernel below forms it
+struct T1Pair {
+    double CA[3], CB[3], CA2, CB2, kv[3], k, ai, aj, ci, cj;
+    bool skip;
+};
+
+__device__ __forceinline__ T1Pair t1_pair(const Type1NumArgs &a, int A, int B, int C, int j)
+{
+    T1Pair p;
+    const double *oA = a.shell_origin + 3 * A, *oB = a.shell_origin + 3 * B, *oC = a.centre_origin + 3 * C;
+    const double CAx = oC[0] - oA[0], CAy = oC[1] - oA[1], CAz = oC[2] - oA[2];
+    const double CBx = oC[0] - oB[0], CBy = oC[1] - oB[1], CBz = oC[2] - oB[2];
+    p.CA2 = CAx * CAx + CAy * CAy + CAz * CAz;
+    p.CB2 = CBx * CBx + CBy * CBy + CBz * CBz;
+    const int nb = a.shell_nprim[B], i = j / nb, pa = a.shell_prim_off[A] + i, pb = a.shell_prim_off[B] + j - i * nb;
+    p.ci = a.prim_coef[pa];
+    p.cj = a.prim_coef[pb];
+    p.ai = a.prim_alpha[pa];
+    p.aj = a.prim_alpha[pb];
+    p.skip = fabs(p.ci * p.cj) < a.pair_skip;
+    const double kv[3] = {-2.0 * fma(p.ai, CAx, rn_mul(p.aj, CBx)), -2.0 * fma(p.ai, CAy, rn_mul(p.aj, CBy)),
+                          -2.0 * fma(p.ai, CAz, rn_mul(p.aj, CBz))};
+    p.k = sqrt(kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2]);
+    const double ca[3] = {CAx, CAy, CAz}, cb[3] = {CBx, CBy, CBz};
+    for (int d = 0; d < 3; d++) {
+        p.CA[d] = ca[d];
+        p.CB[d] = cb[d];
+        p.kv[d] = kv[d];
+    }
+    return p;
+}
+
+// Radial integrals, one warp per primitive pair: the lanes evaluate 32 points, then each lane adds
+// the 32 terms of its entries in point order, so every sum has libgrpp's order. Bound by the FP64
+// pipe (Bessel rows and the 2 operations per entry and point); the chain of additions of one pair
+// hides behind the other warps of the SM. A batch whose integrand underflows everywhere adds
+// zeros and is passed over. Before, a block walked all pairs of a task one after another with
+// one thread per entry, and evaluated the potential and the powers of r for every pair: 300 tasks
+// of s..f shells with 36 pairs each took 33.7 ms; 3.26 ms here and 0.13 ms in the kernels around it.
+// The kernels keep the operations of one pair's sums and factors as they were (k = -2 (a CA + b CB) with one
+// rounding of b CB included): re-centring amplifies their last bits by up to 1e7.
+template <int E>
+__global__ void __launch_bounds__(32 * kT1Warps) t1_radial_kernel(Type1NumArgs a, int64_t n_units)
+{
+    extern __shared__ double t1_sm[];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t u = (int64_t)blockIdx.x * kT1Warps + wp;
+    if (u >= n_units) return;
+    const int t = t1_find(a.unit_off, a.n_tasks, u), j = (int)(u - (a.unit_off[t] - a.unit_off[0]));
+    const int A = a.task_a[t], B = a.task_b[t];
+    const int la = a.shell_L[A], lb = a.shell_L[B], lmax = la + lb, nq = t1_nq(lmax);
+    const T1Pair p = t1_pair(a, A, B, a.task_c[t], j);
+    if (p.skip) return;
+    const double Dabc = 4 * kPi * gaussian_norm(la, p.ai) * gaussian_norm(lb, p.aj);
+    double *wr = t1_sm + wp * 2 * (a.lmax_tab + 1) * 33, *bes = wr + (lmax + 1) * 33;
+    const double *wpot = a.wpot + (int64_t)a.slot[t] * kT1Pts, *rp = a.points + kT1Pts;
+    double sum[E], prev[E];
+    bool act[E];
+    int rw[E], rb[E];
+#pragma unroll
+    for (int x = 0; x < E; x++) {
+        const int e = lane + 32 * x;
+        const int N = e / t1_row(lmax), lam = (N & 1) + 2 * (e - N * t1_row(lmax));
+        sum[x] = prev[x] = 0.0;
+        act[x] = e < nq && lam <= lmax;
+        rw[x] = act[x] ? N * 33 : 0;
+        rb[x] = act[x] ? lam * 33 : 0;
+    }
+    int base = 0;
+    for (int level = 0; level < 3; level++) {
+        const int npts = level == 0 ? 2047 : (level == 1 ? 2048 : 4096);
+        if (level > 0) {
+#pragma unroll
+            for (int x = 0; x < E; x++)
+                if (act[x]) {
+                    prev[x] = sum[x];
+                    sum[x] = 0.5 * sum[x];
+                }
+        }
+        for (int c0 = 0; c0 < npts; c0 += 32) {
+            const int q = base + c0 + lane;
+            const bool in = c0 + lane < npts;
+            double r = 1.0, wpg = 0.0;
+            if (in) {
+                r = a.points[q];
+                const double power = rn_add(rn_add(rn_add(rn_mul(p.k, r), -rn_mul(rn_mul(p.ai + p.aj, r), r)), -rn_mul(p.ai, p.CA2)),
+                                            -rn_mul(p.aj, p.CB2));
+                const double gto = Dabc * exp(power);
+                wpg = wpot[q] * gto;
+            }
+            if (!__any_sync(0xffffffffu, wpg != 0.0)) continue;
+            if (in) {
+                double M[kT1MaxLam + 1];
+                bessel_scaled_row<kT1MaxLam>(lmax, r * p.k, M);
+#pragma unroll
+                for (int l = 0; l <= kT1MaxLam; l++)
+                    if (l <= lmax) {
+                        bes[l * 33 + lane] = M[l];
+                        wr[l * 33 + lane] = rn_mul(wpg, rp[(int64_t)l * kT1Pts + q]);
+                    }
+            }
+            __syncwarp();
+            const int cn = min(32, npts - c0);
+            if (cn == 32) {
+#pragma unroll 8
+                for (int i = 0; i < 32; i++)
+#pragma unroll
+                    for (int x = 0; x < E; x++) {
+                        const double v = rn_add(sum[x], rn_mul(wr[rw[x] + i], bes[rb[x] + i]));
+                        if (act[x]) sum[x] = v;
+                    }
+            } else {
+                for (int i = 0; i < cn; i++)
+#pragma unroll
+                    for (int x = 0; x < E; x++) {
+                        const double v = rn_add(sum[x], rn_mul(wr[rw[x] + i], bes[rb[x] + i]));
+                        if (act[x]) sum[x] = v;
+                    }
+            }
+            __syncwarp();
+        }
+        base += npts;
+        if (level > 0) {
+            bool any = false;
+#pragma unroll
+            for (int x = 0; x < E; x++) {
+                if (act[x] && fabs(sum[x] - prev[x]) <= a.tol) act[x] = false;
+                any |= act[x];
+            }
+            if (!__any_sync(0xffffffffu, any)) break;
+        }
+    }
+    double *Q = a.scratch + a.scr_off[t] + (int64_t)j * (nq + ncart(la) * ncart(lb));
+#pragma unroll
+    for (int x = 0; x < E; x++)
+        if (lane + 32 * x < nq) Q[lane + 32 * x] = sum[x];
+}
+
+__host__ __device__ inline int t1_radial_smem(int lmax) { return kT1Warps * 2 * (lmax + 1) * 33; }
+__host__ __device__ inline int t1_assemble_smem(int lmax)
+{
+    return 6 * 8 + kT1Group * (3 * (lmax + 1) + (lmax + 1) * (lmax + 1) + n_abc(lmax)) + (n_abc(lmax) + 1) / 2;
+}
+
+// Binomial re-centring of both shells on C (type1_integrals.c:206-262). The inner sum over lambda
+// depends on (I, J, K) only, so it is tabulated per primitive pair before the components are
+// visited, and the binomial factors of a component are formed once for the block's four pairs.
+__global__ void __launch_bounds__(kT1AsmThreads) t1_assemble_kernel(Type1NumArgs a, int64_t n_groups)
 {
     extern __shared__ double t1_sm[];
     const int tid = threadIdx.x;
-    for (int t = blockIdx.x; t < a.n_tasks; t += gridDim.x) {
+    for (int64_t gi = blockIdx.x; gi < n_groups; gi += gridDim.x) {
+        const int t = t1_find(a.group_off, a.n_tasks, gi), j0 = (int)(gi - (a.group_off[t] - a.group_off[0])) * kT1Group;
         const int A = a.task_a[t], B = a.task_b[t], C = a.task_c[t];
         const int la = a.shell_L[A], lb = a.shell_L[B], nA = ncart(la), nB = ncart(lb), np = nA * nB;
-        const int lmax = la + lb, ne = (lmax + 1) * (lmax + 1);
-        double *wpg = t1_sm, *bes = wpg + kT1Threads, *rpw = bes + kT1Threads * (lmax + 1);
-        double *sum = rpw + kT1Threads * (lmax + 1), *prev = sum + ne, *act = prev + ne;
-        double *rsh = act + ne, *om = rsh + (lmax + 1) * (2 * lmax + 1);
-        const double *oA = a.shell_origin + 3 * A, *oB = a.shell_origin + 3 * B, *oC = a.centre_origin + 3 * C;
+        const int lmax = la + lb, nq = t1_nq(lmax), nijk = n_abc(lmax), nlm = (lmax + 1) * (lmax + 1);
+        const int nj = min(kT1Group, (int)(a.unit_off[t + 1] - a.unit_off[t]) - j0);
+        double *pw = t1_sm, *up = pw + 48, *rsh = up + kT1Group * 3 * (lmax + 1), *sq = rsh + kT1Group * nlm;
+        int *tij = (int *)(sq + kT1Group * nijk);  // index under lmax_tab, degree in the top byte
+        double *scr = a.scratch + a.scr_off[t] + (int64_t)j0 * (nq + np);
+        __syncthreads();
+        if (tid < 6) {
+            const T1Pair p = t1_pair(a, A, B, C, j0);
+            const double u = tid < 3 ? p.CA[tid] : p.CB[tid - 3];
+            for (int n = 0; n <= (tid < 3 ? la : lb); n++) pw[tid * 8 + n] = pow(u, (double)n);
+        } else if (tid >= 32 && tid < 32 + 3 * nj) {
+            // powers of the unit vector k/|k| (spherical_harmonics.c:172-220)
+            const int c = (tid - 32) / 3, d = (tid - 32) % 3;
+            const T1Pair p = t1_pair(a, A, B, C, j0 + c);
+            const double ux = p.k > kZeroThresh ? p.kv[d] / p.k : 0.0;
+            double v = 1.0;
+            for (int n = 0; n <= lmax; n++) {
+                up[(c * 3 + d) * (lmax + 1) + n] = v;
+                v *= ux;
+            }
+        }
+        for (int I = tid; I < (lmax + 1) * (lmax + 1); I += kT1AsmThreads) {
+            const int x = I / (lmax + 1), y = I - x * (lmax + 1);
+            for (int z = 0; x + y + z <= lmax; z++)
+                tij[abc_index(lmax, x, y, z)] = abc_index(a.lmax_tab, x, y, z) | (x + y + z) << 24;
+        }
+        __syncthreads();
+        for (int e = tid; e < nlm * nj; e += kT1AsmThreads) {
+            const int c = e / nlm, lm = e - c * nlm;
+            int l = (int)sqrtf((float)lm);
+            while (l * l > lm) l--;
+            while ((l + 1) * (l + 1) <= lm) l++;
+            const int mu = lm - l * l - l, nc = ncart(l);
+            const int8_t *cc = c_tab.rsh_comb + 3 * c_tab.rsh_comb_off[l];
+            const double *y = c_tab.rsh_coef + c_tab.rsh_off[l] + (mu + l) * nc;
+            const double *u = up + c * 3 * (lmax + 1);
+            double v = 0.0;
+            for (int q = 0; q < nc; q++)
+                v = rn_add(v, rn_mul(rn_mul(rn_mul(y[q], u[cc[3 * q]]), u[lmax + 1 + cc[3 * q + 1]]), u[2 * (lmax + 1) + cc[3 * q + 2]]));
+            rsh[e] = v;
+        }
+        __syncthreads();
+        for (int e = tid; e < nijk; e += kT1AsmThreads) {
+            const int ti = tij[e] & 0xffffff, N = tij[e] >> 24;
+            double s[kT1Group];
+            for (int c = 0; c < kT1Group; c++) s[c] = 0.0;
+            for (int l = N & 1; l <= lmax; l += 2) {
+                double om[kT1Group];
+#pragma unroll
+                for (int c = 0; c < kT1Group; c++) om[c] = 0.0;
+                for (int m = 0; m <= 2 * l; m++) {
+                    const double f = a.ang1[ang1_index(a.lmax_tab, l, m, ti)];
+                    if (f == 0.0) continue;
+#pragma unroll
+                    for (int c = 0; c < kT1Group; c++)
+                        if (c < nj) om[c] = rn_add(om[c], rn_mul(f, rsh[c * nlm + l * l + m]));
+                }
+#pragma unroll
+                for (int c = 0; c < kT1Group; c++)
+                    if (c < nj) {
+                        const double Q = scr[(int64_t)c * (nq + np) + N * t1_row(lmax) + l / 2];
+                        if (!(fabs(Q) < 1e-16)) s[c] = rn_add(s[c], rn_mul(om[c], Q));
+                    }
+            }
+#pragma unroll
+            for (int c = 0; c < kT1Group; c++) sq[c * nijk + e] = s[c];
+        }
+        __syncthreads();
+        double cc[kT1Group];
+        bool skip[kT1Group];
+#pragma unroll
+        for (int c = 0; c < kT1Group; c++) {
+            const T1Pair p = t1_pair(a, A, B, C, j0 + min(c, nj - 1));
+            cc[c] = p.ci * p.cj;
+            skip[c] = p.skip;
+        }
         const int8_t *ca = a.cart + 3 * a.shell_cart_off[A], *cb = a.cart + 3 * a.shell_cart_off[B];
-        const double *prm = a.centre_param + 4 * C;
-        double *out = a.out + a.out_off[t];
-        for (int p = tid; p < np; p += kT1Threads) out[p] = 0.0;
-        const double CAx = oC[0] - oA[0], CAy = oC[1] - oA[1], CAz = oC[2] - oA[2];
-        const double CBx = oC[0] - oB[0], CBy = oC[1] - oB[1], CBz = oC[2] - oB[2];
-        const double CA2 = CAx * CAx + CAy * CAy + CAz * CAz, CB2 = CBx * CBx + CBy * CBy + CBz * CBz;
-        const int pa = a.shell_prim_off[A], pb = a.shell_prim_off[B];
-        for (int i = 0; i < a.shell_nprim[A]; i++)
-            for (int j = 0; j < a.shell_nprim[B]; j++) {
-                const double ci = a.prim_coef[pa + i], cj = a.prim_coef[pb + j];
-                if (fabs(ci * cj) < a.pair_skip) continue;
-                const double ai = a.prim_alpha[pa + i], aj = a.prim_alpha[pb + j];
-                const double kv[3] = {-2.0 * (ai * CAx + aj * CBx), -2.0 * (ai * CAy + aj * CBy), -2.0 * (ai * CAz + aj * CBz)};
-                const double k = sqrt(kv[0] * kv[0] + kv[1] * kv[1] + kv[2] * kv[2]);
-                const double Dabc = 4 * kPi * gaussian_norm(la, ai) * gaussian_norm(lb, aj);
-                __syncthreads();
-                for (int e = tid; e < ne; e += kT1Threads) {
-                    sum[e] = 0.0;
-                    act[e] = 1.0;
-                }
-                // ---- radial integrals, level by level
-                int any = 1;
-                for (int level = 0; level < 3 && any; level++) {
-                    const int nr = level == 0 ? 2047 : (level == 1 ? 4095 : 8191);
-                    const int npts = level == 0 ? nr : (nr + 1) / 2;
-                    __syncthreads();
-                    if (level > 0)
-                        for (int e = tid; e < ne; e += kT1Threads)
-                            if (act[e] != 0.0) {
-                                prev[e] = sum[e];
-                                sum[e] = 0.5 * sum[e];
-                            }
-                    for (int c0 = 0; c0 < npts; c0 += kT1Threads) {
-                        __syncthreads();
-                        const int q = c0 + tid;
-                        if (q < npts) {
-                            const int ip = level == 0 ? q + 1 : 2 * q + 1;
-                            const double xi = ip / (nr + 1.0), xi3 = xi * xi * xi, ln = log(1 - xi3);
-                            const double R = 5.0, R3 = R * R * R;
-                            const double w = 3 * R3 * xi * xi * ln * ln / ((1 - xi3) * (nr + 1.0)), r = -R * ln;
-                            double pot;
-                            if (a.model == kPotGrpp) {
-                                pot = 0.0;
-                                const int o = a.centre_pot_off[C];
-                                const double r2 = r * r;
-                                for (int u = 0; u < a.centre_pot_n[C]; u++)
-                                    pot = rn_add(pot, rn_mul(rn_mul(a.pot_coef[o + u], pow(r, (double)(a.pot_pow[o + u] - 2))),
-                                                             exp(-a.pot_alpha[o + u] * r2)));
-                            } else {
-                                pot = nuclear_potential(a.model, prm, r, a.fermi);
-                            }
-                            const double power = rn_add(rn_add(rn_add(rn_mul(k, r), -rn_mul(rn_mul(ai + aj, r), r)),
-                                                               -rn_mul(ai, CA2)),
-                                                        -rn_mul(aj, CB2));
-                            const double gto = Dabc * exp(power);
-                            wpg[tid] = w * pot * gto;
-                            double M[kT1MaxLam + 1];
-                            bessel_scaled_row<kT1MaxLam>(lmax, r * k, M);
-                            for (int l = 0; l <= lmax; l++) bes[l * kT1Threads + tid] = M[l];
-                            for (int n = 0; n <= lmax; n++) rpw[n * kT1Threads + tid] = pow(r, (double)n);
-                        }
-                        __syncthreads();
-                        const int cn = min(kT1Threads, npts - c0);
-                        for (int e = tid; e < ne; e += kT1Threads) {
-                            if (act[e] == 0.0) continue;
-                            const int lam = e / (lmax + 1), n = e - lam * (lmax + 1);
-                            double s = sum[e];
-                            for (int u = 0; u < cn; u++)
-                                s = rn_add(s, rn_mul(rn_mul(wpg[u], rpw[n * kT1Threads + u]), bes[lam * kT1Threads + u]));
-                            sum[e] = s;
-                        }
-                    }
-                    __syncthreads();
-                    if (level > 0) {
-                        for (int e = tid; e < ne; e += kT1Threads)
-                            if (act[e] != 0.0 && fabs(sum[e] - prev[e]) <= a.tol) act[e] = 0.0;
-                        __syncthreads();
-                        any = 0;
-                        for (int e = 0; e < ne; e++)
-                            if (act[e] != 0.0) any = 1;
-                    }
-                }
-                __syncthreads();
-                // ---- angular factors at k/|k| (spherical_harmonics.c:172-220)
-                {
-                    const double len = k;
-                    double ux = 0.0, uy = 0.0, uz = 0.0;
-                    if (len > kZeroThresh) {
-                        ux = kv[0] / len;
-                        uy = kv[1] / len;
-                        uz = kv[2] / len;
-                    }
-                    const int st = 2 * lmax + 1;
-                    for (int e = tid; e < (lmax + 1) * st; e += kT1Threads) {
-                        const int l = e / st, mu = e % st - l;
-                        double v = 0.0;
-                        if (mu <= l) {
-                            const int nc = ncart(l);
-                            const int8_t *cc = c_tab.rsh_comb + 3 * c_tab.rsh_comb_off[l];
-                            const double *y = c_tab.rsh_coef + c_tab.rsh_off[l] + (mu + l) * nc;
-                            for (int q = 0; q < nc; q++) {
-                                double px = 1.0, py = 1.0, pz = 1.0;
-                                for (int s = 0; s < cc[3 * q]; s++) px *= ux;
-                                for (int s = 0; s < cc[3 * q + 1]; s++) py *= uy;
-                                for (int s = 0; s < cc[3 * q + 2]; s++) pz *= uz;
-                                v = rn_add(v, rn_mul(rn_mul(rn_mul(y[q], px), py), pz));
-                            }
-                        }
-                        rsh[e] = v;
-                    }
-                    __syncthreads();
-                    const int nijk = n_abc(lmax);
-                    for (int e = tid; e < (lmax + 1) * nijk; e += kT1Threads) {
-                        const int l = e / nijk, ijk = e - l * nijk;
-                        // (I, J, K) of the batch table index: the same triple under lmax_tab
-                        int I = 0, J = 0, K = 0, q = 0;
-                        for (int x = 0; x <= lmax && q <= ijk; x++)
-                            for (int y = 0; x + y <= lmax && q <= ijk; y++)
-                                for (int z = 0; x + y + z <= lmax && q <= ijk; z++, q++)
-                                    if (q == ijk) {
-                                        I = x;
-                                        J = y;
-                                        K = z;
-                                    }
-                        const int tij = abc_index(a.lmax_tab, I, J, K);
-                        double v = 0.0;
-                        for (int mu = -l; mu <= l; mu++)
-                            v = rn_add(v, rn_mul(a.ang1[ang1_index(a.lmax_tab, l, mu + l, tij)], rsh[l * st + mu + l]));
-                        om[e] = v;
-                    }
-                }
-                __syncthreads();
-                // ---- binomial re-centring of both shells on C (type1_integrals.c:206-262)
-                const double cc = ci * cj;
-                const int nijk = n_abc(lmax);
-                for (int p = tid; p < np; p += kT1Threads) {
-                    const int m = p / nB, n = p - m * nB;
-                    const int nxA = ca[3 * m], nyA = ca[3 * m + 1], nzA = ca[3 * m + 2];
-                    const int nxB = cb[3 * n], nyB = cb[3 * n + 1], nzB = cb[3 * n + 2];
-                    double chi = 0.0;
-                    for (int aa = 0; aa <= nxA; aa++) {
-                        const double C1 = c_tab.binom[nxA * kBinN + aa], P1 = pow(CAx, (double)(nxA - aa));
-                        for (int bb = 0; bb <= nyA; bb++) {
-                            const double C2 = c_tab.binom[nyA * kBinN + bb], P2 = pow(CAy, (double)(nyA - bb));
-                            for (int cq = 0; cq <= nzA; cq++) {
-                                const double C3 = c_tab.binom[nzA * kBinN + cq], P3 = pow(CAz, (double)(nzA - cq));
-                                for (int d = 0; d <= nxB; d++) {
-                                    const double C4 = c_tab.binom[nxB * kBinN + d], P4 = pow(CBx, (double)(nxB - d));
-                                    for (int e = 0; e <= nyB; e++) {
-                                        const double C5 = c_tab.binom[nyB * kBinN + e], P5 = pow(CBy, (double)(nyB - e));
-                                        for (int f = 0; f <= nzB; f++) {
-                                            const double C6 = c_tab.binom[nzB * kBinN + f], P6 = pow(CBz, (double)(nzB - f));
-                                            const double factor = C1 * C2 * C3 * C4 * C5 * C6 * P1 * P2 * P3 * P4 * P5 * P6;
-                                            if (fabs(factor) < 1e-13) continue;
-                                            const int N = aa + bb + cq + d + e + f;
-                                            const int ijk = abc_index(lmax, aa + d, bb + e, cq + f);
-                                            double sq = 0.0;
-                                            for (int lam = 0; lam <= lmax; lam++) {
-                                                const double Q = sum[lam * (lmax + 1) + N];
-                                                if (fabs(Q) < 1e-16) continue;
-                                                sq = rn_add(sq, rn_mul(om[lam * nijk + ijk], Q));
-                                            }
-                                            chi = rn_add(chi, rn_mul(factor, sq));
-                                        }
-                                    }
+        for (int p = tid; p < np; p += kT1AsmThreads) {
+            const int m = p / nB, n = p - m * nB;
+            const int nxA = ca[3 * m], nyA = ca[3 * m + 1], nzA = ca[3 * m + 2];
+            const int nxB = cb[3 * n], nyB = cb[3 * n + 1], nzB = cb[3 * n + 2];
+            double chi[kT1Group];
+#pragma unroll
+            for (int c = 0; c < kT1Group; c++) chi[c] = 0.0;
+            for (int aa = 0; aa <= nxA; aa++) {
+                const double C1 = c_tab.binom[nxA * kBinN + aa], P1 = pw[nxA - aa];
+                for (int bb = 0; bb <= nyA; bb++) {
+                    const double C2 = C1 * c_tab.binom[nyA * kBinN + bb], P2 = pw[8 + nyA - bb];
+                    for (int cq = 0; cq <= nzA; cq++) {
+                        const double C3 = C2 * c_tab.binom[nzA * kBinN + cq], P3 = pw[16 + nzA - cq];
+                        for (int d = 0; d <= nxB; d++) {
+                            const double C4 = C3 * c_tab.binom[nxB * kBinN + d], P4 = pw[24 + nxB - d];
+                            for (int e = 0; e <= nyB; e++) {
+                                const double C5 = C4 * c_tab.binom[nyB * kBinN + e], P5 = pw[32 + nyB - e];
+                                const double *row = sq + abc_index(lmax, aa + d, bb + e, cq);
+                                for (int f = 0; f <= nzB; f++) {
+                                    const double C6 = c_tab.binom[nzB * kBinN + f], P6 = pw[40 + nzB - f];
+                                    const double factor = C5 * C6 * P1 * P2 * P3 * P4 * P5 * P6;
+                                    if (fabs(factor) < 1e-13) continue;
+#pragma unroll
+                                    for (int c = 0; c < kT1Group; c++) chi[c] = rn_add(chi[c], rn_mul(factor, row[c * nijk + f]));
                                 }
                             }
                         }
                     }
-                    out[p] = rn_add(out[p], rn_mul(cc, chi));
                 }
             }
+#pragma unroll
+            for (int c = 0; c < kT1Group; c++)
+                if (c < nj) scr[(int64_t)c * (nq + np) + nq + p] = skip[c] ? 0.0 : rn_mul(cc[c], chi[c]);
+        }
+    }
+}
+
+// contributions of a task's primitive pairs, added in their order
+__global__ void t1_sum_kernel(Type1NumArgs a)
+{
+    for (int t = blockIdx.x; t < a.n_tasks; t += gridDim.x) {
+        const int la = a.shell_L[a.task_a[t]], lb = a.shell_L[a.task_b[t]], np = ncart(la) * ncart(lb), nq = t1_nq(la + lb);
+        const int nu = (int)(a.unit_off[t + 1] - a.unit_off[t]);
+        const double *scr = a.scratch + a.scr_off[t] + nq;
+        for (int p = threadIdx.x; p < np; p += blockDim.x) {
+            double v = 0.0;
+            for (int j = 0; j < nu; j++) v = rn_add(v, scr[(int64_t)j * (nq + np) + p]);
+            a.out[a.out_off[t] + p] = v;
+        }
     }
 }
 
