@@ -2,11 +2,11 @@
 //
 //   onee_os_kernel     overlap, kinetic energy and momentum blocks by the Obara-Saika
 //                      recurrences (libgrpp/overlap.c:39-139, kinetic.c:48-162,
-//                      momentum.c:48-181). One warp per shell pair: three lanes build the
-//                      per-axis tables S_ij (and D1_ij or D2_ij) of one primitive pair in
-//                      shared memory, then every lane owns Cartesian pairs of the block and
-//                      adds c_i c_j N_i N_j S S S with libgrpp's rounding (primitive pairs
-//                      outer, products left to right, no fused multiply-add).
+//                      momentum.c:48-181). One warp per shell pair: up to ten primitive pairs
+//                      at a time, one lane per pair and axis builds the tables S_ij (and D1_ij
+//                      or D2_ij) in shared memory, then every lane owns Cartesian pairs of
+//                      the block and adds c_i c_j N_i N_j S S S with libgrpp's rounding
+//                      (primitive pairs in order, products left to right, no fused multiply-add).
 //   type1_ang_kernel   k-independent angular factors of the numeric type 1 integral,
 //                      A1[lambda][mu][IJK] = sum_rst y_{lambda mu, rst} I(I+r, J+s, K+t)
 //                      (libgrpp/angular_integrals.c:35-56), once per batch.
@@ -47,100 +47,135 @@ struct OneeArgs {
 };
 
 constexpr int kOneeWarps = 4;
-constexpr int kOneeT = kMaxL + 3;  // table rows 0..L+2 (kinetic)
+constexpr int kOneeTab = 1350;  // doubles of tables per warp
+constexpr int kOneeQ = 10;      // primitive pairs at a time: three lanes each
+static_assert(3 * (((kMaxL + 3) * (kMaxL + 3) + (kMaxL + 1) * (kMaxL + 1)) | 1) <= kOneeTab, "tables of one primitive pair");
 
+// Bound by the chain of the recurrences and by issue of the component products, about evenly
+// at six or more primitive pairs. Before, three lanes built one primitive pair's tables while 29 waited, every
+// lane computed the norms, and each product was added to the block in global memory: every
+// ordered shell pair of 48 atoms (s..g) took 3.07 ms, 0.54 ms here. 1350 doubles hold six pairs of g
+// shells and leave room for five blocks on an SM.
 __global__ void __launch_bounds__(32 * kOneeWarps) onee_os_kernel(OneeArgs a)
 {
-    __shared__ double sS[kOneeWarps][3][kOneeT][kOneeT];
-    __shared__ double sD[kOneeWarps][3][kOneeT][kOneeT];
+    __shared__ double s_tab[kOneeWarps][kOneeTab];
+    __shared__ double s_fac[kOneeWarps][2 * kOneeQ];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ext = a.kind == kOneeKinetic ? 2 : (a.kind == kOneeMomentum ? 1 : 0);
+    double *tab = s_tab[w], *fac = s_fac[w];
     for (int t = blockIdx.x * kOneeWarps + w; t < a.n_tasks; t += gridDim.x * kOneeWarps) {
         const int A = a.task_a[t], B = a.task_b[t];
-        const int la = a.shell_L[A], lb = a.shell_L[B], nA = ncart(la), nB = ncart(lb), np = nA * nB;
-        const int ext = a.kind == kOneeKinetic ? 2 : (a.kind == kOneeMomentum ? 1 : 0);
+        const int la = a.shell_L[A], lb = a.shell_L[B], nB = ncart(lb), np = ncart(la) * nB;
         const double *oA = a.shell_origin + 3 * A, *oB = a.shell_origin + 3 * B;
         const int8_t *ca = a.cart + 3 * a.shell_cart_off[A], *cb = a.cart + 3 * a.shell_cart_off[B];
         double *o0 = a.out0 + a.out_off[t];
         double *o1 = a.kind == kOneeMomentum ? a.out1 + a.out_off[t] : nullptr;
         double *o2 = a.kind == kOneeMomentum ? a.out2 + a.out_off[t] : nullptr;
-        for (int p = lane; p < np; p += 32) {
-            o0[p] = 0.0;
-            if (o1) {
-                o1[p] = 0.0;
-                o2[p] = 0.0;
+        const int pa = a.shell_prim_off[A], pb = a.shell_prim_off[B], nb = a.shell_nprim[B], npr = a.shell_nprim[A] * nb;
+        // per pair and axis: S[ii][jj], rows of ws, then D[ii][jj], rows of wd
+        const int ws = lb + ext + 1, wd = lb + 1, nS = (la + ext + 1) * ws, axis = (nS + (la + 1) * wd) | 1;
+        const int nq = min(kOneeQ, kOneeTab / (3 * axis));
+        if (npr == 0)
+            for (int p = lane; p < np; p += 32) {
+                o0[p] = 0.0;
+                if (o1) {
+                    o1[p] = 0.0;
+                    o2[p] = 0.0;
+                }
+            }
+        for (int q0 = 0; q0 < npr; q0 += nq) {
+            const int cnt = min(nq, npr - q0);
+            __syncwarp();
+            if (lane < 3 * cnt) {
+                const int q = lane / 3, c = lane - 3 * q, i = (q0 + q) / nb, j = q0 + q - i * nb;
+                double *S = tab + lane * axis, *D = S + nS;
+                const double ai = a.prim_alpha[pa + i], aj = a.prim_alpha[pb + j];
+                const double p = ai + aj, mu = ai * aj / p;
+                const double P = rn_add(rn_mul(ai, oA[c]), rn_mul(aj, oB[c])) / p;
+                const double xab = oA[c] - oB[c], xpa = P - oA[c], xpb = P - oB[c], pf = 1.0 / (2.0 * p);
+                double s1 = sqrt(kPi / p) * exp(-mu * xab * xab), s2 = 0.0;
+                S[0] = s1;
+                for (int jj = 1; jj < ws; jj++) {
+                    double s = rn_mul(xpb, s1);
+                    if (jj > 1) s = rn_add(s, rn_mul(rn_mul(jj - 1, pf), s2));
+                    S[jj] = s;
+                    s2 = s1;
+                    s1 = s;
+                }
+                for (int ii = 1; ii <= la + ext; ii++) {
+                    const double fi = rn_mul(ii - 1, pf);
+                    double *r = S + ii * ws;
+#pragma unroll 4
+                    for (int jj = 0; jj < ws; jj++) {
+                        double s = rn_mul(xpa, r[jj - ws]);
+                        if (ii > 1) s = rn_add(s, rn_mul(fi, r[jj - 2 * ws]));
+                        if (jj > 0) s = rn_add(s, rn_mul(rn_mul(jj, pf), r[jj - ws - 1]));
+                        r[jj] = s;
+                    }
+                }
+                if (a.kind == kOneeKinetic) {
+                    for (int ii = 0; ii <= la; ii++)
+                        for (int jj = 0; jj <= lb; jj++) {
+                            double d = rn_mul(rn_mul(4.0 * ai, ai), S[(ii + 2) * ws + jj]);
+                            d = rn_add(d, -rn_mul(rn_mul(2.0 * ai, 2 * ii + 1), S[ii * ws + jj]));
+                            if (ii >= 2) d = rn_add(d, rn_mul(ii * (ii - 1), S[(ii - 2) * ws + jj]));
+                            D[ii * wd + jj] = d;
+                        }
+                } else if (a.kind == kOneeMomentum) {
+                    for (int ii = 0; ii <= la; ii++)
+                        for (int jj = 0; jj <= lb; jj++) {
+                            double d = rn_mul(2.0 * ai, S[(ii + 1) * ws + jj]);
+                            if (ii >= 1) d = rn_add(d, -rn_mul(ii, S[(ii - 1) * ws + jj]));
+                            D[ii * wd + jj] = d;
+                        }
+                }
+            }
+            if (lane < cnt) {
+                const int i = (q0 + lane) / nb, j = q0 + lane - i * nb;
+                const double NA = gaussian_norm(la, a.prim_alpha[pa + i]), NB = gaussian_norm(lb, a.prim_alpha[pb + j]);
+                fac[2 * lane] = rn_mul(a.prim_coef[pa + i], a.prim_coef[pb + j]);
+                fac[2 * lane + 1] = a.kind == kOneeOverlap ? rn_mul(NA, NB)
+                                                           : rn_mul(a.kind == kOneeKinetic ? -0.5 * NA : -NA, NB);
+            }
+            __syncwarp();
+            for (int p = lane; p < np; p += 32) {
+                const int m = p / nB, n = p - m * nB;
+                const int x1 = ca[3 * m], y1 = ca[3 * m + 1], z1 = ca[3 * m + 2];
+                const int x2 = cb[3 * n], y2 = cb[3 * n + 1], z2 = cb[3 * n + 2];
+                const double *Sx = tab + x1 * ws + x2, *Sy = tab + axis + y1 * ws + y2, *Sz = tab + 2 * axis + z1 * ws + z2;
+                const double *Dx = tab + nS + x1 * wd + x2, *Dy = tab + axis + nS + y1 * wd + y2,
+                             *Dz = tab + 2 * axis + nS + z1 * wd + z2;
+                double v0 = 0.0, v1 = 0.0, v2 = 0.0;
+                if (q0 > 0) {
+                    v0 = o0[p];
+                    if (o1) {
+                        v1 = o1[p];
+                        v2 = o2[p];
+                    }
+                }
+                for (int q = 0; q < cnt; q++) {
+                    const int o = 3 * q * axis;
+                    const double cc = fac[2 * q], f = fac[2 * q + 1], sx = Sx[o], sy = Sy[o], sz = Sz[o];
+                    if (a.kind == kOneeOverlap) {
+                        v0 = rn_add(v0, rn_mul(cc, rn_mul(rn_mul(rn_mul(f, sx), sy), sz)));
+                    } else if (a.kind == kOneeKinetic) {
+                        double s = rn_mul(rn_mul(Dx[o], sy), sz);
+                        s = rn_add(s, rn_mul(rn_mul(sx, Dy[o]), sz));
+                        s = rn_add(s, rn_mul(rn_mul(sx, sy), Dz[o]));
+                        v0 = rn_add(v0, rn_mul(cc, rn_mul(f, s)));
+                    } else {
+                        v0 = rn_add(v0, rn_mul(cc, rn_mul(rn_mul(rn_mul(f, Dx[o]), sy), sz)));
+                        v1 = rn_add(v1, rn_mul(cc, rn_mul(rn_mul(rn_mul(f, sx), Dy[o]), sz)));
+                        v2 = rn_add(v2, rn_mul(cc, rn_mul(rn_mul(rn_mul(f, sx), sy), Dz[o])));
+                    }
+                }
+                o0[p] = v0;
+                if (o1) {
+                    o1[p] = v1;
+                    o2[p] = v2;
+                }
             }
         }
-        double(*S)[kOneeT][kOneeT] = sS[w];
-        double(*D)[kOneeT][kOneeT] = sD[w];
-        const int pa = a.shell_prim_off[A], pb = a.shell_prim_off[B];
-        for (int i = 0; i < a.shell_nprim[A]; i++)
-            for (int j = 0; j < a.shell_nprim[B]; j++) {
-                const double ai = a.prim_alpha[pa + i], aj = a.prim_alpha[pb + j];
-                const double cc = rn_mul(a.prim_coef[pa + i], a.prim_coef[pb + j]);
-                __syncwarp();
-                if (lane < 3) {
-                    const int c = lane;
-                    const double p = ai + aj, mu = ai * aj / p;
-                    const double P = rn_add(rn_mul(ai, oA[c]), rn_mul(aj, oB[c])) / p;
-                    const double xab = oA[c] - oB[c], xpa = P - oA[c], xpb = P - oB[c], pf = 1.0 / (2.0 * p);
-                    for (int ii = 0; ii <= la + ext; ii++)
-                        for (int jj = 0; jj <= lb + ext; jj++) {
-                            double s = 0.0;
-                            if (ii + jj == 0) {
-                                s = sqrt(kPi / p) * exp(-mu * xab * xab);
-                            } else if (ii == 0) {
-                                s = rn_mul(xpb, S[c][0][jj - 1]);
-                                if (jj - 1 > 0) s = rn_add(s, rn_mul(rn_mul(jj - 1, pf), S[c][0][jj - 2]));
-                            } else {
-                                s = rn_mul(xpa, S[c][ii - 1][jj]);
-                                if (ii - 1 > 0) s = rn_add(s, rn_mul(rn_mul(ii - 1, pf), S[c][ii - 2][jj]));
-                                if (jj > 0) s = rn_add(s, rn_mul(rn_mul(jj, pf), S[c][ii - 1][jj - 1]));
-                            }
-                            S[c][ii][jj] = s;
-                        }
-                    if (a.kind == kOneeKinetic) {
-                        for (int ii = 0; ii <= la; ii++)
-                            for (int jj = 0; jj <= lb; jj++) {
-                                double d = rn_mul(rn_mul(4.0 * ai, ai), S[c][ii + 2][jj]);
-                                d = rn_add(d, -rn_mul(rn_mul(2.0 * ai, 2 * ii + 1), S[c][ii][jj]));
-                                if (ii >= 2) d = rn_add(d, rn_mul(ii * (ii - 1), S[c][ii - 2][jj]));
-                                D[c][ii][jj] = d;
-                            }
-                    } else if (a.kind == kOneeMomentum) {
-                        for (int ii = 0; ii <= la; ii++)
-                            for (int jj = 0; jj <= lb; jj++) {
-                                double d = rn_mul(2.0 * ai, S[c][ii + 1][jj]);
-                                if (ii >= 1) d = rn_add(d, -rn_mul(ii, S[c][ii - 1][jj]));
-                                D[c][ii][jj] = d;
-                            }
-                    }
-                }
-                __syncwarp();
-                const double NA = gaussian_norm(la, ai), NB = gaussian_norm(lb, aj), NN = rn_mul(NA, NB);
-                for (int p = lane; p < np; p += 32) {
-                    const int m = p / nB, n = p - m * nB;
-                    const int x1 = ca[3 * m], y1 = ca[3 * m + 1], z1 = ca[3 * m + 2];
-                    const int x2 = cb[3 * n], y2 = cb[3 * n + 1], z2 = cb[3 * n + 2];
-                    const double Sx = S[0][x1][x2], Sy = S[1][y1][y2], Sz = S[2][z1][z2];
-                    if (a.kind == kOneeOverlap) {
-                        const double v = rn_mul(rn_mul(rn_mul(NN, Sx), Sy), Sz);
-                        o0[p] = rn_add(o0[p], rn_mul(cc, v));
-                    } else if (a.kind == kOneeKinetic) {
-                        const double Dx = D[0][x1][x2], Dy = D[1][y1][y2], Dz = D[2][z1][z2];
-                        double s = rn_mul(rn_mul(Dx, Sy), Sz);
-                        s = rn_add(s, rn_mul(rn_mul(Sx, Dy), Sz));
-                        s = rn_add(s, rn_mul(rn_mul(Sx, Sy), Dz));
-                        const double v = rn_mul(rn_mul(-0.5 * NA, NB), s);
-                        o0[p] = rn_add(o0[p], rn_mul(cc, v));
-                    } else {
-                        const double Dx = D[0][x1][x2], Dy = D[1][y1][y2], Dz = D[2][z1][z2];
-                        const double mNN = rn_mul(-NA, NB);
-                        o0[p] = rn_add(o0[p], rn_mul(cc, rn_mul(rn_mul(rn_mul(mNN, Dx), Sy), Sz)));
-                        o1[p] = rn_add(o1[p], rn_mul(cc, rn_mul(rn_mul(rn_mul(mNN, Sx), Dy), Sz)));
-                        o2[p] = rn_add(o2[p], rn_mul(cc, rn_mul(rn_mul(rn_mul(mNN, Sx), Sy), Dz)));
-                    }
-                }
-            }
     }
 }
 
