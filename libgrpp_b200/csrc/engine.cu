@@ -1,8 +1,8 @@
 // GRPP engine: the single CUDA translation unit (device tables, kernels, host
 // orchestration of a batch of (shell A, shell B, centre C) tasks).
 //
-// Pipeline of one batch (kernels and uploads on the state's stream; the batched call's
-// downloads of finished chunks on a second stream):
+// Pipeline of one batch (uploads and the longest chain of kernels on the state's stream, the others
+// beside it, plan_launch_kernels; the batched call's downloads of finished chunks on a copy stream):
 //   1. atab_kernel    k-independent angular tensors, cached per device and (L, l)
 //   2. mmd_kernel     type 1 blocks <A|U_L|B> written straight into the arep output,
 //                     and <S|U_oc|oc>, <S|oc> Cartesian blocks for every (shell, centre)
@@ -116,7 +116,9 @@ struct DeviceState {
     bool ready = false;
     cudaStream_t stream = nullptr;       // all kernels and uploads
     cudaStream_t copy_stream = nullptr;  // downloads of finished chunks
-    cudaEvent_t ev[2][6];                // per buffer set: phase boundaries of one execution
+    cudaStream_t side[2] = {nullptr, nullptr};  // independent kernels of one execution (plan_launch)
+    cudaEvent_t side_ev[2][4];           // per buffer set: fork, walk inputs ready, the two side streams' ends
+    cudaEvent_t ev[2][7];                // per buffer set: phase boundaries of one execution
     cudaEvent_t done[2];                 // per buffer set: execution and its status copy finished
     cudaEvent_t uploaded[2];             // per buffer set: the staging buffer's last upload finished
     std::vector<void *> table_bufs;
@@ -197,10 +199,14 @@ int init_device_state(DeviceState &st, int device)
     GRPP_CUDA(upload_vec(st, h.fermi, &st.fermi));
     GRPP_CUDA(cudaMemcpyToSymbol(c_tab, &d, sizeof(d)));
     GRPP_CUDA(ang_upload_tables(&d, sizeof(d)));
-    GRPP_CUDA(cudaStreamCreateWithFlags(&st.stream, cudaStreamNonBlocking));
+    int prio_low = 0, prio_high = 0;
+    GRPP_CUDA(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
+    GRPP_CUDA(cudaStreamCreateWithPriority(&st.stream, cudaStreamNonBlocking, prio_high));
+    for (auto &q : st.side) GRPP_CUDA(cudaStreamCreateWithPriority(&q, cudaStreamNonBlocking, prio_low));
     GRPP_CUDA(cudaStreamCreateWithFlags(&st.copy_stream, cudaStreamNonBlocking));
     for (int k = 0; k < 2; k++) {
         for (auto &e : st.ev[k]) GRPP_CUDA(cudaEventCreate(&e));
+        for (auto &e : st.side_ev[k]) GRPP_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         GRPP_CUDA(cudaEventCreateWithFlags(&st.done[k], cudaEventDisableTiming));
         GRPP_CUDA(cudaEventCreateWithFlags(&st.uploaded[k], cudaEventDisableTiming));
         GRPP_CUDA(cudaHostAlloc((void **)&st.hstat[k], 16 * sizeof(int) + kRadCntNum * sizeof(unsigned long long),
@@ -557,6 +563,7 @@ struct Plan {
     const GradArgs *grad = nullptr;  // contraction to run after the assembly, its host arrays (page-locked)
     const void *grad_tasks = nullptr;
     double *grad_out = nullptr;
+    bool fork = false;  // independent kernels on the side streams
     bool send_outputs = false;  // copy the (small) outputs to the state's page-locked buffer with the status
     bool count_ops = false;  // run the type 1 kernel's counting instantiation
 };
@@ -1484,43 +1491,69 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     return 0;
 }
 
-// Enqueue one execution of a plan on the state's stream (no host synchronisation).
-int plan_launch(Plan &P)
+// Enqueue one execution of a plan (no host synchronisation): everything on the state's stream s, or,
+// with P.fork, on three streams that meet again on s:
+//   s        screening, (prediction), walk, assembly
+//   side[0]  type 1 items, outercore projections
+//   side[1]  potential and F_l tables (wanted by the walk), one-centre radial items, omega tables
+// The chain screening -> walk -> assembly is the longest; the others leave most of the chip idle on
+// small batches and fill the last waves of large ones. s has the higher priority, so their blocks
+// wait for its blocks. Kept plans run on s alone: their phase times are those of one kernel
+// after the other. One f x d block: 723 us on one
+// stream, 555 us here; a three-atom molecule 1.69 and 1.29 ms, a 5-atom one 6.5 and 4.5 ms; above 20 ms a few percent.
+static int plan_launch_kernels(Plan &P)
 {
     DeviceState &st = *P.st;
-    cudaStream_t s = st.stream;
-    cudaEvent_t *ev = st.ev[P.set];
-    if (P.n_tasks == 0) return 0;
+    cudaStream_t s = st.stream, sa = P.fork ? st.side[0] : s, sb = P.fork ? st.side[1] : s;
+    cudaEvent_t *ev = st.ev[P.set], *sev = st.side_ev[P.set];
+    const bool radial = P.rad_blocks > 0;
     GRPP_CUDA(cudaMemsetAsync(P.status, 0, 64 * sizeof(int), s));  // status, counters, assembly queues
     GRPP_CUDA(cudaEventRecord(ev[0], s));
-    if (P.mmd_blocks > 0) {
-        if (P.count_ops) mmd_kernel<true><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, s>>>(P.mmd);
-        else mmd_kernel<false><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, s>>>(P.mmd);
-        GRPP_CUDA(cudaGetLastError());
-    }
-    GRPP_CUDA(cudaEventRecord(ev[1], s));
-    if (P.ocp_blocks > 0) {
-        GRPP_CUDA(ang_launch_oc_proj(P.ocp_blocks, 64, s, &P.ocp, sizeof(P.ocp)));
-    }
-    if (P.rad_blocks > 0) {
+    auto type1 = [&]() -> int {
+        if (P.mmd_blocks > 0) {
+            if (P.count_ops) mmd_kernel<true><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
+            else mmd_kernel<false><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
+            GRPP_CUDA(cudaGetLastError());
+        }
+        GRPP_CUDA(cudaEventRecord(ev[1], sa));
+        if (!P.fork) GRPP_CUDA(cudaEventRecord(ev[6], s));
+        if (P.ocp_blocks > 0) GRPP_CUDA(ang_launch_oc_proj(P.ocp_blocks, 64, sa, &P.ocp, sizeof(P.ocp)));
+        return 0;
+    };
+    int rc = 0;
+    if (!P.fork && (rc = type1())) return rc;
+    if (radial) {
         GRPP_CUDA(cudaMemsetAsync(P.rad.walk, 0, (size_t)P.n_radial, s));
         GRPP_CUDA(cudaMemsetAsync(P.lm_ctl, 0, (16 + (P.wlk.item_level ? (size_t)P.n_radial : 0)) * sizeof(int), s));
         GRPP_CUDA(cudaMemsetAsync(P.rad.eflag, 0, (size_t)P.n_entries, s));  // unread entries stay inactive
+    }
+    if (P.fork) {
+        GRPP_CUDA(cudaEventRecord(ev[6], s));
+        GRPP_CUDA(cudaEventRecord(sev[0], s));
+        GRPP_CUDA(cudaStreamWaitEvent(sa, sev[0], 0));
+        GRPP_CUDA(cudaStreamWaitEvent(sb, sev[0], 0));
+    }
+    if (radial) {
         if (P.scru_blocks > 0) {
             radial_screen_unit_kernel<<<P.scru_blocks, 32 * kScrWarps, P.scru_smem, s>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
         }
+        if (P.wu) GRPP_CUDA(nofma_launch_wu_table(P.wu_blocks, 256, sb, &P.rad, sizeof(P.rad), P.wu_grpps, P.wu));
+        if (P.ftab) GRPP_CUDA(nofma_launch_ftab(P.ft_blocks, kRadThreads, P.ft_smem, sb, &P.rad, sizeof(P.rad), P.ftab));
+        if (P.fork) GRPP_CUDA(cudaEventRecord(sev[1], sb));
         if (P.scr_blocks > 0) {
-            radial_one_centre_kernel<<<P.scr_blocks, kRadThreads, 0, s>>>(P.rad);
+            radial_one_centre_kernel<<<P.scr_blocks, kRadThreads, 0, sb>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
         }
         GRPP_CUDA(cudaEventRecord(ev[4], s));
+    }
+    if (P.fork && (rc = type1())) return rc;
+    if (P.omtab && P.fork)
+        GRPP_CUDA(ang_launch_omega_tab(P.om_blocks, kFinThreads, P.om_smem, sb, &P.fin, sizeof(P.fin), &P.fin_smem_layout,
+                                       sizeof(P.fin_smem_layout), P.om_shell, P.om_centre, P.om_pairs, P.om_sl, P.omtab));
+    if (radial) {
         RadialArgs ra = P.rad;
         if (P.opt.radial_mode == LIBGRPP_B200_RADIAL_LEARNED) {
-            if (!st.lm_ready) {
-                set_error(LIBGRPP_B200_ERR_INVALID, "learned radial mode needs a level model (libgrpp_b200_set_level_model)");
-                return LIBGRPP_B200_ERR_INVALID;
-            }
             // predict every walked task's level, order deepest first, walk from the queue
             LevelModelDev lm{st.lm_norm, st.lm_w};
             const int pblocks = (int)std::min<int64_t>((P.n_radial + 3) / 4, (int64_t)st.nsm * 16);
@@ -1532,20 +1565,20 @@ int plan_launch(Plan &P)
             ra.pred_level = P.pred_level;
             GRPP_CUDA(cudaEventRecord(ev[5], s));
         }
-        if (P.wu) {
-            GRPP_CUDA(nofma_launch_wu_table(P.wu_blocks, 256, s, &P.rad, sizeof(P.rad), P.wu_grpps, P.wu));
-        }
-        if (P.ftab) {
-            GRPP_CUDA(nofma_launch_ftab(P.ft_blocks, kRadThreads, P.ft_smem, s, &P.rad, sizeof(P.rad), P.ftab));
-        }
+        if (P.fork) GRPP_CUDA(cudaStreamWaitEvent(s, sev[1], 0));
         if (P.walk_groups) radial_walk_group_kernel<<<P.rad_blocks, kWalkThreads, P.walk_smem, s>>>(ra, P.wlk);
         else radial_walk_kernel<<<P.rad_blocks, kRadThreads, P.rad_smem, s>>>(ra);
         GRPP_CUDA(cudaGetLastError());
     }
     GRPP_CUDA(cudaEventRecord(ev[2], s));
-    if (P.omtab) {
+    if (P.omtab && !P.fork)
         GRPP_CUDA(ang_launch_omega_tab(P.om_blocks, kFinThreads, P.om_smem, s, &P.fin, sizeof(P.fin), &P.fin_smem_layout,
                                        sizeof(P.fin_smem_layout), P.om_shell, P.om_centre, P.om_pairs, P.om_sl, P.omtab));
+    if (P.fork) {
+        GRPP_CUDA(cudaEventRecord(sev[2], sa));
+        GRPP_CUDA(cudaEventRecord(sev[3], sb));
+        GRPP_CUDA(cudaStreamWaitEvent(s, sev[2], 0));
+        GRPP_CUDA(cudaStreamWaitEvent(s, sev[3], 0));
     }
     for (size_t gi = 0; gi < P.fin_groups.size(); gi++) {
         const FinGroup &G = P.fin_groups[gi];
@@ -1577,6 +1610,19 @@ int plan_launch(Plan &P)
     return 0;
 }
 
+int plan_launch(Plan &P)
+{
+    if (P.n_tasks == 0) return 0;
+    if (P.rad_blocks > 0 && P.opt.radial_mode == LIBGRPP_B200_RADIAL_LEARNED && !P.st->lm_ready) {
+        set_error(LIBGRPP_B200_ERR_INVALID, "learned radial mode needs a level model (libgrpp_b200_set_level_model)");
+        return LIBGRPP_B200_ERR_INVALID;
+    }
+    const int rc = plan_launch_kernels(P);
+    if (rc && P.fork)  // what the side streams still run uses this set's buffers
+        for (cudaStream_t q : P.st->side) cudaStreamSynchronize(q);
+    return rc;
+}
+
 // Wait for a launched execution; its timings, counters and status.
 int plan_finish(Plan &P)
 {
@@ -1587,8 +1633,8 @@ int plan_finish(Plan &P)
     const int *hstatus = st.hstat[P.set];
     memcpy(P.stats.radial_counters, hstatus + 16, kRadCntNum * sizeof(unsigned long long));
     cudaEventElapsedTime(&P.stats.ms_mmd, ev[0], ev[1]);
-    cudaEventElapsedTime(&P.stats.ms_radial, ev[1], ev[2]);
-    if (P.rad_blocks > 0) cudaEventElapsedTime(&P.stats.ms_screen, ev[1], ev[4]);
+    cudaEventElapsedTime(&P.stats.ms_radial, ev[6], ev[2]);
+    if (P.rad_blocks > 0) cudaEventElapsedTime(&P.stats.ms_screen, ev[6], ev[4]);
     P.stats.ms_predict = 0.f;
     if (P.rad_blocks > 0 && P.opt.radial_mode == LIBGRPP_B200_RADIAL_LEARNED)
         cudaEventElapsedTime(&P.stats.ms_predict, ev[4], ev[5]);
@@ -1715,6 +1761,7 @@ int run_full_batch(const libgrpp_b200_batch_t *b, const RunOptions &opt, double 
         P[k] = Plan();
         rc = plan_build(*stp, &v, opt, false, P[k], k);
         if (rc) return rc;
+        P[k].fork = true;
         P[k].send_outputs = P[k].out_tot <= kSmallOut;
         rc = plan_launch(P[k]);
         if (rc) return rc;
@@ -2115,6 +2162,7 @@ int run_grad_contract(int64_t n_chunks, int64_t max_tasks, const GradFill &fill,
             ga.D = Dd;
             ga.n_bf = n_bf;
             ga.g = (double *)(dev + tab_b + d_b + 2 * task_b + k * out_b);
+            P[k].fork = true;
             P[k].grad = &ga;
             P[k].grad_tasks = host + k * task_b;
             P[k].grad_out = (double *)(host + 2 * task_b + k * out_b);

@@ -66,3 +66,30 @@ def test_outputs_with_the_status_or_after_it(gpu_lib, copies):
     for x, y in zip(one, many):
         y = y.reshape(copies, 36)
         assert np.max(np.abs(y - x)) <= 1e-13 * max(np.max(np.abs(x)), 1e-300)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("which", ["all", "one_centre", "local_only", "one_task"])
+def test_three_streams_equal_one(gpu_lib, which, mode):
+    """A batched call spreads its kernels over three streams, a kept plan runs them one after
+    another: the same operations in the same order, so the same bits."""
+    S = synthetic.moderate_heavy_system(3)
+    a, b, c = S.all_tasks()
+    if which == "one_centre":
+        at = np.array([[np.allclose(s.origin, x) for x, _ in S.centres] for s in S.shells])
+        keep = at[a, c] & at[b, c]
+        a, b, c = a[keep], b[keep], c[keep]
+    elif which == "local_only":
+        for g in S.grpps:
+            g.arep, g.so, g.oc = [], [], []
+    elif which == "one_task":
+        a, b, c = a[17:18], b[17:18], c[17:18]
+    batch = S.batch(a, b, c)
+    got = gpu_lib.full_grpp_batch(batch, mode)
+    plan = gpu_lib.plan(batch, mode)
+    plan.execute()
+    want = plan.outputs()
+    assert len(a) and max(np.abs(x).max() for x in want) > 0.0
+    for x, y in zip(got, want):
+        assert np.array_equal(x, y)
