@@ -12,17 +12,19 @@
 //     r_i = -5 ln(1 - x_i^3), levels of 31, 63, ..., 8191 points, stopping when
 //     |S_L - S_{L-1}| <= 1e-16 unless |S|/|estimate| < 1e-3, capped at 8191 points.
 //
-// GPU mapping, two kernels:
+// GPU mapping:
 //  * radial_screen_unit_kernel: one warp per run of entries of one (task, potential), lanes over
-//    primitive triples, triples that cannot matter dropped first; the gate decisions are
+//    entries, triples that cannot matter dropped first; the gate decisions are
 //    libgrpp's. One-centre tasks get their analytic table (radial_one_centre_kernel).
-//  * radial_walk_kernel: one CTA per task that has entries left. The grid is
-//    walked level by level in chunks of one point per thread; a point's
-//    integrand values
+//  * radial_walk_group_kernel: the grid walk of the tasks that have entries left, over tabulated
+//    integrands, a thread per group of entries.
+//  * radial_screen_kernel and radial_walk_kernel: the same by single entries and without tables
+//    (no-allocation path; the walk also for batches whose tables would be too large). One CTA
+//    per task; the grid is walked in chunks of one point per thread; a point's integrand values
 //      w U_p(r) for every potential, F^A_l, F^B_l for every order, r^N,
-//    are evaluated once and shared by all potentials and entries; every thread
-//    then advances the running sums of the entries it owns, point by point in
-//    the reference's order and association ((((w U) F1) F2) r^N).
+//    are evaluated once and shared by all potentials and entries; every thread then advances
+//    the running sums of the entries it owns, point by point in the reference's order and
+//    association ((((w U) F1) F2) r^N).
 #pragma once
 
 #include "grpp_common.cuh"
@@ -1269,12 +1271,14 @@ __device__ __forceinline__ void copy8_async(double *dst, const double *src, bool
                  : "memory");
 }
 
-// The sums of K entries over the point pairs x0..x1-1, each in point order: s += (((w U) F1) F2) r^N
+// The sums of K entries over the point pairs x0..x1-1, each in point order: s += (((w U) F1) F2) r^N.
+// Four pairs of points in flight hide the loads behind the additions where a block is alone on its
+// SM (one f x d block: call 535 us with two, 512 with four, 509 with eight; 65536 s..g tasks 80.3, 79.0, 79.5 ms).
 template <int K>
 __device__ __forceinline__ void walk_advance(int x0, int x1, const double2 *pw, const double2 *p1, const double2 *p2,
                                              const double2 *const *pn, double *s)
 {
-#pragma unroll(K > 2 ? 2 : 4)
+#pragma unroll 4
     for (int x = x0; x < x1; x++) {
         const double2 vw = pw[x], v1 = p1[x], v2 = p2[x];
         const double tx = __dmul_rn(__dmul_rn(vw.x, v1.x), v2.x), ty = __dmul_rn(__dmul_rn(vw.y, v1.y), v2.y);
