@@ -563,6 +563,7 @@ struct Plan {
     const GradArgs *grad = nullptr;  // contraction to run after the assembly, its host arrays (page-locked)
     const void *grad_tasks = nullptr;
     double *grad_out = nullptr;
+    int mmd_cnt_n = 0;  // type 1 items worked on by several blocks
     bool fork = false;  // independent kernels on the side streams
     bool send_outputs = false;  // copy the (small) outputs to the state's page-locked buffer with the status
     bool count_ops = false;  // run the type 1 kernel's counting instantiation
@@ -970,7 +971,12 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 }
     }
     // estimated work per type 1 item: primitive triples x (Hermite + R entries + contraction terms)
-    std::vector<int> mmd_order;
+    // Where the whole batch is a few items, the largest are cut into shares of their triples, so
+    // that no block has more than about a resident block's part of the work (and at least two
+    // groups of triples): XXMMD
+    std::vector<int4> mmd_units;
+    int64_t mmd_part_n = 0;
+    int mmd_cnt_n = 0;
     {
         std::vector<double> cost(items.size());
         for (size_t q = 0; q < items.size(); q++) {
@@ -982,7 +988,28 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 cost[q] = np2 * p_n[it.pot] *
                           (mmd_e_count(la, lb) + mmd_r_size(S) + pairs * (S + 3.0) * (S + 3.0) * (S + 3.0) / 27.0);
         }
-        mmd_order = order_by_cost(cost);
+        double total = 0.0;
+        for (double c : cost) total += c;
+        const double fair = total / (3.0 * st.nsm);
+        std::vector<int4> units;
+        std::vector<double> ucost;
+        for (size_t q = 0; q < items.size(); q++) {
+            const MmdItem &it = items[q];
+            const int64_t triples = (int64_t)sh_np[it.bra] * sh_np[it.ket] * (it.pot < 0 ? 1 : p_n[it.pot]);
+            int64_t n = 1;
+            if (cost[q] > fair) n = std::min<int64_t>({(int64_t)std::ceil(cost[q] / fair), triples / (2 * kMmdGroup), kMmdMaxParts});
+            n = std::max<int64_t>(n, 1);
+            for (int k = 0; k < n; k++) {
+                units.push_back(int4{(int)q, k | (int)n << 8, (int)mmd_part_n, mmd_cnt_n});
+                ucost.push_back(cost[q] / n);
+            }
+            if (n > 1) {
+                mmd_part_n += n * ncart(sh_L[it.bra]) * ncart(sh_L[it.ket]);
+                mmd_cnt_n++;
+            }
+        }
+        mmd_units.reserve(units.size());
+        for (int q : order_by_cost(ucost)) mmd_units.push_back(units[q]);
     }
 
     // omega tables per (shell, centre) pair (omega_tab_kernel): per semilocal potential of the
@@ -1172,7 +1199,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     const size_t o_fps = pk.add(fp_shell), o_fpc = pk.add(fp_centre), o_fpl = pk.add(fp_lmax), o_fpo = pk.add(fp_off),
                  o_ifa = pk.add(item_fa), o_ifb = pk.add(item_fb), o_omo = pk.add(om_off), o_tfa = pk.add(task_fpa),
                  o_tfb = pk.add(task_fpb);
-    const size_t o_mord = pk.add(mmd_order), o_ford = pk.add(fin_order);
+    const size_t o_mord = pk.add(mmd_units), o_ford = pk.add(fin_order);
     DevBuf *bin = own_buffers ? &P.in : &st.in[set], *bscr = own_buffers ? &P.scratch : &st.scratch[set],
            *bout = own_buffers ? &P.out : &st.out[set];
     GRPP_CUDA(bin->ensure(pk.size));
@@ -1199,7 +1226,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     if (wu_words * (int64_t)sizeof(double) > (int64_t(256) << 20)) wu_words = 0;
     const int64_t om_at = (3 * qn + 2 * cn + 2 * sn + 16 + 16 + flag_words + lm_words + wu_words + f_words + 1) & ~int64_t(1);
     const int64_t ls_at = om_at + om_words;  // 16-byte aligned omega tables, then the L matrix products
-    const size_t scratch_bytes = (size_t)(ls_at + 6 * sn) * sizeof(double);
+    const int64_t part_at = ls_at + 6 * sn;  // partial sums of shared type 1 items, their counters
+    const size_t scratch_bytes = (size_t)(part_at + mmd_part_n + (mmd_cnt_n + 1) / 2) * sizeof(double);
     GRPP_CUDA(bscr->ensure(scratch_bytes));
     GRPP_CUDA(bout->ensure((size_t)4 * std::max<int64_t>(out_tot, 1) * sizeof(double)));
     P.scratch_bytes = (int64_t)scratch_bytes;
@@ -1260,13 +1288,17 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         m.out[2] = Scd;
         m.counters = (unsigned long long *)(statusd + 16);
         m.pairs = at<int4>(ib, o_mpair);
-        m.order = at<int>(ib, o_mord);
+        m.units = at<int4>(ib, o_mord);
+        m.n_units = (int)mmd_units.size();
         m.queue = statusd + 8;
+        m.part_out = (double *)bscr->p + part_at;
+        m.part_cnt = (int *)(m.part_out + mmd_part_n);
+        P.mmd_cnt_n = mmd_cnt_n;
         P.mmd = m;
         // persistent grid: the resident blocks pop items until the queue is empty
         int mmd_occ = 0;
         GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<false>, kMmdThreads, mmd_smem));
-        P.mmd_blocks = (int)std::min<int64_t>((int64_t)items.size(), (int64_t)nsm * std::max(mmd_occ, 1));
+        P.mmd_blocks = (int)std::min<int64_t>((int64_t)mmd_units.size(), (int64_t)nsm * std::max(mmd_occ, 1));
         P.mmd_smem = mmd_smem;
     }
 
@@ -1511,6 +1543,7 @@ static int plan_launch_kernels(Plan &P)
     GRPP_CUDA(cudaEventRecord(ev[0], s));
     auto type1 = [&]() -> int {
         if (P.mmd_blocks > 0) {
+            if (P.mmd_cnt_n > 0) GRPP_CUDA(cudaMemsetAsync(P.mmd.part_cnt, 0, P.mmd_cnt_n * sizeof(int), sa));
             if (P.count_ops) mmd_kernel<true><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
             else mmd_kernel<false><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
             GRPP_CUDA(cudaGetLastError());

@@ -60,6 +60,7 @@ constexpr int kMmdMaxL = 8;               // largest angular momentum whose tabl
 constexpr int kMmdCls = kMmdMaxL + 1;
 constexpr int kMmdMaxPrims = 64;          // primitives per shell (the engine's limit)
 constexpr int kMmdMaxLgT = 6;
+constexpr int kMmdMaxParts = 16;          // shares of one item's triples
 constexpr int kMmdSmem = 70 * 1024;       // dynamic shared memory at most: three blocks per SM
 constexpr int kMmdGroup = 64;             // triples whose scalars and auxiliary values are formed together
 constexpr int kMmdRing = 512;             // live triples waiting: at most kMmdGroup - 1 + kMmdThreads
@@ -97,9 +98,15 @@ struct MmdArgs {
     // per class of (bra, ket) Cartesian tables, one int4 per pair (mmd_pair)
     const int4 *pairs;
     // dynamic schedule: blocks pop positions from *queue (zeroed before the launch) and take
-    // item order[position]; the host orders items by decreasing estimated work
-    const int *order;
+    // units[position]; the host orders them by decreasing estimated work. A unit is an item or, in
+    // small batches, one of up to kMmdMaxParts equal shares of its triples: x item, y share |
+    // number of shares << 8, z offset of the item's partial sums in part_out, w its counter in
+    // part_cnt (zeroed before the launch)
+    const int4 *units;
+    int n_units;
     int *queue;
+    double *part_out;
+    int *part_cnt;
 };
 
 __host__ __device__ inline int mmd_tet(int m) { return (m + 1) * (m + 2) * (m + 3) / 6; }
@@ -194,7 +201,8 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
     extern __shared__ double smem[];
     __shared__ int ring[kMmdRing];
     __shared__ int s_cnt[kMmdThreads / 32];
-    __shared__ int s_item;
+    __shared__ int4 s_unit;
+    __shared__ int s_last;
     __shared__ double normA[kMmdMaxPrims], normB[kMmdMaxPrims];
     __shared__ double rcp[2 * kMmdMaxL + 1];  // 1/t
     __shared__ unsigned long long s_fl;
@@ -205,12 +213,13 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
     for (;;) {
         if (tid == 0) {
             const int k = atomicAdd(a.queue, 1);
-            s_item = k < a.n_items ? a.order[k] : -1;
+            s_unit = k < a.n_units ? a.units[k] : int4{-1, 0, 0, 0};
         }
         __syncthreads();
-        const int it = s_item;
-        if (it < 0) break;
-        const MmdItem item = a.items[it];
+        const int4 unit = s_unit;
+        if (unit.x < 0) break;
+        const int part = unit.y & 255, nparts = unit.y >> 8;
+        const MmdItem item = a.items[unit.x];
         const MmdClass &cl = a.classes[item.cls];
         const int la = cl.la, lb = cl.lb, S = cl.S, npairs = ncart(la) * ncart(lb);
         const int G = mmd_sum_groups(cl);
@@ -250,13 +259,14 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
             const int lg = cl.lgT[kind], T = 1 << lg, tr = tid & (T - 1), e0 = tid >> lg, est = NT >> lg;
             const int nax = kind == 0 ? (la + 1) * (lb + 1) : mmd_e_axis(la, lb);
             double *R0 = E + cl.nE * T, *X = R0 + cl.nR0 * T, *Rb = X;  // kind 1; X shares the R levels' space
-            int head = 0, tail = 0, base = 0;
+            const int cend = (int)((int64_t)ncand * (part + 1) / nparts);
+            int head = 0, tail = 0, base = (int)((int64_t)ncand * part / nparts);
             for (;;) {
-                if (tail - head < GS && base < ncand) {
+                if (tail - head < GS && base < cend) {
                     // the next NT triples (term outer, primitive pair inner): keep the live ones, in order
                     const int c = base + tid;
                     bool live = false;
-                    if (c < ncand) {
+                    if (c < cend) {
                         const int k = c / np2, r = c - k * np2, i = r / npB, j = r - i * npB;
                         if (overlap || (!(fabs(cA[i]) < kZeroThresh) && !(fabs(cB[j]) < kZeroThresh))) {
                             const double al = xA[i], be = xB[j];
@@ -459,12 +469,28 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
         }
         __syncthreads();
         double *out = a.out[item.out_kind] + item.out_off;
+        double *po = a.part_out + unit.z;
         for (int p = tid; p < npairs; p += NT) {
             double s = acc[p * G];
             for (int g = 1; g < G; g++) s += acc[p * G + g];
-            out[__ldg(pt + p).w] = s;
+            if (nparts == 1) out[__ldg(pt + p).w] = s;
+            else po[part * npairs + p] = s;
         }
-        __syncthreads();  // acc and s_item are consumed
+        if (nparts > 1) {  // the share that comes last adds all of them, in order
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(a.part_cnt + unit.w, 1) == nparts - 1;
+            __syncthreads();
+            if (s_last) {
+                __threadfence();
+                for (int p = tid; p < npairs; p += NT) {
+                    double s = 0.0;
+                    for (int q = 0; q < nparts; q++) s += __ldcg(po + q * npairs + p);
+                    out[__ldg(pt + p).w] = s;
+                }
+            }
+        }
+        __syncthreads();  // acc and s_unit are consumed
     }
     if (COUNT && a.counters) {
         for (int o = 16; o > 0; o >>= 1) {

@@ -1,13 +1,14 @@
 """A task alone against the same task in a batch: small calls share an item's grid walk between
 blocks, cut the screening runs finer and take larger assembly blocks.
 
-Every sum that reaches an output has one order whatever the batch, except the screening estimates
-(their last bits decide nothing unless an estimate lies within them of a threshold, when one radial
+Every sum that reaches an output has one order whatever the batch, except the type 1 sums of items
+that several blocks share (last bits) and the screening estimates (their last bits decide nothing unless an estimate lies within them of a threshold, when one radial
 integral changes by its threshold, 1e-16): the tolerance is 1e-13 of the block's largest value."""
 import numpy as np
 import pytest
 
 from libgrpp_b200 import synthetic
+from libgrpp_b200.system import GRPP, Potential, Shell, System
 
 
 @pytest.mark.gpu
@@ -93,3 +94,24 @@ def test_three_streams_equal_one(gpu_lib, which, mode):
     assert len(a) and max(np.abs(x).max() for x in want) > 0.0
     for x, y in zip(got, want):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("la,lb,nprim", [(0, 0, 3), (1, 2, 8), (4, 3, 11), (6, 6, 5), (6, 6, 9)])
+def test_shared_type1_items(gpu_lib, la, lb, nprim):
+    """A few type 1 items are cut into shares of their triples, many are not: one task against 700
+    copies of it. Coefficients of one sign, so the shares' sums do not cancel: the orders differ
+    by at most n_triples eps of the terms, which the block's largest element bounds within a factor of 10."""
+    rng = np.random.default_rng(10 * la + lb + nprim)
+    al = lambda n: np.exp(rng.uniform(np.log(0.2), np.log(3.0), n))
+    A = Shell([0.0, 0.1, -0.2], la, rng.uniform(0.2, 1.0, nprim), al(nprim))
+    B = Shell([0.7, -0.3, 0.4], lb, rng.uniform(0.2, 1.0, nprim), al(nprim))
+    U = Potential(0, 0, [0, 1, 2, 2, 1], rng.uniform(0.5, 2.0, 5), al(5))
+    S = System(shells=[A, B], grpps=[GRPP(UL=U)], centres=[(np.array([0.2, 0.3, 0.1]), 0)])
+    task = [np.array([x], np.int32) for x in (0, 1, 0)]
+    one = gpu_lib.full_grpp_batch(S.batch(*task))[0]
+    many = gpu_lib.full_grpp_batch(S.batch(*[np.repeat(x, 700) for x in task]))[0].reshape(700, -1)
+    tol = 10 * 5 * nprim * nprim * 2.3e-16 * np.abs(one).max()
+    assert np.abs(one).max() > 0.0
+    assert np.all(many == many[0])
+    assert np.max(np.abs(many[0] - one)) <= tol
