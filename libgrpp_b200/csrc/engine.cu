@@ -1553,6 +1553,11 @@ static int plan_launch_kernels(Plan &P)
         if (P.ocp_blocks > 0) GRPP_CUDA(ang_launch_oc_proj(P.ocp_blocks, 64, sa, &P.ocp, sizeof(P.ocp)));
         return 0;
     };
+    auto tables = [&]() -> int {
+        if (P.wu) GRPP_CUDA(nofma_launch_wu_table(P.wu_blocks, 256, sb, &P.rad, sizeof(P.rad), P.wu_grpps, P.wu));
+        if (P.ftab) GRPP_CUDA(nofma_launch_ftab(P.ft_blocks, kRadThreads, P.ft_smem, sb, &P.rad, sizeof(P.rad), P.ftab));
+        return 0;
+    };
     int rc = 0;
     if (!P.fork && (rc = type1())) return rc;
     if (radial) {
@@ -1571,9 +1576,10 @@ static int plan_launch_kernels(Plan &P)
             radial_screen_unit_kernel<<<P.scru_blocks, 32 * kScrWarps, P.scru_smem, s>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
         }
-        if (P.wu) GRPP_CUDA(nofma_launch_wu_table(P.wu_blocks, 256, sb, &P.rad, sizeof(P.rad), P.wu_grpps, P.wu));
-        if (P.ftab) GRPP_CUDA(nofma_launch_ftab(P.ft_blocks, kRadThreads, P.ft_smem, sb, &P.rad, sizeof(P.rad), P.ftab));
-        if (P.fork) GRPP_CUDA(cudaEventRecord(sev[1], sb));
+        if (P.fork) {
+            if ((rc = tables())) return rc;
+            GRPP_CUDA(cudaEventRecord(sev[1], sb));
+        }
         if (P.scr_blocks > 0) {
             radial_one_centre_kernel<<<P.scr_blocks, kRadThreads, 0, sb>>>(P.rad);
             GRPP_CUDA(cudaGetLastError());
@@ -1598,7 +1604,9 @@ static int plan_launch_kernels(Plan &P)
             ra.pred_level = P.pred_level;
             GRPP_CUDA(cudaEventRecord(ev[5], s));
         }
+        // a kept plan's tables count as part of its walk
         if (P.fork) GRPP_CUDA(cudaStreamWaitEvent(s, sev[1], 0));
+        else if ((rc = tables())) return rc;
         if (P.walk_groups) radial_walk_group_kernel<<<P.rad_blocks, kWalkThreads, P.walk_smem, s>>>(ra, P.wlk);
         else radial_walk_kernel<<<P.rad_blocks, kRadThreads, P.rad_smem, s>>>(ra);
         GRPP_CUDA(cudaGetLastError());
