@@ -136,7 +136,7 @@ class ClockSampler:
 def cpu_reference_rate(batch_fn, n_sample: int, threads: int, seed: int = 0):
     """libgrpp (oracle/_ref) on a seeded sample of a step's tasks: (tasks/s, sample description)."""
     from libgrpp_b200.capi import LibGRPP
-    ref = LibGRPP(os.path.join(ROOT, "oracle", "_ref", "libgrpp_ref.so"))
+    ref = LibGRPP(REF_LIB)
     a, b, c = batch_fn()
     sel = np.sort(np.random.default_rng(seed).choice(len(a), n_sample, replace=False))
     batch = system().batch(a[sel], b[sel], c[sel])
@@ -162,7 +162,7 @@ def cpu_reference_stratified(S, a, b, c, per_class: int, threads: int, seed: int
     (tasks in the class) x (mean seconds per task of the class); the all-cores time as that
     over threads x efficiency. Returns the serial and all-cores tasks/s and a description."""
     from libgrpp_b200.capi import LibGRPP
-    ref = LibGRPP(os.path.join(ROOT, "oracle", "_ref", "libgrpp_ref.so"))
+    ref = LibGRPP(REF_LIB)
     cls = task_classes(S, a, b, c)
     rng = np.random.default_rng(seed)
     keys, counts = np.unique(cls, return_counts=True)
@@ -202,8 +202,15 @@ def host_threads():
         return os.cpu_count() or 1
 
 
+REF_LIB = os.path.join(ROOT, "oracle", "_ref", "libgrpp_ref.so")
+
+
 def run_reference(args, rank, world):
     if rank != 0:
+        return
+    if not os.path.exists(REF_LIB):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref (libgrpp compiled from its sources) is not built here"}),
+              flush=True)
         return
     threads = host_threads()
     S = system()
@@ -412,7 +419,9 @@ def run_ours(args, rank, world, local):
                          "kernel_ms_per_step": P["kernel_ms_per_step"], "clocks": P["clocks"]}
         line["learned_over_plain"] = R["value"] / P["value"]
         line["learned_fallbacks_per_step"] = R["fallbacks_per_step"]
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not os.path.exists(REF_LIB):
+        line["cpu_baseline"] = {"unavailable": "oracle/_ref (libgrpp compiled from its sources) is not built here"}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         threads = host_threads()
         r = cpu_reference_stratified(S, *step_tasks(idxs[0]), args.ref_per_class, threads)
         line["cpu_baseline"] = {"value": r["all_cores"], "unit": "tasks/s", "cores": threads, "kind": "reference",
@@ -422,7 +431,7 @@ def run_ours(args, rank, world, local):
     line["roofline"] = roofline(R["kernel_ms_per_step"], R["counters"], peak)
     line["roofline"]["traffic"] = TRAFFIC_PER_TASK.get(line["roofline"]["kernel"], 0.0) * n_tasks[0] or None
     if line["roofline"]["traffic"]:
-        line["roofline"]["traffic_source"] = TRAFFIC_SOURCE
+        line["roofline"]["traffic_source"] = TRAFFIC_SOURCE[line["roofline"]["kernel"]]
     if rank == 0 and world == 1 and not args.no_extra:
         # north_star's other workloads in the same run: the gradient (config 3) and the uneven batch (config 4)
         line["config3"], _ = gradient_leg(args, lib, local, flush, max(1, min(args.steps, 3)))
@@ -436,10 +445,13 @@ def run_ours(args, rank, world, local):
 
 # DRAM bytes per task of the dominant kernel, from one ncu capture of it (dram__bytes_read.sum +
 # dram__bytes_write.sum over the captured launch / its tasks); see profiles/
-TRAFFIC_PER_TASK = {"ms_screen": (15.772672e6 + 14.599936e6) / 4096}
-TRAFFIC_SOURCE = ("ncu --set full of radial_screen_unit_kernel (the screening of the long runs, about 85% of the "
-                  "screening time) on 4096 tasks of the first config-1 step: 30.37 MB DRAM read+write, scaled to "
-                  "the step's tasks (profiles/screen_unit_kernel_full_4096tasks.md)")
+TRAFFIC_PER_TASK = {"ms_screen": (22.991616e6 + 20.618496e6) / 4096, "ms_walk": (292.135168e6 + 21.524480e6) / 4096}
+TRAFFIC_SOURCE = {
+    "ms_screen": "ncu --set full of radial_screen_unit_kernel on 4096 tasks of the first config-1 step: 43.61 MB DRAM "
+                 "read+write, scaled to the step's tasks (profiles/screen_unit_kernel_full_4096tasks.md)",
+    "ms_walk": "ncu --set full of radial_walk_group_kernel on 4096 tasks of the first config-1 step: 313.66 MB DRAM "
+               "read+write from a cold L2, scaled to the step's tasks, an upper bound: the F_l tables are shared by more "
+               "tasks there (profiles/walk_group_kernel_full_4096tasks.md)"}
 
 # FLOP model of the radial path (count of FP64 add/mul, FMA = 2, each exp/pow/sqrt/log/erf = 1,
 # per operation of libgrpp's algorithm, libgrpp/radial_type2_integral.c and screening.c):
