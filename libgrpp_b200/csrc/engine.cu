@@ -973,7 +973,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     // estimated work per type 1 item: primitive triples x (Hermite + R entries + contraction terms)
     // Where the whole batch is a few items, the largest are cut into shares of their triples, so
     // that no block has more than about a resident block's part of the work (and at least two
-    // groups of triples): XXMMD
+    // groups of triples). All matrices of a 5-atom molecule with shells up to i (225 tasks, 435 items):
+    // the largest item kept one block busy for 1.4 ms; call 4.3 -> 3.1 ms. Large batches are not cut.
     std::vector<int4> mmd_units;
     int64_t mmd_part_n = 0;
     int mmd_cnt_n = 0;
