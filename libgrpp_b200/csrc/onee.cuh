@@ -185,6 +185,7 @@ constexpr int kT1Pts = 8192;        // row length of the point tables (8191 poin
 constexpr int kT1Warps = 4;         // warps of a radial block
 constexpr int kT1Group = 4;         // primitive pairs of an assembly block
 constexpr int kT1AsmThreads = 128;
+constexpr int kT1PowRow = kMaxL + 1; // powers 0..kMaxL of one component of CA or CB: one shell may have all of L_A + L_B
 
 struct Type1NumArgs {
     int n_tasks, model;
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(32 * kT1Warps) t1_radial_kernel(Type1NumArgs a
 __host__ __device__ inline int t1_radial_smem(int lmax) { return kT1Warps * 2 * (lmax + 1) * 33; }
 __host__ __device__ inline int t1_assemble_smem(int lmax)
 {
-    return 6 * 8 + kT1Group * (3 * (lmax + 1) + (lmax + 1) * (lmax + 1) + n_abc(lmax)) + (n_abc(lmax) + 1) / 2;
+    return 6 * kT1PowRow + kT1Group * (3 * (lmax + 1) + (lmax + 1) * (lmax + 1) + n_abc(lmax)) + (n_abc(lmax) + 1) / 2;
 }
 
 // Binomial re-centring of both shells on C (type1_integrals.c:206-262). The inner sum over lambda
@@ -468,14 +469,14 @@ __global__ void __launch_bounds__(kT1AsmThreads) t1_assemble_kernel(Type1NumArgs
         const int la = a.shell_L[A], lb = a.shell_L[B], nA = ncart(la), nB = ncart(lb), np = nA * nB;
         const int lmax = la + lb, nq = t1_nq(lmax), nijk = n_abc(lmax), nlm = (lmax + 1) * (lmax + 1);
         const int nj = min(kT1Group, (int)(a.unit_off[t + 1] - a.unit_off[t]) - j0);
-        double *pw = t1_sm, *up = pw + 48, *rsh = up + kT1Group * 3 * (lmax + 1), *sq = rsh + kT1Group * nlm;
+        double *pw = t1_sm, *up = pw + 6 * kT1PowRow, *rsh = up + kT1Group * 3 * (lmax + 1), *sq = rsh + kT1Group * nlm;
         int *tij = (int *)(sq + kT1Group * nijk);  // index under lmax_tab, degree in the top byte
         double *scr = a.scratch + a.scr_off[t] + (int64_t)j0 * (nq + np);
         __syncthreads();
         if (tid < 6) {
             const T1Pair p = t1_pair(a, A, B, C, j0);
             const double u = tid < 3 ? p.CA[tid] : p.CB[tid - 3];
-            for (int n = 0; n <= (tid < 3 ? la : lb); n++) pw[tid * 8 + n] = pow(u, (double)n);
+            for (int n = 0; n <= (tid < 3 ? la : lb); n++) pw[tid * kT1PowRow + n] = pow(u, (double)n);
         } else if (tid >= 32 && tid < 32 + 3 * nj) {
             // powers of the unit vector k/|k| (spherical_harmonics.c:172-220)
             const int c = (tid - 32) / 3, d = (tid - 32) % 3;
@@ -553,16 +554,16 @@ __global__ void __launch_bounds__(kT1AsmThreads) t1_assemble_kernel(Type1NumArgs
             for (int aa = 0; aa <= nxA; aa++) {
                 const double C1 = c_tab.binom[nxA * kBinN + aa], P1 = pw[nxA - aa];
                 for (int bb = 0; bb <= nyA; bb++) {
-                    const double C2 = C1 * c_tab.binom[nyA * kBinN + bb], P2 = pw[8 + nyA - bb];
+                    const double C2 = C1 * c_tab.binom[nyA * kBinN + bb], P2 = pw[kT1PowRow + nyA - bb];
                     for (int cq = 0; cq <= nzA; cq++) {
-                        const double C3 = C2 * c_tab.binom[nzA * kBinN + cq], P3 = pw[16 + nzA - cq];
+                        const double C3 = C2 * c_tab.binom[nzA * kBinN + cq], P3 = pw[2 * kT1PowRow + nzA - cq];
                         for (int d = 0; d <= nxB; d++) {
-                            const double C4 = C3 * c_tab.binom[nxB * kBinN + d], P4 = pw[24 + nxB - d];
+                            const double C4 = C3 * c_tab.binom[nxB * kBinN + d], P4 = pw[3 * kT1PowRow + nxB - d];
                             for (int e = 0; e <= nyB; e++) {
-                                const double C5 = C4 * c_tab.binom[nyB * kBinN + e], P5 = pw[32 + nyB - e];
+                                const double C5 = C4 * c_tab.binom[nyB * kBinN + e], P5 = pw[4 * kT1PowRow + nyB - e];
                                 const double *row = sq + abc_index(lmax, aa + d, bb + e, cq);
                                 for (int f = 0; f <= nzB; f++) {
-                                    const double C6 = c_tab.binom[nzB * kBinN + f], P6 = pw[40 + nzB - f];
+                                    const double C6 = c_tab.binom[nzB * kBinN + f], P6 = pw[5 * kT1PowRow + nzB - f];
                                     const double factor = C5 * C6 * P1 * P2 * P3 * P4 * P5 * P6;
                                     if (fabs(factor) < 1e-13) continue;
 #pragma unroll
