@@ -281,21 +281,24 @@ __device__ __forceinline__ double scr_gaussian_integral(int n, double p)
 // division (two Taylor sums or asymptotic series per side and a division before); relative error
 // below 3e-12 at every order. Below x = 1.25 libgrpp's own 4th-order
 // Taylor sums of M_l lose digits (down to 0/0 for high l near 0, an undefined estimate): there
-// its quotient is formed as libgrpp does. inv_x: 1/x, read for x > 16 only.
+// its quotient is formed as libgrpp does. inv_x: 1/x, read for x > 16 only. An undefined
+// estimate leaves r0 NaN (the entry is then walked): no table row is taken from a NaN, and scr_row
+// keeps every row number inside its table.
+__device__ __forceinline__ int scr_row(double g, unsigned n) { return (int)min(__double2uint_rz(g), n - 1u); }
 __device__ __forceinline__ double scr_poly(const double *c, double h)
 {
     return __ldg(c) + h * (__ldg(c + 1) + h * (__ldg(c + 2) + h * (__ldg(c + 3) + h * __ldg(c + 4))));
 }
 __device__ __forceinline__ double scr_t(int l, double x, double inv_x)
 {
-    if (x < kRatXmin) {
+    if (!(x >= kRatXmin)) {
         double num, den;
         scr_ratio_parts(l, x, num, den);
         return num * x / den;
     }
     // one polynomial for both ranges, so that lanes on either side of 16 stay together
     const bool lo = x <= 16.0;
-    const int i = lo ? (int)(x * 100.0 + 0.5) : (int)(inv_x * kRatYInv + 0.5);
+    const int i = scr_row(lo ? x * 100.0 + 0.5 : inv_x * kRatYInv + 0.5, lo ? kBesNX : kRatYN);
     const double h = lo ? x - i * 0.01 : inv_x - i * (1.0 / kRatYInv);
     return (lo ? 0.0 : x) + scr_poly((lo ? c_tab.ratio : c_tab.ratio_y) + (i * kRatL + l) * 5, h);
 }
@@ -303,14 +306,15 @@ __device__ __forceinline__ double scr_t(int l, double x, double inv_x)
 __device__ __forceinline__ double scr_m(int l, double x, double inv_x)
 {
     const bool lo = x <= 16.0;
-    const int i = lo ? (int)(x * 100.0 + 0.5) : (int)(inv_x * kBesYInv + 0.5);
+    const int i = scr_row(lo ? x * 100.0 + 0.5 : inv_x * kBesYInv + 0.5, lo ? kBesNX : kBesYN);
     const double h = lo ? x - i * 0.01 : inv_x - i * (1.0 / kBesYInv);
     return scr_poly((lo ? c_tab.bes_t : c_tab.bes_y) + (i * kRatL + l) * 5, h) * (lo ? 1.0 : 0.5 * inv_x);
 }
 
 // The envelope of screening.c:308-318 at the fixed point r0, with sqpi = sqrt(pi / p) and
-// sqp = sqrt(p). Every factor is finite and non-negative: a Gaussian factor that underflowed to
-// exactly 0 makes the product exactly 0, so the other factors are not needed; and 1 + erf(z) is
+// sqp = sqrt(p). Every factor is finite and non-negative where the Gaussian factor is positive; one that
+// underflowed to exactly 0 makes the product exactly 0, and a NaN one (r0 undefined) makes it NaN, so the other
+// factors are not needed there; and 1 + erf(z) is
 // exactly 2 once erfc(z) < 2^-54 (z > 5.9), taken here as p r0^2 > 36 (z > 6). The product keeps
 // libgrpp's order (screening.c:333-338).
 __device__ __forceinline__ double scr_envelope(int l1, int l2, int n, double CA, double CB, double aA, double aB,
@@ -319,7 +323,7 @@ __device__ __forceinline__ double scr_envelope(int l1, int l2, int n, double CA,
 {
     const double e1 = r0 - CA, e2 = r0 - CB;
     const double ex = exp(-eta * r0 * r0 - aA * e1 * e1 - aB * e2 * e2);
-    if (ex == 0.0) return 0.0;
+    if (!(ex > 0.0)) return ex;
     const double z2 = p * r0 * r0;
     const double erf_part = z2 > 36.0 ? 2.0 : 1 + erf(sqp * r0);
     const double ir = 1.0 / r0;
@@ -368,6 +372,26 @@ __device__ __forceinline__ void scr_store(const RadialArgs &a, int item, int64_t
         a.eflag[g] = kEntActive | (fail ? 0 : kEntScrOk);
         a.walk[item] = 1;
     }
+}
+
+// Whether a triple's estimate is below 1e-40 and its iteration ends at the first step, for every
+// entry with l1 <= l1m, l2 <= l2m and N between nlo and nhi (pw: the term's power; c: the triple's
+// coefficient). The bounds on the Bessel ratios hold for the tabulated values too when their
+// arguments are at least 0.5 (or the side's distance is 0, where entries with l > 0 are 0) and
+// the orders at most 16: their relative error is then below 1e-6, against a margin of 0.5%.
+__device__ __forceinline__ bool scr_dead(double CA, double CB, double aA, double aB, double eta, double c, int pw, int l1m,
+                                         int l2m, int nlo, int nhi)
+{
+    const double p = aA + aB + eta, inv_p = 1.0 / p, inv2p = 0.5 * inv_p;
+    const double r = (aA * CA + aB * CB) * inv_p, k1 = 2 * aA * CA, k2 = 2 * aB * CB;
+    const bool in1 = k1 * r >= 0.5, in2 = k2 * r >= 0.5;
+    if (!(in1 || k1 <= kZeroThresh) || !(in2 || k2 <= kZeroThresh) || !(in1 || in2) || l1m > 16 || l2m > 16) return false;
+    if (!((nhi + pw + l1m + l2m) * inv2p <= 0.0199 * r + 0.99e-4) || !((2 - nlo - pw) * inv2p <= 0.0199 * r - 1e-4)) return false;
+    const double eA = r - CA, eB = r - CB;
+    const float g = (float)(-eta * r * r - aA * eA * eA - aB * eB * eB);
+    const float b = 0.5f * __logf(3.1416f * (float)inv_p) + (nhi + pw) * __logf(fmaxf(1.f, (float)r + 0.01f)) +
+                    __logf(fmaxf((float)fabs(c), 1e-37f));
+    return g + b < -92.f;
 }
 
 #ifndef GRPP_RADIAL_TABLES_ONLY
@@ -430,26 +454,6 @@ constexpr int kScrArr = 13;     // staged scalars per triple
 // shared memory of a warp, in doubles: T_l [side][order][32], scalars, sums, then ints
 // (r power, waiting triples, failed entries)
 __host__ __device__ inline int scr_warp_doubles(int lw) { return 2 * lw * 32 + kScrArr * 32 + kScrRunMax + (32 + 64 + kScrRunMax) / 2; }
-
-// Whether a triple's estimate is below 1e-40 and its iteration ends at the first step, for every
-// entry with l1 <= l1m, l2 <= l2m and N between nlo and nhi (pw: the term's power; c: the triple's
-// coefficient). The bounds on the Bessel ratios hold for the tabulated values too when their
-// arguments are at least 0.5 (or the side's distance is 0, where entries with l > 0 are 0) and
-// the orders at most 16: their relative error is then below 1e-6, against a margin of 0.5%.
-__device__ __forceinline__ bool scr_dead(double CA, double CB, double aA, double aB, double eta, double c, int pw, int l1m,
-                                         int l2m, int nlo, int nhi)
-{
-    const double p = aA + aB + eta, inv_p = 1.0 / p, inv2p = 0.5 * inv_p;
-    const double r = (aA * CA + aB * CB) * inv_p, k1 = 2 * aA * CA, k2 = 2 * aB * CB;
-    const bool in1 = k1 * r >= 0.5, in2 = k2 * r >= 0.5;
-    if (!(in1 || k1 <= kZeroThresh) || !(in2 || k2 <= kZeroThresh) || !(in1 || in2) || l1m > 16 || l2m > 16) return false;
-    if (!((nhi + pw + l1m + l2m) * inv2p <= 0.0199 * r + 0.99e-4) || !((2 - nlo - pw) * inv2p <= 0.0199 * r - 1e-4)) return false;
-    const double eA = r - CA, eB = r - CB;
-    const float g = (float)(-eta * r * r - aA * eA * eA - aB * eB * eB);
-    const float b = 0.5f * __logf(3.1416f * (float)inv_p) + (nhi + pw) * __logf(fmaxf(1.f, (float)r + 0.01f)) +
-                    __logf(fmaxf((float)fabs(c), 1e-37f));
-    return g + b < -92.f;
-}
 
 __global__ void __launch_bounds__(32 * kScrWarps, 5) radial_screen_unit_kernel(RadialArgs a)
 {
