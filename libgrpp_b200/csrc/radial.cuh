@@ -389,8 +389,9 @@ __device__ __forceinline__ bool scr_dead(double CA, double CB, double aA, double
     if (!((nhi + pw + l1m + l2m) * inv2p <= 0.0199 * r + 0.99e-4) || !((2 - nlo - pw) * inv2p <= 0.0199 * r - 1e-4)) return false;
     const double eA = r - CA, eB = r - CB;
     const float g = (float)(-eta * r * r - aA * eA * eA - aB * eB * eB);
+    const float cm = (float)fabs(c);  // NaN stays NaN: such a triple is kept, as an infinite one is
     const float b = 0.5f * __logf(3.1416f * (float)inv_p) + (nhi + pw) * __logf(fmaxf(1.f, (float)r + 0.01f)) +
-                    __logf(fmaxf((float)fabs(c), 1e-37f));
+                    __logf(cm <= 1e-37f ? 1e-37f : cm);
     return g + b < -92.f;
 }
 

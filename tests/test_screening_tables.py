@@ -3,7 +3,8 @@ undefined-behaviour checks, over the tables of tables.cpp, every read checked ag
 
 libgrpp's quotient of two Bessel functions is 0/0 for orders l >= 6 at 1e-7 < x < 0.005, so the fixed
 point, the arguments k r and 1/(k r) may be NaN or infinite. A row number is never formed from those
-without a limit, an undefined r0 gives an undefined estimate, r0 = inf one of 0."""
+without a limit, an undefined r0 gives an undefined estimate, r0 = inf one of 0, and a triple whose
+coefficient is not finite is not dropped."""
 import os
 import shutil
 import subprocess
@@ -90,8 +91,9 @@ int main()
                         for (double r0 : {1e-320, 1e-9, 0.3, 5.0, 40.0}) env(r0);
                         env(0.0);
                     }
-    // a far, tight triple is dropped
+    // a far, tight triple is dropped, unless its coefficient is not finite
     for (double c : {0.0, 1.0, -1e3, 1e-300}) REQUIRE(scr_dead(3.0, 4.0, 50.0, 60.0, 20.0, c, 0, 2, 2, 0, 2));
+    for (double c : {nan, inf, -inf}) REQUIRE(!scr_dead(3.0, 4.0, 50.0, 60.0, 20.0, c, 0, 2, 2, 0, 2));
     REQUIRE(!scr_dead(3.0, 4.0, nan, 60.0, 20.0, 1.0, 0, 2, 2, 0, 2));
     std::printf("ok\n");
     return 0;

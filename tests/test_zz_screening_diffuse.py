@@ -2,7 +2,10 @@
 l >= 6, arguments below 0.005) and the estimate undefined: those entries are walked. Against the
 no-allocation path, which screens with libgrpp's expressions entry by entry; the tolerance of record,
 max(1e-10, 1e-9 |ref|). Shells within 1.2 bohr of the centre, much less than their extent, so that the
-re-centring sums keep their digits (the largest of them is 30 times the block's largest element)."""
+re-centring sums keep their digits.
+
+A potential whose coefficient is NaN makes every element of its blocks NaN, also where none of its
+triples could have mattered."""
 import numpy as np
 import pytest
 
@@ -32,3 +35,14 @@ def test_undefined_estimates_are_walked(gpu_lib, l_proj, eta):
     print(f"projector {l_proj}, exponents {eta:g}: max abs {err.max():.2e} of {np.abs(want).max():.2e}")
     assert np.all(np.isfinite(want)) and np.abs(want).max() > 0.0
     assert np.all(err <= strict_tol(want)), float((err / strict_tol(want)).max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("distance", [1.0, 30.0])
+def test_nan_coefficient_reaches_the_result(gpu_lib, distance):
+    xyz = np.array([0.0, 0.3, 1.0]) * distance
+    shells = [Shell(xyz, l, [0.7, 0.4], [3.0, 8.0]) for l in (0, 1)]
+    arep = [Potential(1, 0, [2, 2], [1.0, np.nan], [5.0, 9.0])]
+    S = System(shells, [GRPP(arep=arep)], [(np.zeros(3), 0)])
+    out = gpu_lib.full_grpp_batch(S.batch(*S.all_tasks()))[0]
+    assert np.all(np.isnan(out))
