@@ -1468,7 +1468,6 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         f.pot_L = at<int>(ib, o_pL);
         f.Q = Qd;
         f.atab_off = (const int64_t *)st.atab_off_dev.p;
-        f.atab = (const double *)st.atab.p;
         f.proj_off = at<int64_t>(ib, o_poffp);
         f.S_sph = Ssd;
         f.U_sph = Usd;
@@ -1540,6 +1539,7 @@ static int plan_launch_kernels(Plan &P)
     cudaStream_t s = st.stream, sa = P.fork ? st.side[0] : s, sb = P.fork ? st.side[1] : s;
     cudaEvent_t *ev = st.ev[P.set], *sev = st.side_ev[P.set];
     const bool radial = P.rad_blocks > 0;
+    P.fin.atab = (const double *)st.atab.p;  // a batch built after a kept plan may have moved the tensors (ensure_atab)
     GRPP_CUDA(cudaMemsetAsync(P.status, 0, 64 * sizeof(int), s));  // status, counters, assembly queues
     GRPP_CUDA(cudaEventRecord(ev[0], s));
     auto type1 = [&]() -> int {
