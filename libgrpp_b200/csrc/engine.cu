@@ -215,8 +215,8 @@ int init_device_state(DeviceState &st, int device)
     for (int k = 0; k < 2; k++)
         GRPP_CUDA(cudaHostAlloc((void **)&st.hout[k], 4 * kSmallOut * sizeof(double), cudaHostAllocDefault));
     st.atab_off.assign((kMaxL + 2) * (kMaxL + 2), -1);
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmdSmem));
-    GRPP_CUDA(cudaFuncSetAttribute(mmd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmdSmem));
+    for (auto kernel : {mmd_kernel<false, false>, mmd_kernel<false, true>, mmd_kernel<true, true>})
+        GRPP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMmdSmem));
     MmdTables mt;
     mmd_build_classes(mt);
     st.mmd_cls = mt.classes;
@@ -971,10 +971,10 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 }
     }
     // estimated work per type 1 item: primitive triples x (Hermite + R entries + contraction terms)
-    // Where the whole batch is a few items, the largest are cut into shares of their triples, so
-    // that no block has more than about a resident block's part of the work (and at least two
-    // groups of triples). All matrices of a 5-atom molecule with shells up to i (225 tasks, 435 items):
-    // the largest item kept one block busy for 1.4 ms; call 4.3 -> 3.1 ms. Large batches are not cut.
+    // Where the whole batch is a few items, the parts of the largest are shared out, so that no block has
+    // more than about a resident block's part of the work (and at least a group of triples). All matrices
+    // of a 5-atom molecule with shells up to i (225 tasks, 435 items): the largest item kept one block busy
+    // for 1.4 ms; call 4.3 -> 2.5 ms. Large batches are not shared out.
     std::vector<int4> mmd_units;
     int64_t mmd_part_n = 0;
     int mmd_cnt_n = 0;
@@ -998,14 +998,14 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             const MmdItem &it = items[q];
             const int64_t triples = (int64_t)sh_np[it.bra] * sh_np[it.ket] * (it.pot < 0 ? 1 : p_n[it.pot]);
             int64_t n = 1;
-            if (cost[q] > fair) n = std::min<int64_t>({(int64_t)std::ceil(cost[q] / fair), triples / (2 * kMmdGroup), kMmdMaxParts});
+            if (cost[q] > fair) n = std::min<int64_t>({(int64_t)std::ceil(cost[q] / fair), triples / kMmdGroup, kMmdMaxShares});
             n = std::max<int64_t>(n, 1);
             for (int k = 0; k < n; k++) {
                 units.push_back(int4{(int)q, k | (int)n << 8, (int)mmd_part_n, mmd_cnt_n});
                 ucost.push_back(cost[q] / n);
             }
             if (n > 1) {
-                mmd_part_n += n * ncart(sh_L[it.bra]) * ncart(sh_L[it.ket]);
+                mmd_part_n += (int64_t)kMmdMaxParts * ncart(sh_L[it.bra]) * ncart(sh_L[it.ket]);
                 mmd_cnt_n++;
             }
         }
@@ -1298,7 +1298,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         P.mmd = m;
         // persistent grid: the resident blocks pop items until the queue is empty
         int mmd_occ = 0;
-        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<false>, kMmdThreads, mmd_smem));
+        GRPP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&mmd_occ, mmd_kernel<false, true>, kMmdThreads, mmd_smem));
         P.mmd_blocks = (int)std::min<int64_t>((int64_t)mmd_units.size(), (int64_t)nsm * std::max(mmd_occ, 1));
         P.mmd_smem = mmd_smem;
     }
@@ -1545,8 +1545,8 @@ static int plan_launch_kernels(Plan &P)
     auto type1 = [&]() -> int {
         if (P.mmd_blocks > 0) {
             if (P.mmd_cnt_n > 0) GRPP_CUDA(cudaMemsetAsync(P.mmd.part_cnt, 0, P.mmd_cnt_n * sizeof(int), sa));
-            if (P.count_ops) mmd_kernel<true><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
-            else mmd_kernel<false><<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
+            auto kernel = P.count_ops ? mmd_kernel<true, true> : (P.mmd_cnt_n > 0 ? mmd_kernel<false, true> : mmd_kernel<false, false>);
+            kernel<<<P.mmd_blocks, kMmdThreads, P.mmd_smem, sa>>>(P.mmd);
             GRPP_CUDA(cudaGetLastError());
         }
         GRPP_CUDA(cudaEventRecord(ev[1], sa));

@@ -60,7 +60,8 @@ constexpr int kMmdMaxL = 8;               // largest angular momentum whose tabl
 constexpr int kMmdCls = kMmdMaxL + 1;
 constexpr int kMmdMaxPrims = 64;          // primitives per shell (the engine's limit)
 constexpr int kMmdMaxLgT = 6;
-constexpr int kMmdMaxParts = 16;          // shares of one item's triples
+constexpr int kMmdMaxParts = 32;          // parts of one item's triples, each with a sum of its own
+constexpr int kMmdMaxShares = 16;         // blocks that share one item's parts
 constexpr int kMmdSmem = 70 * 1024;       // dynamic shared memory at most: three blocks per SM
 constexpr int kMmdGroup = 64;             // triples whose scalars and auxiliary values are formed together
 constexpr int kMmdRing = 512;             // live triples waiting: at most kMmdGroup - 1 + kMmdThreads
@@ -99,7 +100,7 @@ struct MmdArgs {
     const int4 *pairs;
     // dynamic schedule: blocks pop positions from *queue (zeroed before the launch) and take
     // units[position]; the host orders them by decreasing estimated work. A unit is an item or, in
-    // small batches, one of up to kMmdMaxParts equal shares of its triples: x item, y share |
+    // small batches, one of up to kMmdMaxShares shares of its parts (below): x item, y share |
     // number of shares << 8, z offset of the item's partial sums in part_out, w its counter in
     // part_cnt (zeroed before the launch)
     const int4 *units;
@@ -124,6 +125,17 @@ __host__ __device__ __forceinline__ int r0_row(int S, int t, int u)
 }
 // index of (u + v = k, v) within level s
 __host__ __device__ __forceinline__ int r_in_level(int u, int v) { return (u + v) * (u + v + 1) / 2 + v; }
+
+// Triples per part of an item with n triples (all terms): a group, half of one where a batch of the class
+// has at most 8 triples (high l, few triples that take long), or as many of these as make at most
+// kMmdMaxParts parts (the two kinds of terms apart). The sums of the parts are added in order, so that an
+// item has the same bits whether one block takes all of its parts or several share them. Twice the size left
+// shares of molecules with i shells uneven (2.65 against 2.5 ms for five atoms); half of it gained nothing.
+__host__ __device__ inline int mmd_part_size(int64_t n, int lgT)
+{
+    const int unit = lgT <= 3 ? kMmdGroup / 2 : kMmdGroup;
+    return unit * (int)((n / unit + 2) / (kMmdMaxParts - 1) + 1);
+}
 
 // doubles of shared memory: per triple of a group (scalars and R^n_000), and of a batch (tables)
 __host__ __device__ inline int mmd_group_doubles(const MmdClass &c) { return 15 + c.S + 1; }
@@ -194,8 +206,10 @@ __host__ __device__ inline int mmd_r_size(int smax)
     return tot;
 }
 
-// COUNT: keep the operation counters (a separate instantiation, so the timed kernel carries none)
-template <bool COUNT>
+// COUNT: keep the operation counters (a separate instantiation, so the timed kernel carries none). SHARE:
+// units may be shares of an item (apart, because its positions cost the others 1.5 ms of 82 in the gradient
+// of an 18-atom molecule).
+template <bool COUNT, bool SHARE>
 __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
 {
     extern __shared__ double smem[];
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
         __syncthreads();
         const int4 unit = s_unit;
         if (unit.x < 0) break;
-        const int part = unit.y & 255, nparts = unit.y >> 8;
+        const int share = SHARE ? unit.y & 255 : 0, nshares = SHARE ? unit.y >> 8 : 1;
         const MmdItem item = a.items[unit.x];
         const MmdClass &cl = a.classes[item.cls];
         const int la = cl.la, lb = cl.lb, S = cl.S, npairs = ncart(la) * ncart(lb);
@@ -254,34 +268,74 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
         constexpr int GS = kMmdGroup;
         double *sQA = ws, *sQB = sQA + 3 * GS, *sQC = sQB + 3 * GS, *sK = sQC + 3 * GS, *sW = sK + 3 * GS, *sI = sW + GS,
                *sC = sI + GS, *sR = sC + GS, *E = sR + (S + 1) * GS;
+        // candidate c of the terms from k0 on (term outer, primitive pair inner)
+        auto alive = [&](int k0, int c) {
+            const int k = c / np2, r = c - k * np2, i = r / npB, j = r - i * npB;
+            if (!overlap && (fabs(cA[i]) < kZeroThresh || fabs(cB[j]) < kZeroThresh)) return false;
+            const double al = xA[i], be = xB[j];
+            const double z = overlap ? 0.0 : a.pot_alpha[poff + a.pot_perm[poff + k0 + k]];
+            double ab = 0.0, ac = 0.0, bc = 0.0;
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const double u = Ao[d] - Bo[d], v = Ao[d] - Co[d], w = Bo[d] - Co[d];
+                ab += u * u;
+                ac += v * v;
+                bc += w * w;
+            }
+            return !(al * be * ab + al * z * ac + be * z * bc > kMmdDropArg * (al + be + z));
+        };
+        double *out = a.out[item.out_kind] + item.out_off;
+        double *po = a.part_out + unit.z;
+        // a share counts the live triples to find its parts of each kind
+        int parts[2] = {0, 0};
+        if (nshares > 1)
+            for (int kind = 0; kind < 2; kind++) {
+                const int k0 = kind == 0 ? 0 : n2, ncand = (kind == 0 ? n2 : nterms - n2) * np2;
+                int n = 0;
+                for (int c = tid; c - tid < ncand; c += NT) n += __syncthreads_count(c < ncand && alive(k0, c));
+                const int ps = mmd_part_size((int64_t)nterms * np2, cl.lgT[kind]);
+                parts[kind] = (n + ps - 1) / ps;
+            }
+        int part = 0;  // next part whose sums are complete
+        // the sums of a part, complete after a barrier: to the output or the shares' buffer
+        auto flush = [&]() {
+            for (int p = tid; p < npairs; p += NT) {
+                double s = 0.0;
+                for (int g = 0; g < G; g++) {
+                    s = g == 0 ? acc[p * G] : s + acc[p * G + g];
+                    acc[p * G + g] = 0.0;
+                }
+                if (nshares > 1) {
+                    po[part * npairs + p] = s;
+                } else {
+                    double *o = out + __ldg(pt + p).w;
+                    *o = part == 0 ? s : *o + s;
+                }
+            }
+            part++;
+        };
         for (int kind = 0; kind < 2; kind++) {
             const int k0 = kind == 0 ? 0 : n2, ncand = (kind == 0 ? n2 : nterms - n2) * np2;
             const int lg = cl.lgT[kind], T = 1 << lg, tr = tid & (T - 1), e0 = tid >> lg, est = NT >> lg;
             const int nax = kind == 0 ? (la + 1) * (lb + 1) : mmd_e_axis(la, lb);
             double *R0 = E + cl.nE * T, *X = R0 + cl.nR0 * T, *Rb = X;  // kind 1; X shares the R levels' space
-            const int cend = (int)((int64_t)ncand * (part + 1) / nparts);
-            int head = 0, tail = 0, base = (int)((int64_t)ncand * part / nparts);
+            const int ps = mmd_part_size((int64_t)nterms * np2, lg);
+            // live triples lo <= index < hi of this kind: all, or a share's parts
+            int lo = 0, hi = 1 << 30;
+            if (nshares > 1) {
+                const int k = kind == 0 ? nshares - 1 - share : share;  // who has fewer parts of one kind has more of the other
+                part = parts[kind] * k / nshares;
+                lo = part * ps;
+                hi = parts[kind] * (k + 1) / nshares * ps;
+                if (kind == 1) part += parts[0];
+            }
+            int head = lo, tail = lo, base = 0, seen = 0, pend = 0;
             for (;;) {
-                if (tail - head < GS && base < cend) {
+                if (tail - head < GS && base < ncand && seen < hi) {
                     // the next NT triples (term outer, primitive pair inner): keep the live ones, in order
                     const int c = base + tid;
                     bool live = false;
-                    if (c < cend) {
-                        const int k = c / np2, r = c - k * np2, i = r / npB, j = r - i * npB;
-                        if (overlap || (!(fabs(cA[i]) < kZeroThresh) && !(fabs(cB[j]) < kZeroThresh))) {
-                            const double al = xA[i], be = xB[j];
-                            const double z = overlap ? 0.0 : a.pot_alpha[poff + a.pot_perm[poff + k0 + k]];
-                            double ab = 0.0, ac = 0.0, bc = 0.0;
-#pragma unroll
-                            for (int d = 0; d < 3; d++) {
-                                const double u = Ao[d] - Bo[d], v = Ao[d] - Co[d], w = Bo[d] - Co[d];
-                                ab += u * u;
-                                ac += v * v;
-                                bc += w * w;
-                            }
-                            live = !(al * be * ab + al * z * ac + be * z * bc > kMmdDropArg * (al + be + z));
-                        }
-                    }
+                    if (c < ncand) live = alive(k0, c);
                     const unsigned m = __ballot_sync(0xffffffffu, live);
                     if (lane == 0) s_cnt[warp] = __popc(m);
                     __syncthreads();
@@ -292,8 +346,10 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
                         pre += w < warp ? v : 0;
                         tot += v;
                     }
-                    if (live) ring[(tail + pre + __popc(m & ((1u << lane) - 1))) & (kMmdRing - 1)] = c;
-                    tail += tot;
+                    const int at = seen + pre + __popc(m & ((1u << lane) - 1));
+                    if (live && at >= lo && at < hi) ring[at & (kMmdRing - 1)] = c;
+                    seen += tot;
+                    tail = max(lo, min(seen, hi));
                     base += NT;
                     __syncthreads();
                     continue;
@@ -463,29 +519,29 @@ __global__ void __launch_bounds__(kMmdThreads, 3) mmd_kernel(MmdArgs a)
                         if (p < npairs && (tr & 31) == 0) acc[p * G + (tr >> 5)] += s;
                     }
                     __syncthreads();  // the batch's tables are consumed
+                    pend += T;
+                    if (pend == ps) {
+                        flush();
+                        pend = 0;
+                    }
                 }
                 head += ng;
             }
+            if (pend > 0) flush();
         }
-        __syncthreads();
-        double *out = a.out[item.out_kind] + item.out_off;
-        double *po = a.part_out + unit.z;
-        for (int p = tid; p < npairs; p += NT) {
-            double s = acc[p * G];
-            for (int g = 1; g < G; g++) s += acc[p * G + g];
-            if (nparts == 1) out[__ldg(pt + p).w] = s;
-            else po[part * npairs + p] = s;
-        }
-        if (nparts > 1) {  // the share that comes last adds all of them, in order
+        if (part == 0 && nshares == 1)  // no triple is left
+            for (int p = tid; p < npairs; p += NT) out[__ldg(pt + p).w] = 0.0;
+        if (nshares > 1) {  // the share that comes last adds all parts, in order
             __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(a.part_cnt + unit.w, 1) == nparts - 1;
+            if (tid == 0) s_last = atomicAdd(a.part_cnt + unit.w, 1) == nshares - 1;
             __syncthreads();
             if (s_last) {
                 __threadfence();
+                const int np_all = parts[0] + parts[1];
                 for (int p = tid; p < npairs; p += NT) {
                     double s = 0.0;
-                    for (int q = 0; q < nparts; q++) s += __ldcg(po + q * npairs + p);
+                    for (int q = 0; q < np_all; q++) s = q == 0 ? __ldcg(po + p) : s + __ldcg(po + q * npairs + p);
                     out[__ldg(pt + p).w] = s;
                 }
             }
