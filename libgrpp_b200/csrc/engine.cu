@@ -1426,7 +1426,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                                                                                         (int64_t)10 * nsm / (int64_t)rad_task.size()));
         P.wlk.list_max = (int)walk_list_max;
         P.wlk.chunk_doubles = wrows * kWalkRow;
-        P.wlk.item_level = opt.radial_mode == LIBGRPP_B200_RADIAL_LEARNED && P.wlk.nparts > 1 ? lmctld + 16 : nullptr;
+        P.wlk.item_level = P.wlk.nparts > 1 ? (unsigned *)(lmctld + 16) : nullptr;
         P.walk_smem = gsmem;
         if (P.walk_groups) {
             int occ = 0;

@@ -1265,7 +1265,7 @@ struct WalkArgs {
     int nparts;          // CTAs per item
     int list_max;        // capacity of the active-group lists (groups of one item at most)
     int chunk_doubles;   // doubles of point rows before the lists
-    int *item_level;     // learned mode and nparts > 1: deepest level + 1 of an item so far (else null)
+    unsigned *item_level;  // nparts > 1: levels that an item's finished parts reached (a bit each) and, from bit 16, how many have finished
 };
 
 // 8 bytes from global to shared memory, asynchronously (zero: writes 0)
@@ -1360,11 +1360,6 @@ __global__ void __launch_bounds__(kWalkThreads, 4) radial_walk_group_kernel(Radi
         double *Q = a.Q + qo, *Sp = a.S_prev + qo;
         const double *SC = a.scr + qo;
         uint8_t *EF = a.eflag + qo;
-        int l1m = 0, l2m = 0;
-        for (int p = 0; p < npot; p++) {
-            l1m = max(l1m, pL[p] + la);
-            l2m = max(l2m, pL[p] + lb);
-        }
         const long long t0 = clock64();
         unsigned long long c_acc = 0;
         const int G = gpre[npot], glo = (int)((int64_t)G * part / w.nparts), ghi = (int)((int64_t)G * (part + 1) / w.nparts);
@@ -1518,26 +1513,36 @@ __global__ void __launch_bounds__(kWalkThreads, 4) radial_walk_group_kernel(Radi
             if (my_lvl) atomicMax(&s_lvl, my_lvl);
             __syncthreads();  // the next list and needs are complete; the rows are consumed
         }
-        // deepest level walked: the cap if the last chunk was walked, else the last convergence
-        const int level_reached = any ? kRadMaxLevel : s_lvl;
-        if (tid == 0) {
-            if (w.nparts == 1 && a.stop_level) a.stop_level[item] = (int8_t)level_reached;
-            if (a.pred_level && level_reached > a.pred_level[item] + 1 &&
-                (!w.item_level || atomicMax(w.item_level + item, level_reached + 1) <= a.pred_level[item] + 2))
-                atomicAdd(a.fallback_count, 1);
-        }
         if (a.counters) {
             unsigned long long v = c_acc;
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
             if (lane == 0) atomicAdd(a.counters + kRadCntAccum, v);
             if (tid == 0) atomicAdd(a.counters + kRadCntQuadCycles, (unsigned long long)(clock64() - t0));
-            if (tid == 0 && part == 0) {
+        }
+        if (tid == 0) {
+            // deepest level walked: the cap if the last chunk was walked, else the last convergence; the
+            // item's is known to the CTA that finishes its last part
+            int level_reached = any ? kRadMaxLevel : s_lvl;
+            bool last = true;
+            if (w.nparts > 1) {
+                atomicOr(w.item_level + item, 1u << level_reached);
+                const unsigned v = atomicAdd(w.item_level + item, 1u << 16);
+                last = (int)(v >> 16) == w.nparts - 1;
+                level_reached = 31 - __clz(v & 0xffffu);
+            }
+            if (last && a.stop_level) a.stop_level[item] = (int8_t)level_reached;
+            if (last && a.pred_level && level_reached > a.pred_level[item] + 1) atomicAdd(a.fallback_count, 1);
+            if (last && a.counters) {
                 // algorithmic work of the shared grid up to the stop level (every point once,
                 // every order and potential term at every point)
                 const unsigned long long pts = (unsigned long long)((1 << (level_reached + 5)) - 1);
                 const int np_a = a.rp_n[a.task_a[t]], np_b = a.rp_n[a.task_b[t]];
-                int terms = 0;
-                for (int p = 0; p < npot; p++) terms += a.pot_nprim[a.sl_pot[a.grpp_sl_off[gr] + p]];
+                int terms = 0, l1m = 0, l2m = 0;
+                for (int p = 0; p < npot; p++) {
+                    terms += a.pot_nprim[a.sl_pot[a.grpp_sl_off[gr] + p]];
+                    l1m = max(l1m, pL[p] + la);
+                    l2m = max(l2m, pL[p] + lb);
+                }
                 atomicAdd(a.counters + kRadCntPoints, pts);
                 atomicAdd(a.counters + kRadCntBessel, pts * (unsigned long long)(np_a * (l1m + 1) + np_b * (l2m + 1)));
                 atomicAdd(a.counters + kRadCntPrimPts, pts * (unsigned long long)(np_a + np_b));
