@@ -927,8 +927,9 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
     // Cartesian pair tables of the type 1 items, one per (bra, ket) table class
     std::vector<int4> mmd_pairs;
     size_t mmd_smem = 0;
-    CHECK_INPUT(items.empty() || (mmd_lmax <= kMmdMaxL && mmd_accept_bytes(mmd_lmax, mmd_smax) <= 200 * 1024),
-                "type 1 workspace of this batch's angular momenta exceeds one block's shared memory");
+    CHECK_INPUT(items.empty() || mmd_accepts(mmd_lmax, mmd_smax),
+                "type 1 and outercore overlap items of a batch: L <= 6, or L <= 7 with every L_A + L_B <= 11, or L <= 8 with every "
+                "L_A + L_B <= 8");
     {
         std::map<std::vector<int8_t>, int> tab_id;  // a shell's Cartesian table -> class
         std::vector<int> sh_tab(ns);

@@ -143,14 +143,9 @@ static void mmd_build_classes(MmdTables &T)
         }
 }
 
-// Largest shared workspace of the angular momenta (lmax, smax = largest la + lb) of one batch that
-// the entry points accept, in bytes: the limit of the supported classes (la, lb <= kMmdMaxL).
-static size_t mmd_accept_bytes(int lmax, int smax)
-{
-    const size_t kpl = ncart(lmax) * ncart(lmax) <= 256 ? 8 : 32;
-    const size_t ws = 3 * (lmax + 1) * (lmax + 1) * (2 * lmax + 1) + mmd_r_size(smax) + mmd_tet(smax) + 2 * (smax + 2) + 16 +
-                      2 * kMmdMaxPrims + 12 + (smax + 1) + 7 * 32;
-    return 4 * (ws + 32 * kpl) * sizeof(double);
-}
+// Supported angular momenta of one batch's type 1 and overlap items: lmax the largest L, smax the largest
+// L_A + L_B. Every pair up to i shells; one L = 7 shell with L_A + L_B <= 11, L = 8 with L_A + L_B <= 8. Every
+// class within these fits kMmdSmem.
+static bool mmd_accepts(int lmax, int smax) { return lmax <= 6 || (lmax == 7 && smax <= 11) || (lmax == kMmdMaxL && smax <= 8); }
 
 }  // namespace grpp
