@@ -46,6 +46,7 @@ namespace grpp {
 // doubles per output array that a chunk sends back with its status: one copy of at most 256 KB instead of four
 // that wait for the launches (a single f x d block: 46 us of downloads before)
 constexpr int64_t kSmallOut = 8192;
+constexpr size_t kOneeKeep = size_t(128) << 20;  // bytes of the one-electron buffer kept after a numeric type 1 call
 constexpr size_t kFinSmemMax = 220 * 1024;  // dynamic shared memory of the assembly kernel (+ its static 3 kB)
 
 // ------------------------------------------------------------------ errors
@@ -88,6 +89,12 @@ struct DevBuf {
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) cap = want;
         return e;
+    }
+    void release()
+    {
+        if (p) cudaFree(p);
+        p = nullptr;
+        cap = 0;
     }
 };
 
@@ -2408,11 +2415,14 @@ int run_type1_numeric_batch(const libgrpp_b200_batch_t *b, int model, const doub
     cudaStream_t s = stp->stream;
     const int64_t nt = b->n_tasks, nout = k.off[nt];
     const int Lt = k.lmax_pair;
-    // chunks of consecutive tasks: up to kT1Scratch doubles of per-pair scratch and kT1Slots centres
+    // chunks of consecutive tasks: up to kT1Scratch doubles of per-pair scratch and kT1Slots centres (64 kB of
+    // tables each). 64 MB of scratch are 65 000 f x f pairs, twenty times the resident warps (14400 tasks of s..f
+    // shells: 110.5 ms, 111.2 with 32 MB, 109.5 with 256). Few centres per chunk would cut a list that
+    // runs over its centres first into small chunks (500 centres, 128 per chunk: 370 ms against 260).
     struct T1Chunk {
         int64_t t0, t1, s0, s1;
     };
-    constexpr int64_t kT1Scratch = int64_t(1) << 25;
+    constexpr int64_t kT1Scratch = int64_t(1) << 23;
     constexpr int kT1Slots = 1024;
     std::vector<int64_t> unit_off(nt + 1, 0), group_off(nt + 1, 0), scr_off(nt);
     std::vector<int> slot(nt), slot_centre, slot_of(nc, -1);
@@ -2519,6 +2529,7 @@ int run_type1_numeric_batch(const libgrpp_b200_batch_t *b, int model, const doub
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, a.out, nout * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (stp->onee.cap > kOneeKeep) stp->onee.release();
     if (e != cudaSuccess) {
         set_error(LIBGRPP_B200_ERR_CUDA, std::string("numeric type 1 integrals: ") + cudaGetErrorString(e));
         return LIBGRPP_B200_ERR_CUDA;
