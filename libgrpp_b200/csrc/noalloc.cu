@@ -286,6 +286,7 @@ int run(const libgrpp_b200_batch_t *b, double *h_arep)
     std::vector<std::pair<int, int>> atab_need;
     int64_t qtot = 0;
     int l1m = 0, l2m = 0, dn = 1, npot = 0, fin_lam = 0, fin_nq = 1;
+    int fin_task = 2;  // doubles of a task's own tables in the assembly, the largest of the batch
     for (int64_t t = 0; t < nt; t++) {
         NA_CHECK(ta[t] >= 0 && ta[t] < ns && tb[t] >= 0 && tb[t] < ns && tc[t] >= 0 && tc[t] < b->n_centres, "task index out of range");
         const int la = sh_L[ta[t]], lb = sh_L[tb[t]], g = b->centre_grpp[tc[t]];
@@ -293,16 +294,21 @@ int run(const libgrpp_b200_batch_t *b, double *h_arep)
         out_off[t + 1] = out_off[t] + (int64_t)ncart(la) * ncart(lb);
         if (g_sl_n[g] == 0) continue;
         int64_t e = 0;
+        int om = 0, nq = 0;
         for (int i = 0; i < g_sl_n[g]; i++) {
             const int L = p_L[sl_pot[g_sl_off[g] + i]];
             e += (int64_t)(L + la + 1) * (L + lb + 1) * (la + lb + 1);
             l1m = std::max(l1m, L + la);
             l2m = std::max(l2m, L + lb);
             fin_lam = std::max(fin_lam, L + std::max(la, lb));
-            fin_nq = std::max(fin_nq, (L + la + 1) * (L + lb + 1) * (la + lb + 1));
+            nq = std::max(nq, (L + la + 1) * (L + lb + 1) * (la + lb + 1));
+            om = std::max(om, om_size(L, la) + om_size(L, lb));
             atab_need.push_back({L, la});
             atab_need.push_back({L, lb});
         }
+        fin_nq = std::max(fin_nq, nq);
+        const int terms = fin_terms(cart.data() + 3 * sh_co[ta[t]], ncart(la)) + fin_terms(cart.data() + 3 * sh_co[tb[t]], ncart(lb));
+        fin_task = std::max(fin_task, (fin_task_doubles(om, nq, terms) + 1) & ~1);
         NA_CHECK(e <= kRadMaxEntries, "radial table larger than 16384 entries for one task");
         q_off[t] = qtot;
         rad_task.push_back((int)t);
@@ -443,18 +449,15 @@ int run(const libgrpp_b200_batch_t *b, double *h_arep)
     FinalSmem fs{};
     fs.rsh_stride = 2 * fin_lam + 1;
     fs.n_rsh = (fin_lam + 1) * fs.rsh_stride;
-    int n_om = 1, n_om2 = 1, nabmax = 1, terms = 1;
+    int n_om = 1, nabmax = 1;
     for (auto &lp : atab_need) {
         n_om = std::max(n_om, n_abc(lp.second) * lam_slots(lp.first, lp.second) * (2 * lp.first + 1));
-        n_om2 = std::max(n_om2, om_size(lp.first, lp.second));
         nabmax = std::max(nabmax, n_abc(lp.second));
     }
-    for (int i = 0; i < b->n_shells; i++)
-        terms = std::max(terms, fin_terms(cart.data() + 3 * sh_co[i], ncart(sh_L[i])));
     // the classes that fit: dense omega rows, the harmonics, the radial table and V
     const size_t need = (size_t)(2 * fs.n_rsh + 2 * n_om + fin_nq + std::max(6144, 3 * nabmax)) * sizeof(double);
     const int vmin = (fin_v_row(nabmax, 1) + 1) & ~1;
-    fs.n_task = (fin_task_doubles(2 * n_om2, fin_nq, 2 * terms) + 1) & ~1;
+    fs.n_task = fin_task;
     fs.n_v = std::max(6144, vmin);
     auto bytes = [&]() { return (size_t)(2 * fs.n_rsh + fs.n_task + fs.n_v) * sizeof(double); };
     while (bytes() > kNaFinSmem && fs.n_v > vmin) fs.n_v = std::max(vmin, fs.n_v - 256);
