@@ -330,8 +330,10 @@ static int fin_default_nt(int la, int lb, int64_t n_tasks, int nsm)
     return n_abc(la) * n_abc(lb) >= 1000 || n_tasks <= 2 * nsm ? 512 : 128;
 }
 
-// Limit of the supported classes: what a launch may need with dense omega rows on both sides, the
-// harmonics, the radial table and 6144 values of V
+// Limit of the supported classes: what the tasks of one accept group may need with dense omega rows on
+// both sides, the harmonics, the radial table and 6144 values of V (maxima over the group). An accept
+// group holds the classes of one range of V entries (or set block size) and one memory tier; it does not depend on
+// how the launches are grouped, and every launch group of accepted classes fits: 196 kB at most.
 struct FinNeed {
     int n_rsh = 0, n_omega = 0, n_q = 0, n_v = 0;
     size_t bytes() const { return (size_t)(2 * n_rsh + 2 * n_omega + n_q + n_v) * sizeof(double); }
@@ -1047,7 +1049,7 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
         std::vector<double> cost(nt);
         std::map<int, int> gidx;
         std::vector<std::vector<int>> members;
-        std::vector<FinNeed> needs;
+        std::map<int, FinNeed> needs;  // per accept group
         std::vector<int> v_min, sh_terms(ns);
         for (int i = 0; i < ns; i++) sh_terms[i] = fin_terms(cart.data() + 3 * sh_co[i], ncart(sh_L[i]));
         // GRPPs of equal semilocal orders and spin-orbit parts share one shape
@@ -1088,14 +1090,18 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             int ntb = opt.fin_nt;
             if (ntb == 0) {
                 auto it = st.fin_tune.find(cls);
-                ntb = it != st.fin_tune.end() ? it->second : fin_default_nt(la, lb, nt, st.nsm);
+                if (it != st.fin_tune.end()) ntb = it->second;
             }
+            const int w = n_abc(la) * n_abc(lb), range = ntb ? ntb : (w < 1000 ? 128 : (w < 3000 ? 256 : 512));
+            if (ntb == 0) ntb = fin_default_nt(la, lb, nt, st.nsm);
             CHECK_INPUT(ntb == 128 || ntb == 256 || ntb == 512, "assembly block size must be 128, 256 or 512");
             const FinNeed fn = fin_need(lam, nom, nq, n_abc(la), n_abc(lb), so ? 3 : 1);
             const int task_dbl = fin_task_doubles(om2, nq, sh_terms[ta[t]] + sh_terms[tb[t]]);
             const size_t bytes = fn.bytes();
             const int tier = bytes <= 32 * 1024 ? 0 : (bytes <= 96 * 1024 ? 1 : 2);
             const int key = opt.fin_by_class ? cls * 8 + ntb / 128 : ntb * 4 + tier;
+            FinNeed &need = needs[opt.fin_by_class ? cls * 8 + range / 128 : range * 4 + tier];
+            need = fin_merge(need, fn);
             auto it = gidx.find(key);
             int gi;
             if (it == gidx.end()) {
@@ -1107,10 +1113,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 fin_groups.push_back(G);
                 members.emplace_back();
                 v_min.push_back(0);
-                needs.push_back(fn);
             } else {
                 gi = it->second;
-                needs[gi] = fin_merge(needs[gi], fn);
             }
             FinalSmem &fs = fin_groups[gi].fs;
             fs.n_task = std::max(fs.n_task, (task_dbl + 1) & ~1);
@@ -1122,6 +1126,8 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             cn.nq = nq;
             cn.cost = cost[t];
         }
+        for (const auto &q : needs)
+            CHECK_INPUT(q.second.bytes() <= kFinSmemMax, "assembly tables of this batch exceed the shared memory of one block");
         for (size_t gi = 0; gi < fin_groups.size(); gi++) {
             auto &m = members[gi];
             std::vector<double> mc(m.size());
@@ -1130,7 +1136,6 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
             fin_groups[gi].count = (int)m.size();
             for (int i : order_by_cost(mc)) fin_order.push_back(m[i]);
             FinalSmem &fs = fin_groups[gi].fs;
-            CHECK_INPUT(needs[gi].bytes() <= kFinSmemMax, "assembly tables of this batch exceed the shared memory of one block");
             if (om_words == 0) {
                 fs.rsh_stride = 2 * fin_lam + 1;
                 fs.n_rsh = (fin_lam + 1) * fs.rsh_stride;
