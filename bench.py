@@ -445,11 +445,11 @@ def run_ours(args, rank, world, local):
 
 # DRAM bytes per task of the dominant kernel, from one ncu capture of it (dram__bytes_read.sum +
 # dram__bytes_write.sum over the captured launch / its tasks); see profiles/
-TRAFFIC_PER_TASK = {"ms_screen": (22.991616e6 + 20.618496e6) / 4096, "ms_walk": (292.135168e6 + 21.524480e6) / 4096}
+TRAFFIC_PER_TASK = {"ms_screen": (22.980096e6 + 20.604928e6) / 4096, "ms_walk": (292.851968e6 + 25.079552e6) / 4096}
 TRAFFIC_SOURCE = {
-    "ms_screen": "ncu --set full of radial_screen_unit_kernel on 4096 tasks of the first config-1 step: 43.61 MB DRAM "
+    "ms_screen": "ncu --set full of radial_screen_unit_kernel on 4096 tasks of the first config-1 step: 43.59 MB DRAM "
                  "read+write, scaled to the step's tasks (profiles/screen_unit_kernel_full_4096tasks.md)",
-    "ms_walk": "ncu --set full of radial_walk_group_kernel on 4096 tasks of the first config-1 step: 313.66 MB DRAM "
+    "ms_walk": "ncu --set full of radial_walk_group_kernel on 4096 tasks of the first config-1 step: 317.93 MB DRAM "
                "read+write from a cold L2, scaled to the step's tasks, an upper bound: the F_l tables are shared by more "
                "tasks there (profiles/walk_group_kernel_full_4096tasks.md)"}
 

@@ -121,9 +121,9 @@ struct DeviceState {
     int device = -1;
     int nsm = 148;                       // multiprocessors of the device (set at initialisation)
     bool ready = false;
-    cudaStream_t stream = nullptr;       // all kernels and uploads
+    cudaStream_t stream = nullptr;       // uploads and the main chain of kernels (plan_launch_kernels)
     cudaStream_t copy_stream = nullptr;  // downloads of finished chunks
-    cudaStream_t side[2] = {nullptr, nullptr};  // independent kernels of one execution (plan_launch)
+    cudaStream_t side[2] = {nullptr, nullptr};  // independent kernels of one execution (plan_launch_kernels)
     cudaEvent_t side_ev[2][4];           // per buffer set: fork, walk inputs ready, the two side streams' ends
     cudaEvent_t ev[2][7];                // per buffer set: phase boundaries of one execution
     cudaEvent_t done[2];                 // per buffer set: execution and its status copy finished

@@ -181,8 +181,9 @@ __global__ void __launch_bounds__(128) level_predict_kernel(RadialArgs a, LevelM
     }
 }
 
-// Deepest-predicted-first order of the walked items, within a level in the order of perm (items by
-// centre): counting sort over levels 8..0. cursor[0..9] must be zero on entry; one CTA of 256 threads.
+// Deepest-predicted-first order of the walked items, within a level roughly in the order of perm (items by
+// centre; concurrent threads take positions from a counter): counting sort over levels 8..0. cursor[0..9] must be
+// zero on entry; one CTA (of 1024 threads).
 __global__ void level_order_kernel(int n_items, const int *perm, const int8_t *pred, int *order, int *n_order, int *cursor)
 {
     __shared__ int hist[kLmOut], start[kLmOut];

@@ -27,6 +27,8 @@
 // X[t,u][az,bz] = sum_v E^z_v R^0_tuv and, per Cartesian pair, sum_t E^x_t sum_u E^y_u X.
 // Splitting the contraction at z makes it about 4 operations per pair where the triple sum
 // needs 14 (g x g) to 60 (i x i).
+// The sums of an item are formed in parts that the item alone fixes (mmd_part_size), so that they do not depend
+// on how many blocks take it.
 // Triples whose Gaussian product exponents sum to more than 800 are dropped: K_x K_y K_z < 1e-347
 // there, so their contributions underflow.
 //

@@ -185,7 +185,7 @@ constexpr int kT1Pts = 8192;        // row length of the point tables (8191 poin
 constexpr int kT1Warps = 4;         // warps of a radial block
 constexpr int kT1Group = 4;         // primitive pairs of an assembly block
 constexpr int kT1AsmThreads = 128;
-constexpr int kT1PowRow = kMaxL + 1; // powers 0..kMaxL of one component of CA or CB: one shell may have all of L_A + L_B
+constexpr int kT1PowRow = kMaxL + 1;  // powers 0..kMaxL of one component of CA or CB: one shell may have all of L_A + L_B
 
 struct Type1NumArgs {
     int n_tasks, model;
