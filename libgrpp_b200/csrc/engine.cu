@@ -1015,7 +1015,10 @@ int plan_build(DeviceState &st, const libgrpp_b200_batch_t *b, const RunOptions 
                 ucost.push_back(cost[q] / n);
             }
             if (n > 1) {
-                mmd_part_n += (int64_t)kMmdMaxParts * ncart(sh_L[it.bra]) * ncart(sh_L[it.ket]);
+                // room for as many parts as the triples can make: ceil(x / ps) + ceil(y / ps) <= (x + y) / ps + 2
+                const MmdClass &mc = st.mmd_cls[it.cls];
+                const int ps = std::min(mmd_part_size(triples, mc.lgT[0]), mmd_part_size(triples, mc.lgT[1]));
+                mmd_part_n += std::min<int64_t>(kMmdMaxParts, triples / ps + 2) * ncart(sh_L[it.bra]) * ncart(sh_L[it.ket]);
                 mmd_cnt_n++;
             }
         }
